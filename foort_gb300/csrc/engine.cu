@@ -207,6 +207,7 @@ RunConst make_run_const(const foort_run_desc& d) {
     R.gp_every = d.geopos_freq.every_n;
     R.gp_start = d.geopos_freq.at_start;
     R.gp_finish = d.geopos_freq.at_finish;
+    fill_mixed_run(R);
     return R;
 }
 
@@ -214,7 +215,8 @@ RunConst make_run_const(const foort_run_desc& d) {
 // (the latter takes every step in FP64).
 bool analytic_family(int precision) { return precision == FOORT_PREC_MIXED || precision == FOORT_PREC_FP64_ANALYTIC; }
 
-const void* select_kernel(const RunConst& R) {
+const void* select_kernel(const RunConst& R, bool positions) {
+    if (const void* lean = positions ? nullptr : mixed_lean_kernel(R, false)) return lean;
     if (analytic_family(R.precision))
         return mixed_kernel_variant(R.metric_id, R.integrator, (R.mixed_options & FOORT_MIXED_FP64_DECISIONS) != 0);
     return fp64_kernel(R.metric_id, R.integrator);
@@ -222,7 +224,8 @@ const void* select_kernel(const RunConst& R) {
 
 // The two-lanes-per-geodesic kernel for these options, or nullptr (FP64, FP64-analytic,
 // Verlet, the called plugins, the strong-field FP64 steps).
-const void* select_pair_kernel(const RunConst& R) {
+const void* select_pair_kernel(const RunConst& R, bool positions) {
+    if (const void* lean = positions ? nullptr : mixed_lean_kernel(R, true)) return lean;
     if (R.precision != FOORT_PREC_MIXED || R.mixed_fp64_margin > 0.0 ||
         (R.mixed_options & FOORT_MIXED_FP64_TURNING_POINTS))
         return nullptr;
@@ -234,29 +237,42 @@ struct LaunchShape {
     uint32_t grid = 0, block = 0, lanes = 1, refill = 1, poll = kDefaultPollSteps;
 };
 
+// Geodesics up to which a launch takes two lanes each, where that kernel exists and the
+// launch leaves the choice open.
+// - General kernels: as many as the GPU's resident lanes hold that way. Then a step's
+//   latency, not the GPU's throughput, sets the pace, and two lanes halve its metric work.
+// - Lean kernels: one lane already evaluates two stages at a time, so two lanes pay only
+//   while they leave each scheduler one warp (n <= 64 x SMs), and only in log r, where
+//   each half of a packed stage needs its own exponentials and division: Kerr, 3,721
+//   geodesics in log r 1.31 ms on two lanes and 1.58 on one. In plain r both take the same
+//   within 3 % (3,000 geodesics 66 and 64 ms, 1.00 and 0.97 us a step): the smallest launches
+//   stay on two, the rest take one.
+uint64_t pair_limit(const RunConst& R, bool positions, int per_sm, int num_sms, uint32_t bs) {
+    const uint64_t sms = static_cast<uint64_t>(num_sms);
+    if (!positions && mixed_lean_kernel(R, true)) return (R.rlog ? 64 : 24) * sms;
+    return static_cast<uint64_t>(per_sm) * sms * bs / 2;
+}
+
 // Kernel and grid of a launch of n geodesics in the requested shape (zero fields: the
 // built-in rule): a persistent grid of at most the resident CTAs. The rule takes 128
-// threads, as many CTAs per SM as fit, and two lanes per geodesic where that kernel exists
-// and all n geodesics fit on the GPU's resident lanes that way (then a step's latency,
-// not the GPU's throughput, sets the pace, and two lanes halve the metric work on it).
+// threads, as many CTAs per SM as fit, and two lanes per geodesic up to pair_limit().
 int choose_launch(foort_ctx* ctx, const RunConst& R, uint64_t n, int num_sms, const foort_launch_shape& want,
-                  LaunchShape& out) {
+                  LaunchShape& out, bool positions = false) {
     const uint32_t bs = want.block_size ? want.block_size : 128;
     auto resident = [&](const void* fn, int& per_sm) -> int {
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, static_cast<int>(bs), 0));
         if (want.blocks_per_sm) per_sm = std::min<int>(per_sm, static_cast<int>(want.blocks_per_sm));
         return FOORT_OK;
     };
-    const void* fn = select_kernel(R);
+    const void* fn = select_kernel(R, positions);
     if (!fn) return fail(ctx, FOORT_E_UNSUPPORTED, "no kernel for this metric / integrator / precision");
     int per_sm = 0, rc = 0;
     uint32_t lanes = 1;
-    const void* fn2 = (want.lanes != 1) ? select_pair_kernel(R) : nullptr;
+    const void* fn2 = (want.lanes != 1) ? select_pair_kernel(R, positions) : nullptr;
     if (fn2) {
         int per_sm2 = 0;
         if ((rc = resident(fn2, per_sm2))) return rc;
-        const uint64_t cap2 = static_cast<uint64_t>(per_sm2) * static_cast<uint64_t>(num_sms) * bs;
-        if (per_sm2 > 0 && (want.lanes == 2 || 2 * n <= cap2)) {
+        if (per_sm2 > 0 && (want.lanes == 2 || n <= pair_limit(R, positions, per_sm2, num_sms, bs))) {
             fn = fn2;
             per_sm = per_sm2;
             lanes = 2;
@@ -314,7 +330,7 @@ int launch(foort_ctx* ctx, const foort_pixel* d_px, uint64_t n, foort_result* d_
     const foort_launch_shape want = shape ? *shape : requested_shape(ctx, n, &cached);
     if (!shape && !cached && ctx->autotune && !gp_plan && n > 0) return autotune_launch(ctx, d_px, n, d_out, st, nullptr);
     LaunchShape ls;
-    int rc = choose_launch(ctx, ctx->rc, n, ctx->num_sms, want, ls);
+    int rc = choose_launch(ctx, ctx->rc, n, ctx->num_sms, want, ls, gp_plan != nullptr);
     if (rc) return rc;
     const void* fn = ls.fn;
     const uint32_t bs = ls.block, grid = ls.grid;
@@ -412,7 +428,7 @@ int autotune_launch(foort_ctx* ctx, const foort_pixel* d_px, uint64_t n, foort_r
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, probe.fn, 128, 0));
     const uint64_t resident = static_cast<uint64_t>(std::max(per_sm, 1)) * ctx->num_sms * 128;
     const uint64_t m = std::min<uint64_t>(n, FOORT_TUNE_SAMPLE_LANES_X * resident);
-    const bool has_pair = select_pair_kernel(ctx->rc) != nullptr;
+    const bool has_pair = select_pair_kernel(ctx->rc, false) != nullptr;
     std::vector<foort_launch_shape> tried;
     auto time_shape = [&](foort_launch_shape s, double& ms) -> int {
         int r = launch(ctx, d_px, m, d_out, st, nullptr, &s);
@@ -534,7 +550,7 @@ int foort_gpu_create(const foort_run_desc* desc, foort_ctx** out_ctx) {
     if (e != cudaSuccess) return bail(cuda_fail(ctx, e, "cudaGetDevice"));
     e = cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount, ctx->device);
     if (e != cudaSuccess) return bail(cuda_fail(ctx, e, "cudaDeviceGetAttribute"));
-    if (!select_kernel(ctx->rc)) return bail(fail(ctx, FOORT_E_UNSUPPORTED, "no kernel for this metric / integrator / precision"));
+    if (!select_kernel(ctx->rc, false)) return bail(fail(ctx, FOORT_E_UNSUPPORTED, "no kernel for this metric / integrator / precision"));
     e = cudaMalloc(&ctx->d_images, ctx->hic.size() * sizeof(ImageConst));
     if (e != cudaSuccess) return bail(cuda_fail(ctx, e, "cudaMalloc(images)"));
     e = cudaMemcpy(ctx->d_images, ctx->hic.data(), ctx->hic.size() * sizeof(ImageConst), cudaMemcpyHostToDevice);
@@ -950,7 +966,7 @@ extern "C" int foort_gpu_integrate_noalloc(const foort_run_desc* desc, const foo
                         " images that the allocation-free entry point has room for");
     if (n && (!d_px || !d_out)) return fail(nullptr, FOORT_E_BADARG, "NULL pixel or result buffer");
     const RunConst R0 = make_run_const(*desc);
-    const void* fn = select_kernel(R0);
+    const void* fn = select_kernel(R0, false);
     if (!fn) return fail(nullptr, FOORT_E_UNSUPPORTED, "no kernel for this metric / integrator / precision");
 
     int dev = 0;

@@ -48,6 +48,15 @@ struct ImageConst {
     MixedConst mx;
 };
 
+// The run's constants in FP32 (pairs are float-float splits, as in MixedConst), read by the
+// lean mixed kernels from the kernel's parameters.
+struct MixedRun {
+    float bthr[2], theps[2], pi[2], mpio2[2], eqthr[2], eps[2];
+    float hmin, vtol2;
+    float eqfar;  // beyond this distance from pi / 2, theta's high part decides EquatorialPasses
+    float thfar;  // beyond this distance from 0 and pi, theta's high part excludes ThetaSingularity
+};
+
 // Run options (process globals in the reference, Config.cpp:11-28 and
 // Integrators.h:31-57), passed by value to every launch.
 struct RunConst {
@@ -76,6 +85,7 @@ struct RunConst {
     double mixed_fp64_margin;
     uint64_t gp_every;  // GeodesicPosition update frequency (recorded on a second pass)
     int32_t gp_start, gp_finish;
+    MixedRun mr;
 };
 
 // Scratch counters of one launch (device memory, zeroed before each launch).

@@ -248,6 +248,9 @@ __device__ __forceinline__ bool finite4(const double a[4]) {
 //   finish(L, R, out)                  write the lane's record
 //   stop(L, R, out, err)               write a partial record (budget / cancel)
 //   counters: L.rhs, L.fp64            accumulated per lane, flushed at each poll
+// A lean engine (E::kLean, kernel_lean.cuh) has step(L, R) instead: its lanes keep the
+// image constants they need, record no positions and take kRhsPerStep right-hand sides a
+// step.
 //
 // Every warp takes pixels from one global counter (one atomic per warp, shared by the
 // lanes that need work) and keeps integrating until the queue is empty. Lanes whose
@@ -263,6 +266,15 @@ __device__ __forceinline__ bool finite4(const double a[4]) {
 // PAIR: lanes 2k and 2k+1 integrate one geodesic together (E::step_pair). Both take the
 // same pixel, hold the same state and so leave the loop together; the even lane writes
 // the record and counts the step.
+template <class E>
+constexpr bool is_lean(...) {
+    return false;
+}
+template <class E>
+constexpr bool is_lean(decltype(E::kLean)*) {
+    return true;
+}
+
 template <class E, bool PAIR = false>
 __device__ __forceinline__ void persistent_loop(const LaunchArgs& A, const RunConst& R) {
     const unsigned lane = threadIdx.x & 31u;
@@ -271,6 +283,7 @@ __device__ __forceinline__ void persistent_loop(const LaunchArgs& A, const RunCo
     const unsigned lt_mask = (1u << slot_lane) - 1u;
     const unsigned slots = PAIR ? 0x55555555u : kFullMask;  // one bit per geodesic slot
     const unsigned pmask = 3u << (lane & ~1u);
+    constexpr bool kLean = is_lean<E>(nullptr);
     typename E::Lane L;
     ImageConst Ic;  // PAIR: the lane's image constants in registers, copied at each refill
     bool active = false;
@@ -278,8 +291,20 @@ __device__ __forceinline__ void persistent_loop(const LaunchArgs& A, const RunCo
     bool stopping = false;
     uint32_t stop_err = 0;
     uint64_t idx = 0;
-    unsigned long long lane_steps = 0, lane_done = 0;
+    unsigned lane_steps = 0, lane_done = 0;
     int since_poll = 0, since_refill = 0;
+    // The warp's right-hand sides and FP64 steps since the last count: the lanes' counters,
+    // or (lean engines) a fixed number per step.
+    auto rhs_counts = [](typename E::Lane& l, unsigned long long steps, unsigned long long& rhs, unsigned long long& fp64) {
+        if constexpr (kLean) {
+            rhs = steps * E::kRhsPerStep;
+        } else {
+            rhs = __reduce_add_sync(kFullMask, l.rhs);
+            fp64 = __reduce_add_sync(kFullMask, l.fp64);
+            l.rhs = 0;
+            l.fp64 = 0;
+        }
+    };
 
     for (;;) {
         // Refill idle lanes from the queue.
@@ -305,11 +330,11 @@ __device__ __forceinline__ void persistent_loop(const LaunchArgs& A, const RunCo
                             idx = my;
                             // i and cnt start at 0 as literals: copying them from the record
                             // made the Johannsen Verlet kernel 3 % slower on GB300
-                            L.gp = (A.gp_plan && !odd && A.gp_plan[my].M > 0 && A.gp_plan[my].j > 0)
+                            if constexpr (!kLean) L.gp = (A.gp_plan && !odd && A.gp_plan[my].M > 0 && A.gp_plan[my].j > 0)
                                        ? GeoposRec{A.gp_plan[my].dst, A.gp_plan[my].j, A.gp_plan[my].M, 0, 0}
                                        : GeoposRec{nullptr, 1, 0, 0, 0};
                             E::init(L, A.images[p.image], R, p);
-                            if constexpr (PAIR) Ic = A.images[p.image];
+                            if constexpr (PAIR && !kLean) Ic = A.images[p.image];
                             active = true;
                         }
                     }
@@ -324,10 +349,16 @@ __device__ __forceinline__ void persistent_loop(const LaunchArgs& A, const RunCo
         for (;;) {
             if (active) {
                 bool more;
-                if constexpr (PAIR) {
+                if constexpr (PAIR && kLean) {
+                    more = E::step_pair(L, R, odd, pmask);
+                } else if constexpr (PAIR) {
                     more = E::step_pair(L, Ic, R, odd, pmask);
                 } else {
-                    more = E::step(L, A.images[L.img], R);
+                    if constexpr (kLean) {
+                        more = E::step(L, R);
+                    } else {
+                        more = E::step(L, A.images[L.img], R);
+                    }
                 }
                 lane_steps += odd ? 0u : 1u;
                 if (!more) {
@@ -348,14 +379,12 @@ __device__ __forceinline__ void persistent_loop(const LaunchArgs& A, const RunCo
         if (since_poll >= R.poll_steps || drained) {
             since_poll = 0;
             // Publish progress; read the global stop request.
-            unsigned long long ws = __reduce_add_sync(kFullMask, static_cast<unsigned>(lane_steps));
-            unsigned long long wr = __reduce_add_sync(kFullMask, static_cast<unsigned>(L.rhs));
-            unsigned long long wf = __reduce_add_sync(kFullMask, static_cast<unsigned>(L.fp64));
-            unsigned long long wd = __reduce_add_sync(kFullMask, static_cast<unsigned>(lane_done));
+            unsigned long long ws = __reduce_add_sync(kFullMask, lane_steps);
+            unsigned long long wr = 0, wf = 0;
+            rhs_counts(L, ws, wr, wf);
+            unsigned long long wd = __reduce_add_sync(kFullMask, lane_done);
             lane_steps = 0;
             lane_done = 0;
-            L.rhs = 0;
-            L.fp64 = 0;
             unsigned long long st = 0;
             if (lane == 0) {
                 unsigned long long before = atomicAdd(&A.ctr[kCtrSteps], ws);
@@ -378,10 +407,10 @@ __device__ __forceinline__ void persistent_loop(const LaunchArgs& A, const RunCo
         }
     }
     // Flush what is left.
-    unsigned long long ws = __reduce_add_sync(kFullMask, static_cast<unsigned>(lane_steps));
-    unsigned long long wr = __reduce_add_sync(kFullMask, static_cast<unsigned>(L.rhs));
-    unsigned long long wf = __reduce_add_sync(kFullMask, static_cast<unsigned>(L.fp64));
-    unsigned long long wd = __reduce_add_sync(kFullMask, static_cast<unsigned>(lane_done));
+    unsigned long long ws = __reduce_add_sync(kFullMask, lane_steps);
+    unsigned long long wr = 0, wf = 0;
+    rhs_counts(L, ws, wr, wf);
+    unsigned long long wd = __reduce_add_sync(kFullMask, lane_done);
     if (lane == 0) {
         if (ws) atomicAdd(&A.ctr[kCtrSteps], ws);
         if (wr) atomicAdd(&A.ctr[kCtrRhs], wr);

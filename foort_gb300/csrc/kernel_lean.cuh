@@ -1,0 +1,395 @@
+// Lean mixed-precision kernels: the mixed kernel's arithmetic (kernel_mixed.cuh) for the
+// options nearly every run has, with packed FP32 instructions (packed.cuh).
+//
+// Lean options (lean_options, engine.cu): every termination and diagnostic in use updates
+// at each step, decisions on the float-float state, no FP64 steps, no recorded positions.
+// A lane then carries no update counters, no position record and no copy of the options'
+// constants (they sit in the kernel's parameters, RunConst::mr). Results are the general
+// kernel's bit for bit: each rounding is written out as the compiler contracts the scalar
+// code (gen_packed.py), and the shortcuts below only skip work whose outcome is known.
+//
+// RK4, one lane per geodesic: the metric parts of stages 1 and 2 need only the step's
+// start, those of stages 3 and 4 only k1 and k2, so each of the two pairs is evaluated
+// packed, one stage per half. On two lanes per geodesic each lane evaluates one stage of a
+// pair, and only the state's update is packed.
+//
+// What bounds it: a warp alone on its scheduler waits for fixed latencies (0.89 of 2.36
+// cycles per issue; 809 instructions and 1,914 cycles a step, 0.95 us, where the general
+// kernels took 1.66 us on one lane and 1.17 us on two); three warps per scheduler take
+// 1,441 cycles per warp and step, near the FP32 pipe (476 packed and 154 scalar
+// instructions) with what mixing scalar and packed ones costs it. Kerr a = 0.99 view of
+// half-width 12 M from r = 1000, random pixels, GB300 at 2,070 MHz: 16,384 geodesics 65 ms
+// (general kernels: 82 to 94), 58,368 geodesics 140 ms.
+#pragma once
+
+#include "kernel_mixed.cuh"
+#include "packed.cuh"
+#include "gen_packed.inc"
+
+namespace foort {
+
+template <int MID>
+struct PackedMetric;
+
+#define FOORT_DEFINE_PACKED_METRIC(ID, NAME)                                                              \
+    template <>                                                                                           \
+    struct PackedMetric<ID> {                                                                             \
+        static constexpr int kSlots = FOORT_PACKED_SLOTS_##NAME;                                          \
+        static __device__ __forceinline__ void constants(const float* q, float* k) {                      \
+            (void)q; (void)k;                                                                             \
+            FOORT_PACKED_CONST_##NAME                                                                     \
+        }                                                                                                 \
+        template <typename T>                                                                             \
+        static __device__ __forceinline__ void eval(const float* k, T r, T dp, T dm, T s, T c, G5T<T>& dr, \
+                                                    G5T<T>& dh, G5T<T>& gu) {                             \
+            (void)k; (void)dp; (void)dm;                                                                  \
+            FOORT_PACKED_BODY_##NAME                                                                      \
+        }                                                                                                 \
+    };
+#define MUL p_mul
+#define ADD p_add
+#define FMA p_fma
+#define RCP p_rcp
+#define K p_all<T>
+#define B(i) p_all<T>(k[i])
+FOORT_DEFINE_PACKED_METRIC(kKerr, KERR)
+FOORT_DEFINE_PACKED_METRIC(kFlat, FLAT)
+#undef MUL
+#undef ADD
+#undef FMA
+#undef RCP
+#undef K
+#undef B
+
+// accel_part (kernel_mixed.cuh) with the compiler's contraction written out. m.gu.rr and
+// m.gu.hh come multiplied by -1/2 (halved_gu); the other factors of 2 and 1/2, which are
+// exact, are left out where they cancel.
+template <bool RLOG>
+__device__ __forceinline__ void accel_lean(const MetricAt<float>& m, const float u[4], float a[4]) {
+    const float w1t = __fmaf_rn(m.d1.tt, u[0], __fmul_rn(m.d1.tp, u[3]));
+    const float w1p = __fmaf_rn(m.d1.tp, u[0], __fmul_rn(m.d1.pp, u[3]));
+    const float w2t = __fmaf_rn(m.d2.tt, u[0], __fmul_rn(m.d2.tp, u[3]));
+    const float w2p = __fmaf_rn(m.d2.tp, u[0], __fmul_rn(m.d2.pp, u[3]));
+    const float w1r = __fmul_rn(m.d1.rr, u[1]), w1h = __fmul_rn(m.d1.hh, u[2]);
+    const float w2r = __fmul_rn(m.d2.rr, u[1]), w2h = __fmul_rn(m.d2.hh, u[2]);
+    const float p1r = __fmul_rn(u[1], w1r), p2h = __fmul_rn(u[2], w2h);
+    const float q1 = __fmaf_rn(u[3], w1p, __fmaf_rn(u[2], w1h, __fmaf_rn(u[0], w1t, p1r)));
+    const float q2 = __fmaf_rn(u[3], w2p, __fadd_rn(__fmaf_rn(u[0], w2t, __fmul_rn(u[1], w2r)), p2h));
+    const float Ft = __fmaf_rn(u[1], w1t, __fmul_rn(u[2], w2t));
+    const float Fp = __fmaf_rn(u[1], w1p, __fmul_rn(u[2], w2p));
+    const float Fr = __fmaf_rn(2.f, __fmaf_rn(u[1], w1r, __fmul_rn(u[2], w2r)), -q1);
+    const float Fh = __fmaf_rn(2.f, __fmaf_rn(u[1], w1h, p2h), -q2);
+    a[0] = -__fmaf_rn(m.gu.tt, Ft, __fmul_rn(m.gu.tp, Fp));
+    a[3] = -__fmaf_rn(m.gu.tp, Ft, __fmul_rn(m.gu.pp, Fp));
+    a[1] = __fmul_rn(m.gu.rr, Fr);
+    a[2] = __fmul_rn(m.gu.hh, Fh);
+    if (RLOG) a[1] = __fmaf_rn(-u[1], u[1], a[1]);
+}
+
+// Image constants a lane keeps.
+template <int MID>
+struct LeanConst {
+    float k[PackedMetric<MID>::kSlots ? PackedMetric<MID>::kSlots : 1];
+    float rp[2], rm[2], hthr[2];
+    float lrp[2];  // log-r only
+};
+
+// metric_part (kernel_mixed.cuh) with a plugin of PackedMetric, on every half.
+template <int MID, bool RLOG, typename T>
+__device__ __forceinline__ MetricAt<T> metric_lean(const LeanConst<MID>& C, T x1h, T x1l, T thh, T thl) {
+    T r, dp, dm;
+    if (!RLOG) {
+        r = p_add(x1h, x1l);
+        dp = p_add(p_sub(x1h, p_all<T>(C.rp[0])), p_sub(x1l, p_all<T>(C.rp[1])));
+        dm = p_add(p_sub(x1h, p_all<T>(C.rm[0])), p_sub(x1l, p_all<T>(C.rm[1])));
+    } else {
+        const T e = p_each([](float x) { return expf(x); }, x1h);
+        r = p_fma(e, x1l, e);
+        const T yp = p_add(p_sub(x1h, p_all<T>(C.lrp[0])), p_sub(x1l, p_all<T>(C.lrp[1])));
+        const float rp = C.rp[0];
+        dp = p_each([rp](float y, float rr) { return (y > 1.f) ? __fsub_rn(rr, rp) : __fmul_rn(rp, expm1f(y)); }, yp, r);
+        dm = p_sub(r, p_all<T>(C.rm[0]));
+    }
+    T s, c;
+    p_sincos(thh, thl, s, c);
+    MetricAt<T> m;
+    PackedMetric<MID>::template eval<T>(C.k, r, dp, dm, s, c, m.d1, m.d2, m.gu);
+    if (RLOG) {  // scale_log_r
+        const T r2 = p_mul(r, r);
+        m.d1.tt = p_mul(m.d1.tt, r);
+        m.d1.tp = p_mul(m.d1.tp, r);
+        m.d1.hh = p_mul(m.d1.hh, r);
+        m.d1.pp = p_mul(m.d1.pp, r);
+        m.d1.rr = p_mul(m.d1.rr, p_mul(r2, r));
+        m.d2.rr = p_mul(m.d2.rr, r2);
+        m.gu.rr = p_each([](float a, float b) { return __fdiv_rn(a, b); }, m.gu.rr, r2);
+    }
+    m.gu.rr = p_mul(p_all<T>(-0.5f), m.gu.rr);
+    m.gu.hh = p_mul(p_all<T>(-0.5f), m.gu.hh);
+    return m;
+}
+
+// One half of a packed metric part.
+__device__ __forceinline__ G5T<float> half_of(const G5T<f2>& g, bool hi) {
+    auto h = [hi](f2 a) { return hi ? hi2(a) : lo2(a); };
+    return {h(g.tt), h(g.tp), h(g.rr), h(g.hh), h(g.pp)};
+}
+__device__ __forceinline__ MetricAt<float> half_of(const MetricAt<f2>& m, bool hi) {
+    return {half_of(m.d1, hi), half_of(m.d2, hi), half_of(m.gu, hi)};
+}
+
+// adaptive_step_f32 (kernel_mixed.cuh) with the run's constants.
+__device__ __forceinline__ float adaptive_step_lean(const MixedRun& G, float thh, float thl, float v1, float v2, float v3) {
+    const float t = __fadd_rn(thh, thl), pt = __fadd_rn(__fsub_rn(G.pi[0], thh), __fsub_rn(G.pi[1], thl));
+    const float m = fabsf((pt < t) ? pt : t);
+    const float s1 = __fadd_rn(fabsf(v1), 1e-20f);
+    const float s2 = __fadd_rn(fabsf(v2), 1e-20f);
+    const float s3 = fabsf(__fadd_rn(v3, 1e-20f));
+    const float den = __fmaf_rn(m, __fadd_rn(s1, s3), s2);
+    const float inv = rcp(den);
+    const float num = __fmul_rn(G.eps[0], m);
+    const float q0 = __fmul_rn(num, inv);
+    const float res = __fmaf_rn(-q0, den, num);
+    const float h = __fmaf_rn(__fmaf_rn(G.eps[1], m, res), inv, q0);
+    return (h < G.hmin) ? G.hmin : h;
+}
+
+template <int MID, bool RLOG>
+struct LeanEngine {
+    static constexpr bool kLean = true;
+    static constexpr unsigned kRhsPerStep = 4;
+
+    // x and v: [0] holds components 0 and 1, [1] components 2 and 3, high and low parts.
+    struct Lane {
+        f2 xh[2], xl[2], vh[2], vl[2];
+        ff lam;
+        ff rmin;
+        LeanConst<MID> C;
+        uint64_t steps;
+        uint32_t err;
+        int32_t term;
+        int32_t passes;
+        int32_t side;  // EquatorialPasses' last sample: 0 none (or theta <= 0), 1 below, 2 above pi/2
+    };
+
+    static __device__ __forceinline__ void init(Lane& L, const ImageConst& I, const RunConst& R, const foort_pixel& p) {
+        double x[4], v[4];
+        initial_conditions(I, p, x, v);
+        ff fx[4], fv[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            ff_split(x[i], fx[i].hi, fx[i].lo);
+            ff_split(v[i], fv[i].hi, fv[i].lo);
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            L.xh[i] = pack2(fx[2 * i].hi, fx[2 * i + 1].hi);
+            L.xl[i] = pack2(fx[2 * i].lo, fx[2 * i + 1].lo);
+            L.vh[i] = pack2(fv[2 * i].hi, fv[2 * i + 1].hi);
+            L.vl[i] = pack2(fv[2 * i].lo, fv[2 * i + 1].lo);
+        }
+        PackedMetric<MID>::constants(I.mx.q, L.C.k);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            L.C.rp[i] = I.mx.rp[i];
+            L.C.rm[i] = I.mx.rm[i];
+            L.C.lrp[i] = I.mx.lrp[i];
+            L.C.hthr[i] = I.mx.hthr[i];
+        }
+        // without a horizon (r_h = 0) either threshold ends the ray: the larger one decides
+        if (I.m.rh == 0.0 && ff_lt(ff_of(I.mx.hthr), ff_of(I.mx.hthr0))) {
+            L.C.hthr[0] = I.mx.hthr0[0];
+            L.C.hthr[1] = I.mx.hthr0[1];
+        }
+        L.lam = {0.f, 0.f};
+        L.steps = 0;
+        L.err = 0;
+        L.term = FOORT_TERMCODE_CONTINUE;
+        L.passes = 0;
+        L.side = 0;
+        L.rmin = fx[1];  // Geodesic::Reset's start sample
+        diags(L, R);
+    }
+
+    // EquatorialPasses and ClosestRadius (MixedEngine::diags) on the new state.
+    static __device__ __forceinline__ void diags(Lane& L, const RunConst& R) {
+        if (R.diag_flags & FOORT_DIAG_EQUATORIAL_PASSES) {
+            const MixedRun& G = R.mr;
+            const float thh = lo2(L.xh[1]), d0 = __fadd_rn(thh, G.mpio2[0]);
+            bool upd = true, neg = d0 < 0.f;
+            if (!(fabsf(d0) > G.eqfar)) {  // near the equator: the float-float difference decides
+                const ff dt = ff_add(ff{thh, lo2(L.xl[1])}, ff_of(G.mpio2));
+                upd = ff_lt(ff_of(G.eqthr), ff_abs(dt));
+                neg = ff_neg_sign(dt);
+            }
+            const int32_t side = neg ? 1 : 2;
+            L.passes += (upd & (L.side + side == 3)) ? 1 : 0;
+            L.side = upd ? (thh > 0.f ? side : 0) : L.side;
+        }
+        if (R.diag_flags & FOORT_DIAG_CLOSEST_RADIUS) {
+            const ff x1 = {hi2(L.xh[0]), hi2(L.xl[0])};
+            const bool upd = ff_lt(x1, L.rmin);
+            L.rmin.hi = upd ? x1.hi : L.rmin.hi;
+            L.rmin.lo = upd ? x1.lo : L.rmin.lo;
+        }
+    }
+
+    // MixedEngine::terms with every termination checked at each step; L.steps counts the
+    // steps before this one, as TimeOut's counter does.
+    static __device__ __forceinline__ int terms(const Lane& L, const RunConst& R) {
+        const MixedRun& G = R.mr;
+        int code = FOORT_TERMCODE_CONTINUE;
+        if (R.term_flags & FOORT_TERM_THETA_SINGULARITY) {
+            // within theps of 0 or pi; well away from both, the high part alone says no
+            const float thh = lo2(L.xh[1]);
+            if (!(fminf(fabsf(thh), fabsf(__fadd_rn(thh, -G.pi[0]))) > G.thfar)) {
+                const ff th = {thh, lo2(L.xl[1])}, e = ff_of(G.theps);
+                const bool hit = ff_lt(ff_abs(th), e) | ff_lt(ff_abs(ff_add(ff_of(G.pi), ff_neg(th))), e);
+                code = hit ? FOORT_TERMCODE_THETA_SINGULARITY : code;
+            }
+        }
+        if (R.term_flags & FOORT_TERM_TIMEOUT)
+            code = (static_cast<uint32_t>(L.steps) >= R.t_max) ? FOORT_TERMCODE_TIMEOUT : code;
+        const ff x1 = {hi2(L.xh[0]), hi2(L.xl[0])};
+        if (R.term_flags & FOORT_TERM_BOUNDARY_SPHERE)
+            code = ff_lt(ff_of(G.bthr), x1) ? FOORT_TERMCODE_BOUNDARY_SPHERE : code;
+        if (R.term_flags & FOORT_TERM_HORIZON) code = ff_lt(x1, ff_of(L.C.hthr)) ? FOORT_TERMCODE_HORIZON : code;
+        return code;
+    }
+
+    static __device__ __forceinline__ bool step(Lane& L, const RunConst& R) {
+        const f2 uf01 = p_add(L.vh[0], L.vl[0]), uf23 = p_add(L.vh[1], L.vl[1]);
+        const float uf[4] = {lo2(uf01), hi2(uf01), lo2(uf23), hi2(uf23)};
+        const float x1h = hi2(L.xh[0]), x1l = hi2(L.xl[0]), thh = lo2(L.xh[1]), thl = lo2(L.xl[1]);
+        const float h = adaptive_step_lean(R.mr, thh, thl, uf[1], uf[2], uf[3]);
+        const float hh = 0.5f * h;
+        const f2 hh2 = pack2(hh, hh), h2 = pack2(h, h);
+        float k1[4], k2[4], k3[4], k4[4], us[4];
+        // stages 1 (low half) and 2 (high half)
+        f2 ph, pl;
+        p_ff_add_f(pack2(x1h, thh), pack2(x1l, thl), p_mul(hh2, pack2(uf[1], uf[2])), ph, pl);
+        MetricAt<f2> m = metric_lean<MID, RLOG, f2>(L.C, pack2(x1h, lo2(ph)), pack2(x1l, lo2(pl)), pack2(thh, hi2(ph)),
+                                                    pack2(thl, hi2(pl)));
+        accel_lean<RLOG>(half_of(m, false), uf, k1);
+        stage(hh2, uf01, uf23, k1, us);
+        accel_lean<RLOG>(half_of(m, true), us, k2);
+        // stages 3 and 4: x + h/2 (u + h/2 k1), x + h (u + h/2 k2)
+        const f2 hs = pack2(hh, h);
+        f2 rh, rl, qh, ql;
+        p_ff_add_f(pack2(x1h, x1h), pack2(x1l, x1l),
+                   p_mul(hs, p_fma(hh2, pack2(k1[1], k2[1]), pack2(uf[1], uf[1]))), rh, rl);
+        p_ff_add_f(pack2(thh, thh), pack2(thl, thl),
+                   p_mul(hs, p_fma(hh2, pack2(k1[2], k2[2]), pack2(uf[2], uf[2]))), qh, ql);
+        m = metric_lean<MID, RLOG, f2>(L.C, rh, rl, qh, ql);
+        stage(hh2, uf01, uf23, k2, us);
+        accel_lean<RLOG>(half_of(m, false), us, k3);
+        stage(h2, uf01, uf23, k3, us);
+        accel_lean<RLOG>(half_of(m, true), us, k4);
+        return advance(L, R, h, k1, k2, k3, k4);
+    }
+
+    // The step on two lanes (MixedEngine::step_pair): in each of two rounds the even lane
+    // evaluates stage 1 (then 3) and the odd lane stage 2 (then 4).
+    static __device__ __forceinline__ bool step_pair(Lane& L, const RunConst& R, bool odd, unsigned pmask) {
+        const f2 uf01 = p_add(L.vh[0], L.vl[0]), uf23 = p_add(L.vh[1], L.vl[1]);
+        const float uf[4] = {lo2(uf01), hi2(uf01), lo2(uf23), hi2(uf23)};
+        const f2 x12h = pack2(hi2(L.xh[0]), lo2(L.xh[1])), x12l = pack2(hi2(L.xl[0]), lo2(L.xl[1]));
+        const float h = adaptive_step_lean(R.mr, hi2(x12h), hi2(x12l), uf[1], uf[2], uf[3]);
+        const float hh = 0.5f * h;
+        const f2 hh2 = pack2(hh, hh), h2 = pack2(h, h), uf12 = pack2(uf[1], uf[2]);
+        float k1[4], k2[4], k3[4], k4[4], us[4], ka[4];
+        auto share = [&](float k[4], int from) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) k[i] = __shfl_sync(pmask, ka[i], from, 2);
+        };
+        f2 ph, pl;
+        p_ff_add_f(x12h, x12l, p_mul(hh2, uf12), ph, pl);
+        MetricAt<float> m = metric_lean<MID, RLOG, float>(L.C, odd ? lo2(ph) : lo2(x12h), odd ? lo2(pl) : lo2(x12l),
+                                                          odd ? hi2(ph) : hi2(x12h), odd ? hi2(pl) : hi2(x12l));
+        accel_lean<RLOG>(m, uf, ka);
+        share(k1, 0);
+        stage(hh2, uf01, uf23, k1, us);
+        accel_lean<RLOG>(m, us, ka);
+        share(k2, 1);
+        const float hs = odd ? h : hh;
+        const f2 k12 = odd ? pack2(k2[1], k2[2]) : pack2(k1[1], k1[2]);
+        p_ff_add_f(x12h, x12l, p_mul(pack2(hs, hs), p_fma(hh2, k12, uf12)), ph, pl);
+        m = metric_lean<MID, RLOG, float>(L.C, lo2(ph), lo2(pl), hi2(ph), hi2(pl));
+        stage(hh2, uf01, uf23, k2, us);
+        accel_lean<RLOG>(m, us, ka);
+        share(k3, 0);
+        stage(h2, uf01, uf23, k3, us);
+        accel_lean<RLOG>(m, us, ka);
+        share(k4, 1);
+        return advance(L, R, h, k1, k2, k3, k4);
+    }
+
+    // us = u + t k
+    static __device__ __forceinline__ void stage(f2 t, f2 uf01, f2 uf23, const float k[4], float us[4]) {
+        const f2 a = p_fma(t, pack2(k[0], k[1]), uf01), b = p_fma(t, pack2(k[2], k[3]), uf23);
+        us[0] = lo2(a);
+        us[1] = hi2(a);
+        us[2] = lo2(b);
+        us[3] = hi2(b);
+    }
+
+    // MixedEngine::rk4_combine, advance and after_step.
+    static __device__ __forceinline__ bool advance(Lane& L, const RunConst& R, float h, const float k1[4],
+                                                   const float k2[4], const float k3[4], const float k4[4]) {
+        const float q0 = __fmul_rn(h, 0.166666672f);
+        const float h6 = __fmaf_rn(__fmaf_rn(-6.f, q0, h), 0.166666672f, q0), hh6 = __fmul_rn(h, h6);
+        const f2 two = p_all<f2>(2.f), ph = p_all<f2>(h), ph6 = p_all<f2>(h6), phh6 = p_all<f2>(hh6);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const f2 a1 = pack2(k1[2 * i], k1[2 * i + 1]), a2 = pack2(k2[2 * i], k2[2 * i + 1]);
+            const f2 a3 = pack2(k3[2 * i], k3[2 * i + 1]), a4 = pack2(k4[2 * i], k4[2 * i + 1]);
+            const f2 du = p_mul(ph6, p_add(p_fma(two, a3, p_fma(two, a2, a1)), a4));
+            const f2 dxc = p_mul(phh6, p_add(p_add(a1, a2), a3));
+            const f2 th = p_mul(ph, L.vh[i]), tl = p_fma(ph, L.vh[i], -th);
+            const f2 bl = p_add(tl, p_fma(ph, L.vl[i], dxc));
+            f2 s, e;
+            p_two_sum(L.xh[i], th, s, e);
+            p_fast_two_sum(s, p_add(e, p_add(L.xl[i], bl)), L.xh[i], L.xl[i]);
+            p_ff_add_f(L.vh[i], L.vl[i], du, L.vh[i], L.vl[i]);
+        }
+        L.lam = ff_add_f(L.lam, h);
+        L.term = terms(L, R);
+        ++L.steps;
+        diags(L, R);
+        const bool bad = !(isfinite(hi2(L.xh[0])) & isfinite(hi2(L.vh[0])));
+        L.err |= bad ? FOORT_ERR_NONFINITE : 0u;
+        return (L.term == FOORT_TERMCODE_CONTINUE) & !(bad & !(R.term_flags & FOORT_TERM_TIMEOUT));
+    }
+
+    static __device__ __forceinline__ void write(const Lane& L, const RunConst& R, foort_result* o, int term,
+                                                 uint32_t err) {
+        double x[4], v[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float2 xh = unpack2(L.xh[i / 2]), xl = unpack2(L.xl[i / 2]);
+            const float2 vh = unpack2(L.vh[i / 2]), vl = unpack2(L.vl[i / 2]);
+            x[i] = (i & 1) ? ff_d({xh.y, xl.y}) : ff_d({xh.x, xl.x});
+            v[i] = (i & 1) ? ff_d({vh.y, vl.y}) : ff_d({vh.x, vl.x});
+        }
+        if (!(finite4(x) && finite4(v))) err |= FOORT_ERR_NONFINITE;
+        DiagState D;
+        D.quad = 0;
+        if ((R.diag_flags & FOORT_DIAG_FOUR_COLOR_SCREEN) && term == FOORT_TERMCODE_BOUNDARY_SPHERE)
+            D.quad = four_color_quadrant(x[2], x[3]);
+        D.passes = (term == FOORT_TERMCODE_HORIZON) ? -L.passes : L.passes;
+        D.rmin = -1.0;
+        if (R.diag_flags & FOORT_DIAG_CLOSEST_RADIUS) {
+            D.rmin = RLOG ? exp(ff_d(L.rmin)) : ff_d(L.rmin);
+            if (term == FOORT_TERMCODE_HORIZON) D.rmin = 0.0;
+        }
+        write_result(o, term, err, L.steps, ff_d(L.lam), x, v, D);
+    }
+    static __device__ __forceinline__ void finish(const Lane& L, const RunConst& R, foort_result* o) {
+        write(L, R, o, L.term, L.err);
+    }
+    static __device__ __forceinline__ void stop(const Lane& L, const RunConst& R, foort_result* o, uint32_t err) {
+        write(L, R, o, FOORT_TERMCODE_CONTINUE, L.err | err);
+    }
+};
+
+}  // namespace foort

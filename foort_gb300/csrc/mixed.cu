@@ -42,6 +42,52 @@ const void* mixed_pair_kernel_variant(int metric_id, int integ, bool decide64) {
     }
 }
 
+const void* mixed_lean_kernel_kerr(bool rlog);
+const void* mixed_lean_kernel_flat();
+const void* mixed_lean_pair_kernel_kerr(bool rlog);
+const void* mixed_lean_pair_kernel_flat();
+
+// Lean options: every termination and diagnostic in use updates at each step (the
+// default), and nothing needs FP64 steps or FP64 decisions.
+static bool lean_options(const RunConst& R) {
+    if (R.precision != FOORT_PREC_MIXED || R.mixed_fp64_margin > 0.0 ||
+        (R.mixed_options & (FOORT_MIXED_FP64_DECISIONS | FOORT_MIXED_FP64_TURNING_POINTS)))
+        return false;
+    auto each_step = [](uint32_t flags, uint32_t flag, uint64_t every) { return !(flags & flag) || every == 1; };
+    return each_step(R.term_flags, FOORT_TERM_HORIZON, R.h_every) &&
+           each_step(R.term_flags, FOORT_TERM_BOUNDARY_SPHERE, R.b_every) &&
+           each_step(R.term_flags, FOORT_TERM_TIMEOUT, R.t_every) &&
+           each_step(R.term_flags, FOORT_TERM_THETA_SINGULARITY, R.th_every) &&
+           each_step(R.diag_flags, FOORT_DIAG_EQUATORIAL_PASSES, R.eq_every) &&
+           each_step(R.diag_flags, FOORT_DIAG_CLOSEST_RADIUS, R.cr_every);
+}
+
+const void* mixed_lean_kernel(const RunConst& R, bool pair) {
+    if (!lean_options(R) || R.integrator != FOORT_INTEGRATOR_RK4) return nullptr;
+    switch (R.metric_id) {
+    case kKerr: return pair ? mixed_lean_pair_kernel_kerr(R.rlog != 0) : mixed_lean_kernel_kerr(R.rlog != 0);
+    case kFlat: return R.rlog ? nullptr : pair ? mixed_lean_pair_kernel_flat() : mixed_lean_kernel_flat();
+    default: return nullptr;
+    }
+}
+
+void fill_mixed_run(RunConst& rc) {
+    MixedRun& m = rc.mr;
+    ff_split(rc.rlog ? std::log(rc.b_rad) : rc.b_rad, m.bthr[0], m.bthr[1]);
+    ff_split(rc.th_eps, m.theps[0], m.theps[1]);
+    ff_split(kRefPi, m.pi[0], m.pi[1]);
+    ff_split(-(kRefPi / 2.0), m.mpio2[0], m.mpio2[1]);
+    ff_split(kRefPi / 2.0 * rc.eq_thr, m.eqthr[0], m.eqthr[1]);
+    ff_split(rc.eps, m.eps[0], m.eps[1]);
+    m.hmin = static_cast<float>(rc.hmin);
+    // a positive tolerance whose square is below FP32's range still iterates (as with 0)
+    m.vtol2 = rc.vtol > 0.0 ? std::max(static_cast<float>(rc.vtol * rc.vtol), FLT_MIN) : 0.f;
+    // theta's high part differs from theta by 6e-8 of it, so a distance from pi / 2 (or
+    // from 0 and pi) this much above the threshold leaves no doubt
+    m.eqfar = std::max(m.eqthr[0], 0.f) * 1.00001f + 4e-6f;
+    m.thfar = std::max(m.theps[0], 0.f) * 1.00001f + 4e-6f;
+}
+
 void fill_mixed_constants(int metric_id, ImageConst& ic, const RunConst& rc) {
     MixedConst& mx = ic.mx;
     mixed_metric_constants(metric_id, ic.m, ic.qa);
@@ -67,15 +113,18 @@ void fill_mixed_constants(int metric_id, ImageConst& ic, const RunConst& rc) {
     const double rh = ic.m.rh;
     ff_split(coord(rh * (1 + ic.h_eps)), mx.hthr[0], mx.hthr[1]);
     ff_split(ic.h_eps > 0 ? coord(ic.h_eps) : (rlog ? -HUGE_VAL : 0.0), mx.hthr0[0], mx.hthr0[1]);
-    ff_split(coord(rc.b_rad), mx.bthr[0], mx.bthr[1]);
-    ff_split(rc.th_eps, mx.theps[0], mx.theps[1]);
-    ff_split(kRefPi, mx.pi[0], mx.pi[1]);
-    ff_split(-(kRefPi / 2.0), mx.mpio2[0], mx.mpio2[1]);
-    ff_split(kRefPi / 2.0 * rc.eq_thr, mx.eqthr[0], mx.eqthr[1]);
-    ff_split(rc.eps, mx.eps[0], mx.eps[1]);
-    mx.hmin = static_cast<float>(rc.hmin);
-    // a positive tolerance whose square is below FP32's range still iterates (as with 0)
-    mx.vtol2 = rc.vtol > 0.0 ? std::max(static_cast<float>(rc.vtol * rc.vtol), FLT_MIN) : 0.f;
+    // the run's constants, also where the general kernels read them
+    const MixedRun& m = rc.mr;
+    for (int i = 0; i < 2; ++i) {
+        mx.bthr[i] = m.bthr[i];
+        mx.theps[i] = m.theps[i];
+        mx.pi[i] = m.pi[i];
+        mx.mpio2[i] = m.mpio2[i];
+        mx.eqthr[i] = m.eqthr[i];
+        mx.eps[i] = m.eps[i];
+    }
+    mx.hmin = m.hmin;
+    mx.vtol2 = m.vtol2;
 }
 
 }  // namespace foort

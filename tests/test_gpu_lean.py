@@ -1,0 +1,96 @@
+"""The lean mixed kernels (kernel_lean.cuh) against the general ones: the same records bit
+for bit. FOORT_MIXED_FP64_DECISIONS takes the general kernel, whose decisions agree with
+the float-float ones except within 2^-48 of a threshold, so no tolerance is needed."""
+import os
+import subprocess
+import sys
+
+import numpy as np
+import pytest
+
+from conftest import ROOT
+from foort_gb300 import abi, workloads
+
+ALL_DIAGS = abi.DIAG_FOUR_COLOR_SCREEN | abi.DIAG_EQUATORIAL_PASSES | abi.DIAG_CLOSEST_RADIUS
+
+
+@pytest.fixture(scope="module")
+def eng():
+    import foort_gb300
+    from foort_gb300 import build as engine_build
+    engine_build.build()
+    foort_gb300.check_layout()
+    return foort_gb300
+
+
+def describe(metric, params, rlog, inclination, integrator=abi.INTEGRATOR_RK4, timeout=None):
+    d = workloads.base_desc(abi.PREC_MIXED)
+    d.metric_id, d.rlog, d.integrator_id = metric, rlog, integrator
+    d.timeout_max_steps = timeout or (10000 if rlog else 100000)
+    d.diag_flags = ALL_DIAGS
+    if rlog:
+        d.term_flags |= abi.TERM_THETA_SINGULARITY
+    keep = abi.attach_images(d, [abi.make_image(params, r=1000.0, theta=np.radians(inclination), half_width=9.0)])
+    return d, keep
+
+
+def same_records(a, b):
+    for name in abi.RESULT_DTYPE.names:
+        np.testing.assert_array_equal(a[name], b[name], err_msg=name)
+
+
+# spins from none to near-extremal, views along the axis and from the equator (where every
+# step is inside EquatorialPasses' threshold), a ray that ends after one step
+@pytest.mark.gpu
+@pytest.mark.parametrize("metric,params,rlog,inclination,side,timeout", [
+    (abi.METRIC_KERR, (0.0,), 1, 63.0, 23, None),
+    (abi.METRIC_KERR, (0.998,), 1, 17.0, 37, None),
+    (abi.METRIC_KERR, (0.7,), 1, 90.0, 21, None),
+    (abi.METRIC_KERR, (0.9,), 1, 2.0, 21, None),
+    (abi.METRIC_KERR, (0.9,), 0, 80.0, 9, None),
+    (abi.METRIC_KERR, (0.9,), 0, 60.0, 2, None),
+    (abi.METRIC_KERR, (0.9,), 1, 60.0, 33, 0),
+    (abi.METRIC_KERR, (0.9,), 1, 60.0, 33, 400),
+    (abi.METRIC_FLAT, (), 0, 63.0, 7, None),
+])
+def test_lean_kernels_give_the_general_kernels_records(eng, metric, params, rlog, inclination, side, timeout):
+    px = abi.square_pixels(side)
+    d, keep = describe(metric, params, rlog, inclination, timeout=timeout)
+    got = {}
+    for lanes in (1, 2):
+        with eng.Engine(d) as e:
+            e.set_lanes(lanes)
+            got[lanes] = e.integrate(px)
+            counts = e.stats()
+            assert counts["rhs_evals"] == 4 * counts["steps"] == 4 * int(got[lanes]["steps"].sum())
+    d.mixed_options = abi.MIXED_FP64_DECISIONS
+    with eng.Engine(d) as e:
+        e.set_lanes(1)
+        want = e.integrate(px)
+    same_records(got[1], want)
+    same_records(got[2], want)
+    del keep
+
+
+@pytest.mark.gpu
+def test_a_full_gpu_of_refilled_lanes_gives_the_general_kernels_records(eng):
+    """More pixels than resident lanes, so that every lane is refilled, with two images of
+    different spins side by side."""
+    d, _ = describe(abi.METRIC_KERR, (0.9,), 1, 70.0)
+    keep = abi.attach_images(d, [abi.make_image((a,), r=1000.0, theta=1.2, half_width=8.0) for a in (0.9, 0.2)])
+    px = np.concatenate([abi.square_pixels(260, image=i) for i in (0, 1)])
+    px = px[np.random.default_rng(5).permutation(len(px))]
+    with eng.Engine(d) as e:
+        got = e.integrate(px)
+    d.mixed_options = abi.MIXED_FP64_DECISIONS
+    with eng.Engine(d) as e:
+        same_records(got, e.integrate(px))
+    del keep
+
+
+def test_packed_bodies_match_the_generator():
+    """gen_packed.inc is what gen_packed.py prints for the committed gen_christoffel.inc."""
+    gen = os.path.join(ROOT, "foort_gb300", "gen", "gen_packed.py")
+    out = subprocess.run([sys.executable, gen], check=True, capture_output=True, text=True).stdout
+    with open(os.path.join(ROOT, "foort_gb300", "csrc", "gen_packed.inc")) as f:
+        assert f.read() == out
