@@ -247,9 +247,12 @@ struct LaunchShape {
 //   geodesics in log r 1.31 ms on two lanes and 1.58 on one. In plain r both take the same
 //   within 3 % (3,000 geodesics 66 and 64 ms, 1.00 and 0.97 us a step): the smallest launches
 //   stay on two, the rest take one.
+// - Lean kernels with a called plugin exist on two lanes only and cost a geodesic no more
+//   than the general one-lane kernel: every size.
 uint64_t pair_limit(const RunConst& R, bool positions, int per_sm, int num_sms, uint32_t bs) {
     const uint64_t sms = static_cast<uint64_t>(num_sms);
-    if (!positions && mixed_lean_kernel(R, true)) return (R.rlog ? 64 : 24) * sms;
+    if (!positions && mixed_lean_kernel(R, true))
+        return mixed_lean_kernel(R, false) ? (R.rlog ? 64 : 24) * sms : UINT64_MAX;
     return static_cast<uint64_t>(per_sm) * sms * bs / 2;
 }
 

@@ -61,37 +61,57 @@ FOORT_DEFINE_PACKED_METRIC(kFlat, FLAT)
 #undef K
 #undef B
 
-// accel_part (kernel_mixed.cuh) with the compiler's contraction written out. m.gu.rr and
-// m.gu.hh come multiplied by -1/2 (halved_gu); the other factors of 2 and 1/2, which are
-// exact, are left out where they cancel.
-template <bool RLOG>
+// accel_part (kernel_mixed.cuh) with the compiler's contraction written out. Where a sum has
+// two products, it depends on the code around which of them joins as a fused multiply-add:
+// FORM 0 is the step with an inlined plugin, 1 and 2 the called right-hand side of
+// Johannsen and of Rasheed-Larsen. m.gu.rr and m.gu.hh come multiplied by -1/2; the other
+// factors of 2 and 1/2, which are exact, are left out where they cancel.
+template <int FORM>
 __device__ __forceinline__ void accel_lean(const MetricAt<float>& m, const float u[4], float a[4]) {
-    const float w1t = __fmaf_rn(m.d1.tt, u[0], __fmul_rn(m.d1.tp, u[3]));
-    const float w1p = __fmaf_rn(m.d1.tp, u[0], __fmul_rn(m.d1.pp, u[3]));
-    const float w2t = __fmaf_rn(m.d2.tt, u[0], __fmul_rn(m.d2.tp, u[3]));
-    const float w2p = __fmaf_rn(m.d2.tp, u[0], __fmul_rn(m.d2.pp, u[3]));
+    // x y + z w with the first or the second product fused
+    auto first = [](float x, float y, float z, float w) { return __fmaf_rn(x, y, __fmul_rn(z, w)); };
+    auto second = [](float x, float y, float z, float w) { return __fmaf_rn(z, w, __fmul_rn(x, y)); };
+    const float w1t = first(m.d1.tt, u[0], m.d1.tp, u[3]), w1p = first(m.d1.tp, u[0], m.d1.pp, u[3]);
+    const float w2t = first(m.d2.tt, u[0], m.d2.tp, u[3]);
+    const float w2p = (FORM == 1) ? second(m.d2.tp, u[0], m.d2.pp, u[3]) : first(m.d2.tp, u[0], m.d2.pp, u[3]);
     const float w1r = __fmul_rn(m.d1.rr, u[1]), w1h = __fmul_rn(m.d1.hh, u[2]);
     const float w2r = __fmul_rn(m.d2.rr, u[1]), w2h = __fmul_rn(m.d2.hh, u[2]);
-    const float p1r = __fmul_rn(u[1], w1r), p2h = __fmul_rn(u[2], w2h);
-    const float q1 = __fmaf_rn(u[3], w1p, __fmaf_rn(u[2], w1h, __fmaf_rn(u[0], w1t, p1r)));
-    const float q2 = __fmaf_rn(u[3], w2p, __fadd_rn(__fmaf_rn(u[0], w2t, __fmul_rn(u[1], w2r)), p2h));
-    const float Ft = __fmaf_rn(u[1], w1t, __fmul_rn(u[2], w2t));
-    const float Fp = __fmaf_rn(u[1], w1p, __fmul_rn(u[2], w2p));
-    const float Fr = __fmaf_rn(2.f, __fmaf_rn(u[1], w1r, __fmul_rn(u[2], w2r)), -q1);
-    const float Fh = __fmaf_rn(2.f, __fmaf_rn(u[1], w1h, p2h), -q2);
-    a[0] = -__fmaf_rn(m.gu.tt, Ft, __fmul_rn(m.gu.tp, Fp));
-    a[3] = -__fmaf_rn(m.gu.tp, Ft, __fmul_rn(m.gu.pp, Fp));
+    const float q1 = __fmaf_rn(u[3], w1p, __fmaf_rn(u[2], w1h, first(u[0], w1t, u[1], w1r)));
+    const float q2a = first(u[0], w2t, u[1], w2r);
+    const float q2b = FORM ? __fmaf_rn(u[2], w2h, q2a) : __fadd_rn(q2a, __fmul_rn(u[2], w2h));
+    const float q2 = __fmaf_rn(u[3], w2p, q2b);
+    const float Ft = FORM ? second(u[1], w1t, u[2], w2t) : first(u[1], w1t, u[2], w2t);
+    const float Fp = FORM ? second(u[1], w1p, u[2], w2p) : first(u[1], w1p, u[2], w2p);
+    const float Fr = __fmaf_rn(2.f, first(u[1], w1r, u[2], w2r), -q1);
+    const float Fh = __fmaf_rn(2.f, FORM ? second(u[1], w1h, u[2], w2h) : first(u[1], w1h, u[2], w2h), -q2);
+    a[0] = -first(m.gu.tt, Ft, m.gu.tp, Fp);
+    a[3] = -first(m.gu.tp, Ft, m.gu.pp, Fp);
     a[1] = __fmul_rn(m.gu.rr, Fr);
     a[2] = __fmul_rn(m.gu.hh, Fh);
-    if (RLOG) a[1] = __fmaf_rn(-u[1], u[1], a[1]);
+}
+// In log-r mode the coordinate term -(u^1)^2 joins a^1 (accel_log_r).
+template <int FORM>
+__device__ __forceinline__ void accel_lean(const MetricAt<float>& m, bool rlog, const float u[4], float a[4]) {
+    accel_lean<FORM>(m, u, a);
+    if (rlog) a[1] = __fmaf_rn(-u[1], u[1], a[1]);
 }
 
-// Image constants a lane keeps.
+// Image constants a lane of a packed plugin keeps.
 template <int MID>
 struct LeanConst {
     float k[PackedMetric<MID>::kSlots ? PackedMetric<MID>::kSlots : 1];
-    float rp[2], rm[2], hthr[2];
+    float rp[2], rm[2];
     float lrp[2];  // log-r only
+
+    __device__ __forceinline__ void load(const ImageConst& I) {
+        PackedMetric<MID>::constants(I.mx.q, k);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            rp[i] = I.mx.rp[i];
+            rm[i] = I.mx.rm[i];
+            lrp[i] = I.mx.lrp[i];
+        }
+    }
 };
 
 // metric_part (kernel_mixed.cuh) with a plugin of PackedMetric, on every half.
@@ -154,17 +174,19 @@ __device__ __forceinline__ float adaptive_step_lean(const MixedRun& G, float thh
     return (h < G.hmin) ? G.hmin : h;
 }
 
-template <int MID, bool RLOG>
-struct LeanEngine {
+// A lane's state and everything of a step but its right-hand sides. C: the image constants
+// that those need.
+template <class C>
+struct LeanState {
     static constexpr bool kLean = true;
-    static constexpr unsigned kRhsPerStep = 4;
 
     // x and v: [0] holds components 0 and 1, [1] components 2 and 3, high and low parts.
     struct Lane {
         f2 xh[2], xl[2], vh[2], vl[2];
         ff lam;
         ff rmin;
-        LeanConst<MID> C;
+        float hthr[2];
+        C c;
         uint64_t steps;
         uint32_t err;
         int32_t term;
@@ -188,18 +210,13 @@ struct LeanEngine {
             L.vh[i] = pack2(fv[2 * i].hi, fv[2 * i + 1].hi);
             L.vl[i] = pack2(fv[2 * i].lo, fv[2 * i + 1].lo);
         }
-        PackedMetric<MID>::constants(I.mx.q, L.C.k);
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            L.C.rp[i] = I.mx.rp[i];
-            L.C.rm[i] = I.mx.rm[i];
-            L.C.lrp[i] = I.mx.lrp[i];
-            L.C.hthr[i] = I.mx.hthr[i];
-        }
+        L.c.load(I);
+        L.hthr[0] = I.mx.hthr[0];
+        L.hthr[1] = I.mx.hthr[1];
         // without a horizon (r_h = 0) either threshold ends the ray: the larger one decides
         if (I.m.rh == 0.0 && ff_lt(ff_of(I.mx.hthr), ff_of(I.mx.hthr0))) {
-            L.C.hthr[0] = I.mx.hthr0[0];
-            L.C.hthr[1] = I.mx.hthr0[1];
+            L.hthr[0] = I.mx.hthr0[0];
+            L.hthr[1] = I.mx.hthr0[1];
         }
         L.lam = {0.f, 0.f};
         L.steps = 0;
@@ -253,75 +270,8 @@ struct LeanEngine {
         const ff x1 = {hi2(L.xh[0]), hi2(L.xl[0])};
         if (R.term_flags & FOORT_TERM_BOUNDARY_SPHERE)
             code = ff_lt(ff_of(G.bthr), x1) ? FOORT_TERMCODE_BOUNDARY_SPHERE : code;
-        if (R.term_flags & FOORT_TERM_HORIZON) code = ff_lt(x1, ff_of(L.C.hthr)) ? FOORT_TERMCODE_HORIZON : code;
+        if (R.term_flags & FOORT_TERM_HORIZON) code = ff_lt(x1, ff_of(L.hthr)) ? FOORT_TERMCODE_HORIZON : code;
         return code;
-    }
-
-    static __device__ __forceinline__ bool step(Lane& L, const RunConst& R) {
-        const f2 uf01 = p_add(L.vh[0], L.vl[0]), uf23 = p_add(L.vh[1], L.vl[1]);
-        const float uf[4] = {lo2(uf01), hi2(uf01), lo2(uf23), hi2(uf23)};
-        const float x1h = hi2(L.xh[0]), x1l = hi2(L.xl[0]), thh = lo2(L.xh[1]), thl = lo2(L.xl[1]);
-        const float h = adaptive_step_lean(R.mr, thh, thl, uf[1], uf[2], uf[3]);
-        const float hh = 0.5f * h;
-        const f2 hh2 = pack2(hh, hh), h2 = pack2(h, h);
-        float k1[4], k2[4], k3[4], k4[4], us[4];
-        // stages 1 (low half) and 2 (high half)
-        f2 ph, pl;
-        p_ff_add_f(pack2(x1h, thh), pack2(x1l, thl), p_mul(hh2, pack2(uf[1], uf[2])), ph, pl);
-        MetricAt<f2> m = metric_lean<MID, RLOG, f2>(L.C, pack2(x1h, lo2(ph)), pack2(x1l, lo2(pl)), pack2(thh, hi2(ph)),
-                                                    pack2(thl, hi2(pl)));
-        accel_lean<RLOG>(half_of(m, false), uf, k1);
-        stage(hh2, uf01, uf23, k1, us);
-        accel_lean<RLOG>(half_of(m, true), us, k2);
-        // stages 3 and 4: x + h/2 (u + h/2 k1), x + h (u + h/2 k2)
-        const f2 hs = pack2(hh, h);
-        f2 rh, rl, qh, ql;
-        p_ff_add_f(pack2(x1h, x1h), pack2(x1l, x1l),
-                   p_mul(hs, p_fma(hh2, pack2(k1[1], k2[1]), pack2(uf[1], uf[1]))), rh, rl);
-        p_ff_add_f(pack2(thh, thh), pack2(thl, thl),
-                   p_mul(hs, p_fma(hh2, pack2(k1[2], k2[2]), pack2(uf[2], uf[2]))), qh, ql);
-        m = metric_lean<MID, RLOG, f2>(L.C, rh, rl, qh, ql);
-        stage(hh2, uf01, uf23, k2, us);
-        accel_lean<RLOG>(half_of(m, false), us, k3);
-        stage(h2, uf01, uf23, k3, us);
-        accel_lean<RLOG>(half_of(m, true), us, k4);
-        return advance(L, R, h, k1, k2, k3, k4);
-    }
-
-    // The step on two lanes (MixedEngine::step_pair): in each of two rounds the even lane
-    // evaluates stage 1 (then 3) and the odd lane stage 2 (then 4).
-    static __device__ __forceinline__ bool step_pair(Lane& L, const RunConst& R, bool odd, unsigned pmask) {
-        const f2 uf01 = p_add(L.vh[0], L.vl[0]), uf23 = p_add(L.vh[1], L.vl[1]);
-        const float uf[4] = {lo2(uf01), hi2(uf01), lo2(uf23), hi2(uf23)};
-        const f2 x12h = pack2(hi2(L.xh[0]), lo2(L.xh[1])), x12l = pack2(hi2(L.xl[0]), lo2(L.xl[1]));
-        const float h = adaptive_step_lean(R.mr, hi2(x12h), hi2(x12l), uf[1], uf[2], uf[3]);
-        const float hh = 0.5f * h;
-        const f2 hh2 = pack2(hh, hh), h2 = pack2(h, h), uf12 = pack2(uf[1], uf[2]);
-        float k1[4], k2[4], k3[4], k4[4], us[4], ka[4];
-        auto share = [&](float k[4], int from) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) k[i] = __shfl_sync(pmask, ka[i], from, 2);
-        };
-        f2 ph, pl;
-        p_ff_add_f(x12h, x12l, p_mul(hh2, uf12), ph, pl);
-        MetricAt<float> m = metric_lean<MID, RLOG, float>(L.C, odd ? lo2(ph) : lo2(x12h), odd ? lo2(pl) : lo2(x12l),
-                                                          odd ? hi2(ph) : hi2(x12h), odd ? hi2(pl) : hi2(x12l));
-        accel_lean<RLOG>(m, uf, ka);
-        share(k1, 0);
-        stage(hh2, uf01, uf23, k1, us);
-        accel_lean<RLOG>(m, us, ka);
-        share(k2, 1);
-        const float hs = odd ? h : hh;
-        const f2 k12 = odd ? pack2(k2[1], k2[2]) : pack2(k1[1], k1[2]);
-        p_ff_add_f(x12h, x12l, p_mul(pack2(hs, hs), p_fma(hh2, k12, uf12)), ph, pl);
-        m = metric_lean<MID, RLOG, float>(L.C, lo2(ph), lo2(pl), hi2(ph), hi2(pl));
-        stage(hh2, uf01, uf23, k2, us);
-        accel_lean<RLOG>(m, us, ka);
-        share(k3, 0);
-        stage(h2, uf01, uf23, k3, us);
-        accel_lean<RLOG>(m, us, ka);
-        share(k4, 1);
-        return advance(L, R, h, k1, k2, k3, k4);
     }
 
     // us = u + t k
@@ -379,7 +329,7 @@ struct LeanEngine {
         D.passes = (term == FOORT_TERMCODE_HORIZON) ? -L.passes : L.passes;
         D.rmin = -1.0;
         if (R.diag_flags & FOORT_DIAG_CLOSEST_RADIUS) {
-            D.rmin = RLOG ? exp(ff_d(L.rmin)) : ff_d(L.rmin);
+            D.rmin = R.rlog ? exp(ff_d(L.rmin)) : ff_d(L.rmin);
             if (term == FOORT_TERMCODE_HORIZON) D.rmin = 0.0;
         }
         write_result(o, term, err, L.steps, ff_d(L.lam), x, v, D);
@@ -389,6 +339,153 @@ struct LeanEngine {
     }
     static __device__ __forceinline__ void stop(const Lane& L, const RunConst& R, foort_result* o, uint32_t err) {
         write(L, R, o, FOORT_TERMCODE_CONTINUE, L.err | err);
+    }
+};
+
+// RK4 with a packed plugin.
+template <int MID, bool RLOG>
+struct LeanEngine : LeanState<LeanConst<MID>> {
+    using Base = LeanState<LeanConst<MID>>;
+    using Lane = typename Base::Lane;
+    using Base::advance;
+    using Base::stage;
+    static constexpr unsigned kRhsPerStep = 4;
+
+    static __device__ __forceinline__ bool step(Lane& L, const RunConst& R) {
+        const f2 uf01 = p_add(L.vh[0], L.vl[0]), uf23 = p_add(L.vh[1], L.vl[1]);
+        const float uf[4] = {lo2(uf01), hi2(uf01), lo2(uf23), hi2(uf23)};
+        const float x1h = hi2(L.xh[0]), x1l = hi2(L.xl[0]), thh = lo2(L.xh[1]), thl = lo2(L.xl[1]);
+        const float h = adaptive_step_lean(R.mr, thh, thl, uf[1], uf[2], uf[3]);
+        const float hh = 0.5f * h;
+        const f2 hh2 = pack2(hh, hh), h2 = pack2(h, h);
+        float k1[4], k2[4], k3[4], k4[4], us[4];
+        // stages 1 (low half) and 2 (high half)
+        f2 ph, pl;
+        p_ff_add_f(pack2(x1h, thh), pack2(x1l, thl), p_mul(hh2, pack2(uf[1], uf[2])), ph, pl);
+        MetricAt<f2> m = metric_lean<MID, RLOG, f2>(L.c, pack2(x1h, lo2(ph)), pack2(x1l, lo2(pl)), pack2(thh, hi2(ph)),
+                                                    pack2(thl, hi2(pl)));
+        accel_lean<0>(half_of(m, false), RLOG, uf, k1);
+        stage(hh2, uf01, uf23, k1, us);
+        accel_lean<0>(half_of(m, true), RLOG, us, k2);
+        // stages 3 and 4: x + h/2 (u + h/2 k1), x + h (u + h/2 k2)
+        const f2 hs = pack2(hh, h);
+        f2 rh, rl, qh, ql;
+        p_ff_add_f(pack2(x1h, x1h), pack2(x1l, x1l),
+                   p_mul(hs, p_fma(hh2, pack2(k1[1], k2[1]), pack2(uf[1], uf[1]))), rh, rl);
+        p_ff_add_f(pack2(thh, thh), pack2(thl, thl),
+                   p_mul(hs, p_fma(hh2, pack2(k1[2], k2[2]), pack2(uf[2], uf[2]))), qh, ql);
+        m = metric_lean<MID, RLOG, f2>(L.c, rh, rl, qh, ql);
+        stage(hh2, uf01, uf23, k2, us);
+        accel_lean<0>(half_of(m, false), RLOG, us, k3);
+        stage(h2, uf01, uf23, k3, us);
+        accel_lean<0>(half_of(m, true), RLOG, us, k4);
+        return advance(L, R, h, k1, k2, k3, k4);
+    }
+
+    // The step on two lanes (MixedEngine::step_pair): in each of two rounds the even lane
+    // evaluates stage 1 (then 3) and the odd lane stage 2 (then 4).
+    static __device__ __forceinline__ bool step_pair(Lane& L, const RunConst& R, bool odd, unsigned pmask) {
+        const f2 uf01 = p_add(L.vh[0], L.vl[0]), uf23 = p_add(L.vh[1], L.vl[1]);
+        const float uf[4] = {lo2(uf01), hi2(uf01), lo2(uf23), hi2(uf23)};
+        const f2 x12h = pack2(hi2(L.xh[0]), lo2(L.xh[1])), x12l = pack2(hi2(L.xl[0]), lo2(L.xl[1]));
+        const float h = adaptive_step_lean(R.mr, hi2(x12h), hi2(x12l), uf[1], uf[2], uf[3]);
+        const float hh = 0.5f * h;
+        const f2 hh2 = pack2(hh, hh), h2 = pack2(h, h), uf12 = pack2(uf[1], uf[2]);
+        float k1[4], k2[4], k3[4], k4[4], us[4], ka[4];
+        auto share = [&](float k[4], int from) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) k[i] = __shfl_sync(pmask, ka[i], from, 2);
+        };
+        f2 ph, pl;
+        p_ff_add_f(x12h, x12l, p_mul(hh2, uf12), ph, pl);
+        MetricAt<float> m = metric_lean<MID, RLOG, float>(L.c, odd ? lo2(ph) : lo2(x12h), odd ? lo2(pl) : lo2(x12l),
+                                                          odd ? hi2(ph) : hi2(x12h), odd ? hi2(pl) : hi2(x12l));
+        accel_lean<0>(m, RLOG, uf, ka);
+        share(k1, 0);
+        stage(hh2, uf01, uf23, k1, us);
+        accel_lean<0>(m, RLOG, us, ka);
+        share(k2, 1);
+        const float hs = odd ? h : hh;
+        const f2 k12 = odd ? pack2(k2[1], k2[2]) : pack2(k1[1], k1[2]);
+        p_ff_add_f(x12h, x12l, p_mul(pack2(hs, hs), p_fma(hh2, k12, uf12)), ph, pl);
+        m = metric_lean<MID, RLOG, float>(L.c, lo2(ph), lo2(pl), hi2(ph), hi2(pl));
+        stage(hh2, uf01, uf23, k2, us);
+        accel_lean<0>(m, RLOG, us, ka);
+        share(k3, 0);
+        stage(h2, uf01, uf23, k3, us);
+        accel_lean<0>(m, RLOG, us, ka);
+        share(k4, 1);
+        return advance(L, R, h, k1, k2, k3, k4);
+    }
+};
+
+// RK4 on two lanes with a plugin too large to pack or to inline (Johannsen,
+// Rasheed-Larsen): the compiler's scalar body, in one function that both rounds of a step
+// call. Its ~900 and ~1,800 instructions set the pace; on one lane the general kernel calls
+// it four times in sequence, which costs as many instructions per geodesic, so two lanes
+// are taken at every size. GB300, log r, one lane before and two lanes now: Johannsen
+// 3,721 geodesics 6.0 and 2.9 ms, 90,000 15.1 and 11.0 ms; Rasheed-Larsen 14.7 and 7.2,
+// 39.7 and 24.5 ms. Without a register cap (226 and 255): capped to three CTAs per SM the
+// largest of these take 11.5 and 29.4 ms.
+struct ImageRef {
+    const MixedConst* mx;
+    __device__ __forceinline__ void load(const ImageConst& I) { mx = &I.mx; }
+};
+
+struct TwoK {
+    F4 a, b;
+};
+
+// One round: the metric part at this lane's stage, contracted with the velocity u (the even
+// lane's acceleration counts, k_a) and then with uf + t k_a (the odd lane's, k_b).
+template <int MID>
+__device__ __noinline__ TwoK round_called(const MixedConst& mc, bool rlog, ff x1, ff th, F4 uf, F4 u, float t,
+                                          unsigned pmask) {
+    MetricAt<float> m = metric_part<MID, float>(mc.q, mc, rlog, x1, th);
+    m.gu.rr = __fmul_rn(-0.5f, m.gu.rr);
+    m.gu.hh = __fmul_rn(-0.5f, m.gu.hh);
+    auto contract = [&](const float v[4], int from) {
+        float a[4];
+        accel_lean<MID == kJohannsen ? 1 : 2>(m, rlog, v, a);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) a[i] = __shfl_sync(pmask, a[i], from, 2);
+        return F4{a[0], a[1], a[2], a[3]};
+    };
+    const float ua[4] = {u.x, u.y, u.z, u.w};
+    TwoK k;
+    k.a = contract(ua, 0);
+    const float ub[4] = {__fmaf_rn(t, k.a.x, uf.x), __fmaf_rn(t, k.a.y, uf.y), __fmaf_rn(t, k.a.z, uf.z),
+                         __fmaf_rn(t, k.a.w, uf.w)};
+    k.b = contract(ub, 1);
+    return k;
+}
+
+template <int MID>
+struct LeanCalledEngine : LeanState<ImageRef> {
+    static constexpr unsigned kRhsPerStep = 4;
+
+    static __device__ __forceinline__ bool step_pair(Lane& L, const RunConst& R, bool odd, unsigned pmask) {
+        const bool rlog = R.rlog != 0;
+        const f2 uf01 = p_add(L.vh[0], L.vl[0]), uf23 = p_add(L.vh[1], L.vl[1]);
+        const F4 uf = {lo2(uf01), hi2(uf01), lo2(uf23), hi2(uf23)};
+        const f2 x12h = pack2(hi2(L.xh[0]), lo2(L.xh[1])), x12l = pack2(hi2(L.xl[0]), lo2(L.xl[1]));
+        const float h = adaptive_step_lean(R.mr, hi2(x12h), hi2(x12l), uf.y, uf.z, uf.w);
+        const float hh = 0.5f * h;
+        const f2 hh2 = pack2(hh, hh), uf12 = pack2(uf.y, uf.z);
+        f2 ph, pl;
+        p_ff_add_f(x12h, x12l, p_mul(hh2, uf12), ph, pl);
+        const ff r12 = odd ? ff{lo2(ph), lo2(pl)} : ff{lo2(x12h), lo2(x12l)};
+        const ff t12 = odd ? ff{hi2(ph), hi2(pl)} : ff{hi2(x12h), hi2(x12l)};
+        const TwoK k12 = round_called<MID>(*L.c.mx, rlog, r12, t12, uf, uf, hh, pmask);
+        const float hs = odd ? h : hh;
+        const f2 kp = odd ? pack2(k12.b.y, k12.b.z) : pack2(k12.a.y, k12.a.z);
+        p_ff_add_f(x12h, x12l, p_mul(pack2(hs, hs), p_fma(hh2, kp, uf12)), ph, pl);
+        const f2 us01 = p_fma(hh2, pack2(k12.b.x, k12.b.y), uf01), us23 = p_fma(hh2, pack2(k12.b.z, k12.b.w), uf23);
+        const TwoK k34 = round_called<MID>(*L.c.mx, rlog, ff{lo2(ph), lo2(pl)}, ff{hi2(ph), hi2(pl)}, uf,
+                                           F4{lo2(us01), hi2(us01), lo2(us23), hi2(us23)}, h, pmask);
+        const float k1[4] = {k12.a.x, k12.a.y, k12.a.z, k12.a.w}, k2[4] = {k12.b.x, k12.b.y, k12.b.z, k12.b.w};
+        const float k3[4] = {k34.a.x, k34.a.y, k34.a.z, k34.a.w}, k4[4] = {k34.b.x, k34.b.y, k34.b.z, k34.b.w};
+        return advance(L, R, h, k1, k2, k3, k4);
     }
 };
 

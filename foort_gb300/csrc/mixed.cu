@@ -46,6 +46,8 @@ const void* mixed_lean_kernel_kerr(bool rlog);
 const void* mixed_lean_kernel_flat();
 const void* mixed_lean_pair_kernel_kerr(bool rlog);
 const void* mixed_lean_pair_kernel_flat();
+const void* mixed_lean_pair_kernel_joh();
+const void* mixed_lean_pair_kernel_rl();
 
 // Lean options: every termination and diagnostic in use updates at each step (the
 // default), and nothing needs FP64 steps or FP64 decisions.
@@ -67,6 +69,8 @@ const void* mixed_lean_kernel(const RunConst& R, bool pair) {
     switch (R.metric_id) {
     case kKerr: return pair ? mixed_lean_pair_kernel_kerr(R.rlog != 0) : mixed_lean_kernel_kerr(R.rlog != 0);
     case kFlat: return R.rlog ? nullptr : pair ? mixed_lean_pair_kernel_flat() : mixed_lean_kernel_flat();
+    case kJohannsen: return pair ? mixed_lean_pair_kernel_joh() : nullptr;
+    case kRasheedLarsen: return pair ? mixed_lean_pair_kernel_rl() : nullptr;
     default: return nullptr;
     }
 }

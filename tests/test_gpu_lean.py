@@ -12,6 +12,7 @@ from conftest import ROOT
 from foort_gb300 import abi, workloads
 
 ALL_DIAGS = abi.DIAG_FOUR_COLOR_SCREEN | abi.DIAG_EQUATORIAL_PASSES | abi.DIAG_CLOSEST_RADIUS
+LORENZO = (0.3556562853309941, 0.2969060968239216, 3.057664971085168, 0.942335028914832)
 
 
 @pytest.fixture(scope="module")
@@ -52,6 +53,11 @@ def same_records(a, b):
     (abi.METRIC_KERR, (0.9,), 1, 60.0, 33, 0),
     (abi.METRIC_KERR, (0.9,), 1, 60.0, 33, 400),
     (abi.METRIC_FLAT, (), 0, 63.0, 7, None),
+    (abi.METRIC_JOHANNSEN, (0.8, 1.0, 0.5, 0.2, 0.1), 1, 63.0, 33, None),
+    (abi.METRIC_JOHANNSEN, (0.7, 2.0, 0.0, 0.0, 0.0), 1, 90.0, 21, None),
+    (abi.METRIC_JOHANNSEN, (0.8, 1.0, 0.5, 0.2, 0.1), 0, 63.0, 3, 20000),
+    (abi.METRIC_RASHEED_LARSEN, LORENZO, 1, 63.0, 33, None),
+    (abi.METRIC_RASHEED_LARSEN, LORENZO, 0, 63.0, 3, 20000),
 ])
 def test_lean_kernels_give_the_general_kernels_records(eng, metric, params, rlog, inclination, side, timeout):
     px = abi.square_pixels(side)
