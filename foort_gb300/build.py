@@ -48,7 +48,7 @@ MIXED_FLAGS = ["-ftz=true"]
 
 def _compile(src, obj, extra, verbose):
     if src.endswith(".cu"):
-        more = MIXED_FLAGS if os.path.basename(src).startswith(("k_mixed_", "k_lean_")) else []
+        more = MIXED_FLAGS if os.path.basename(src).startswith(("k_mixed_", "k_lean_", "k_analytic_")) else []
         cmd = [nvcc()] + NVFLAGS + more + extra + ["-c", src, "-o", obj]
     else:
         cmd = ["g++"] + CXXFLAGS + ["-I" + os.path.join(HERE, "..", "include"), "-I/usr/local/cuda/include",

@@ -226,6 +226,7 @@ const void* select_kernel(const RunConst& R, bool positions) {
 // Verlet, the called plugins, the strong-field FP64 steps).
 const void* select_pair_kernel(const RunConst& R, bool positions) {
     if (const void* lean = positions ? nullptr : mixed_lean_kernel(R, true)) return lean;
+    if (R.precision == FOORT_PREC_FP64) return fp64_pair_kernel(R.metric_id, R.integrator);
     if (R.precision != FOORT_PREC_MIXED || R.mixed_fp64_margin > 0.0 ||
         (R.mixed_options & FOORT_MIXED_FP64_TURNING_POINTS))
         return nullptr;
@@ -241,6 +242,12 @@ struct LaunchShape {
 // launch leaves the choice open.
 // - General kernels: as many as the GPU's resident lanes hold that way. Then a step's
 //   latency, not the GPU's throughput, sets the pace, and two lanes halve its metric work.
+// - FP64 kernels: an FP64 instruction occupies its scheduler's pipe for 64 cycles however
+//   many lanes are active, so two lanes halve the metric work of a launch that leaves lanes
+//   idle, and shorten the last rays of a larger one. Past several refills they only add the
+//   parts that both lanes do: log r, Kerr 10,201 geodesics 102.7 ms on one lane and 64.9 on
+//   two, 62,500 204 and 175, 122,500 293 and 325; Johannsen 126 and 75.5, 275 and 216, 388
+//   and 396.
 // - Lean kernels: one lane already evaluates two stages at a time, so two lanes pay only
 //   while they leave each scheduler one warp (n <= 64 x SMs), and only in log r, where
 //   each half of a packed stage needs its own exponentials and division: Kerr, 3,721
@@ -251,6 +258,7 @@ struct LaunchShape {
 //   than the general one-lane kernel: every size.
 uint64_t pair_limit(const RunConst& R, bool positions, int per_sm, int num_sms, uint32_t bs) {
     const uint64_t sms = static_cast<uint64_t>(num_sms);
+    if (R.precision != FOORT_PREC_MIXED) return 512 * sms;
     if (!positions && mixed_lean_kernel(R, true))
         return mixed_lean_kernel(R, false) ? (R.rlog ? 64 : 24) * sms : UINT64_MAX;
     return static_cast<uint64_t>(per_sm) * sms * bs / 2;
@@ -259,11 +267,17 @@ uint64_t pair_limit(const RunConst& R, bool positions, int per_sm, int num_sms, 
 // Kernel and grid of a launch of n geodesics in the requested shape (zero fields: the
 // built-in rule): a persistent grid of at most the resident CTAs. The rule takes 128
 // threads, as many CTAs per SM as fit, and two lanes per geodesic up to pair_limit().
+// FP64 kernels take CTAs of 32 threads, four per SM: one warp per scheduler already fills
+// its FP64 pipe, more only leave rays unevenly spread over lanes at the end (62,500
+// Johannsen rays in FP64 130 ms with two CTAs of 128 per SM, 110 with four of 32), and small
+// CTAs spread a launch that does not fill the GPU evenly (4,096 Kerr rays 65.8 and 62.5 ms).
 int choose_launch(foort_ctx* ctx, const RunConst& R, uint64_t n, int num_sms, const foort_launch_shape& want,
                   LaunchShape& out, bool positions = false) {
-    const uint32_t bs = want.block_size ? want.block_size : 128;
+    const bool fp64 = R.precision != FOORT_PREC_MIXED;
+    const uint32_t bs = want.block_size ? want.block_size : fp64 ? 32 : 128;
     auto resident = [&](const void* fn, int& per_sm) -> int {
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, static_cast<int>(bs), 0));
+        if (fp64 && !want.blocks_per_sm) per_sm = std::min<int>(per_sm, std::max<int>(1, 128 / static_cast<int>(bs)));
         if (want.blocks_per_sm) per_sm = std::min<int>(per_sm, static_cast<int>(want.blocks_per_sm));
         return FOORT_OK;
     };
@@ -902,6 +916,24 @@ const void* fp64_kernel(int metric_id, int integ) {
     case kRasheedLarsen: return fp64_kernel_rl(integ);
     case kJohannsen: return fp64_kernel_joh(integ);
     case kMankoNovikov: return fp64_kernel_mn(integ);
+    default: return nullptr;
+    }
+}
+
+const void* fp64_pair_kernel_kerr();
+const void* fp64_pair_kernel_flat();
+const void* fp64_pair_kernel_rl();
+const void* fp64_pair_kernel_joh();
+
+// Two lanes per geodesic: RK4. Not for Manko-Novikov, whose much larger metric the compiler
+// contracts differently there, so that its results would not be the one-lane kernel's.
+const void* fp64_pair_kernel(int metric_id, int integ) {
+    if (integ != FOORT_INTEGRATOR_RK4) return nullptr;
+    switch (metric_id) {
+    case kKerr: return fp64_pair_kernel_kerr();
+    case kFlat: return fp64_pair_kernel_flat();
+    case kRasheedLarsen: return fp64_pair_kernel_rl();
+    case kJohannsen: return fp64_pair_kernel_joh();
     default: return nullptr;
     }
 }

@@ -10,4 +10,6 @@ const void* fp64_kernel_flat(int integrator) {
     return reinterpret_cast<const void*>(&integrate_fp64_kernel<kFlat, FOORT_INTEGRATOR_VERLET>);
 }
 
+const void* fp64_pair_kernel_flat() { return reinterpret_cast<const void*>(&integrate_fp64_pair_kernel<kFlat>); }
+
 }  // namespace foort

@@ -10,4 +10,6 @@ const void* fp64_kernel_joh(int integrator) {
     return reinterpret_cast<const void*>(&integrate_fp64_kernel<kJohannsen, FOORT_INTEGRATOR_VERLET>);
 }
 
+const void* fp64_pair_kernel_joh() { return reinterpret_cast<const void*>(&integrate_fp64_pair_kernel<kJohannsen>); }
+
 }  // namespace foort

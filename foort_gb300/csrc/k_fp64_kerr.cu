@@ -10,4 +10,6 @@ const void* fp64_kernel_kerr(int integrator) {
     return reinterpret_cast<const void*>(&integrate_fp64_kernel<kKerr, FOORT_INTEGRATOR_VERLET>);
 }
 
+const void* fp64_pair_kernel_kerr() { return reinterpret_cast<const void*>(&integrate_fp64_pair_kernel<kKerr>); }
+
 }  // namespace foort

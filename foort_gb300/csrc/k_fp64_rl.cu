@@ -10,4 +10,6 @@ const void* fp64_kernel_rl(int integrator) {
     return reinterpret_cast<const void*>(&integrate_fp64_kernel<kRasheedLarsen, FOORT_INTEGRATOR_VERLET>);
 }
 
+const void* fp64_pair_kernel_rl() { return reinterpret_cast<const void*>(&integrate_fp64_pair_kernel<kRasheedLarsen>); }
+
 }  // namespace foort

@@ -275,6 +275,16 @@ constexpr bool is_lean(decltype(E::kLean)*) {
     return true;
 }
 
+// Lean engines whose every step is an FP64 step (E::kFp64Steps).
+template <class E>
+constexpr bool is_fp64_steps(...) {
+    return false;
+}
+template <class E>
+constexpr bool is_fp64_steps(decltype(E::kFp64Steps)*) {
+    return true;
+}
+
 template <class E, bool PAIR = false>
 __device__ __forceinline__ void persistent_loop(const LaunchArgs& A, const RunConst& R) {
     const unsigned lane = threadIdx.x & 31u;
@@ -285,7 +295,7 @@ __device__ __forceinline__ void persistent_loop(const LaunchArgs& A, const RunCo
     const unsigned pmask = 3u << (lane & ~1u);
     constexpr bool kLean = is_lean<E>(nullptr);
     typename E::Lane L;
-    ImageConst Ic;  // PAIR: the lane's image constants in registers, copied at each refill
+    ImageConst Ic;  // PAIR, E::kCopyImage: the lane's image constants in registers, copied at each refill
     bool active = false;
     bool drained = false;
     bool stopping = false;
@@ -298,6 +308,7 @@ __device__ __forceinline__ void persistent_loop(const LaunchArgs& A, const RunCo
     auto rhs_counts = [](typename E::Lane& l, unsigned long long steps, unsigned long long& rhs, unsigned long long& fp64) {
         if constexpr (kLean) {
             rhs = steps * E::kRhsPerStep;
+            if constexpr (is_fp64_steps<E>(nullptr)) fp64 = steps;
         } else {
             rhs = __reduce_add_sync(kFullMask, l.rhs);
             fp64 = __reduce_add_sync(kFullMask, l.fp64);
@@ -334,7 +345,7 @@ __device__ __forceinline__ void persistent_loop(const LaunchArgs& A, const RunCo
                                        ? GeoposRec{A.gp_plan[my].dst, A.gp_plan[my].j, A.gp_plan[my].M, 0, 0}
                                        : GeoposRec{nullptr, 1, 0, 0, 0};
                             E::init(L, A.images[p.image], R, p);
-                            if constexpr (PAIR && !kLean) Ic = A.images[p.image];
+                            if constexpr (PAIR && E::kCopyImage) Ic = A.images[p.image];
                             active = true;
                         }
                     }
@@ -352,7 +363,7 @@ __device__ __forceinline__ void persistent_loop(const LaunchArgs& A, const RunCo
                 if constexpr (PAIR && kLean) {
                     more = E::step_pair(L, R, odd, pmask);
                 } else if constexpr (PAIR) {
-                    more = E::step_pair(L, Ic, R, odd, pmask);
+                    more = E::step_pair(L, E::kCopyImage ? Ic : A.images[L.img], R, odd, pmask);
                 } else {
                     if constexpr (kLean) {
                         more = E::step(L, R);

@@ -66,34 +66,36 @@ FOORT_DEFINE_PACKED_METRIC(kFlat, FLAT)
 // FORM 0 is the step with an inlined plugin, 1 and 2 the called right-hand side of
 // Johannsen and of Rasheed-Larsen. m.gu.rr and m.gu.hh come multiplied by -1/2; the other
 // factors of 2 and 1/2, which are exact, are left out where they cancel.
-template <int FORM>
-__device__ __forceinline__ void accel_lean(const MetricAt<float>& m, const float u[4], float a[4]) {
+// a[2] is the product of m.gu.hh and *f2 (where asked for).
+template <int FORM, typename T>
+__device__ __forceinline__ void accel_lean(const MetricAt<T>& m, const T u[4], T a[4], T* f2 = nullptr) {
     // x y + z w with the first or the second product fused
-    auto first = [](float x, float y, float z, float w) { return __fmaf_rn(x, y, __fmul_rn(z, w)); };
-    auto second = [](float x, float y, float z, float w) { return __fmaf_rn(z, w, __fmul_rn(x, y)); };
-    const float w1t = first(m.d1.tt, u[0], m.d1.tp, u[3]), w1p = first(m.d1.tp, u[0], m.d1.pp, u[3]);
-    const float w2t = first(m.d2.tt, u[0], m.d2.tp, u[3]);
-    const float w2p = (FORM == 1) ? second(m.d2.tp, u[0], m.d2.pp, u[3]) : first(m.d2.tp, u[0], m.d2.pp, u[3]);
-    const float w1r = __fmul_rn(m.d1.rr, u[1]), w1h = __fmul_rn(m.d1.hh, u[2]);
-    const float w2r = __fmul_rn(m.d2.rr, u[1]), w2h = __fmul_rn(m.d2.hh, u[2]);
-    const float q1 = __fmaf_rn(u[3], w1p, __fmaf_rn(u[2], w1h, first(u[0], w1t, u[1], w1r)));
-    const float q2a = first(u[0], w2t, u[1], w2r);
-    const float q2b = FORM ? __fmaf_rn(u[2], w2h, q2a) : __fadd_rn(q2a, __fmul_rn(u[2], w2h));
-    const float q2 = __fmaf_rn(u[3], w2p, q2b);
-    const float Ft = FORM ? second(u[1], w1t, u[2], w2t) : first(u[1], w1t, u[2], w2t);
-    const float Fp = FORM ? second(u[1], w1p, u[2], w2p) : first(u[1], w1p, u[2], w2p);
-    const float Fr = __fmaf_rn(2.f, first(u[1], w1r, u[2], w2r), -q1);
-    const float Fh = __fmaf_rn(2.f, FORM ? second(u[1], w1h, u[2], w2h) : first(u[1], w1h, u[2], w2h), -q2);
+    auto first = [](T x, T y, T z, T w) { return p_fma(x, y, p_mul(z, w)); };
+    auto second = [](T x, T y, T z, T w) { return p_fma(z, w, p_mul(x, y)); };
+    const T w1t = first(m.d1.tt, u[0], m.d1.tp, u[3]), w1p = first(m.d1.tp, u[0], m.d1.pp, u[3]);
+    const T w2t = first(m.d2.tt, u[0], m.d2.tp, u[3]);
+    const T w2p = (FORM == 1) ? second(m.d2.tp, u[0], m.d2.pp, u[3]) : first(m.d2.tp, u[0], m.d2.pp, u[3]);
+    const T w1r = p_mul(m.d1.rr, u[1]), w1h = p_mul(m.d1.hh, u[2]);
+    const T w2r = p_mul(m.d2.rr, u[1]), w2h = p_mul(m.d2.hh, u[2]);
+    const T q1 = p_fma(u[3], w1p, p_fma(u[2], w1h, first(u[0], w1t, u[1], w1r)));
+    const T q2a = first(u[0], w2t, u[1], w2r);
+    const T q2b = FORM ? p_fma(u[2], w2h, q2a) : p_add(q2a, p_mul(u[2], w2h));
+    const T q2 = p_fma(u[3], w2p, q2b);
+    const T Ft = FORM ? second(u[1], w1t, u[2], w2t) : first(u[1], w1t, u[2], w2t);
+    const T Fp = FORM ? second(u[1], w1p, u[2], w2p) : first(u[1], w1p, u[2], w2p);
+    const T Fr = p_fma(T(2), first(u[1], w1r, u[2], w2r), -q1);
+    const T Fh = p_fma(T(2), FORM ? second(u[1], w1h, u[2], w2h) : first(u[1], w1h, u[2], w2h), -q2);
     a[0] = -first(m.gu.tt, Ft, m.gu.tp, Fp);
     a[3] = -first(m.gu.tp, Ft, m.gu.pp, Fp);
-    a[1] = __fmul_rn(m.gu.rr, Fr);
-    a[2] = __fmul_rn(m.gu.hh, Fh);
+    a[1] = p_mul(m.gu.rr, Fr);
+    a[2] = p_mul(m.gu.hh, Fh);
+    if (f2) *f2 = Fh;
 }
 // In log-r mode the coordinate term -(u^1)^2 joins a^1 (accel_log_r).
-template <int FORM>
-__device__ __forceinline__ void accel_lean(const MetricAt<float>& m, bool rlog, const float u[4], float a[4]) {
-    accel_lean<FORM>(m, u, a);
-    if (rlog) a[1] = __fmaf_rn(-u[1], u[1], a[1]);
+template <int FORM, typename T>
+__device__ __forceinline__ void accel_lean(const MetricAt<T>& m, bool rlog, const T u[4], T a[4], T* f2 = nullptr) {
+    accel_lean<FORM>(m, u, a, f2);
+    if (rlog) a[1] = p_fma(-u[1], u[1], a[1]);
 }
 
 // Image constants a lane of a packed plugin keeps.
@@ -179,6 +181,7 @@ __device__ __forceinline__ float adaptive_step_lean(const MixedRun& G, float thh
 template <class C>
 struct LeanState {
     static constexpr bool kLean = true;
+    static constexpr bool kCopyImage = false;
 
     // x and v: [0] holds components 0 and 1, [1] components 2 and 3, high and low parts.
     struct Lane {
@@ -283,7 +286,7 @@ struct LeanState {
         us[3] = hi2(b);
     }
 
-    // MixedEngine::rk4_combine, advance and after_step.
+    // MixedEngine::rk4_combine and advance.
     static __device__ __forceinline__ bool advance(Lane& L, const RunConst& R, float h, const float k1[4],
                                                    const float k2[4], const float k3[4], const float k4[4]) {
         const float q0 = __fmul_rn(h, 0.166666672f);
@@ -302,7 +305,12 @@ struct LeanState {
             p_fast_two_sum(s, p_add(e, p_add(L.xl[i], bl)), L.xh[i], L.xl[i]);
             p_ff_add_f(L.vh[i], L.vl[i], du, L.vh[i], L.vl[i]);
         }
-        L.lam = ff_add_f(L.lam, h);
+        return after_step(L, R, ff_add_f(L.lam, h));
+    }
+
+    // MixedEngine::after_step
+    static __device__ __forceinline__ bool after_step(Lane& L, const RunConst& R, ff lam) {
+        L.lam = lam;
         L.term = terms(L, R);
         ++L.steps;
         diags(L, R);
@@ -429,7 +437,11 @@ struct LeanEngine : LeanState<LeanConst<MID>> {
 // largest of these take 11.5 and 29.4 ms.
 struct ImageRef {
     const MixedConst* mx;
-    __device__ __forceinline__ void load(const ImageConst& I) { mx = &I.mx; }
+    const double* qa;
+    __device__ __forceinline__ void load(const ImageConst& I) {
+        mx = &I.mx;
+        qa = I.qa;
+    }
 };
 
 struct TwoK {
@@ -486,6 +498,93 @@ struct LeanCalledEngine : LeanState<ImageRef> {
         const float k1[4] = {k12.a.x, k12.a.y, k12.a.z, k12.a.w}, k2[4] = {k12.b.x, k12.b.y, k12.b.z, k12.b.w};
         const float k3[4] = {k34.a.x, k34.a.y, k34.a.z, k34.a.w}, k4[4] = {k34.b.x, k34.b.y, k34.b.z, k34.b.w};
         return advance(L, R, h, k1, k2, k3, k4);
+    }
+};
+
+// FOORT_PREC_FP64_ANALYTIC with RK4 on two lanes per geodesic: step_fp64 (kernel_mixed.cuh)
+// with the metric parts of stages 1 and 2, and of 3 and 4, side by side. GB300 takes 64
+// cycles per warp for an FP64 instruction however many lanes are active, so a step costs
+// its FP64 instructions: about 1,400 on one lane, 850 here.
+struct D4 {
+    double x, y, z, w;
+};
+struct TwoKD {
+    D4 a, b;
+    double bg, bf;  // b.z unrounded: the product of these
+};
+template <int MID>
+__device__ __noinline__ TwoKD round_fp64(const double* q, const MixedConst& mc, bool rlog, double x1, double th, D4 uf,
+                                         D4 u, double t, unsigned pmask) {
+    MetricAt<double> m = metric_part_d<MID>(q, mc, rlog, x1, th);
+    m.gu.rr = __dmul_rn(-0.5, m.gu.rr);
+    m.gu.hh = __dmul_rn(-0.5, m.gu.hh);
+    double f;
+    auto contract = [&](const double v[4], int from) {
+        double a[4];
+        accel_lean<0>(m, rlog, v, a, &f);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) a[i] = __shfl_sync(pmask, a[i], from, 2);
+        return D4{a[0], a[1], a[2], a[3]};
+    };
+    const double ua[4] = {u.x, u.y, u.z, u.w};
+    TwoKD k;
+    k.a = contract(ua, 0);
+    const double ub[4] = {__fma_rn(t, k.a.x, uf.x), __fma_rn(t, k.a.y, uf.y), __fma_rn(t, k.a.z, uf.z),
+                          __fma_rn(t, k.a.w, uf.w)};
+    k.b = contract(ub, 1);
+    k.bg = __shfl_sync(pmask, m.gu.hh, 1, 2);
+    k.bf = __shfl_sync(pmask, f, 1, 2);
+    return k;
+}
+
+template <int MID>
+struct AnalyticPairEngine : LeanState<ImageRef> {
+    static constexpr unsigned kRhsPerStep = 4;
+    static constexpr bool kFp64Steps = true;
+
+    static __device__ __forceinline__ bool step_pair(Lane& L, const RunConst& R, bool odd, unsigned pmask) {
+        const bool rlog = R.rlog != 0;
+        double x[4], u[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            x[i] = half_d(L.xh[i / 2], L.xl[i / 2], i & 1);
+            u[i] = half_d(L.vh[i / 2], L.vl[i / 2], i & 1);
+        }
+        const double h = adaptive_step_fp64(R, x, u), hh = 0.5 * h;
+        const D4 uf = {u[0], u[1], u[2], u[3]};
+        auto ahead = [](double a, double t, double b) { return __fma_rn(t, b, a); };  // a + t b
+        const TwoKD k12 = round_fp64<MID>(L.c.qa, *L.c.mx, rlog, odd ? ahead(x[1], hh, u[1]) : x[1],
+                                          odd ? ahead(x[2], hh, u[2]) : x[2], uf, uf, hh, pmask);
+        const double ts = odd ? h : hh, ky = odd ? k12.b.y : k12.a.y, kz = odd ? k12.b.z : k12.a.z;
+        const D4 us = {ahead(u[0], hh, k12.b.x), ahead(u[1], hh, k12.b.y), ahead(u[2], hh, k12.b.z),
+                       ahead(u[3], hh, k12.b.w)};
+        const TwoKD k34 = round_fp64<MID>(L.c.qa, *L.c.mx, rlog, ahead(x[1], ts, ahead(u[1], hh, ky)),
+                                          ahead(x[2], ts, ahead(u[2], hh, kz)), uf, us, h, pmask);
+        const double k1[4] = {k12.a.x, k12.a.y, k12.a.z, k12.a.w}, k2[4] = {k12.b.x, k12.b.y, k12.b.z, k12.b.w};
+        const double k3[4] = {k34.a.x, k34.a.y, k34.a.z, k34.a.w}, k4[4] = {k34.b.x, k34.b.y, k34.b.z, k34.b.w};
+        const double h6 = h / 6.0, hh6 = __dmul_rn(h, h6);
+        ff nx[4], nv[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const double s3 = __fma_rn(k3[i], 2.0, __fma_rn(k2[i], 2.0, k1[i]));
+            // step_fp64's sum takes k4[2], a product used only here, unrounded
+            const double dv = __dmul_rn(i == 2 ? __fma_rn(k34.bg, k34.bf, s3) : __dadd_rn(s3, k4[i]), h6);
+            const double dx = __fma_rn(u[i], h, __dmul_rn(__dadd_rn(__dadd_rn(k1[i], k2[i]), k3[i]), hh6));
+            nx[i] = ff_from_d(__dadd_rn(x[i], dx));
+            nv[i] = ff_from_d(__dadd_rn(u[i], dv));
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            L.xh[i] = pack2(nx[2 * i].hi, nx[2 * i + 1].hi);
+            L.xl[i] = pack2(nx[2 * i].lo, nx[2 * i + 1].lo);
+            L.vh[i] = pack2(nv[2 * i].hi, nv[2 * i + 1].hi);
+            L.vl[i] = pack2(nv[2 * i].lo, nv[2 * i + 1].lo);
+        }
+        return after_step(L, R, ff_add(L.lam, ff_from_d(h)));
+    }
+
+    static __device__ __forceinline__ double half_d(f2 h, f2 l, bool hi) {
+        return hi ? ff_d({hi2(h), hi2(l)}) : ff_d({lo2(h), lo2(l)});
     }
 };
 

@@ -346,6 +346,8 @@ struct MixedEngine {
     // (kept out of it, their call raised the two-lane kernel from 111 to 158 registers)
     static constexpr bool kPairCapable = INTEG == FOORT_INTEGRATOR_RK4 && MixedMetric<MID>::kInline;
 
+    static constexpr bool kCopyImage = true;
+
     struct Lane {
         ff x[4], v[4];
         ff lam;

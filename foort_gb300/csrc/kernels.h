@@ -8,6 +8,8 @@ namespace foort {
 
 // Returns the __global__ function for (metric, integrator), or nullptr.
 const void* fp64_kernel(int metric_id, int integrator);
+// two lanes per geodesic, or nullptr where that kernel does not exist
+const void* fp64_pair_kernel(int metric_id, int integrator);
 const void* mixed_kernel(int metric_id, int integrator);
 // decide64: terminations and diagnostics decided in FP64 (else in float-float)
 const void* mixed_kernel_variant(int metric_id, int integrator, bool decide64);

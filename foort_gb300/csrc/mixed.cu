@@ -48,13 +48,14 @@ const void* mixed_lean_pair_kernel_kerr(bool rlog);
 const void* mixed_lean_pair_kernel_flat();
 const void* mixed_lean_pair_kernel_joh();
 const void* mixed_lean_pair_kernel_rl();
+const void* analytic_pair_kernel_kerr();
+const void* analytic_pair_kernel_joh();
+const void* analytic_pair_kernel_flat();
 
 // Lean options: every termination and diagnostic in use updates at each step (the
-// default), and nothing needs FP64 steps or FP64 decisions.
+// default), with decisions on the float-float state.
 static bool lean_options(const RunConst& R) {
-    if (R.precision != FOORT_PREC_MIXED || R.mixed_fp64_margin > 0.0 ||
-        (R.mixed_options & (FOORT_MIXED_FP64_DECISIONS | FOORT_MIXED_FP64_TURNING_POINTS)))
-        return false;
+    if (R.mixed_options & FOORT_MIXED_FP64_DECISIONS) return false;
     auto each_step = [](uint32_t flags, uint32_t flag, uint64_t every) { return !(flags & flag) || every == 1; };
     return each_step(R.term_flags, FOORT_TERM_HORIZON, R.h_every) &&
            each_step(R.term_flags, FOORT_TERM_BOUNDARY_SPHERE, R.b_every) &&
@@ -66,6 +67,19 @@ static bool lean_options(const RunConst& R) {
 
 const void* mixed_lean_kernel(const RunConst& R, bool pair) {
     if (!lean_options(R) || R.integrator != FOORT_INTEGRATOR_RK4) return nullptr;
+    if (R.precision == FOORT_PREC_FP64_ANALYTIC) {
+        if (!pair) return nullptr;
+        switch (R.metric_id) {
+        case kKerr: return analytic_pair_kernel_kerr();
+        case kJohannsen: return analytic_pair_kernel_joh();
+        case kFlat: return analytic_pair_kernel_flat();
+        default: return nullptr;
+        }
+    }
+    // no FP64 steps near the horizon or at turning points
+    if (R.precision != FOORT_PREC_MIXED || R.mixed_fp64_margin > 0.0 ||
+        (R.mixed_options & FOORT_MIXED_FP64_TURNING_POINTS))
+        return nullptr;
     switch (R.metric_id) {
     case kKerr: return pair ? mixed_lean_pair_kernel_kerr(R.rlog != 0) : mixed_lean_kernel_kerr(R.rlog != 0);
     case kFlat: return R.rlog ? nullptr : pair ? mixed_lean_pair_kernel_flat() : mixed_lean_kernel_flat();

@@ -61,6 +61,9 @@ __device__ __forceinline__ float p_fma(float a, float b, float c) { return __fma
 __device__ __forceinline__ float p_mul(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ float p_add(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ float p_sub(float a, float b) { return __fsub_rn(a, b); }
+__device__ __forceinline__ double p_fma(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ double p_mul(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ double p_add(double a, double b) { return __dadd_rn(a, b); }
 
 // A float in every half, and a function of a float on every half.
 template <typename T>

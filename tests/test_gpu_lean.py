@@ -94,6 +94,58 @@ def test_a_full_gpu_of_refilled_lanes_gives_the_general_kernels_records(eng):
     del keep
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [abi.PREC_FP64, abi.PREC_FP64_ANALYTIC])
+@pytest.mark.parametrize("metric,params,rlog,side,timeout", [
+    (abi.METRIC_KERR, (0.9,), 1, 17, None),
+    (abi.METRIC_KERR, (0.0,), 1, 7, 0),
+    (abi.METRIC_KERR, (0.99,), 0, 2, 3000),
+    (abi.METRIC_JOHANNSEN, (0.8, 1.0, 0.5, 0.2, 0.1), 1, 17, None),
+    (abi.METRIC_RASHEED_LARSEN, LORENZO, 1, 9, None),
+    (abi.METRIC_FLAT, (), 0, 3, 3000),
+])
+def test_two_lanes_in_fp64_give_the_one_lane_results(eng, metric, params, rlog, side, timeout, precision):
+    """The FP64 and FP64-analytic kernels on two lanes per geodesic (where they exist)
+    against one lane. In FP64-analytic the compiler may contract Johannsen's body differently
+    in the two (one rounding of FP64 in an acceleration): its records agree to the 48 bits of
+    the state times the rays' amplification, taken as 1e4 here, and exactly in the rest."""
+    px = abi.square_pixels(side)
+    d, keep = describe(metric, params, rlog, 63.0, timeout=timeout)
+    d.precision = precision
+    got = {}
+    for lanes in (1, 2):
+        with eng.Engine(d) as e:
+            e.set_lanes(lanes)
+            got[lanes] = e.integrate(px)
+            counts = e.stats()
+            assert counts["rhs_evals"] == 4 * counts["steps"] == 4 * int(got[lanes]["steps"].sum())
+            assert counts["fp64_steps"] == (counts["steps"] if precision == abi.PREC_FP64_ANALYTIC else 0)
+    if precision == abi.PREC_FP64_ANALYTIC and metric == abi.METRIC_JOHANNSEN:
+        for name in abi.RESULT_DTYPE.names:
+            np.testing.assert_allclose(got[2][name], got[1][name], rtol=1e4 * 2.0**-48, atol=1e4 * 2.0**-48,
+                                       err_msg=name)
+    else:
+        same_records(got[2], got[1])
+    del keep
+
+
+@pytest.mark.gpu
+def test_fp64_launches_in_every_block_size_give_the_same_records(eng):
+    """FP64 launches take CTAs of 32 threads, four per SM, unless a shape is asked for."""
+    px = abi.square_pixels(41)
+    d, keep = describe(abi.METRIC_KERR, (0.9,), 1, 63.0, integrator=abi.INTEGRATOR_VERLET)
+    d.precision = abi.PREC_FP64
+    got = {}
+    for block in (0, 32, 64, 128):
+        with eng.Engine(d) as e:
+            e.set_launch(block, 0)
+            got[block] = e.integrate(px)
+            assert e.stats()["block_size"] == (block or 32)
+    for block in got:
+        same_records(got[block], got[0])
+    del keep
+
+
 def test_packed_bodies_match_the_generator():
     """gen_packed.inc is what gen_packed.py prints for the committed gen_christoffel.inc."""
     gen = os.path.join(ROOT, "foort_gb300", "gen", "gen_packed.py")
