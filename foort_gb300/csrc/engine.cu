@@ -171,6 +171,10 @@ int validate(const foort_run_desc* d, std::string& why) {
 
 RunConst make_run_const(const foort_run_desc& d) {
     RunConst R{};
+    R.only_alpha13 = 1;
+    for (uint32_t i = 0; i < d.n_images; ++i)
+        for (int k = 2; k < 5; ++k)  // alpha22, alpha52, epsilon3
+            if (d.images[i].metric_params[k] != 0.0) R.only_alpha13 = 0;
     R.metric_id = d.metric_id;
     // Flat space is not a SphericalHorizonMetric: no log-r scale (ViewScreen.h:49-50)
     // and no Horizon termination (Config.cpp:649-657).
@@ -254,13 +258,21 @@ struct LaunchShape {
 //   geodesics in log r 1.31 ms on two lanes and 1.58 on one. In plain r both take the same
 //   within 3 % (3,000 geodesics 66 and 64 ms, 1.00 and 0.97 us a step): the smallest launches
 //   stay on two, the rest take one.
+// - Johannsen with alpha13 alone: its packed body spills on one lane at three CTAs per SM and
+//   is held to two, so two lanes pay as long as they fit on the GPU (192 x SMs geodesics;
+//   plain r, 19,600 geodesics 174 ms on two and 211 on one, 39,204 291 and 255), and in log r,
+//   where the longest rays end a launch alone, several refills further (62,500 4.9 and 5.9 ms,
+//   160,000 9.0 and 9.2).
 // - Lean kernels with a called plugin exist on two lanes only and cost a geodesic no more
 //   than the general one-lane kernel: every size.
 uint64_t pair_limit(const RunConst& R, bool positions, int per_sm, int num_sms, uint32_t bs) {
     const uint64_t sms = static_cast<uint64_t>(num_sms);
     if (R.precision != FOORT_PREC_MIXED) return 512 * sms;
-    if (!positions && mixed_lean_kernel(R, true))
-        return mixed_lean_kernel(R, false) ? (R.rlog ? 64 : 24) * sms : UINT64_MAX;
+    if (!positions && mixed_lean_kernel(R, true)) {
+        if (!mixed_lean_kernel(R, false)) return UINT64_MAX;
+        if (R.metric_id == kJohannsen) return (R.rlog ? 1024 : 192) * sms;
+        return (R.rlog ? 64 : 24) * sms;
+    }
     return static_cast<uint64_t>(per_sm) * sms * bs / 2;
 }
 

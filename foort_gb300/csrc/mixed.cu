@@ -47,6 +47,8 @@ const void* mixed_lean_kernel_flat();
 const void* mixed_lean_pair_kernel_kerr(bool rlog);
 const void* mixed_lean_pair_kernel_flat();
 const void* mixed_lean_pair_kernel_joh();
+const void* mixed_lean_kernel_joh13(bool rlog);
+const void* mixed_lean_pair_kernel_joh13(bool rlog);
 const void* mixed_lean_pair_kernel_rl();
 const void* analytic_pair_kernel_kerr();
 const void* analytic_pair_kernel_joh();
@@ -83,7 +85,10 @@ const void* mixed_lean_kernel(const RunConst& R, bool pair) {
     switch (R.metric_id) {
     case kKerr: return pair ? mixed_lean_pair_kernel_kerr(R.rlog != 0) : mixed_lean_kernel_kerr(R.rlog != 0);
     case kFlat: return R.rlog ? nullptr : pair ? mixed_lean_pair_kernel_flat() : mixed_lean_kernel_flat();
-    case kJohannsen: return pair ? mixed_lean_pair_kernel_joh() : nullptr;
+    case kJohannsen:
+        if (R.only_alpha13)
+            return pair ? mixed_lean_pair_kernel_joh13(R.rlog != 0) : mixed_lean_kernel_joh13(R.rlog != 0);
+        return pair ? mixed_lean_pair_kernel_joh() : nullptr;
     case kRasheedLarsen: return pair ? mixed_lean_pair_kernel_rl() : nullptr;
     default: return nullptr;
     }

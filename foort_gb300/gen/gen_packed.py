@@ -6,9 +6,8 @@ multiply-adds at all, while the compiler contracts the scalar bodies of
 gen_christoffel.inc, so a pair body written with operators would round differently from
 the scalar one. This script writes the bodies with every rounding spelled out (MUL, ADD,
 FMA, RCP on a type T that is a float or a pair of floats), contracting as the compiler
-does: a product joins a sum as an FMA where the sum is its only use, or where all of its
-(fewer than five) uses are sums; with two such products the one that only this sum uses
-joins, the left one first. A step's results are then the scalar body's bit for bit.
+does: a product joins a sum as an FMA where all of its (fewer than five) uses are sums, or
+where the sum comes far behind it; of two such products the left one. A step's results are then the scalar body's bit for bit.
 
 Products of the metric constants q[] alone are split off (FOORT_PACKED_CONST_*): a lane
 computes them once per geodesic.
@@ -131,97 +130,216 @@ def reachable(g):
     return seen
 
 
-def contraction(g):
-    """add node -> index (0 or 1) of the product operand that joins it, or None."""
-    live, users = reachable(g), {}
+# Where the compiled Johannsen body departs from contraction()'s rule, found by comparing
+# 262,144 evaluations (four spins and alpha13, r_+ + 0.002 to 1000) bit for bit: sum -> the
+# operand whose product joins it.
+EXCEPTIONS = {"JOHANNSEN": {89: 1, 614: 1, 1036: 1, 1045: 1}}
+FAR = 500  # operations between a product and a sum that make the compiler fuse it all the same
+
+
+def contraction(g, name):
+    """add node -> index (0 or 1) of the product operand that joins it, or None. Sums are
+    taken from the last to the first: a sum that has taken a product no longer counts as a
+    sum for its other operand."""
+    live, users, order = reachable(g), {}, {}
 
     def positive(x):
         return x[0] > 0 or g.is_const(x)
 
-    for i in live:
+    at = 0
+    for i in sorted(live):
         k = g.nodes[i]
+        if k[0] in ("mul", "add", "rcp"):
+            order[i] = at
+            at += 4 if k[0] == "rcp" else 1
         kind = "add" if k[0] == "add" and positive(k[1]) and positive(k[2]) else "other"
         for o in g.operands(i):
-            users.setdefault(o, []).append(kind)
+            users.setdefault(o, []).append([i, kind])
     for _, x in g.outputs:
-        users.setdefault(x[1], []).append("other")
+        users.setdefault(x[1], []).append([None, "other"])
+
+    def joins(m, total):
+        if g.nodes[m][0] != "mul" or len(users[m]) >= 5:
+            return False
+        if all(kind == "add" for _, kind in users[m]):
+            return True
+        if order[total] - order[m] < FAR:
+            return False
+        return any(g.nodes[o][0] == "const" or any(u is None or order[u] > order[total] for u, _ in users[o])
+                   for o in g.nodes[m][1:])
+
     out = {}
-    for i in live:
+    for i in sorted((i for i in live if g.nodes[i][0] == "add"), reverse=True):
         k = g.nodes[i]
-        if k[0] != "add":
-            continue
         ops = [x[1] for x in k[1:]]
-        product = [g.nodes[o][0] == "mul" for o in ops]
-        single = [p and len(users[o]) == 1 for p, o in zip(product, ops)]
-        sums = [p and len(users[o]) < 5 and all(u == "add" for u in users[o]) and positive(k[1]) and positive(k[2])
-                for p, o in zip(product, ops)]
-        out[i] = 0 if single[0] else 1 if single[1] else 0 if sums[0] else 1 if sums[1] else None
+        if positive(k[1]) and positive(k[2]):
+            join = next((n for n in (0, 1) if joins(ops[n], i)), None)
+        else:  # a difference takes a product that only it uses
+            join = next((n for n in (0, 1) if g.nodes[ops[n]][0] == "mul" and len(users[ops[n]]) == 1), None)
+        join = EXCEPTIONS.get(name, {}).get(i, join)
+        out[i] = join
+        if join is not None:
+            users[ops[join]] = [u for u in users[ops[join]] if u[0] != i]
+            for o in g.nodes[ops[join]][1:]:
+                users[o].append([i, "fma"])
+            for u in users[ops[1 - join]]:
+                if u[0] == i:
+                    u[1] = "fma"
     return out
 
 
-def emit(name):
-    g = read_body(name)
-    fuse, live = contraction(g), reachable(g)
-    only_q = {}
+class Ops:
+    """The operations of a contracted body, each once. Values are ("c", number) or
+    ("v", sign, text); operations with a zero or a one fold away, exactly."""
 
-    def constant(i):
-        """Made of q[] alone."""
-        if i not in only_q:
-            k = g.nodes[i]
-            only_q[i] = k[1].startswith("q[") if k[0] == "leaf" else k[0] == "mul" and all(map(constant, k[1:]))
-        return only_q[i]
+    def __init__(self, g, fuse, zeros):
+        self.g, self.fuse, self.zeros = g, fuse, zeros
+        self.done, self.index, self.list = {}, {}, []
 
-    needed = sorted({o for i in live if not constant(i) for o in operands_after(g, fuse, i) if constant(o)})
-    consts, body, done = [], [], {}
+    def op(self, *key):
+        if key not in self.index:
+            self.index[key] = "n%d" % len(self.list)
+            self.list.append((self.index[key], key))
+        return self.index[key]
 
-    def value(i, lines):
-        if i in done:
-            return done[i]
-        k = g.nodes[i]
+    @staticmethod
+    def text(v):
+        if v[0] == "c":
+            return ("-" if v[1] < 0 else "") + "K(%rf)" % abs(v[1])
+        return ("-" if v[1] < 0 else "") + v[2]
+
+    @staticmethod
+    def negated(v):
+        return ("c", -v[1]) if v[0] == "c" else ("v", -v[1], v[2])
+
+    def factors(self, a, b):
+        """(sign, a, b) with the signs taken out, or the product where it folds."""
+        if ("c", 0.0) in (a, b):
+            return ("c", 0.0)
+        for x, y in ((a, b), (b, a)):
+            if x[0] == "c" and abs(x[1]) == 1.0:
+                return y if x[1] > 0 else self.negated(y)
+        sign, texts = 1, []
+        for v in (a, b):
+            texts.append(self.text(v).lstrip("-"))
+            sign *= -1 if self.text(v).startswith("-") else 1
+        return sign, texts[0], texts[1]
+
+    def mul(self, a, b):
+        f = self.factors(a, b)
+        if f[0] in ("c", "v"):
+            return f
+        sign, x, y = f
+        return "v", sign, self.index.get(("MUL", y, x)) or self.op("MUL", x, y)
+
+    def add(self, a, b):
+        if a == ("c", 0.0):
+            return b
+        return a if b == ("c", 0.0) else ("v", 1, self.op("ADD", self.text(a), self.text(b)))
+
+    def fma(self, a, b, c):
+        if c == ("c", 0.0):
+            return self.mul(a, b)
+        f = self.factors(a, b)
+        if f[0] in ("c", "v"):
+            return self.add(f, c)
+        return "v", 1, self.op("FMA", ("-" if f[0] < 0 else "") + f[1], f[2], self.text(c))
+
+    def signed(self, x):
+        v = self.value(x[1])
+        return v if x[0] > 0 else self.negated(v)
+
+    def value(self, i):
+        if i in self.done:
+            return self.done[i]
+        k = self.g.nodes[i]
         if k[0] == "leaf":
-            return k[1]
-        if k[0] == "const":
-            return "K(%sf)" % k[1]
-        if k[0] == "mul":
-            text = "MUL(%s, %s)" % (value(k[1], lines), value(k[2], lines))
+            v = ("c", 0.0) if k[1] in self.zeros else ("v", 1, k[1])
+        elif k[0] == "const":
+            v = ("c", k[1])
+        elif k[0] == "mul":
+            v = self.mul(self.value(k[1]), self.value(k[2]))
         elif k[0] == "rcp":
-            text = "RCP(%s)" % signed(k[1], lines)
-        elif fuse[i] is None:
-            text = "ADD(%s, %s)" % (signed(k[1], lines), signed(k[2], lines))
+            x = self.signed(k[1])
+            v = ("c", 1.0) if x == ("c", 1.0) else ("v", 1, self.op("RCP", self.text(x)))
+        elif self.fuse[i] is None:
+            v = self.add(self.signed(k[1]), self.signed(k[2]))
         else:
-            m, o = (k[1], k[2]) if fuse[i] == 0 else (k[2], k[1])
-            a, b = g.nodes[m[1]][1:]
-            text = "FMA(%s%s, %s, %s)" % ("-" if m[0] < 0 else "", value(a, lines), value(b, lines), signed(o, lines))
-        lines.append("const T n%d = %s;" % (i, text))
-        done[i] = "n%d" % i
-        return done[i]
+            m, o = (k[1], k[2]) if self.fuse[i] == 0 else (k[2], k[1])
+            x, y = (self.value(j) for j in self.g.nodes[m[1]][1:])
+            v = self.fma(x if m[0] > 0 else self.negated(x), y, self.signed(o))
+        self.done[i] = v
+        return v
 
-    def signed(x, lines):
-        return ("-" if x[0] < 0 else "") + value(x[1], lines)
 
-    for slot, i in enumerate(needed):
-        text = value(i, consts)
-        consts.append("k[%d] = %s;" % (slot, text))
-    consts = [line.replace("const T ", "const float ") for line in consts]
-    for slot, i in enumerate(needed):
-        done[i] = "B(%d)" % slot
-    body += ["%s = %s;" % (target, signed(x, body)) for target, x in g.outputs]
-    print("// %d operations on T" % sum(line.startswith("const") for line in body))
-    print("#define FOORT_PACKED_SLOTS_%s %d" % (name, len(needed)))
-    print("#define FOORT_PACKED_CONST_%s \\" % name)
+def emit(name, label=None, zeros=()):
+    g = read_body(name)
+    ops = Ops(g, contraction(g, name), zeros)
+    outputs = [(target, ops.text(ops.signed(x))) for target, x in g.outputs]
+    made = dict(ops.list)
+    word = re.compile(r"\bn\d+\b|q\[\d+\]")
+
+    def inputs(key):
+        return [w for arg in key[1:] for w in word.findall(arg)]
+
+    live, todo = set(), [w for _, e in outputs for w in word.findall(e)]
+    while todo:
+        w = todo.pop()
+        if w not in live:
+            live.add(w)
+            todo += inputs(made[w]) if w in made else []
+    # the lane's constants: made of q[] alone and used by the rest, but for small multiples
+    only_q = {w for w in live if w.startswith("q[")}
+    for w, key in ops.list:
+        if w in live and not re.search(r"\b(r|dp|dm|s|c)\b", " ".join(key[1:])) and key[0] != "RCP" \
+                and all(v in only_q for v in inputs(key)):
+            only_q.add(w)
+    multiple = {w for w in only_q if w in made and made[w][0] == "MUL" and made[w][1].startswith("K(")}
+    kept, seen = [], set()
+
+    def need(w):
+        if w not in only_q or w in seen:
+            return
+        seen.add(w)
+        if w in multiple:
+            for v in inputs(made[w]):
+                need(v)
+        else:
+            kept.append(w)
+
+    rest = [w for w, _ in ops.list if w in live and w not in only_q]
+    for w in rest:
+        for v in inputs(made[w]):
+            need(v)
+    order = {w: n for n, (w, _) in enumerate(ops.list)}
+    kept.sort(key=lambda w: order.get(w, -1))
+    slot = {w: "B(%d)" % n for n, w in enumerate(kept)}
+    consts, have = [], set()
+
+    def const_line(w):
+        if w in made and w not in have:
+            have.add(w)
+            for v in inputs(made[w]):
+                const_line(v)
+            consts.append("const float %s = %s(%s);" % (w, made[w][0], ", ".join(made[w][1:])))
+
+    for n, w in enumerate(kept):
+        const_line(w)
+        consts.append("k[%d] = %s;" % (n, w))
+
+    def put(text):
+        return word.sub(lambda m: slot.get(m.group(0), m.group(0)), text)
+
+    body = ["const T %s = %s(%s);" % (w, key[0], ", ".join(map(put, key[1:]))) for w, key in ops.list
+            if w in live and (w not in only_q or w in multiple and w in seen)]
+    print("// %d operations on T" % len(body))
+    label = label or name
+    print("#define FOORT_PACKED_SLOTS_%s %d" % (label, len(kept)))
+    print("#define FOORT_PACKED_CONST_%s \\" % label)
     print(" \\\n".join("    " + line for line in consts or [";"]))
-    print("#define FOORT_PACKED_BODY_%s \\" % name)
-    print(" \\\n".join("    " + line for line in body))
+    print("#define FOORT_PACKED_BODY_%s \\" % label)
+    print(" \\\n".join("    " + line for line in body + ["%s = %s;" % (t, put(e)) for t, e in outputs]))
     print()
-
-
-def operands_after(g, fuse, i):
-    """Operands of node i once products have joined sums."""
-    k = g.nodes[i]
-    if k[0] == "add" and fuse[i] is not None:
-        m, o = (k[1], k[2]) if fuse[i] == 0 else (k[2], k[1])
-        return list(g.nodes[m[1]][1:]) + [o[1]]
-    return g.operands(i)
 
 
 def main():
@@ -231,6 +349,9 @@ def main():
     print("// lane's constant i as a T. Out: dr, dh, gu as in gen_christoffel.inc.")
     for name in ("KERR", "FLAT"):
         emit(name)
+    # Johannsen's metric with alpha13 alone: the shipped configurations and the studies of
+    # one deviation at a time
+    emit("JOHANNSEN", "JOHANNSEN13", ("q[2]", "q[3]", "q[4]"))
 
 
 if __name__ == "__main__":

@@ -56,6 +56,10 @@ def same_records(a, b):
     (abi.METRIC_JOHANNSEN, (0.8, 1.0, 0.5, 0.2, 0.1), 1, 63.0, 33, None),
     (abi.METRIC_JOHANNSEN, (0.7, 2.0, 0.0, 0.0, 0.0), 1, 90.0, 21, None),
     (abi.METRIC_JOHANNSEN, (0.8, 1.0, 0.5, 0.2, 0.1), 0, 63.0, 3, 20000),
+    (abi.METRIC_JOHANNSEN, (0.3, -0.9, 0.0, 0.0, 0.0), 1, 30.0, 33, None),
+    (abi.METRIC_JOHANNSEN, (0.99, 0.0, 0.0, 0.0, 0.0), 1, 2.0, 17, None),
+    (abi.METRIC_JOHANNSEN, (0.9, 0.4, 0.0, 0.0, 0.0), 0, 30.0, 9, None),
+    (abi.METRIC_JOHANNSEN, (0.7, 2.0, 0.0, 0.0, 1e-3), 1, 90.0, 9, None),
     (abi.METRIC_RASHEED_LARSEN, LORENZO, 1, 63.0, 33, None),
     (abi.METRIC_RASHEED_LARSEN, LORENZO, 0, 63.0, 3, 20000),
 ])
