@@ -18,6 +18,17 @@ __global__ void __launch_bounds__(128) integrate_lean_pair_kernel(const __grid_c
     persistent_loop<LeanEngine<MID, RLOG>, true>(A, R);
 }
 
+template <int MID, bool RLOG>
+__global__ void __launch_bounds__(128, 3) integrate_lean_verlet_kernel(const __grid_constant__ LaunchArgs A,
+                                                                       const __grid_constant__ RunConst R) {
+    persistent_loop<LeanVerletEngine<MID, RLOG>>(A, R);
+}
+
+const void* mixed_lean_verlet_kernel_joh13(bool rlog) {
+    return rlog ? reinterpret_cast<const void*>(&integrate_lean_verlet_kernel<kJohannsen, true>)
+                : reinterpret_cast<const void*>(&integrate_lean_verlet_kernel<kJohannsen, false>);
+}
+
 const void* mixed_lean_kernel_joh13(bool rlog) {
     return rlog ? reinterpret_cast<const void*>(&integrate_lean_kernel<kJohannsen, true>)
                 : reinterpret_cast<const void*>(&integrate_lean_kernel<kJohannsen, false>);

@@ -275,6 +275,16 @@ constexpr bool is_lean(decltype(E::kLean)*) {
     return true;
 }
 
+// Lean engines that count their right-hand sides (E::kCountsRhs).
+template <class E>
+constexpr bool is_counting(...) {
+    return false;
+}
+template <class E>
+constexpr bool is_counting(decltype(E::kCountsRhs)*) {
+    return true;
+}
+
 // Lean engines whose every step is an FP64 step (E::kFp64Steps).
 template <class E>
 constexpr bool is_fp64_steps(...) {
@@ -306,7 +316,10 @@ __device__ __forceinline__ void persistent_loop(const LaunchArgs& A, const RunCo
     // The warp's right-hand sides and FP64 steps since the last count: the lanes' counters,
     // or (lean engines) a fixed number per step.
     auto rhs_counts = [](typename E::Lane& l, unsigned long long steps, unsigned long long& rhs, unsigned long long& fp64) {
-        if constexpr (kLean) {
+        if constexpr (is_counting<E>(nullptr)) {
+            rhs = __reduce_add_sync(kFullMask, l.rhs);
+            l.rhs = 0;
+        } else if constexpr (kLean) {
             rhs = steps * E::kRhsPerStep;
             if constexpr (is_fp64_steps<E>(nullptr)) fp64 = steps;
         } else {

@@ -80,6 +80,7 @@ __device__ __forceinline__ void accel_lean(const MetricAt<T>& m, const T u[4], T
     auto second = [](T x, T y, T z, T w) { return p_fma(z, w, p_mul(x, y)); };
     const T w1t = first(m.d1.tt, u[0], m.d1.tp, u[3]), w1p = first(m.d1.tp, u[0], m.d1.pp, u[3]);
     const T w2t = first(m.d2.tt, u[0], m.d2.tp, u[3]);
+    constexpr bool kSecond = FORM == 1 || FORM == 2;
     const T w2p = (FORM == 1) ? second(m.d2.tp, u[0], m.d2.pp, u[3]) : first(m.d2.tp, u[0], m.d2.pp, u[3]);
     const T w1r = p_mul(m.d1.rr, u[1]), w1h = p_mul(m.d1.hh, u[2]);
     const T w2r = p_mul(m.d2.rr, u[1]), w2h = p_mul(m.d2.hh, u[2]);
@@ -87,10 +88,10 @@ __device__ __forceinline__ void accel_lean(const MetricAt<T>& m, const T u[4], T
     const T q2a = first(u[0], w2t, u[1], w2r);
     const T q2b = FORM ? p_fma(u[2], w2h, q2a) : p_add(q2a, p_mul(u[2], w2h));
     const T q2 = p_fma(u[3], w2p, q2b);
-    const T Ft = FORM ? second(u[1], w1t, u[2], w2t) : first(u[1], w1t, u[2], w2t);
-    const T Fp = FORM ? second(u[1], w1p, u[2], w2p) : first(u[1], w1p, u[2], w2p);
+    const T Ft = kSecond ? second(u[1], w1t, u[2], w2t) : first(u[1], w1t, u[2], w2t);
+    const T Fp = kSecond ? second(u[1], w1p, u[2], w2p) : first(u[1], w1p, u[2], w2p);
     const T Fr = p_fma(T(2), first(u[1], w1r, u[2], w2r), -q1);
-    const T Fh = p_fma(T(2), FORM ? second(u[1], w1h, u[2], w2h) : first(u[1], w1h, u[2], w2h), -q2);
+    const T Fh = p_fma(T(2), kSecond ? second(u[1], w1h, u[2], w2h) : first(u[1], w1h, u[2], w2h), -q2);
     a[0] = -first(m.gu.tt, Ft, m.gu.tp, Fp);
     a[3] = -first(m.gu.tp, Ft, m.gu.pp, Fp);
     a[1] = p_mul(m.gu.rr, Fr);
@@ -191,7 +192,8 @@ struct LeanState {
     static constexpr bool kLean = true;
     static constexpr bool kCopyImage = false;
 
-    // x and v: [0] holds components 0 and 1, [1] components 2 and 3, high and low parts.
+    // x and v: [0] holds components 0 (t) and 3 (phi), [1] components 1 (r or ln r) and 2
+    // (theta), high and low parts.
     struct Lane {
         f2 xh[2], xl[2], vh[2], vl[2];
         ff lam;
@@ -216,10 +218,11 @@ struct LeanState {
         }
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
-            L.xh[i] = pack2(fx[2 * i].hi, fx[2 * i + 1].hi);
-            L.xl[i] = pack2(fx[2 * i].lo, fx[2 * i + 1].lo);
-            L.vh[i] = pack2(fv[2 * i].hi, fv[2 * i + 1].hi);
-            L.vl[i] = pack2(fv[2 * i].lo, fv[2 * i + 1].lo);
+            const int a = i, b = 3 - i;
+            L.xh[i] = pack2(fx[a].hi, fx[b].hi);
+            L.xl[i] = pack2(fx[a].lo, fx[b].lo);
+            L.vh[i] = pack2(fv[a].hi, fv[b].hi);
+            L.vl[i] = pack2(fv[a].lo, fv[b].lo);
         }
         L.c.load(I);
         L.hthr[0] = I.mx.hthr[0];
@@ -243,10 +246,10 @@ struct LeanState {
     static __device__ __forceinline__ void diags(Lane& L, const RunConst& R) {
         if (R.diag_flags & FOORT_DIAG_EQUATORIAL_PASSES) {
             const MixedRun& G = R.mr;
-            const float thh = lo2(L.xh[1]), d0 = __fadd_rn(thh, G.mpio2[0]);
+            const float thh = hi2(L.xh[1]), d0 = __fadd_rn(thh, G.mpio2[0]);
             bool upd = true, neg = d0 < 0.f;
             if (!(fabsf(d0) > G.eqfar)) {  // near the equator: the float-float difference decides
-                const ff dt = ff_add(ff{thh, lo2(L.xl[1])}, ff_of(G.mpio2));
+                const ff dt = ff_add(ff{thh, hi2(L.xl[1])}, ff_of(G.mpio2));
                 upd = ff_lt(ff_of(G.eqthr), ff_abs(dt));
                 neg = ff_neg_sign(dt);
             }
@@ -255,7 +258,7 @@ struct LeanState {
             L.side = upd ? (thh > 0.f ? side : 0) : L.side;
         }
         if (R.diag_flags & FOORT_DIAG_CLOSEST_RADIUS) {
-            const ff x1 = {hi2(L.xh[0]), hi2(L.xl[0])};
+            const ff x1 = {lo2(L.xh[1]), lo2(L.xl[1])};
             const bool upd = ff_lt(x1, L.rmin);
             L.rmin.hi = upd ? x1.hi : L.rmin.hi;
             L.rmin.lo = upd ? x1.lo : L.rmin.lo;
@@ -269,16 +272,16 @@ struct LeanState {
         int code = FOORT_TERMCODE_CONTINUE;
         if (R.term_flags & FOORT_TERM_THETA_SINGULARITY) {
             // within theps of 0 or pi; well away from both, the high part alone says no
-            const float thh = lo2(L.xh[1]);
+            const float thh = hi2(L.xh[1]);
             if (!(fminf(fabsf(thh), fabsf(__fadd_rn(thh, -G.pi[0]))) > G.thfar)) {
-                const ff th = {thh, lo2(L.xl[1])}, e = ff_of(G.theps);
+                const ff th = {thh, hi2(L.xl[1])}, e = ff_of(G.theps);
                 const bool hit = ff_lt(ff_abs(th), e) | ff_lt(ff_abs(ff_add(ff_of(G.pi), ff_neg(th))), e);
                 code = hit ? FOORT_TERMCODE_THETA_SINGULARITY : code;
             }
         }
         if (R.term_flags & FOORT_TERM_TIMEOUT)
             code = (static_cast<uint32_t>(L.steps) >= R.t_max) ? FOORT_TERMCODE_TIMEOUT : code;
-        const ff x1 = {hi2(L.xh[0]), hi2(L.xl[0])};
+        const ff x1 = {lo2(L.xh[1]), lo2(L.xl[1])};
         if (R.term_flags & FOORT_TERM_BOUNDARY_SPHERE)
             code = ff_lt(ff_of(G.bthr), x1) ? FOORT_TERMCODE_BOUNDARY_SPHERE : code;
         if (R.term_flags & FOORT_TERM_HORIZON) code = ff_lt(x1, ff_of(L.hthr)) ? FOORT_TERMCODE_HORIZON : code;
@@ -286,12 +289,12 @@ struct LeanState {
     }
 
     // us = u + t k
-    static __device__ __forceinline__ void stage(f2 t, f2 uf01, f2 uf23, const float k[4], float us[4]) {
-        const f2 a = p_fma(t, pack2(k[0], k[1]), uf01), b = p_fma(t, pack2(k[2], k[3]), uf23);
+    static __device__ __forceinline__ void stage(f2 t, f2 uf03, f2 uf12, const float k[4], float us[4]) {
+        const f2 a = p_fma(t, pack2(k[0], k[3]), uf03), b = p_fma(t, pack2(k[1], k[2]), uf12);
         us[0] = lo2(a);
-        us[1] = hi2(a);
-        us[2] = lo2(b);
-        us[3] = hi2(b);
+        us[3] = hi2(a);
+        us[1] = lo2(b);
+        us[2] = hi2(b);
     }
 
     // MixedEngine::rk4_combine and advance.
@@ -302,8 +305,8 @@ struct LeanState {
         const f2 two = p_all<f2>(2.f), ph = p_all<f2>(h), ph6 = p_all<f2>(h6), phh6 = p_all<f2>(hh6);
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
-            const f2 a1 = pack2(k1[2 * i], k1[2 * i + 1]), a2 = pack2(k2[2 * i], k2[2 * i + 1]);
-            const f2 a3 = pack2(k3[2 * i], k3[2 * i + 1]), a4 = pack2(k4[2 * i], k4[2 * i + 1]);
+            const f2 a1 = pack2(k1[i], k1[3 - i]), a2 = pack2(k2[i], k2[3 - i]);
+            const f2 a3 = pack2(k3[i], k3[3 - i]), a4 = pack2(k4[i], k4[3 - i]);
             const f2 du = p_mul(ph6, p_add(p_fma(two, a3, p_fma(two, a2, a1)), a4));
             const f2 dxc = p_mul(phh6, p_add(p_add(a1, a2), a3));
             const f2 th = p_mul(ph, L.vh[i]), tl = p_fma(ph, L.vh[i], -th);
@@ -322,9 +325,15 @@ struct LeanState {
         L.term = terms(L, R);
         ++L.steps;
         diags(L, R);
-        const bool bad = !(isfinite(hi2(L.xh[0])) & isfinite(hi2(L.vh[0])));
+        const bool bad = !(isfinite(lo2(L.xh[1])) & isfinite(lo2(L.vh[1])));
         L.err |= bad ? FOORT_ERR_NONFINITE : 0u;
         return (L.term == FOORT_TERMCODE_CONTINUE) & !(bad & !(R.term_flags & FOORT_TERM_TIMEOUT));
+    }
+
+    // Component i of the state as a double.
+    static __device__ __forceinline__ double component(const f2 h[2], const f2 l[2], int i) {
+        const int k = (i == 1 || i == 2) ? 1 : 0;
+        return (i < 2) ? ff_d({lo2(h[k]), lo2(l[k])}) : ff_d({hi2(h[k]), hi2(l[k])});
     }
 
     static __device__ __forceinline__ void write(const Lane& L, const RunConst& R, foort_result* o, int term,
@@ -332,10 +341,8 @@ struct LeanState {
         double x[4], v[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const float2 xh = unpack2(L.xh[i / 2]), xl = unpack2(L.xl[i / 2]);
-            const float2 vh = unpack2(L.vh[i / 2]), vl = unpack2(L.vl[i / 2]);
-            x[i] = (i & 1) ? ff_d({xh.y, xl.y}) : ff_d({xh.x, xl.x});
-            v[i] = (i & 1) ? ff_d({vh.y, vl.y}) : ff_d({vh.x, vl.x});
+            x[i] = component(L.xh, L.xl, i);
+            v[i] = component(L.vh, L.vl, i);
         }
         if (!(finite4(x) && finite4(v))) err |= FOORT_ERR_NONFINITE;
         DiagState D;
@@ -368,20 +375,20 @@ struct LeanEngine : LeanState<LeanConst<MID>> {
     static constexpr unsigned kRhsPerStep = 4;
 
     static __device__ __forceinline__ bool step(Lane& L, const RunConst& R) {
-        const f2 uf01 = p_add(L.vh[0], L.vl[0]), uf23 = p_add(L.vh[1], L.vl[1]);
-        const float uf[4] = {lo2(uf01), hi2(uf01), lo2(uf23), hi2(uf23)};
-        const float x1h = hi2(L.xh[0]), x1l = hi2(L.xl[0]), thh = lo2(L.xh[1]), thl = lo2(L.xl[1]);
+        const f2 uf03 = p_add(L.vh[0], L.vl[0]), uf12 = p_add(L.vh[1], L.vl[1]);
+        const float uf[4] = {lo2(uf03), lo2(uf12), hi2(uf12), hi2(uf03)};
+        const float x1h = lo2(L.xh[1]), x1l = lo2(L.xl[1]), thh = hi2(L.xh[1]), thl = hi2(L.xl[1]);
         const float h = adaptive_step_lean(R.mr, thh, thl, uf[1], uf[2], uf[3]);
         const float hh = 0.5f * h;
         const f2 hh2 = pack2(hh, hh), h2 = pack2(h, h);
         float k1[4], k2[4], k3[4], k4[4], us[4];
         // stages 1 (low half) and 2 (high half)
         f2 ph, pl;
-        p_ff_add_f(pack2(x1h, thh), pack2(x1l, thl), p_mul(hh2, pack2(uf[1], uf[2])), ph, pl);
+        p_ff_add_f(L.xh[1], L.xl[1], p_mul(hh2, uf12), ph, pl);
         MetricAt<f2> m = metric_lean<MID, RLOG, f2>(L.c, pack2(x1h, lo2(ph)), pack2(x1l, lo2(pl)), pack2(thh, hi2(ph)),
                                                     pack2(thl, hi2(pl)));
         accel_lean<accel_form(MID)>(half_of(m, false), RLOG, uf, k1);
-        stage(hh2, uf01, uf23, k1, us);
+        stage(hh2, uf03, uf12, k1, us);
         accel_lean<accel_form(MID)>(half_of(m, true), RLOG, us, k2);
         // stages 3 and 4: x + h/2 (u + h/2 k1), x + h (u + h/2 k2)
         const f2 hs = pack2(hh, h);
@@ -391,9 +398,9 @@ struct LeanEngine : LeanState<LeanConst<MID>> {
         p_ff_add_f(pack2(thh, thh), pack2(thl, thl),
                    p_mul(hs, p_fma(hh2, pack2(k1[2], k2[2]), pack2(uf[2], uf[2]))), qh, ql);
         m = metric_lean<MID, RLOG, f2>(L.c, rh, rl, qh, ql);
-        stage(hh2, uf01, uf23, k2, us);
+        stage(hh2, uf03, uf12, k2, us);
         accel_lean<accel_form(MID)>(half_of(m, false), RLOG, us, k3);
-        stage(h2, uf01, uf23, k3, us);
+        stage(h2, uf03, uf12, k3, us);
         accel_lean<accel_form(MID)>(half_of(m, true), RLOG, us, k4);
         return advance(L, R, h, k1, k2, k3, k4);
     }
@@ -401,12 +408,12 @@ struct LeanEngine : LeanState<LeanConst<MID>> {
     // The step on two lanes (MixedEngine::step_pair): in each of two rounds the even lane
     // evaluates stage 1 (then 3) and the odd lane stage 2 (then 4).
     static __device__ __forceinline__ bool step_pair(Lane& L, const RunConst& R, bool odd, unsigned pmask) {
-        const f2 uf01 = p_add(L.vh[0], L.vl[0]), uf23 = p_add(L.vh[1], L.vl[1]);
-        const float uf[4] = {lo2(uf01), hi2(uf01), lo2(uf23), hi2(uf23)};
-        const f2 x12h = pack2(hi2(L.xh[0]), lo2(L.xh[1])), x12l = pack2(hi2(L.xl[0]), lo2(L.xl[1]));
+        const f2 uf03 = p_add(L.vh[0], L.vl[0]), uf12 = p_add(L.vh[1], L.vl[1]);
+        const float uf[4] = {lo2(uf03), lo2(uf12), hi2(uf12), hi2(uf03)};
+        const f2 x12h = L.xh[1], x12l = L.xl[1];
         const float h = adaptive_step_lean(R.mr, hi2(x12h), hi2(x12l), uf[1], uf[2], uf[3]);
         const float hh = 0.5f * h;
-        const f2 hh2 = pack2(hh, hh), h2 = pack2(h, h), uf12 = pack2(uf[1], uf[2]);
+        const f2 hh2 = pack2(hh, hh), h2 = pack2(h, h);
         float k1[4], k2[4], k3[4], k4[4], us[4], ka[4];
         auto share = [&](float k[4], int from) {
 #pragma unroll
@@ -418,20 +425,104 @@ struct LeanEngine : LeanState<LeanConst<MID>> {
                                                           odd ? hi2(ph) : hi2(x12h), odd ? hi2(pl) : hi2(x12l));
         accel_lean<accel_form(MID)>(m, RLOG, uf, ka);
         share(k1, 0);
-        stage(hh2, uf01, uf23, k1, us);
+        stage(hh2, uf03, uf12, k1, us);
         accel_lean<accel_form(MID)>(m, RLOG, us, ka);
         share(k2, 1);
         const float hs = odd ? h : hh;
         const f2 k12 = odd ? pack2(k2[1], k2[2]) : pack2(k1[1], k1[2]);
         p_ff_add_f(x12h, x12l, p_mul(pack2(hs, hs), p_fma(hh2, k12, uf12)), ph, pl);
         m = metric_lean<MID, RLOG, float>(L.c, lo2(ph), lo2(pl), hi2(ph), hi2(pl));
-        stage(hh2, uf01, uf23, k2, us);
+        stage(hh2, uf03, uf12, k2, us);
         accel_lean<accel_form(MID)>(m, RLOG, us, ka);
         share(k3, 0);
-        stage(h2, uf01, uf23, k3, us);
+        stage(h2, uf03, uf12, k3, us);
         accel_lean<accel_form(MID)>(m, RLOG, us, ka);
         share(k4, 1);
         return advance(L, R, h, k1, k2, k3, k4);
+    }
+};
+
+// Velocity Verlet with its metric part kept from step to step (MixedEngine::
+// step_verlet_cached): one metric part per step, so nothing of it to pack but the state's
+// update. What it gains over the general kernel are the lean checks and state (for Kerr 67.6
+// -> 45.5 ms, 1,600 rays in plain r) and, for Johannsen with alpha13 alone, the body without
+// zero terms and with it the registers that held three CTAs to 168 with 1,142 bytes of spills
+// (4,096 rays 141 -> 59.5 ms, 147,456 rays 599 -> 281 ms; two CTAs 304, four 275).
+template <int MID, bool RLOG>
+struct LeanVerletEngine : LeanState<LeanConst<MID>> {
+    using Base = LeanState<LeanConst<MID>>;
+    static constexpr bool kCountsRhs = true;
+
+    struct Lane : Base::Lane {
+        MetricAt<float> m;  // at (x1, theta)
+        uint32_t rhs = 0;
+    };
+
+    static __device__ __forceinline__ void init(Lane& L, const ImageConst& I, const RunConst& R, const foort_pixel& p) {
+        Base::init(L, I, R, p);
+        L.m = metric_lean<MID, RLOG, float>(L.c, lo2(L.xh[1]), lo2(L.xl[1]), hi2(L.xh[1]), hi2(L.xl[1]));
+    }
+
+    static __device__ __forceinline__ bool step(Lane& L, const RunConst& R) {
+        const MixedRun& G = R.mr;
+        const f2 uf03 = p_add(L.vh[0], L.vl[0]), uf12 = p_add(L.vh[1], L.vl[1]);
+        const float uf[4] = {lo2(uf03), lo2(uf12), hi2(uf12), hi2(uf03)};
+        const float h = adaptive_step_lean(G, hi2(L.xh[1]), hi2(L.xl[1]), uf[1], uf[2], uf[3]);
+        float a0[4], a1[4], vi[4];
+        accel_lean<0>(L.m, RLOG, uf, a0);
+        const float h2 = 0.5f * h, hh2 = __fmul_rn(h2, h);
+        const f2 ph = p_all<f2>(h), ph2 = p_all<f2>(h2), phh2 = p_all<f2>(hh2);
+        const f2 a03 = pack2(a0[0], a0[3]), a12 = pack2(a0[1], a0[2]);
+        Base::stage(ph, uf03, uf12, a0, vi);
+        // x += h u + h^2/2 a0: x1 and theta as the metric part sees them, then t and phi
+        f2 th = p_mul(ph, L.vh[1]), tl = p_fma(ph, L.vh[1], -th), s, e, f, g;
+        p_two_sum(L.xh[1], th, s, e);  // ff_add
+        p_two_sum(L.xl[1], tl, f, g);
+        p_fast_two_sum(s, p_add(e, f), s, e);
+        p_fast_two_sum(s, p_add(e, g), s, e);
+        p_ff_add_f(s, e, p_fma(ph, L.vl[1], p_mul(phh2, a12)), L.xh[1], L.xl[1]);
+        th = p_mul(ph, L.vh[0]);
+        tl = p_add(p_fma(ph, L.vh[0], -th), p_fma(ph, L.vl[0], p_mul(phh2, a03)));
+        p_two_sum(L.xh[0], th, s, e);
+        p_fast_two_sum(s, p_add(e, p_add(L.xl[0], tl)), L.xh[0], L.xl[0]);
+        L.m = metric_lean<MID, RLOG, float>(L.c, lo2(L.xh[1]), lo2(L.xl[1]), hi2(L.xh[1]), hi2(L.xl[1]));
+        accel_lean<0>(L.m, RLOG, vi, a1);
+        L.rhs += 2;
+        f2 b03 = pack2(a1[0], a1[3]), b12 = pack2(a1[1], a1[2]);
+        f2 du03 = p_mul(ph2, p_add(a03, b03)), du12 = p_mul(ph2, p_add(a12, b12));
+        if (G.vtol2 > 0.f) {
+            f2 dv03 = p_mul(ph2, p_sub(b03, a03)), dv12 = p_mul(ph2, p_sub(b12, a12));
+            for (int it = 0;; ++it) {
+                const f2 n03 = p_add(uf03, du03), n12 = p_add(uf12, du12);
+                const float nv[4] = {lo2(n03), lo2(n12), hi2(n12), hi2(n03)};
+                const float dv[4] = {lo2(dv03), lo2(dv12), hi2(dv12), hi2(dv03)};
+                float num = __fmul_rn(dv[0], dv[0]), den = __fmul_rn(nv[0], nv[0]);
+#pragma unroll
+                for (int i = 1; i < 4; ++i) {
+                    num = __fmaf_rn(dv[i], dv[i], num);
+                    den = __fmaf_rn(nv[i], nv[i], den);
+                }
+                if (!(num > __fmul_rn(G.vtol2, den))) break;  // num / den > tol^2 with den = |v|^2 > 0
+                if (it >= R.verlet_cap) {
+                    L.err |= FOORT_ERR_VERLET_ITER;
+                    break;
+                }
+                // (in log-r mode the compiled loop rounds (u^1)^2 before it subtracts it)
+                accel_lean<0>(L.m, false, nv, a1);
+                if (RLOG) a1[1] = __fsub_rn(a1[1], __fmul_rn(nv[1], nv[1]));
+                const f2 c03 = pack2(a1[0], a1[3]), c12 = pack2(a1[1], a1[2]);
+                dv03 = p_mul(ph2, p_sub(c03, b03));
+                dv12 = p_mul(ph2, p_sub(c12, b12));
+                b03 = c03;
+                b12 = c12;
+                du03 = p_mul(ph2, p_add(a03, b03));
+                du12 = p_mul(ph2, p_add(a12, b12));
+                L.rhs += 1;
+            }
+        }
+        p_ff_add_f(L.vh[0], L.vl[0], du03, L.vh[0], L.vl[0]);
+        p_ff_add_f(L.vh[1], L.vl[1], du12, L.vh[1], L.vl[1]);
+        return Base::after_step(L, R, ff_add_f(L.lam, h));
     }
 };
 
@@ -486,12 +577,12 @@ struct LeanCalledEngine : LeanState<ImageRef> {
 
     static __device__ __forceinline__ bool step_pair(Lane& L, const RunConst& R, bool odd, unsigned pmask) {
         const bool rlog = R.rlog != 0;
-        const f2 uf01 = p_add(L.vh[0], L.vl[0]), uf23 = p_add(L.vh[1], L.vl[1]);
-        const F4 uf = {lo2(uf01), hi2(uf01), lo2(uf23), hi2(uf23)};
-        const f2 x12h = pack2(hi2(L.xh[0]), lo2(L.xh[1])), x12l = pack2(hi2(L.xl[0]), lo2(L.xl[1]));
+        const f2 uf03 = p_add(L.vh[0], L.vl[0]), uf12 = p_add(L.vh[1], L.vl[1]);
+        const F4 uf = {lo2(uf03), lo2(uf12), hi2(uf12), hi2(uf03)};
+        const f2 x12h = L.xh[1], x12l = L.xl[1];
         const float h = adaptive_step_lean(R.mr, hi2(x12h), hi2(x12l), uf.y, uf.z, uf.w);
         const float hh = 0.5f * h;
-        const f2 hh2 = pack2(hh, hh), uf12 = pack2(uf.y, uf.z);
+        const f2 hh2 = pack2(hh, hh);
         f2 ph, pl;
         p_ff_add_f(x12h, x12l, p_mul(hh2, uf12), ph, pl);
         const ff r12 = odd ? ff{lo2(ph), lo2(pl)} : ff{lo2(x12h), lo2(x12l)};
@@ -500,9 +591,9 @@ struct LeanCalledEngine : LeanState<ImageRef> {
         const float hs = odd ? h : hh;
         const f2 kp = odd ? pack2(k12.b.y, k12.b.z) : pack2(k12.a.y, k12.a.z);
         p_ff_add_f(x12h, x12l, p_mul(pack2(hs, hs), p_fma(hh2, kp, uf12)), ph, pl);
-        const f2 us01 = p_fma(hh2, pack2(k12.b.x, k12.b.y), uf01), us23 = p_fma(hh2, pack2(k12.b.z, k12.b.w), uf23);
+        const f2 us03 = p_fma(hh2, pack2(k12.b.x, k12.b.w), uf03), us12 = p_fma(hh2, pack2(k12.b.y, k12.b.z), uf12);
         const TwoK k34 = round_called<MID>(*L.c.mx, rlog, ff{lo2(ph), lo2(pl)}, ff{hi2(ph), hi2(pl)}, uf,
-                                           F4{lo2(us01), hi2(us01), lo2(us23), hi2(us23)}, h, pmask);
+                                           F4{lo2(us03), lo2(us12), hi2(us12), hi2(us03)}, h, pmask);
         const float k1[4] = {k12.a.x, k12.a.y, k12.a.z, k12.a.w}, k2[4] = {k12.b.x, k12.b.y, k12.b.z, k12.b.w};
         const float k3[4] = {k34.a.x, k34.a.y, k34.a.z, k34.a.w}, k4[4] = {k34.b.x, k34.b.y, k34.b.z, k34.b.w};
         return advance(L, R, h, k1, k2, k3, k4);
@@ -555,8 +646,8 @@ struct AnalyticPairEngine : LeanState<ImageRef> {
         double x[4], u[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            x[i] = half_d(L.xh[i / 2], L.xl[i / 2], i & 1);
-            u[i] = half_d(L.vh[i / 2], L.vl[i / 2], i & 1);
+            x[i] = component(L.xh, L.xl, i);
+            u[i] = component(L.vh, L.vl, i);
         }
         const double h = adaptive_step_fp64(R, x, u), hh = 0.5 * h;
         const D4 uf = {u[0], u[1], u[2], u[3]};
@@ -583,16 +674,12 @@ struct AnalyticPairEngine : LeanState<ImageRef> {
         }
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
-            L.xh[i] = pack2(nx[2 * i].hi, nx[2 * i + 1].hi);
-            L.xl[i] = pack2(nx[2 * i].lo, nx[2 * i + 1].lo);
-            L.vh[i] = pack2(nv[2 * i].hi, nv[2 * i + 1].hi);
-            L.vl[i] = pack2(nv[2 * i].lo, nv[2 * i + 1].lo);
+            L.xh[i] = pack2(nx[i].hi, nx[3 - i].hi);
+            L.xl[i] = pack2(nx[i].lo, nx[3 - i].lo);
+            L.vh[i] = pack2(nv[i].hi, nv[3 - i].hi);
+            L.vl[i] = pack2(nv[i].lo, nv[3 - i].lo);
         }
         return after_step(L, R, ff_add(L.lam, ff_from_d(h)));
-    }
-
-    static __device__ __forceinline__ double half_d(f2 h, f2 l, bool hi) {
-        return hi ? ff_d({hi2(h), hi2(l)}) : ff_d({lo2(h), lo2(l)});
     }
 };
 

@@ -49,6 +49,8 @@ const void* mixed_lean_pair_kernel_flat();
 const void* mixed_lean_pair_kernel_joh();
 const void* mixed_lean_kernel_joh13(bool rlog);
 const void* mixed_lean_pair_kernel_joh13(bool rlog);
+const void* mixed_lean_verlet_kernel_kerr(bool rlog);
+const void* mixed_lean_verlet_kernel_joh13(bool rlog);
 const void* mixed_lean_pair_kernel_rl();
 const void* analytic_pair_kernel_kerr();
 const void* analytic_pair_kernel_joh();
@@ -67,8 +69,19 @@ static bool lean_options(const RunConst& R) {
            each_step(R.diag_flags, FOORT_DIAG_CLOSEST_RADIUS, R.cr_every);
 }
 
+// Whether some steps of a mixed launch are taken in FP64 (near the horizon, at turning points).
+static bool fp64_regions(const RunConst& R) {
+    return R.mixed_fp64_margin > 0.0 || (R.mixed_options & FOORT_MIXED_FP64_TURNING_POINTS);
+}
+
 const void* mixed_lean_kernel(const RunConst& R, bool pair) {
-    if (!lean_options(R) || R.integrator != FOORT_INTEGRATOR_RK4) return nullptr;
+    if (!lean_options(R)) return nullptr;
+    if (R.integrator == FOORT_INTEGRATOR_VERLET) {
+        if (pair || R.precision != FOORT_PREC_MIXED || fp64_regions(R)) return nullptr;
+        if (R.metric_id == kKerr) return mixed_lean_verlet_kernel_kerr(R.rlog != 0);
+        if (R.metric_id == kJohannsen && R.only_alpha13) return mixed_lean_verlet_kernel_joh13(R.rlog != 0);
+        return nullptr;
+    }
     if (R.precision == FOORT_PREC_FP64_ANALYTIC) {
         if (!pair) return nullptr;
         switch (R.metric_id) {
@@ -78,10 +91,7 @@ const void* mixed_lean_kernel(const RunConst& R, bool pair) {
         default: return nullptr;
         }
     }
-    // no FP64 steps near the horizon or at turning points
-    if (R.precision != FOORT_PREC_MIXED || R.mixed_fp64_margin > 0.0 ||
-        (R.mixed_options & FOORT_MIXED_FP64_TURNING_POINTS))
-        return nullptr;
+    if (R.precision != FOORT_PREC_MIXED || fp64_regions(R)) return nullptr;
     switch (R.metric_id) {
     case kKerr: return pair ? mixed_lean_pair_kernel_kerr(R.rlog != 0) : mixed_lean_kernel_kerr(R.rlog != 0);
     case kFlat: return R.rlog ? nullptr : pair ? mixed_lean_pair_kernel_flat() : mixed_lean_kernel_flat();

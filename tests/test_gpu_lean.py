@@ -82,6 +82,31 @@ def test_lean_kernels_give_the_general_kernels_records(eng, metric, params, rlog
     del keep
 
 
+# tolerances: no velocity iterations, a few, many
+@pytest.mark.gpu
+@pytest.mark.parametrize("metric,params,rlog,inclination,side,timeout,tolerance", [
+    (abi.METRIC_KERR, (0.9,), 1, 63.0, 33, None, -1.0),
+    (abi.METRIC_KERR, (0.998,), 1, 17.0, 33, None, 0.001),
+    (abi.METRIC_KERR, (0.0,), 1, 90.0, 17, None, 1e-5),
+    (abi.METRIC_KERR, (0.7,), 0, 63.0, 5, 20000, 0.001),
+    (abi.METRIC_JOHANNSEN, (0.9, 0.4, 0.0, 0.0, 0.0), 1, 63.0, 33, None, -1.0),
+    (abi.METRIC_JOHANNSEN, (0.3, -0.9, 0.0, 0.0, 0.0), 1, 2.0, 33, None, 1e-5),
+    (abi.METRIC_JOHANNSEN, (0.9, 0.4, 0.0, 0.0, 0.0), 0, 30.0, 5, 20000, 0.001),
+    (abi.METRIC_JOHANNSEN, (0.9, 0.4, 0.0, 0.0, 0.0), 1, 63.0, 2, 0, 0.001),
+])
+def test_lean_verlet_gives_the_general_kernels_records(eng, metric, params, rlog, inclination, side, timeout, tolerance):
+    px = abi.square_pixels(side)
+    d, keep = describe(metric, params, rlog, inclination, integrator=abi.INTEGRATOR_VERLET, timeout=timeout)
+    d.verlet_tol = tolerance
+    with eng.Engine(d) as e:
+        got, counts = e.integrate(px), e.stats()
+    d.mixed_options = abi.MIXED_FP64_DECISIONS
+    with eng.Engine(d) as e:
+        same_records(got, e.integrate(px))
+        assert counts["rhs_evals"] == e.stats()["rhs_evals"] and counts["steps"] == e.stats()["steps"]
+    del keep
+
+
 @pytest.mark.gpu
 def test_a_full_gpu_of_refilled_lanes_gives_the_general_kernels_records(eng):
     """More pixels than resident lanes, so that every lane is refilled, with two images of
