@@ -208,7 +208,7 @@ class Engine:
         self._check(self._lib.foort_gpu_set_launch(self._ctx, block_size, blocks_per_sm))
 
     def set_lanes(self, lanes_per_geodesic=0):
-        """0: chosen per launch; 1 or 2 lanes per geodesic where the kernel has both."""
+        """0: chosen per launch; 1: one lane per geodesic; 2: several, where such a kernel exists."""
         self._check(self._lib.foort_gpu_set_lanes(self._ctx, lanes_per_geodesic))
 
     def autotune(self, d_px, n, d_out, stream=0):

@@ -226,8 +226,8 @@ const void* select_kernel(const RunConst& R, bool positions) {
     return fp64_kernel(R.metric_id, R.integrator);
 }
 
-// The two-lanes-per-geodesic kernel for these options, or nullptr (FP64, FP64-analytic,
-// Verlet, the called plugins, the strong-field FP64 steps).
+// The two-lanes-per-geodesic kernel for these options, or nullptr (FP64 and FP64-analytic
+// in part, Verlet, the called plugins, the strong-field FP64 steps).
 const void* select_pair_kernel(const RunConst& R, bool positions) {
     if (const void* lean = positions ? nullptr : mixed_lean_kernel(R, true)) return lean;
     if (R.precision == FOORT_PREC_FP64) return fp64_pair_kernel(R.metric_id, R.integrator);
@@ -237,9 +237,15 @@ const void* select_pair_kernel(const RunConst& R, bool positions) {
     return mixed_pair_kernel_variant(R.metric_id, R.integrator, (R.mixed_options & FOORT_MIXED_FP64_DECISIONS) != 0);
 }
 
+// The four-lanes-per-geodesic kernel, or nullptr. It records no positions.
+const void* select_split_kernel(const RunConst& R, bool positions) {
+    return (R.precision == FOORT_PREC_FP64 && !positions) ? fp64_split_kernel(R) : nullptr;
+}
+
 struct LaunchShape {
     const void* fn = nullptr;
-    uint32_t grid = 0, block = 0, lanes = 1, refill = 1, poll = kDefaultPollSteps;
+    uint32_t grid = 0, block = 0, lanes = 1;  // lanes: 2 stands for several, as in foort_launch_shape
+    uint32_t refill = 1, poll = kDefaultPollSteps;
 };
 
 // Geodesics up to which a launch takes two lanes each, where that kernel exists and the
@@ -276,6 +282,20 @@ uint64_t pair_limit(const RunConst& R, bool positions, int per_sm, int num_sms, 
     return static_cast<uint64_t>(per_sm) * sms * bs / 2;
 }
 
+// Geodesics up to which an FP64 launch takes four lanes each (Kerr, Johannsen). Four lanes
+// finish a step soonest, but cost 1.5 times the instructions of one lane and 1.4 times those
+// of two per geodesic, so they pay while few geodesics share a scheduler. Log r, ms:
+//              Kerr RK4 (4 / 2 / 1 lanes)    Johannsen RK4        Kerr Verlet   Johannsen Verlet
+//     3,721       34 /  47 /  82              49 /  61 / 110       25 / 55        43 /  95
+//    10,000       65 /  71 / 113              90 /  88 / 147       23 / 39        28 /  46
+//    40,000      153 / 125 / 164             209 / 144 / 194       55 / 58        69 /  75
+//    62,500      234 / 175 / 207             321 / 216 / 273       85 / 66       106 /  74
+// The limit is where the next width is as fast.
+uint64_t split_limit(const RunConst& R, int num_sms) {
+    const uint64_t sms = static_cast<uint64_t>(num_sms);
+    return (R.integrator == FOORT_INTEGRATOR_RK4 ? (R.metric_id == kKerr ? 96 : 64) : 256) * sms;
+}
+
 // Kernel and grid of a launch of n geodesics in the requested shape (zero fields: the
 // built-in rule): a persistent grid of at most the resident CTAs. The rule takes 128
 // threads, as many CTAs per SM as fit, and two lanes per geodesic up to pair_limit().
@@ -297,8 +317,16 @@ int choose_launch(foort_ctx* ctx, const RunConst& R, uint64_t n, int num_sms, co
     if (!fn) return fail(ctx, FOORT_E_UNSUPPORTED, "no kernel for this metric / integrator / precision");
     int per_sm = 0, rc = 0;
     uint32_t lanes = 1;
+    const void* split = (want.lanes != 1) ? select_split_kernel(R, positions) : nullptr;
     const void* fn2 = (want.lanes != 1) ? select_pair_kernel(R, positions) : nullptr;
-    if (fn2) {
+    if (split && (n <= split_limit(R, num_sms) || (want.lanes == 2 && !fn2))) {
+        if ((rc = resident(split, per_sm))) return rc;
+        if (per_sm > 0) {
+            fn = split;
+            lanes = 4;
+        }
+    }
+    if (lanes == 1 && fn2) {
         int per_sm2 = 0;
         if ((rc = resident(fn2, per_sm2))) return rc;
         if (per_sm2 > 0 && (want.lanes == 2 || n <= pair_limit(R, positions, per_sm2, num_sms, bs))) {
@@ -314,7 +342,7 @@ int choose_launch(foort_ctx* ctx, const RunConst& R, uint64_t n, int num_sms, co
     out.fn = fn;
     out.grid = static_cast<uint32_t>(std::max<uint64_t>(1, std::min(full, need)));
     out.block = bs;
-    out.lanes = lanes;
+    out.lanes = std::min(lanes, 2u);
     out.refill = want.refill_steps ? want.refill_steps : 1;
     out.poll = want.poll_steps ? want.poll_steps : kDefaultPollSteps;
     return FOORT_OK;
@@ -457,7 +485,7 @@ int autotune_launch(foort_ctx* ctx, const foort_pixel* d_px, uint64_t n, foort_r
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, probe.fn, 128, 0));
     const uint64_t resident = static_cast<uint64_t>(std::max(per_sm, 1)) * ctx->num_sms * 128;
     const uint64_t m = std::min<uint64_t>(n, FOORT_TUNE_SAMPLE_LANES_X * resident);
-    const bool has_pair = select_pair_kernel(ctx->rc, false) != nullptr;
+    const bool has_pair = select_pair_kernel(ctx->rc, false) || select_split_kernel(ctx->rc, false);
     std::vector<foort_launch_shape> tried;
     auto time_shape = [&](foort_launch_shape s, double& ms) -> int {
         int r = launch(ctx, d_px, m, d_out, st, nullptr, &s);
@@ -936,6 +964,18 @@ const void* fp64_pair_kernel_kerr();
 const void* fp64_pair_kernel_flat();
 const void* fp64_pair_kernel_rl();
 const void* fp64_pair_kernel_joh();
+
+const void* fp64_split_kernel_kerr(int);
+const void* fp64_split_kernel_joh(int, bool);
+
+// Four lanes per geodesic.
+const void* fp64_split_kernel(const RunConst& R) {
+    switch (R.metric_id) {
+    case kKerr: return fp64_split_kernel_kerr(R.integrator);
+    case kJohannsen: return fp64_split_kernel_joh(R.integrator, R.only_alpha13 != 0);
+    default: return nullptr;
+    }
+}
 
 // Two lanes per geodesic: RK4. Not for Manko-Novikov, whose much larger metric the compiler
 // contracts differently there, so that its results would not be the one-lane kernel's.

@@ -7,7 +7,7 @@ namespace foort {
 template <int MID>
 __global__ void __launch_bounds__(128) integrate_analytic_pair_kernel(const __grid_constant__ LaunchArgs A,
                                                                       const __grid_constant__ RunConst R) {
-    persistent_loop<AnalyticPairEngine<MID>, true>(A, R);
+    persistent_loop<AnalyticPairEngine<MID>, 2>(A, R);
 }
 
 const void* analytic_pair_kernel_flat() { return reinterpret_cast<const void*>(&integrate_analytic_pair_kernel<kFlat>); }

@@ -13,7 +13,7 @@ __global__ void __launch_bounds__(128, 3) integrate_lean_kernel(const __grid_con
 template <int MID, bool RLOG>
 __global__ void __launch_bounds__(128) integrate_lean_pair_kernel(const __grid_constant__ LaunchArgs A,
                                                                   const __grid_constant__ RunConst R) {
-    persistent_loop<LeanEngine<MID, RLOG>, true>(A, R);
+    persistent_loop<LeanEngine<MID, RLOG>, 2>(A, R);
 }
 
 const void* mixed_lean_kernel_flat() {

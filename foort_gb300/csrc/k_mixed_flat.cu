@@ -18,7 +18,7 @@ __global__ void __launch_bounds__(128, 3) integrate_mixed_kernel(const __grid_co
 template <int MID, bool D64>
 __global__ void __launch_bounds__(128) integrate_mixed_pair_kernel(const __grid_constant__ LaunchArgs A,
                                                                    const __grid_constant__ RunConst R) {
-    persistent_loop<MixedEngine<MID, FOORT_INTEGRATOR_RK4, D64>, true>(A, R);
+    persistent_loop<MixedEngine<MID, FOORT_INTEGRATOR_RK4, D64>, 2>(A, R);
 }
 
 const void* mixed_kernel_flat(int integrator, bool decide64) {

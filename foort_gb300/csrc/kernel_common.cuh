@@ -263,9 +263,10 @@ __device__ __forceinline__ bool finite4(const double a[4]) {
 // learns whether another warp has asked every lane to stop. No loop waits on another
 // thread or on the host.
 //
-// PAIR: lanes 2k and 2k+1 integrate one geodesic together (E::step_pair). Both take the
+// LANES = 2: lanes 2k and 2k+1 integrate one geodesic together (E::step_pair). Both take the
 // same pixel, hold the same state and so leave the loop together; the even lane writes
-// the record and counts the step.
+// the record and counts the step. LANES = 4: four lanes do, each with its component of
+// the state (E::step_split); each writes its part of the record.
 template <class E>
 constexpr bool is_lean(...) {
     return false;
@@ -295,14 +296,17 @@ constexpr bool is_fp64_steps(decltype(E::kFp64Steps)*) {
     return true;
 }
 
-template <class E, bool PAIR = false>
+template <class E, int LANES = 1>
 __device__ __forceinline__ void persistent_loop(const LaunchArgs& A, const RunConst& R) {
+    static_assert(LANES == 1 || LANES == 2 || LANES == 4, "lanes per geodesic");
+    constexpr bool PAIR = LANES == 2, SPLIT = LANES == 4;
     const unsigned lane = threadIdx.x & 31u;
-    const bool odd = PAIR && (lane & 1u);
-    const unsigned slot_lane = PAIR ? (lane & ~1u) : lane;  // the lane that numbers the slot
+    const unsigned sub = lane & (LANES - 1u);
+    const bool odd = sub != 0;  // not the lane that counts the geodesic
+    const unsigned slot_lane = lane - sub;  // the lane that numbers the slot
     const unsigned lt_mask = (1u << slot_lane) - 1u;
-    const unsigned slots = PAIR ? 0x55555555u : kFullMask;  // one bit per geodesic slot
-    const unsigned pmask = 3u << (lane & ~1u);
+    const unsigned slots = SPLIT ? 0x11111111u : PAIR ? 0x55555555u : kFullMask;  // one bit per geodesic slot
+    const unsigned pmask = ((1u << LANES) - 1u) << slot_lane;
     constexpr bool kLean = is_lean<E>(nullptr);
     typename E::Lane L;
     ImageConst Ic;  // PAIR, E::kCopyImage: the lane's image constants in registers, copied at each refill
@@ -354,10 +358,14 @@ __device__ __forceinline__ void persistent_loop(const LaunchArgs& A, const RunCo
                             idx = my;
                             // i and cnt start at 0 as literals: copying them from the record
                             // made the Johannsen Verlet kernel 3 % slower on GB300
-                            if constexpr (!kLean) L.gp = (A.gp_plan && !odd && A.gp_plan[my].M > 0 && A.gp_plan[my].j > 0)
+                            if constexpr (!kLean && !SPLIT) L.gp = (A.gp_plan && !odd && A.gp_plan[my].M > 0 && A.gp_plan[my].j > 0)
                                        ? GeoposRec{A.gp_plan[my].dst, A.gp_plan[my].j, A.gp_plan[my].M, 0, 0}
                                        : GeoposRec{nullptr, 1, 0, 0, 0};
-                            E::init(L, A.images[p.image], R, p);
+                            if constexpr (SPLIT) {
+                                E::init(L, A.images[p.image], R, p, sub, pmask);
+                            } else {
+                                E::init(L, A.images[p.image], R, p);
+                            }
                             if constexpr (PAIR && E::kCopyImage) Ic = A.images[p.image];
                             active = true;
                         }
@@ -373,7 +381,9 @@ __device__ __forceinline__ void persistent_loop(const LaunchArgs& A, const RunCo
         for (;;) {
             if (active) {
                 bool more;
-                if constexpr (PAIR && kLean) {
+                if constexpr (SPLIT) {
+                    more = E::step_split(L, A.images[L.img], R, sub, pmask);
+                } else if constexpr (PAIR && kLean) {
                     more = E::step_pair(L, R, odd, pmask);
                 } else if constexpr (PAIR) {
                     more = E::step_pair(L, E::kCopyImage ? Ic : A.images[L.img], R, odd, pmask);
@@ -386,10 +396,12 @@ __device__ __forceinline__ void persistent_loop(const LaunchArgs& A, const RunCo
                 }
                 lane_steps += odd ? 0u : 1u;
                 if (!more) {
-                    if (!odd) {
-                        E::finish(L, R, &A.out[idx]);
-                        ++lane_done;
+                    if constexpr (SPLIT) {
+                        E::finish(L, R, &A.out[idx], sub);
+                    } else {
+                        if (!odd) E::finish(L, R, &A.out[idx]);
                     }
+                    lane_done += odd ? 0u : 1u;
                     active = false;
                 }
             }
@@ -424,7 +436,11 @@ __device__ __forceinline__ void persistent_loop(const LaunchArgs& A, const RunCo
                 stopping = true;
                 stop_err = (st & kStatusCancelled) ? FOORT_ERR_CANCELLED : FOORT_ERR_BUDGET;
                 if (active) {
-                    if (!odd) E::stop(L, R, &A.out[idx], stop_err);
+                    if constexpr (SPLIT) {
+                        E::stop(L, R, &A.out[idx], stop_err, sub);
+                    } else {
+                        if (!odd) E::stop(L, R, &A.out[idx], stop_err);
+                    }
                     active = false;
                 }
             }

@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(128) integrate_fp64_kernel(const __grid_consta
 template <int MID>
 __global__ void __launch_bounds__(128) integrate_fp64_pair_kernel(const __grid_constant__ LaunchArgs A,
                                                                   const __grid_constant__ RunConst R) {
-    persistent_loop<Fp64Engine<MID, FOORT_INTEGRATOR_RK4>, true>(A, R);
+    persistent_loop<Fp64Engine<MID, FOORT_INTEGRATOR_RK4>, 2>(A, R);
 }
 
 }  // namespace foort

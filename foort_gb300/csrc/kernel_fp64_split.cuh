@@ -1,0 +1,364 @@
+// The plain FP64 kernel on four lanes per geodesic (Kerr, Johannsen).
+//
+// An FP64 instruction occupies its scheduler's pipe for 64 cycles per warp on GB300, however
+// many lanes are active: a launch that leaves lanes idle costs the instructions of one
+// lane's step. Four lanes share a step here:
+// - finite differences: lane 0 evaluates the metric at r + h, lane 1 at r - h, lane 2 at
+//   theta + h, lane 3 at theta - h (one exp, one sincos and one g_dd each instead of 3, 3
+//   and 4);
+// - lane i holds component i of position and velocity, divides out the inverse metric
+//   components that a^i needs and sums the eight terms of a^i;
+// - the step rule's three quotients are lanes 1 to 3's.
+// A step takes 0.41 (RK4) to 0.44 (Verlet) of the one-lane kernel's time while the geodesics
+// fit on the GPU (log r, 3,721 geodesics, one lane to four: Kerr RK4 82 to 34 ms, Verlet 55 to
+// 25; Johannsen 110 to 49 and 95 to 43); still bound by the FP64 instructions in series.
+// The values are the one-lane kernel's bit for bit: each rounding is written out as the
+// compiler contracts Fp64Engine (kernel_fp64.cuh; found by comparing evaluations).
+#pragma once
+
+#include "kernel_common.cuh"
+
+namespace foort {
+
+__device__ __forceinline__ double d_fma(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ double d_mul(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ double d_add(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ double d_sub(double a, double b) { return __dsub_rn(a, b); }
+
+// p q - t s, the difference of g_phiphi's numerator: the compiler fuses the first product
+// where it belongs to this point alone (r + h and r - h), the second where several points
+// share the first.
+__device__ __forceinline__ double product_difference(double p, double t, double s, bool own) {
+    const double a = own ? p : -t, b = own ? p : s;  // the fused product
+    const double c = own ? -t : p, d = own ? s : p;  // the rounded one
+    return d_fma(a, b, d_mul(c, d));
+}
+
+// Metrics: dd(M, r, s, c, rlog, own) = g_dd; uu(M, r, s, c, rlog, i, g1, g2) = the inverse
+// components of lane i: g1 = g^tt, g^rr, g^thth or g^phiphi, g2 = g^tphi.
+template <int MID, bool A13>
+struct SplitMetric;
+
+template <>
+struct SplitMetric<kKerr, false> {
+    static __device__ __forceinline__ G5 dd(const double* q, double r, double s, double c, bool rlog, bool own) {
+        const double a = q[0], aa = d_mul(a, a), rr = d_mul(r, r), r2 = d_mul(2.0, r);
+        const double sig = d_fma(d_mul(aa, c), c, rr), x = d_add(rr, aa), del = d_sub(x, r2);
+        const double A = product_difference(x, d_mul(d_mul(d_mul(del, a), a), s), s, own);
+        G5 g;
+        g.tt = -d_sub(1.0, r2 / sig);
+        g.rr = sig / del;
+        g.hh = sig;
+        g.pp = d_mul(d_mul(A / sig, s), s);
+        g.tp = -(d_mul(d_mul(d_mul(d_mul(2.0, a), r), s), s) / sig);
+        if (rlog) g.rr = d_mul(g.rr, rr);
+        return g;
+    }
+    static __device__ __forceinline__ void uu(const double* q, double r, double s, double c, bool rlog, int i,
+                                              double& g1, double& g2) {
+        const double a = q[0], aa = d_mul(a, a), rr = d_mul(r, r), r2 = d_mul(2.0, r);
+        const double sig = d_fma(d_mul(aa, c), c, rr), x = d_add(rr, aa), del = d_sub(x, r2);
+        const double A = product_difference(x, d_mul(d_mul(d_mul(del, a), a), s), s, false);
+        const double sd = d_mul(sig, del);
+        const double num = (i == 0) ? -A : (i == 1) ? del : (i == 2) ? 1.0 : d_fma(-d_mul(aa, s), s, del);
+        const double den = (i == 0) ? sd : (i == 3) ? d_mul(d_mul(sd, s), s) : sig;
+        g1 = num / den;
+        g2 = -(d_mul(d_mul(2.0, a), r) / sd);
+        if (rlog && i == 1) g1 = d_mul(g1, 1.0 / rr);
+    }
+};
+
+// Johannsen. A13: alpha22, alpha52 and epsilon3 are 0, whose terms vanish exactly.
+template <bool A13>
+struct SplitMetric<kJohannsen, A13> {
+    struct Parts {
+        double A1, A2, A5, rho2, del, ra, aa, rr;
+    };
+    static __device__ __forceinline__ Parts parts(const double* q, double r, double c) {
+        const double a = q[0];
+        Parts p;
+        p.aa = d_mul(a, a);
+        p.rr = d_mul(r, r);
+        p.A1 = d_add(1.0, q[1] / d_mul(p.rr, r));
+        p.rho2 = d_fma(d_mul(p.aa, c), c, p.rr);
+        if (!A13) {
+            p.A2 = d_add(1.0, q[2] / p.rr);
+            p.A5 = d_add(1.0, q[3] / p.rr);
+            p.rho2 = d_add(p.rho2, q[4] / r);
+        }
+        const double x = d_add(p.rr, p.aa);
+        p.del = d_sub(x, d_mul(2.0, r));
+        p.ra = d_mul(x, p.A1);
+        return p;
+    }
+    static __device__ __forceinline__ double times(double x, double A) { return A13 ? x : d_mul(x, A); }
+
+    static __device__ __forceinline__ G5 dd(const double* q, double r, double s, double c, bool rlog, bool own) {
+        const double a = q[0];
+        const Parts p = parts(q, r, c);
+        const double a2 = times(p.aa, p.A2);
+        const double den = d_fma(-d_mul(a2, s), s, p.ra), den2 = d_mul(den, den);
+        G5 g;
+        g.tt = -(d_mul(p.rho2, d_fma(-d_mul(times(a2, p.A2), s), s, p.del)) / den2);
+        g.rr = p.rho2 / times(p.del, p.A5);
+        g.hh = p.rho2;
+        const double n = product_difference(p.ra, d_mul(d_mul(p.aa, p.del), s), s, own);
+        g.pp = d_mul(d_mul(d_mul(p.rho2, s), s), n) / den2;
+        const double w = A13 ? d_sub(p.ra, p.del) : d_fma(p.ra, p.A2, -p.del);
+        g.tp = -(d_mul(d_mul(d_mul(d_mul(a, w), p.rho2), s), s) / den2);
+        if (rlog) g.rr = d_mul(g.rr, p.rr);
+        return g;
+    }
+    static __device__ __forceinline__ void uu(const double* q, double r, double s, double c, bool rlog, int i,
+                                              double& g1, double& g2) {
+        const double a = q[0];
+        const Parts p = parts(q, r, c);
+        const double a2 = times(times(p.aa, p.A2), p.A2);
+        const double n = d_fma(d_mul(d_mul(p.aa, p.del), s), s, -d_mul(p.ra, p.ra));
+        const double dr = d_mul(p.del, p.rho2);
+        const double num = (i == 0)   ? n
+                           : (i == 1) ? times(p.del, p.A5)
+                           : (i == 2) ? 1.0
+                                      : d_fma(-d_mul(a2, s), s, p.del);
+        const double den = (i == 0) ? dr : (i == 3) ? d_mul(d_mul(dr, s), s) : p.rho2;
+        g1 = num / den;
+        const double x = d_add(p.rr, p.aa);
+        const double w = d_fma(A13 ? p.A1 : d_mul(p.A2, p.A1), x, -p.del);
+        g2 = -(d_mul(a, w) / dr);
+        if (rlog && i == 1) g1 = d_mul(g1, 1.0 / p.rr);
+    }
+};
+
+template <int MID, bool A13, int INTEG>
+struct SplitEngine {
+    using Metric = SplitMetric<MID, A13>;
+    static constexpr bool kSplit = true;
+    static constexpr bool kCopyImage = false;
+
+    struct Lane {
+        double x, v;  // this lane's component
+        double C[6];  // Verlet: the lane's Christoffel symbols at the position
+        double r;     // radius there
+        double lam;
+        uint64_t steps;
+        TermState T;
+        DiagState D;
+        uint32_t err = 0;
+        uint32_t img = 0;
+        uint32_t rhs = 0;
+        uint32_t fp64 = 0;
+        int32_t term = 0;
+    };
+
+    static __device__ __forceinline__ double from(double a, int lane, unsigned m) { return __shfl_sync(m, a, lane, 4); }
+
+    // The Christoffel symbols that a^i needs: for t and phi Gamma^i_01, _02, _13, _23 in
+    // C[0..3], for r and theta Gamma^i_00, _03, _11, _12, _22, _33 in C[0..5].
+    static __device__ __forceinline__ void symbols(const MetricConst& M, const RunConst& R, double x1, double th, int i,
+                                                   unsigned m, double C[6], double& r0, double* kept = nullptr) {
+        const bool rlog = R.rlog != 0;
+        const double hr = (i == 0) ? R.hfd : (i == 1) ? -R.hfd : 0.0, ht = (i == 2) ? R.hfd : (i == 3) ? -R.hfd : 0.0;
+        double r = (i < 2) ? d_add(x1, hr) : x1, s, c;
+        if (rlog) r = exp(r);
+        sincos((i < 2) ? th : d_add(th, ht), &s, &c);
+        r0 = from(r, 2, m);
+        const double s0 = from(s, 0, m), c0 = from(c, 0, m);
+        const G5 g = Metric::dd(M.q, r, s, c, rlog, i < 2);
+        double g1, g2;
+        Metric::uu(M.q, r0, s0, c0, rlog, i, g1, g2);
+        // central differences: lanes 0 and 1 form those in r, lanes 2 and 3 those in theta
+        const double inv = 1 / (2 * R.hfd);
+        const bool second = i & 1;
+        auto diff = [&](double a) {
+            const double b = __shfl_xor_sync(m, a, 1, 4);
+            return d_mul(d_sub(second ? b : a, second ? a : b), inv);
+        };
+        G5 d = {diff(g.tt), diff(g.tp), diff(g.rr), diff(g.hh), diff(g.pp)};
+        auto other = [&](double a) { return __shfl_xor_sync(m, a, 2, 4); };
+        const G5 o = {other(d.tt), other(d.tp), other(d.rr), other(d.hh), other(d.pp)};
+        const bool low = i < 2;
+        const G5 dr = {low ? d.tt : o.tt, low ? d.tp : o.tp, low ? d.rr : o.rr, low ? d.hh : o.hh, low ? d.pp : o.pp};
+        const G5 dh = {low ? o.tt : d.tt, low ? o.tp : d.tp, low ? o.rr : d.rr, low ? o.hh : d.hh, low ? o.pp : d.pp};
+        const double h1 = d_mul(0.5, g1), h2 = d_mul(0.5, g2);
+        const bool ends = i == 0 || i == 3;
+        // t: 0.5 g^tt d_. g_t. + 0.5 g^tphi d_. g_phi.; phi: 0.5 g^tphi d_. g_t. + 0.5 g^phiphi d_. g_phi.
+        const double ha = (i == 3) ? h2 : h1, hb = (i == 3) ? h1 : h2;
+        const double a0 = ends ? dr.tt : (i == 1) ? -dr.tt : -dh.tt, b0 = ends ? dr.tp : 0.0;
+        const double a1 = ends ? dh.tt : (i == 1) ? -dr.tp : -dh.tp, b1 = ends ? dh.tp : 0.0;
+        const double a2 = ends ? dr.tp : (i == 1) ? dr.rr : -dh.rr, b2 = ends ? dr.pp : 0.0;
+        const double a3 = ends ? dh.tp : (i == 1) ? dh.rr : dr.hh, b3 = ends ? dh.pp : 0.0;
+        const double a4 = (i == 1) ? -dr.hh : dh.hh, a5 = (i == 1) ? -dr.pp : -dh.pp;
+        // The compiler fuses the first product of a sum, but the second in Kerr's Gamma^t_01 and
+        // Gamma^t_02; not so in Verlet's symbols of the position it starts from, kept for it.
+        const bool swap = MID == kKerr && i == 0;
+        C[0] = two(swap ? hb : ha, swap ? b0 : a0, swap ? ha : hb, swap ? a0 : b0);
+        C[1] = two(swap ? hb : ha, swap ? b1 : a1, swap ? ha : hb, swap ? a1 : b1);
+        if (MID == kKerr && kept) {
+            kept[0] = two(ha, a0, hb, b0);
+            kept[1] = two(ha, a1, hb, b1);
+        }
+        C[2] = two(ha, a2, hb, b2);
+        C[3] = two(ha, a3, hb, b3);
+        C[4] = d_mul(ha, a4);
+        C[5] = d_mul(ha, a5);
+    }
+    static __device__ __forceinline__ double two(double a, double x, double b, double y) {
+        return d_fma(a, x, d_mul(b, y));
+    }
+
+    // a^i = -Gamma^i_jk v^j v^k in the reference's order of terms.
+    static __device__ __forceinline__ double accel(const double C[6], const double v[4], int i) {
+        const bool ends = i == 0 || i == 3;
+        const double q0 = ends ? v[1] : v[0], q1 = ends ? v[2] : v[3], q2 = ends ? v[0] : v[1], q3 = ends ? v[3] : v[2];
+        const double q4 = ends ? v[0] : v[1], q5 = ends ? v[3] : v[2], q6 = ends ? v[1] : v[0], q7 = ends ? v[2] : v[3];
+        const double c2 = ends ? C[0] : C[2], c3 = ends ? C[2] : C[3], c4 = ends ? C[1] : C[3];
+        const double c5 = ends ? C[3] : C[4], c6 = ends ? C[2] : C[1], c7 = ends ? C[3] : C[5];
+        const double t0 = d_mul(C[0], v[0]), t1 = d_mul(C[1], v[0]);
+        double acc = -d_fma(t0, q0, d_mul(t1, q1));
+        acc = d_fma(-d_mul(c2, v[1]), q2, acc);
+        acc = d_fma(-d_mul(c3, v[1]), q3, acc);
+        acc = d_fma(-d_mul(c4, v[2]), q4, acc);
+        acc = d_fma(-d_mul(c5, v[2]), q5, acc);
+        acc = d_fma(-d_mul(c6, v[3]), q6, acc);
+        return d_fma(-d_mul(c7, v[3]), q7, acc);
+    }
+    static __device__ __forceinline__ void gather(double a, unsigned m, double v[4]) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) v[k] = from(a, k, m);
+    }
+
+    // Integrators::GetAdaptiveStep (Integrators.cpp:34-46): lanes 1 to 3 each divide for
+    // their component (lane 0 follows lane 1).
+    static __device__ __forceinline__ double adaptive_step(const RunConst& R, const Lane& L, int i, unsigned m) {
+        const double pt = d_sub(kRefPi, L.x), mth = (pt < L.x) ? pt : L.x;
+        const double num = (i == 2) ? d_mul(R.eps, mth) : R.eps;
+        const double den = fabs(d_add((i == 3) ? L.v : fabs(L.v), 1e-20));
+        const double w = 1 / fabs(num / den);
+        const double h = 1 / d_add(d_add(from(w, 1, m), from(w, 2, m)), from(w, 3, m));
+        return (h < R.hmin) ? R.hmin : h;
+    }
+
+    static __device__ __forceinline__ void init(Lane& L, const ImageConst& I, const RunConst& R, const foort_pixel& p,
+                                                int i, unsigned m) {
+        double x[4], v[4];
+        initial_conditions(I, p, x, v);
+        L.x = (i == 0) ? x[0] : (i == 1) ? x[1] : (i == 2) ? x[2] : x[3];
+        L.v = (i == 0) ? v[0] : (i == 1) ? v[1] : (i == 2) ? v[2] : v[3];
+        if (INTEG == FOORT_INTEGRATOR_VERLET) symbols(I.m, R, x[1], x[2], i, m, L.C, L.r, L.C);
+        L.lam = 0.0;
+        L.steps = 0;
+        L.err = 0;
+        L.term = FOORT_TERMCODE_CONTINUE;
+        L.img = p.image;
+        reset_lane_state(R, x, L.D, L.T);
+    }
+
+    // One Geodesic::Update (Geodesic.cpp:61-88); i: this lane's component, m: the four lanes.
+    static __device__ __forceinline__ bool step_split(Lane& L, const ImageConst& I, const RunConst& R, int i, unsigned m) {
+        const MetricConst& M = I.m;
+        const double h = adaptive_step(R, L, i, m);
+        double va[4], nx, nv, r;
+        gather(L.v, m, va);
+        if (INTEG == FOORT_INTEGRATOR_RK4) {  // Integrators.cpp:51-94
+            const double hh = 0.5 * h, h6 = h / 6.0;
+            double C[6], l[4], k1, k2, k3, k4, l2, l3, l4, t;
+            symbols(M, R, from(L.x, 1, m), from(L.x, 2, m), i, m, C, r);
+            k1 = accel(C, va, i);
+            t = d_fma(L.v, hh, L.x);
+            l2 = d_fma(k1, hh, L.v);
+            gather(l2, m, l);
+            symbols(M, R, from(t, 1, m), from(t, 2, m), i, m, C, r);
+            k2 = accel(C, l, i);
+            t = d_fma(l2, hh, L.x);
+            l3 = d_fma(k2, hh, L.v);
+            gather(l3, m, l);
+            symbols(M, R, from(t, 1, m), from(t, 2, m), i, m, C, r);
+            k3 = accel(C, l, i);
+            t = d_fma(l3, h, L.x);
+            l4 = d_fma(k3, h, L.v);
+            gather(l4, m, l);
+            symbols(M, R, from(t, 1, m), from(t, 2, m), i, m, C, r);
+            k4 = accel(C, l, i);
+            nv = d_fma(d_add(d_fma(k3, 2.0, d_fma(k2, 2.0, k1)), k4), h6, L.v);
+            nx = d_fma(d_add(d_fma(l3, 2.0, d_fma(l2, 2.0, L.v)), l4), h6, L.x);
+            L.rhs += (i == 0) ? 4 : 0;
+        } else {  // Integrators.cpp:99-152
+            const double a0 = accel(L.C, va, i), hh2 = h * h / 2.0, h2 = h / 2.0;
+            double C[6], via[4], nva[4];
+            nx = d_fma(a0, hh2, d_fma(L.v, h, L.x));
+            const double vi = d_fma(a0, h, L.v);
+            gather(vi, m, via);
+            symbols(M, R, from(nx, 1, m), from(nx, 2, m), i, m, C, r, L.C);
+#pragma unroll
+            for (int k = (MID == kKerr) ? 2 : 0; k < 6; ++k) L.C[k] = C[k];
+            double a1 = accel(C, via, i);
+            nv = d_fma(d_add(a0, a1), h2, L.v);
+            L.rhs += (i == 0) ? 2 : 0;
+            if (R.vtol > 0.0) {
+                const double tol2 = R.vtol * R.vtol;
+                for (int it = 0;; ++it) {
+                    gather(nv, m, nva);
+                    double num = 0.0, den = 0.0;
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const double d = d_sub(nva[k], via[k]);
+                        num = k ? d_fma(d, d, num) : d_mul(d, d);
+                        den = k ? d_fma(nva[k], nva[k], den) : d_mul(nva[k], nva[k]);
+                    }
+                    if (!(num / den > tol2)) break;
+                    if (it >= R.verlet_cap) {
+                        L.err |= FOORT_ERR_VERLET_ITER;
+                        break;
+                    }
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) via[k] = nva[k];
+                    a1 = accel(C, via, i);
+                    nv = d_fma(d_add(a0, a1), h2, L.v);
+                    L.rhs += (i == 0) ? 1 : 0;
+                }
+            }
+        }
+        L.lam += h;
+        L.x = nx;
+        L.v = nv;
+        ++L.steps;
+        const double x1 = from(nx, 1, m), th = from(nx, 2, m), ph = from(nx, 3, m);
+        if (INTEG == FOORT_INTEGRATOR_RK4) r = radius_of(R, x1);  // Verlet's symbols have it
+        L.term = check_terms(R, M.rh, I.h_eps, r, th, L.T);
+        update_diags(R, r, th, ph, L.lam, L.term, L.D);
+        const bool bad = (__ballot_sync(m, !(isfinite(nx) && isfinite(nv))) & m) != 0;
+        if (bad) {
+            L.err |= FOORT_ERR_NONFINITE;
+            if (L.term == FOORT_TERMCODE_CONTINUE && !(R.term_flags & FOORT_TERM_TIMEOUT)) return false;
+        }
+        return L.term == FOORT_TERMCODE_CONTINUE;
+    }
+
+    // Every lane writes its component, lane 0 the rest of the record.
+    static __device__ __forceinline__ void write(const Lane& L, foort_result* o, int term, uint32_t err, int i) {
+        o->pos[i] = L.x;
+        o->vel[i] = L.v;
+        if (i) return;
+        o->term = term;
+        o->err = err;
+        o->steps = L.steps;
+        o->lambda = L.lam;
+        o->quadrant = L.D.quad;
+        o->equat_passes = L.D.passes;
+        o->closest_r = L.D.rmin;
+    }
+    static __device__ __forceinline__ void finish(const Lane& L, const RunConst&, foort_result* o, int i) {
+        write(L, o, L.term, L.err, i);
+    }
+    static __device__ __forceinline__ void stop(const Lane& L, const RunConst&, foort_result* o, uint32_t err, int i) {
+        write(L, o, FOORT_TERMCODE_CONTINUE, L.err | err, i);
+    }
+};
+
+template <int MID, bool A13, int INTEG>
+__global__ void __launch_bounds__(128) integrate_fp64_split_kernel(const __grid_constant__ LaunchArgs A,
+                                                                   const __grid_constant__ RunConst R) {
+    persistent_loop<SplitEngine<MID, A13, INTEG>, 4>(A, R);
+}
+
+}  // namespace foort

@@ -193,7 +193,7 @@ typedef struct foort_stats {
     uint32_t status;         /* FOORT_OK or the launch's FOORT_E_* code             */
     uint32_t n_blocks;
     uint32_t block_size;
-    uint32_t lanes_per_geodesic; /* 1, or 2 where two lanes integrated each geodesic   */
+    uint32_t lanes_per_geodesic; /* 1, or 2 where two lanes (or more) share a geodesic */
     uint32_t refill_steps;   /* the launch's regrouping cadence (foort_launch_shape)   */
     uint32_t poll_steps;     /* its steps between budget / cancel polls               */
 } foort_stats;
@@ -286,12 +286,12 @@ int foort_gpu_cancel(foort_ctx* ctx);
  * built-in rule (128 threads, as many CTAs as fit) where the cache has none. */
 int foort_gpu_set_launch(foort_ctx* ctx, uint32_t block_size, uint32_t blocks_per_sm);
 
-/* Lanes per geodesic in mixed precision with RK4 and the Kerr or flat metric: 0 chooses
- * per launch (two lanes when the launch's geodesics, at two lanes each, fit on the GPU's
- * resident lanes: a step's latency then sets the pace, and two lanes halve the metric
- * work on it), 1 or 2 force the choice; other configurations always use one. Results
- * are the same either way. No counterpart in the reference (one OpenMP thread per
- * geodesic, Main.cpp:327-414). */
+/* Lanes per geodesic: 0 chooses per launch, 1 one lane, 2 several (two or four) where such
+ * a kernel exists: RK4 except Manko-Novikov's, Kerr's and Johannsen's FP64 Verlet; other
+ * configurations always use one. Small launches take several: a step's latency then sets
+ * the pace, and lanes that share a step's metric work shorten it. Results are the same
+ * either way. No counterpart in the reference (one OpenMP thread per geodesic,
+ * Main.cpp:327-414). */
 int foort_gpu_set_lanes(foort_ctx* ctx, uint32_t lanes_per_geodesic);
 
 /* ---- launch shapes and the autotuner --------------------------------------------------
@@ -305,7 +305,7 @@ int foort_gpu_set_lanes(foort_ctx* ctx, uint32_t lanes_per_geodesic);
 typedef struct foort_launch_shape {
     uint32_t block_size;    /* threads per CTA: 32, 64, 96 or 128                      */
     uint32_t blocks_per_sm; /* cap on resident CTAs per SM (0 = as many as fit)        */
-    uint32_t lanes;         /* lanes per geodesic: 1, or 2 where the kernel has two    */
+    uint32_t lanes;         /* lanes per geodesic: 1, or 2 where the kernel has several */
     uint32_t refill_steps;  /* >= 1: steps a warp runs between refills of idle lanes   */
     uint32_t poll_steps;    /* >= 1: steps between budget / cancel polls               */
     uint32_t reserved;

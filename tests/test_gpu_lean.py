@@ -181,3 +181,66 @@ def test_packed_bodies_match_the_generator():
     out = subprocess.run([sys.executable, gen], check=True, capture_output=True, text=True).stdout
     with open(os.path.join(ROOT, "foort_gb300", "csrc", "gen_packed.inc")) as f:
         assert f.read() == out
+
+
+def several_lanes_and_one(eng, d, px, **run):
+    got = {}
+    for lanes in (1, 2):
+        with eng.Engine(d) as e:
+            e.set_lanes(lanes)
+            got[lanes] = e.integrate(px, **run)
+            got[lanes, "counts"] = {k: e.stats()[k] for k in ("steps", "rhs_evals", "fp64_steps", "geodesics")}
+    return got
+
+
+# both integrators, no velocity iterations and many, radii to the horizon and through the
+# theta singularity, rays that end after one step, pixel counts that leave a warp part-filled
+@pytest.mark.gpu
+@pytest.mark.parametrize("metric,params,rlog,inclination,side,timeout,integrator,tolerance", [
+    (abi.METRIC_KERR, (0.998,), 1, 17.0, 33, None, abi.INTEGRATOR_VERLET, 1e-5),
+    (abi.METRIC_KERR, (0.0,), 1, 90.0, 9, None, abi.INTEGRATOR_VERLET, -1.0),
+    (abi.METRIC_KERR, (0.7,), 0, 63.0, 3, 3000, abi.INTEGRATOR_VERLET, 0.001),
+    (abi.METRIC_KERR, (0.9,), 1, 2.0, 31, None, abi.INTEGRATOR_RK4, 0.001),
+    (abi.METRIC_JOHANNSEN, (0.8, 1.0, 0.5, 0.2, 0.1), 1, 63.0, 33, None, abi.INTEGRATOR_VERLET, 1e-5),
+    (abi.METRIC_JOHANNSEN, (0.7, 2.0, 0.0, 0.0, 0.0), 1, 90.0, 33, None, abi.INTEGRATOR_VERLET, -1.0),
+    (abi.METRIC_JOHANNSEN, (0.3, -0.9, 0.0, 0.0, 0.0), 1, 2.0, 17, None, abi.INTEGRATOR_RK4, 0.001),
+    (abi.METRIC_JOHANNSEN, (0.9, 0.4, 0.0, 0.0, 0.0), 0, 30.0, 2, 3000, abi.INTEGRATOR_RK4, 0.001),
+    (abi.METRIC_JOHANNSEN, (0.9, 0.4, 0.0, 0.0, 0.0), 1, 30.0, 2, 0, abi.INTEGRATOR_VERLET, 0.001),
+])
+def test_four_lanes_in_fp64_give_the_one_lane_results(eng, metric, params, rlog, inclination, side, timeout, integrator,
+                                                      tolerance):
+    """The FP64 kernels that share a step between four lanes write each rounding out as the
+    one-lane kernel has it: the same records bit for bit, and the same counts."""
+    d, keep = describe(metric, params, rlog, inclination, integrator=integrator, timeout=timeout)
+    d.precision, d.verlet_tol = abi.PREC_FP64, tolerance
+    got = several_lanes_and_one(eng, d, abi.square_pixels(side))
+    same_records(got[2], got[1])
+    assert got[2, "counts"] == got[1, "counts"]
+    del keep
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("metric,integrator", [(abi.METRIC_KERR, abi.INTEGRATOR_RK4),
+                                               (abi.METRIC_JOHANNSEN, abi.INTEGRATOR_VERLET)])
+def test_fp64_lanes_are_refilled_and_run_two_images(eng, metric, integrator):
+    """More pixels than the four-lane kernels hold at a time, two images side by side:
+    one lane, several lanes and the built-in choice give the same records, also where a
+    step budget ends some of them."""
+    d, _ = describe(metric, (0.9,), 1, 70.0, integrator=integrator, timeout=600)
+    d.precision = abi.PREC_FP64
+    pars = [(a,) if metric == abi.METRIC_KERR else (a, 0.5, 0.0, 0.0, 0.0) for a in (0.9, 0.2)]
+    keep = abi.attach_images(d, [abi.make_image(p, r=1000.0, theta=1.2, half_width=8.0) for p in pars])
+    px = np.concatenate([abi.square_pixels(100, image=i) for i in (0, 1)])
+    px = px[np.random.default_rng(5).permutation(len(px))]
+    got = several_lanes_and_one(eng, d, px)
+    same_records(got[2], got[1])
+    assert got[2, "counts"] == got[1, "counts"]
+    with eng.Engine(d) as e:
+        same_records(e.integrate(px), got[1])
+        e.set_lanes(2)
+        e.set_budget(50000)
+        part = e.integrate(px, allow=(abi.FOORT_E_BUDGET,))
+    stopped = (part["err"] & (abi.ERR_BUDGET | abi.ERR_UNFINISHED)) != 0
+    assert stopped.any() and np.all(part["term"][stopped] == abi.TERMCODE_CONTINUE)
+    same_records(part[~stopped], got[1][~stopped])
+    del keep
