@@ -237,15 +237,9 @@ const void* select_pair_kernel(const RunConst& R, bool positions) {
     return mixed_pair_kernel_variant(R.metric_id, R.integrator, (R.mixed_options & FOORT_MIXED_FP64_DECISIONS) != 0);
 }
 
-// The four-lanes-per-geodesic kernel, or nullptr. It records no positions.
-const void* select_split_kernel(const RunConst& R, bool positions) {
-    return (R.precision == FOORT_PREC_FP64 && !positions) ? fp64_split_kernel(R) : nullptr;
-}
-
 struct LaunchShape {
     const void* fn = nullptr;
-    uint32_t grid = 0, block = 0, lanes = 1;  // lanes: 2 stands for several, as in foort_launch_shape
-    uint32_t refill = 1, poll = kDefaultPollSteps;
+    uint32_t grid = 0, block = 0, lanes = 1, refill = 1, poll = kDefaultPollSteps;
 };
 
 // Geodesics up to which a launch takes two lanes each, where that kernel exists and the
@@ -282,18 +276,24 @@ uint64_t pair_limit(const RunConst& R, bool positions, int per_sm, int num_sms, 
     return static_cast<uint64_t>(per_sm) * sms * bs / 2;
 }
 
-// Geodesics up to which an FP64 launch takes four lanes each (Kerr, Johannsen). Four lanes
-// finish a step soonest, but cost 1.5 times the instructions of one lane and 1.4 times those
-// of two per geodesic, so they pay while few geodesics share a scheduler. Log r, ms:
-//              Kerr RK4 (4 / 2 / 1 lanes)    Johannsen RK4        Kerr Verlet   Johannsen Verlet
-//     3,721       34 /  47 /  82              49 /  61 / 110       25 / 55        43 /  95
-//    10,000       65 /  71 / 113              90 /  88 / 147       23 / 39        28 /  46
-//    40,000      153 / 125 / 164             209 / 144 / 194       55 / 58        69 /  75
-//    62,500      234 / 175 / 207             321 / 216 / 273       85 / 66       106 /  74
-// The limit is where the next width is as fast.
-uint64_t split_limit(const RunConst& R, int num_sms) {
+// Lanes per geodesic that an FP64 launch of Kerr or Johannsen starts with in the kernels that
+// end on four lanes per geodesic (kernel_fp64_split.cuh): 4, 2 (RK4) or 1; 0: the plain
+// one-lane kernel, unless several lanes are forced. Four lanes finish a step soonest, but cost
+// 1.5 times the instructions of one lane and 1.4 times those of two per geodesic. Log r, ms
+// (starting with 4 / 2 / 1 lanes; the plain kernel on 2 / 1 lanes):
+//                Kerr RK4                      Johannsen RK4                  Verlet (4 / 1; 1): Kerr, Johannsen
+//     3,600       36 /  42 /  56;  50 /  83     57 /  62 /  81;  71 / 122     14 / 21; 30     16 / 24; 35
+//    10,000       67 /  63 /  92;  72 / 114     91 /  78 / 124;  90 / 149     24 / 33; 39     29 / 41; 47
+//    25,600      103 /  87 / 103;  99 / 124    139 / 113 / 134; 122 / 163     38 / 38; 46     46 / 45; 53
+//    62,500      238 / 174 / 173; 179 / 214    323 / 210 / 218; 212 / 263     88 / 57; 64    108 / 67; 74
+//   250,000      931 / 658 / 600; 658 / 597   1264 / 804 / 815; 803 / 803    344 / 202; 203  424 / 243; 244
+// Past some ten refills of every lane a launch's end is a small part of it.
+int split_start(const RunConst& R, uint64_t n, int num_sms, bool forced) {
     const uint64_t sms = static_cast<uint64_t>(num_sms);
-    return (R.integrator == FOORT_INTEGRATOR_RK4 ? (R.metric_id == kKerr ? 96 : 64) : 256) * sms;
+    const bool rk4 = R.integrator == FOORT_INTEGRATOR_RK4;
+    if (n <= (rk4 ? 64 : 160) * sms) return 4;
+    if (rk4 && n <= 384 * sms) return 2;
+    return (forced || n <= 1024 * sms) ? 1 : 0;
 }
 
 // Kernel and grid of a launch of n geodesics in the requested shape (zero fields: the
@@ -316,33 +316,35 @@ int choose_launch(foort_ctx* ctx, const RunConst& R, uint64_t n, int num_sms, co
     const void* fn = select_kernel(R, positions);
     if (!fn) return fail(ctx, FOORT_E_UNSUPPORTED, "no kernel for this metric / integrator / precision");
     int per_sm = 0, rc = 0;
-    uint32_t lanes = 1;
-    const void* split = (want.lanes != 1) ? select_split_kernel(R, positions) : nullptr;
-    const void* fn2 = (want.lanes != 1) ? select_pair_kernel(R, positions) : nullptr;
-    if (split && (n <= split_limit(R, num_sms) || (want.lanes == 2 && !fn2))) {
-        if ((rc = resident(split, per_sm))) return rc;
-        if (per_sm > 0) {
-            fn = split;
-            lanes = 4;
-        }
-    }
-    if (lanes == 1 && fn2) {
+    uint32_t lanes = 1;    // 2 stands for several, as in foort_launch_shape
+    uint32_t threads = 1;  // per geodesic of a launch that does not fill the GPU
+    const int start = (R.precision == FOORT_PREC_FP64 && !positions && want.lanes != 1)
+                          ? split_start(R, n, num_sms, want.lanes == 2)
+                          : 0;
+    const void* split = start ? fp64_split_kernel(R, start) : nullptr;
+    const void* pair = (split || want.lanes == 1) ? nullptr : select_pair_kernel(R, positions);
+    if (split) {
+        fn = split;
+        lanes = 2;
+        threads = 4;  // no more than eight geodesics per warp while that spreads them wider
+        if ((rc = resident(fn, per_sm))) return rc;
+    } else if (pair) {
         int per_sm2 = 0;
-        if ((rc = resident(fn2, per_sm2))) return rc;
+        if ((rc = resident(pair, per_sm2))) return rc;
         if (per_sm2 > 0 && (want.lanes == 2 || n <= pair_limit(R, positions, per_sm2, num_sms, bs))) {
-            fn = fn2;
+            fn = pair;
             per_sm = per_sm2;
-            lanes = 2;
+            lanes = threads = 2;
         }
     }
     if (lanes == 1 && (rc = resident(fn, per_sm))) return rc;
     if (per_sm <= 0) return fail(ctx, FOORT_E_CUDA, "kernel does not fit on an SM with this block size");
     const uint64_t full = static_cast<uint64_t>(per_sm) * static_cast<uint64_t>(num_sms);
-    const uint64_t need = (lanes * n + bs - 1) / bs;
+    const uint64_t need = (threads * n + bs - 1) / bs;
     out.fn = fn;
     out.grid = static_cast<uint32_t>(std::max<uint64_t>(1, std::min(full, need)));
     out.block = bs;
-    out.lanes = std::min(lanes, 2u);
+    out.lanes = lanes;
     out.refill = want.refill_steps ? want.refill_steps : 1;
     out.poll = want.poll_steps ? want.poll_steps : kDefaultPollSteps;
     return FOORT_OK;
@@ -485,7 +487,8 @@ int autotune_launch(foort_ctx* ctx, const foort_pixel* d_px, uint64_t n, foort_r
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, probe.fn, 128, 0));
     const uint64_t resident = static_cast<uint64_t>(std::max(per_sm, 1)) * ctx->num_sms * 128;
     const uint64_t m = std::min<uint64_t>(n, FOORT_TUNE_SAMPLE_LANES_X * resident);
-    const bool has_pair = select_pair_kernel(ctx->rc, false) || select_split_kernel(ctx->rc, false);
+    const bool has_pair = select_pair_kernel(ctx->rc, false) ||
+                          (ctx->rc.precision == FOORT_PREC_FP64 && fp64_split_kernel(ctx->rc, 1));
     std::vector<foort_launch_shape> tried;
     auto time_shape = [&](foort_launch_shape s, double& ms) -> int {
         int r = launch(ctx, d_px, m, d_out, st, nullptr, &s);
@@ -965,14 +968,14 @@ const void* fp64_pair_kernel_flat();
 const void* fp64_pair_kernel_rl();
 const void* fp64_pair_kernel_joh();
 
-const void* fp64_split_kernel_kerr(int);
-const void* fp64_split_kernel_joh(int, bool);
+const void* fp64_split_kernel_kerr(int, int);
+const void* fp64_split_kernel_joh(int, bool, int);
 
-// Four lanes per geodesic.
-const void* fp64_split_kernel(const RunConst& R) {
+// Four lanes per geodesic in the end: from a start with 4, 2 (RK4 only) or 1.
+const void* fp64_split_kernel(const RunConst& R, int start) {
     switch (R.metric_id) {
-    case kKerr: return fp64_split_kernel_kerr(R.integrator);
-    case kJohannsen: return fp64_split_kernel_joh(R.integrator, R.only_alpha13 != 0);
+    case kKerr: return fp64_split_kernel_kerr(R.integrator, start);
+    case kJohannsen: return fp64_split_kernel_joh(R.integrator, R.only_alpha13 != 0, start);
     default: return nullptr;
     }
 }

@@ -296,8 +296,15 @@ constexpr bool is_fp64_steps(decltype(E::kFp64Steps)*) {
     return true;
 }
 
-template <class E, int LANES = 1>
-__device__ __forceinline__ void persistent_loop(const LaunchArgs& A, const RunConst& R) {
+// TAIL: once the queue is empty and a warp has at most 8 geodesics left, it hands them to
+// Tail, four lanes each (Tail::take_over).
+struct NoTail {
+    static constexpr bool kIs = false;
+};
+
+template <class E, int LANES, class Tail>
+__device__ __forceinline__ void work_loop(const LaunchArgs& A, const RunConst& R, typename E::Lane& L, bool active,
+                                          uint64_t idx, bool drained) {
     static_assert(LANES == 1 || LANES == 2 || LANES == 4, "lanes per geodesic");
     constexpr bool PAIR = LANES == 2, SPLIT = LANES == 4;
     const unsigned lane = threadIdx.x & 31u;
@@ -308,13 +315,18 @@ __device__ __forceinline__ void persistent_loop(const LaunchArgs& A, const RunCo
     const unsigned slots = SPLIT ? 0x11111111u : PAIR ? 0x55555555u : kFullMask;  // one bit per geodesic slot
     const unsigned pmask = ((1u << LANES) - 1u) << slot_lane;
     constexpr bool kLean = is_lean<E>(nullptr);
-    typename E::Lane L;
+    constexpr bool kTail = Tail::kIs;
+    // With a tail: geodesics per warp at a time, an even share of a launch that does not fill
+    // the lanes (but the tail's 8 at least).
+    unsigned share = 32 / LANES;
+    if constexpr (kTail) {
+        const uint64_t warps = static_cast<uint64_t>(gridDim.x) * (blockDim.x >> 5);
+        const uint64_t even = (A.n + warps - 1) / warps;
+        share = (even < 8) ? 8 : (even < share) ? static_cast<unsigned>(even) : share;
+    }
     ImageConst Ic;  // PAIR, E::kCopyImage: the lane's image constants in registers, copied at each refill
-    bool active = false;
-    bool drained = false;
     bool stopping = false;
     uint32_t stop_err = 0;
-    uint64_t idx = 0;
     unsigned lane_steps = 0, lane_done = 0;
     int since_poll = 0, since_refill = 0;
     // The warp's right-hand sides and FP64 steps since the last count: the lanes' counters,
@@ -341,14 +353,16 @@ __device__ __forceinline__ void persistent_loop(const LaunchArgs& A, const RunCo
             const unsigned need = __ballot_sync(kFullMask, !active) & slots;
             if (need) {
                 const int leader = __ffs(need) - 1;
-                const unsigned cnt = __popc(need);
+                unsigned cnt = __popc(need);
+                if constexpr (kTail) cnt = min(cnt, share - __popc(slots & ~need));
                 unsigned long long base = 0;
                 if (lane == static_cast<unsigned>(leader)) base = atomicAdd(&A.ctr[kCtrHead], (unsigned long long)cnt);
                 base = __shfl_sync(kFullMask, base, leader);
                 if (base + cnt >= A.n) drained = true;
                 if (!active) {
-                    const uint64_t my = base + __popc(need & lt_mask);
-                    if (my < A.n) {
+                    const unsigned rank = __popc(need & lt_mask);
+                    const uint64_t my = base + rank;
+                    if (my < A.n && (!kTail || rank < cnt)) {
                         const foort_pixel p = A.px[my];
                         if (stopping) {
                             if (!odd) write_unstarted(&A.out[my], stop_err);
@@ -376,6 +390,9 @@ __device__ __forceinline__ void persistent_loop(const LaunchArgs& A, const RunCo
         if (!__any_sync(kFullMask, active)) {
             if (drained) break;
             continue;
+        }
+        if constexpr (kTail) {
+            if (drained && __popc(__ballot_sync(kFullMask, active) & slots) <= 8) break;
         }
         // Integrate until a lane needs new work (while work remains) or a poll is due.
         for (;;) {
@@ -410,6 +427,11 @@ __device__ __forceinline__ void persistent_loop(const LaunchArgs& A, const RunCo
             if (since_poll >= R.poll_steps) break;
             const unsigned idle = __ballot_sync(kFullMask, !active);
             if (idle == kFullMask) break;
+            if constexpr (kTail) {
+                const unsigned left = __popc(~idle & slots);
+                if (drained ? left <= 8 : left < share && since_refill >= R.refill_steps) break;
+                continue;
+            }
             if (idle && !drained && since_refill >= R.refill_steps) break;
         }
         if (since_poll >= R.poll_steps || drained) {
@@ -457,6 +479,16 @@ __device__ __forceinline__ void persistent_loop(const LaunchArgs& A, const RunCo
         if (wf) atomicAdd(&A.ctr[kCtrFp64Steps], wf);
         if (wd) atomicAdd(&A.ctr[kCtrDone], wd);
     }
+    if constexpr (kTail) {
+        const unsigned left = __ballot_sync(kFullMask, active) & slots;
+        if (left) Tail::run(A, R, L, left, idx);
+    }
+}
+
+template <class E, int LANES = 1, class Tail = NoTail>
+__device__ __forceinline__ void persistent_loop(const LaunchArgs& A, const RunConst& R) {
+    typename E::Lane L;
+    work_loop<E, LANES, Tail>(A, R, L, false, 0, false);
 }
 
 }  // namespace foort

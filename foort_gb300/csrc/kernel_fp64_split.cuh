@@ -1,4 +1,5 @@
-// The plain FP64 kernel on four lanes per geodesic (Kerr, Johannsen).
+// The plain FP64 kernel on four lanes per geodesic (Kerr, Johannsen), throughout or for the
+// last eight geodesics of each warp.
 //
 // An FP64 instruction occupies its scheduler's pipe for 64 cycles per warp on GB300, however
 // many lanes are active: a launch that leaves lanes idle costs the instructions of one
@@ -16,7 +17,7 @@
 // compiler contracts Fp64Engine (kernel_fp64.cuh; found by comparing evaluations).
 #pragma once
 
-#include "kernel_common.cuh"
+#include "kernel_fp64.cuh"
 
 namespace foort {
 
@@ -138,7 +139,6 @@ struct SplitEngine {
     struct Lane {
         double x, v;  // this lane's component
         double C[6];  // Verlet: the lane's Christoffel symbols at the position
-        double r;     // radius there
         double lam;
         uint64_t steps;
         TermState T;
@@ -179,6 +179,10 @@ struct SplitEngine {
         const bool low = i < 2;
         const G5 dr = {low ? d.tt : o.tt, low ? d.tp : o.tp, low ? d.rr : o.rr, low ? d.hh : o.hh, low ? d.pp : o.pp};
         const G5 dh = {low ? o.tt : d.tt, low ? o.tp : d.tp, low ? o.rr : d.rr, low ? o.hh : d.hh, low ? o.pp : d.pp};
+        christoffel(dr, dh, g1, g2, i, C, kept);
+    }
+    static __device__ __forceinline__ void christoffel(const G5& dr, const G5& dh, double g1, double g2, int i,
+                                                       double C[6], double* kept) {
         const double h1 = d_mul(0.5, g1), h2 = d_mul(0.5, g2);
         const bool ends = i == 0 || i == 3;
         // t: 0.5 g^tt d_. g_t. + 0.5 g^tphi d_. g_phi.; phi: 0.5 g^tphi d_. g_t. + 0.5 g^phiphi d_. g_phi.
@@ -244,7 +248,10 @@ struct SplitEngine {
         initial_conditions(I, p, x, v);
         L.x = (i == 0) ? x[0] : (i == 1) ? x[1] : (i == 2) ? x[2] : x[3];
         L.v = (i == 0) ? v[0] : (i == 1) ? v[1] : (i == 2) ? v[2] : v[3];
-        if (INTEG == FOORT_INTEGRATOR_VERLET) symbols(I.m, R, x[1], x[2], i, m, L.C, L.r, L.C);
+        if (INTEG == FOORT_INTEGRATOR_VERLET) {
+            double r;
+            symbols(I.m, R, x[1], x[2], i, m, L.C, r, L.C);
+        }
         L.lam = 0.0;
         L.steps = 0;
         L.err = 0;
@@ -355,10 +362,81 @@ struct SplitEngine {
     }
 };
 
+// The tail of a launch of Fp64Engine (one or two lanes per geodesic): at most 8 geodesics of
+// a warp continue on four lanes each, from the state between two steps. A warp's step takes
+// the same time with one geodesic left as with all its lanes busy, and the longest rays end a
+// launch alone: 62,500 Johannsen rays in FP64 Verlet 122 ms on one lane throughout, 111 on
+// four, 98 on one and then four; 10,000 Kerr rays in RK4 72 on two lanes, 67 on four, 63 on
+// two and then four.
 template <int MID, bool A13, int INTEG>
+struct SplitTail {
+    using S = SplitEngine<MID, A13, INTEG>;
+    static constexpr bool kIs = true;
+
+    template <class T>
+    static __device__ __forceinline__ T from(const T& a, int lane) {
+        static_assert(sizeof(T) % 4 == 0, "whole words");
+        T b;
+        uint32_t w[sizeof(T) / 4];
+        memcpy(w, &a, sizeof(T));
+#pragma unroll
+        for (unsigned k = 0; k < sizeof(T) / 4; ++k) w[k] = __shfl_sync(kFullMask, w[k], lane);
+        memcpy(&b, w, sizeof(T));
+        return b;
+    }
+    static __device__ __forceinline__ double component(const double a[4], int i, int lane) {
+        const double a0 = from(a[0], lane), a1 = from(a[1], lane), a2 = from(a[2], lane), a3 = from(a[3], lane);
+        return (i == 0) ? a0 : (i == 1) ? a1 : (i == 2) ? a2 : a3;
+    }
+
+    // left: the lanes that hold the geodesics; every lane of the warp calls it.
+    static __device__ __forceinline__ void run(const LaunchArgs& A, const RunConst& R,
+                                               const typename Fp64Engine<MID, INTEG>::Lane& L, unsigned left,
+                                               uint64_t idx) {
+        const int lane = threadIdx.x & 31, i = lane & 3, group = lane >> 2;
+        unsigned rest = left;
+        for (int k = 0; k < group; ++k) rest &= rest - 1;  // drops the groups before this one
+        const bool active = rest != 0;
+        const int src = active ? __ffs(rest) - 1 : __ffs(left) - 1;
+        typename S::Lane T;
+        T.x = component(L.x, i, src);
+        T.v = component(L.v, i, src);
+        T.lam = from(L.lam, src);
+        T.steps = from(L.steps, src);
+        T.T = from(L.T, src);
+        T.D = from(L.D, src);
+        T.err = from(L.err, src);
+        T.img = from(L.img, src);
+        T.term = from(L.term, src);
+        if (INTEG == FOORT_INTEGRATOR_VERLET) {
+            const G5 dr = from(L.P.dr, src), dh = from(L.P.dh, src), gu = from(L.P.gu, src);
+            const double g1 = (i == 0) ? gu.tt : (i == 1) ? gu.rr : (i == 2) ? gu.hh : gu.pp;
+            S::christoffel(dr, dh, g1, gu.tp, i, T.C, T.C);
+        }
+        work_loop<S, 4, NoTail>(A, R, T, active, from(idx, src), true);
+    }
+};
+
+// START: lanes per geodesic until a warp has eight geodesics left.
+template <int MID, bool A13, int INTEG, int START>
 __global__ void __launch_bounds__(128) integrate_fp64_split_kernel(const __grid_constant__ LaunchArgs A,
                                                                    const __grid_constant__ RunConst R) {
-    persistent_loop<SplitEngine<MID, A13, INTEG>, 4>(A, R);
+    if constexpr (START == 4) {
+        persistent_loop<SplitEngine<MID, A13, INTEG>, 4>(A, R);
+    } else {
+        persistent_loop<Fp64Engine<MID, INTEG>, START, SplitTail<MID, A13, INTEG>>(A, R);
+    }
+}
+
+template <int MID, bool A13>
+const void* split_kernel(int integrator, int start) {
+    constexpr int kRk4 = FOORT_INTEGRATOR_RK4, kVerlet = FOORT_INTEGRATOR_VERLET;
+    const void* rk4[] = {reinterpret_cast<const void*>(&integrate_fp64_split_kernel<MID, A13, kRk4, 1>),
+                         reinterpret_cast<const void*>(&integrate_fp64_split_kernel<MID, A13, kRk4, 2>),
+                         reinterpret_cast<const void*>(&integrate_fp64_split_kernel<MID, A13, kRk4, 4>)};
+    const void* verlet[] = {reinterpret_cast<const void*>(&integrate_fp64_split_kernel<MID, A13, kVerlet, 1>), nullptr,
+                            reinterpret_cast<const void*>(&integrate_fp64_split_kernel<MID, A13, kVerlet, 4>)};
+    return (integrator == FOORT_INTEGRATOR_RK4 ? rk4 : verlet)[start / 2];
 }
 
 }  // namespace foort
