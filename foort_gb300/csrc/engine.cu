@@ -219,8 +219,21 @@ RunConst make_run_const(const foort_run_desc& d) {
 // (the latter takes every step in FP64).
 bool analytic_family(int precision) { return precision == FOORT_PREC_MIXED || precision == FOORT_PREC_FP64_ANALYTIC; }
 
+// The analytic-derivative kernels record positions in high and low FP32 parts; this brings
+// them to FP64 in place, values never written (all bits set) apart. A recording lane would
+// take the conversion's twelve FP64 instructions alone in its warp: 3,600 rays with 25
+// positions each 1.41 ms recorded in FP64, 1.25 in parts and this kernel.
+__global__ void expand_positions(double* x, uint64_t n) {
+    const uint64_t step = static_cast<uint64_t>(gridDim.x) * blockDim.x;
+    for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += step) {
+        const float2 f = reinterpret_cast<const float2*>(x)[i];
+        if (__float_as_uint(f.x) == 0xffffffffu && __float_as_uint(f.y) == 0xffffffffu) continue;
+        x[i] = static_cast<double>(f.x) + static_cast<double>(f.y);
+    }
+}
+
 const void* select_kernel(const RunConst& R, bool positions) {
-    if (const void* lean = positions ? nullptr : mixed_lean_kernel(R, false)) return lean;
+    if (const void* lean = mixed_lean_kernel(R, false, positions)) return lean;
     if (analytic_family(R.precision))
         return mixed_kernel_variant(R.metric_id, R.integrator, (R.mixed_options & FOORT_MIXED_FP64_DECISIONS) != 0);
     return fp64_kernel(R.metric_id, R.integrator);
@@ -229,7 +242,7 @@ const void* select_kernel(const RunConst& R, bool positions) {
 // The two-lanes-per-geodesic kernel for these options, or nullptr (FP64 and FP64-analytic
 // in part, Verlet, the called plugins, the strong-field FP64 steps).
 const void* select_pair_kernel(const RunConst& R, bool positions) {
-    if (const void* lean = positions ? nullptr : mixed_lean_kernel(R, true)) return lean;
+    if (const void* lean = mixed_lean_kernel(R, true, positions)) return lean;
     if (R.precision == FOORT_PREC_FP64) return fp64_pair_kernel(R.metric_id, R.integrator);
     if (R.precision != FOORT_PREC_MIXED || R.mixed_fp64_margin > 0.0 ||
         (R.mixed_options & FOORT_MIXED_FP64_TURNING_POINTS))
@@ -249,9 +262,10 @@ struct LaunchShape {
 // - FP64 kernels: an FP64 instruction occupies its scheduler's pipe for 64 cycles however
 //   many lanes are active, so two lanes halve the metric work of a launch that leaves lanes
 //   idle, and shorten the last rays of a larger one. Past several refills they only add the
-//   parts that both lanes do: log r, Kerr 10,201 geodesics 102.7 ms on one lane and 64.9 on
-//   two, 62,500 204 and 175, 122,500 293 and 325; Johannsen 126 and 75.5, 275 and 216, 388
-//   and 396.
+//   parts that both lanes do: FP64-analytic Kerr in log r, 25,600 geodesics 82 ms on one lane
+//   and 69 on two, 62,500 123 and 111, 90,000 133 and 154. Johannsen's FP64-analytic body is
+//   called, and two lanes call it half as often each: every size (25,600 273 and 186, 250,000
+//   1,411 and 1,198).
 // - Lean kernels: one lane already evaluates two stages at a time, so two lanes pay only
 //   while they leave each scheduler one warp (n <= 64 x SMs), and only in log r, where
 //   each half of a packed stage needs its own exponentials and division: Kerr, 3,721
@@ -267,9 +281,10 @@ struct LaunchShape {
 //   than the general one-lane kernel: every size.
 uint64_t pair_limit(const RunConst& R, bool positions, int per_sm, int num_sms, uint32_t bs) {
     const uint64_t sms = static_cast<uint64_t>(num_sms);
+    if (R.precision == FOORT_PREC_FP64_ANALYTIC && R.metric_id == kJohannsen) return UINT64_MAX;
     if (R.precision != FOORT_PREC_MIXED) return 512 * sms;
-    if (!positions && mixed_lean_kernel(R, true)) {
-        if (!mixed_lean_kernel(R, false)) return UINT64_MAX;
+    if (mixed_lean_kernel(R, true, positions)) {
+        if (!mixed_lean_kernel(R, false, positions)) return UINT64_MAX;
         if (R.metric_id == kJohannsen) return (R.rlog ? 1024 : 192) * sms;
         return (R.rlog ? 64 : 24) * sms;
     }
@@ -671,7 +686,7 @@ int foort_gpu_positions(foort_ctx* ctx, const foort_pixel* px, uint64_t n, const
         uint64_t M, j, kept;
         geopos_plan(ctx->desc, first[i].steps, first[i].term, M, j, kept);
         first_slot[i] = total;
-        plan[i] = GeoposRec{nullptr, j, M, 0, 0};
+        plan[i] = GeoposRec{nullptr, j, M, 0, 0, 0};
         counts[i] = kept;
         total += kept;
     }
@@ -696,6 +711,11 @@ int foort_gpu_positions(foort_ctx* ctx, const foort_pixel* px, uint64_t n, const
         CK(cudaMemcpyAsync(d_plan, plan.data(), plan.size() * sizeof(GeoposRec), cudaMemcpyHostToDevice, st));
         int r = launch(ctx, ctx->d_px, n, ctx->d_out, st, d_plan);
         if (r) return r;
+        if (analytic_family(ctx->rc.precision)) {
+            const uint64_t blocks = std::min<uint64_t>((4 * total + 255) / 256, 8ull * ctx->num_sms);
+            if (blocks) expand_positions<<<static_cast<unsigned>(blocks), 256, 0, st>>>(d_pts, 4 * total);
+            CK(cudaGetLastError());
+        }
         CK(cudaMemcpyAsync(points, d_pts, total * 4 * sizeof(double), cudaMemcpyDeviceToHost, st));
         CK(cudaMemcpyAsync(again.data(), ctx->d_out, n * sizeof(foort_result), cudaMemcpyDeviceToHost, st));
         return finish(ctx);

@@ -114,10 +114,11 @@ constexpr unsigned long long kStatusNonfinite = 4ull;
 // M into its state and counts i and cnt there. (Keeping only a pointer to the record in
 // the lane made the Kerr a = 0.99 adaptive run (509² grid, 26,547 geodesics) 1.7 % slower on GB300.)
 struct GeoposRec {
-    double* dst;    // the geodesic's first slot (4 doubles per kept position)
-    uint64_t j, M;  // keep sample i where i % j == 0, and the last of M samples
-    uint64_t i;     // samples taken so far
-    uint64_t cnt;   // steps since the last sample (DecideUpdate)
+    double* dst;        // the geodesic's first slot (4 doubles per kept position)
+    uint64_t j, M;      // keep sample i where i % j == 0, and the last of M samples
+    uint64_t i;         // samples taken so far
+    uint64_t cnt;       // steps since the last sample (DecideUpdate)
+    uint64_t next = 0;  // the next sample to keep
 };
 
 struct LaunchArgs {

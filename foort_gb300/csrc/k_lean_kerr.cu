@@ -4,37 +4,18 @@
 
 namespace foort {
 
-template <int MID, bool RLOG>
-__global__ void __launch_bounds__(128, 3) integrate_lean_kernel(const __grid_constant__ LaunchArgs A,
-                                                             const __grid_constant__ RunConst R) {
-    persistent_loop<LeanEngine<MID, RLOG>>(A, R);
+const void* mixed_lean_kernel_kerr(bool rlog, bool positions) {
+    return rlog ? lean_kernel<LeanEngine<kKerr, true>, 1, 3>(positions)
+                : lean_kernel<LeanEngine<kKerr, false>, 1, 3>(positions);
 }
 
-template <int MID, bool RLOG>
-__global__ void __launch_bounds__(128) integrate_lean_pair_kernel(const __grid_constant__ LaunchArgs A,
-                                                                  const __grid_constant__ RunConst R) {
-    persistent_loop<LeanEngine<MID, RLOG>, 2>(A, R);
+const void* mixed_lean_pair_kernel_kerr(bool rlog, bool positions) {
+    return rlog ? lean_kernel<LeanEngine<kKerr, true>, 2>(positions) : lean_kernel<LeanEngine<kKerr, false>, 2>(positions);
 }
 
-template <int MID, bool RLOG>
-__global__ void __launch_bounds__(128, 3) integrate_lean_verlet_kernel(const __grid_constant__ LaunchArgs A,
-                                                                       const __grid_constant__ RunConst R) {
-    persistent_loop<LeanVerletEngine<MID, RLOG>>(A, R);
-}
-
-const void* mixed_lean_verlet_kernel_kerr(bool rlog) {
-    return rlog ? reinterpret_cast<const void*>(&integrate_lean_verlet_kernel<kKerr, true>)
-                : reinterpret_cast<const void*>(&integrate_lean_verlet_kernel<kKerr, false>);
-}
-
-const void* mixed_lean_kernel_kerr(bool rlog) {
-    return rlog ? reinterpret_cast<const void*>(&integrate_lean_kernel<kKerr, true>)
-                : reinterpret_cast<const void*>(&integrate_lean_kernel<kKerr, false>);
-}
-
-const void* mixed_lean_pair_kernel_kerr(bool rlog) {
-    return rlog ? reinterpret_cast<const void*>(&integrate_lean_pair_kernel<kKerr, true>)
-                : reinterpret_cast<const void*>(&integrate_lean_pair_kernel<kKerr, false>);
+const void* mixed_lean_verlet_kernel_kerr(bool rlog, bool positions) {
+    return rlog ? lean_kernel<LeanVerletEngine<kKerr, true>, 1, 3>(positions)
+                : lean_kernel<LeanVerletEngine<kKerr, false>, 1, 3>(positions);
 }
 
 }  // namespace foort

@@ -4,12 +4,6 @@
 
 namespace foort {
 
-template <int MID>
-__global__ void __launch_bounds__(128) integrate_lean_called_kernel(const __grid_constant__ LaunchArgs A,
-                                                                    const __grid_constant__ RunConst R) {
-    persistent_loop<LeanCalledEngine<MID>, 2>(A, R);
-}
-
-const void* mixed_lean_pair_kernel_rl() { return reinterpret_cast<const void*>(&integrate_lean_called_kernel<kRasheedLarsen>); }
+const void* mixed_lean_pair_kernel_rl(bool positions) { return lean_kernel<LeanCalledEngine<kRasheedLarsen>, 2>(positions); }
 
 }  // namespace foort

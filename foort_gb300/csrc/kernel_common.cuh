@@ -105,24 +105,25 @@ __device__ __forceinline__ bool diag_decide(uint64_t every, int32_t at_start, in
 // final sample. The first pass gives M (from the step count), so this pass writes each
 // kept sample straight to its slot: sample i goes to slot i / j, sample M - 1 to slot
 // (M - 1) / j. Samples beyond the M the plan allows are not written.
+// Returns the slot to write, or nullptr. A step that keeps nothing only counts: a 64-bit
+// remainder at each step, and a state brought to FP64 for it whether kept or not, made a
+// recording Verlet launch of 3,600 Kerr rays take 2.06 ms against 1.09 without recording.
+__device__ __forceinline__ double* geopos_slot(GeoposRec& g, const RunConst& R, double lam, int term) {
+    if (R.gp_every != 1 && !diag_decide(R.gp_every, R.gp_start, R.gp_finish, g.cnt, lam, term)) return nullptr;
+    const uint64_t i = g.i++;
+    if (i != g.next) return nullptr;
+    const uint64_t k = (g.j == 1) ? i : i / g.j, up = (k + 1) * g.j;
+    g.next = (up < g.M) ? up : (i + 1 < g.M) ? g.M - 1 : UINT64_MAX;
+    return g.dst + 4 * k;
+}
 __device__ __forceinline__ void geopos_sample(GeoposRec& g, const RunConst& R, const double x[4], double lam,
                                               int term) {
-    if (!diag_decide(R.gp_every, R.gp_start, R.gp_finish, g.cnt, lam, term)) return;
-    const uint64_t i = g.i++;
-    if (i >= g.M) return;
-    uint64_t slot;
-    if (i % g.j == 0) {
-        slot = i / g.j;
-    } else if (i == g.M - 1) {
-        slot = (g.M - 1) / g.j;
-    } else {
-        return;
+    if (double* d = geopos_slot(g, R, lam, term)) {
+        d[0] = x[0];
+        d[1] = x[1];
+        d[2] = x[2];
+        d[3] = x[3];
     }
-    double* d = g.dst + 4 * slot;
-    d[0] = x[0];
-    d[1] = x[1];
-    d[2] = x[2];
-    d[3] = x[3];
 }
 
 // FourColorScreenDiagnostic::UpdateData, Diagnostics.cpp:159-200 (only on BoundarySphere)
@@ -302,6 +303,16 @@ struct NoTail {
     static constexpr bool kIs = false;
 };
 
+// Engines that record positions (E::kRecords): the general ones, and Recording's.
+template <class E>
+constexpr bool is_recording(...) {
+    return false;
+}
+template <class E>
+constexpr bool is_recording(decltype(E::kRecords)*) {
+    return true;
+}
+
 template <class E, int LANES, class Tail>
 __device__ __forceinline__ void work_loop(const LaunchArgs& A, const RunConst& R, typename E::Lane& L, bool active,
                                           uint64_t idx, bool drained) {
@@ -372,9 +383,9 @@ __device__ __forceinline__ void work_loop(const LaunchArgs& A, const RunConst& R
                             idx = my;
                             // i and cnt start at 0 as literals: copying them from the record
                             // made the Johannsen Verlet kernel 3 % slower on GB300
-                            if constexpr (!kLean && !SPLIT) L.gp = (A.gp_plan && !odd && A.gp_plan[my].M > 0 && A.gp_plan[my].j > 0)
-                                       ? GeoposRec{A.gp_plan[my].dst, A.gp_plan[my].j, A.gp_plan[my].M, 0, 0}
-                                       : GeoposRec{nullptr, 1, 0, 0, 0};
+                            if constexpr (is_recording<E>(nullptr)) L.gp = (A.gp_plan && !odd && A.gp_plan[my].M > 0 && A.gp_plan[my].j > 0)
+                                       ? GeoposRec{A.gp_plan[my].dst, A.gp_plan[my].j, A.gp_plan[my].M, 0, 0, 0}
+                                       : GeoposRec{nullptr, 1, 0, 0, 0, 0};
                             if constexpr (SPLIT) {
                                 E::init(L, A.images[p.image], R, p, sub, pmask);
                             } else {

@@ -70,6 +70,7 @@ __device__ __forceinline__ void rhs_fd_fp64(const MetricConst& M, bool rlog, dou
 template <int MID, int INTEG>
 struct Fp64Engine {
     static constexpr bool kCopyImage = false;
+    static constexpr bool kRecords = true;
 
     struct Lane {
         double x[4], v[4];

@@ -683,4 +683,52 @@ struct AnalyticPairEngine : LeanState<ImageRef> {
     }
 };
 
+// A lean engine that records positions (Fp64Engine's and MixedEngine's samples): the second
+// pass of foort_gpu_positions takes the first one's steps. 3,600 Kerr rays in Verlet, ln r, 25
+// positions kept of each: 2.06 ms with the general kernel, 1.25 with this (1.09 without
+// recording).
+template <class E>
+struct Recording : E {
+    static constexpr bool kRecords = true;
+
+    struct Lane : E::Lane {
+        GeoposRec gp;  // set by the loop before init (dst null: not recording)
+    };
+
+    static __device__ __forceinline__ void sample(Lane& L, const RunConst& R, double lam) {
+        if (!L.gp.dst) return;
+        if (double* d = geopos_slot(L.gp, R, lam, L.term)) {  // as MixedEngine::geopos
+            float4* f = reinterpret_cast<float4*>(d);
+            f[0] = make_float4(lo2(L.xh[0]), lo2(L.xl[0]), lo2(L.xh[1]), lo2(L.xl[1]));
+            f[1] = make_float4(hi2(L.xh[1]), hi2(L.xl[1]), hi2(L.xh[0]), hi2(L.xl[0]));
+        }
+    }
+    static __device__ __forceinline__ void init(Lane& L, const ImageConst& I, const RunConst& R, const foort_pixel& p) {
+        E::init(L, I, R, p);
+        sample(L, R, 0.0);
+    }
+    static __device__ __forceinline__ bool step(Lane& L, const RunConst& R) {
+        const bool more = E::step(L, R);
+        sample(L, R, 1.0);  // lambda > 0 after a step; only compared with 0
+        return more;
+    }
+    static __device__ __forceinline__ bool step_pair(Lane& L, const RunConst& R, bool odd, unsigned pmask) {
+        const bool more = E::step_pair(L, R, odd, pmask);
+        sample(L, R, 1.0);
+        return more;
+    }
+};
+
+template <class E, int LANES, int CTAS>
+__global__ void __launch_bounds__(128, CTAS) integrate_lean_kernel(const __grid_constant__ LaunchArgs A,
+                                                                   const __grid_constant__ RunConst R) {
+    persistent_loop<E, LANES>(A, R);
+}
+
+template <class E, int LANES, int CTAS = 1>
+const void* lean_kernel(bool positions) {
+    return positions ? reinterpret_cast<const void*>(&integrate_lean_kernel<Recording<E>, LANES, CTAS>)
+                     : reinterpret_cast<const void*>(&integrate_lean_kernel<E, LANES, CTAS>);
+}
+
 }  // namespace foort

@@ -347,6 +347,7 @@ struct MixedEngine {
     static constexpr bool kPairCapable = INTEG == FOORT_INTEGRATOR_RK4 && MixedMetric<MID>::kInline;
 
     static constexpr bool kCopyImage = true;
+    static constexpr bool kRecords = true;
 
     struct Lane {
         ff x[4], v[4];
@@ -384,12 +385,13 @@ struct MixedEngine {
         }
     }
 
-    // GeodesicPosition sample of the compensated position (second pass only)
+    // GeodesicPosition sample of the compensated position (second pass only): high and low
+    // parts, which expand_positions() brings to FP64
     static __device__ __forceinline__ void geopos(Lane& L, const RunConst& R, double lam) {
-        double x[4];
+        if (double* d = geopos_slot(L.gp, R, lam, L.term)) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) x[i] = ff_d(L.x[i]);
-        geopos_sample(L.gp, R, x, lam, L.term);
+            for (int i = 0; i < 4; ++i) reinterpret_cast<float2*>(d)[i] = make_float2(L.x[i].hi, L.x[i].lo);
+        }
     }
 
     static __device__ __forceinline__ void load_double(const Lane& L, double x[4], double v[4]) {

@@ -20,7 +20,7 @@ const void* mixed_pair_kernel_variant(int metric_id, int integrator, bool decide
 
 // The lean kernel (kernel_lean.cuh) of these options, with one or two lanes per geodesic,
 // or nullptr where they need the general one.
-const void* mixed_lean_kernel(const RunConst& R, bool pair);
+const void* mixed_lean_kernel(const RunConst& R, bool pair, bool positions);
 
 // Host-side helpers of the mixed-precision kernels (per-image FP32 constants).
 void fill_mixed_constants(int metric_id, ImageConst& ic, const RunConst& rc);

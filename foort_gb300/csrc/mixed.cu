@@ -42,19 +42,19 @@ const void* mixed_pair_kernel_variant(int metric_id, int integ, bool decide64) {
     }
 }
 
-const void* mixed_lean_kernel_kerr(bool rlog);
-const void* mixed_lean_kernel_flat();
-const void* mixed_lean_pair_kernel_kerr(bool rlog);
-const void* mixed_lean_pair_kernel_flat();
-const void* mixed_lean_pair_kernel_joh();
-const void* mixed_lean_kernel_joh13(bool rlog);
-const void* mixed_lean_pair_kernel_joh13(bool rlog);
-const void* mixed_lean_verlet_kernel_kerr(bool rlog);
-const void* mixed_lean_verlet_kernel_joh13(bool rlog);
-const void* mixed_lean_pair_kernel_rl();
-const void* analytic_pair_kernel_kerr();
-const void* analytic_pair_kernel_joh();
-const void* analytic_pair_kernel_flat();
+const void* mixed_lean_kernel_kerr(bool rlog, bool positions);
+const void* mixed_lean_kernel_flat(bool positions);
+const void* mixed_lean_pair_kernel_kerr(bool rlog, bool positions);
+const void* mixed_lean_pair_kernel_flat(bool positions);
+const void* mixed_lean_pair_kernel_joh(bool positions);
+const void* mixed_lean_kernel_joh13(bool rlog, bool positions);
+const void* mixed_lean_pair_kernel_joh13(bool rlog, bool positions);
+const void* mixed_lean_verlet_kernel_kerr(bool rlog, bool positions);
+const void* mixed_lean_verlet_kernel_joh13(bool rlog, bool positions);
+const void* mixed_lean_pair_kernel_rl(bool positions);
+const void* analytic_pair_kernel_kerr(bool positions);
+const void* analytic_pair_kernel_joh(bool positions);
+const void* analytic_pair_kernel_flat(bool positions);
 
 // Lean options: every termination and diagnostic in use updates at each step (the
 // default), with decisions on the float-float state.
@@ -74,32 +74,32 @@ static bool fp64_regions(const RunConst& R) {
     return R.mixed_fp64_margin > 0.0 || (R.mixed_options & FOORT_MIXED_FP64_TURNING_POINTS);
 }
 
-const void* mixed_lean_kernel(const RunConst& R, bool pair) {
+const void* mixed_lean_kernel(const RunConst& R, bool pair, bool positions) {
     if (!lean_options(R)) return nullptr;
     if (R.integrator == FOORT_INTEGRATOR_VERLET) {
         if (pair || R.precision != FOORT_PREC_MIXED || fp64_regions(R)) return nullptr;
-        if (R.metric_id == kKerr) return mixed_lean_verlet_kernel_kerr(R.rlog != 0);
-        if (R.metric_id == kJohannsen && R.only_alpha13) return mixed_lean_verlet_kernel_joh13(R.rlog != 0);
+        if (R.metric_id == kKerr) return mixed_lean_verlet_kernel_kerr(R.rlog != 0, positions);
+        if (R.metric_id == kJohannsen && R.only_alpha13) return mixed_lean_verlet_kernel_joh13(R.rlog != 0, positions);
         return nullptr;
     }
     if (R.precision == FOORT_PREC_FP64_ANALYTIC) {
         if (!pair) return nullptr;
         switch (R.metric_id) {
-        case kKerr: return analytic_pair_kernel_kerr();
-        case kJohannsen: return analytic_pair_kernel_joh();
-        case kFlat: return analytic_pair_kernel_flat();
+        case kKerr: return analytic_pair_kernel_kerr(positions);
+        case kJohannsen: return analytic_pair_kernel_joh(positions);
+        case kFlat: return analytic_pair_kernel_flat(positions);
         default: return nullptr;
         }
     }
     if (R.precision != FOORT_PREC_MIXED || fp64_regions(R)) return nullptr;
     switch (R.metric_id) {
-    case kKerr: return pair ? mixed_lean_pair_kernel_kerr(R.rlog != 0) : mixed_lean_kernel_kerr(R.rlog != 0);
-    case kFlat: return R.rlog ? nullptr : pair ? mixed_lean_pair_kernel_flat() : mixed_lean_kernel_flat();
+    case kKerr: return pair ? mixed_lean_pair_kernel_kerr(R.rlog != 0, positions) : mixed_lean_kernel_kerr(R.rlog != 0, positions);
+    case kFlat: return R.rlog ? nullptr : pair ? mixed_lean_pair_kernel_flat(positions) : mixed_lean_kernel_flat(positions);
     case kJohannsen:
         if (R.only_alpha13)
-            return pair ? mixed_lean_pair_kernel_joh13(R.rlog != 0) : mixed_lean_kernel_joh13(R.rlog != 0);
-        return pair ? mixed_lean_pair_kernel_joh() : nullptr;
-    case kRasheedLarsen: return pair ? mixed_lean_pair_kernel_rl() : nullptr;
+            return pair ? mixed_lean_pair_kernel_joh13(R.rlog != 0, positions) : mixed_lean_kernel_joh13(R.rlog != 0, positions);
+        return pair ? mixed_lean_pair_kernel_joh(positions) : nullptr;
+    case kRasheedLarsen: return pair ? mixed_lean_pair_kernel_rl(positions) : nullptr;
     default: return nullptr;
     }
 }

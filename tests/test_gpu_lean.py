@@ -251,3 +251,33 @@ def test_fp64_lanes_are_refilled_and_run_two_images(eng, metric, integrator, sid
     assert stopped.any() and np.all(part["term"][stopped] == abi.TERMCODE_CONTINUE)
     same_records(part[~stopped], got[1][~stopped])
     del keep
+
+
+# every step sampled, each third with the last, one kept position, all of them
+@pytest.mark.gpu
+@pytest.mark.parametrize("keep_steps,freq", [(25, (1, 1, 0)), (7, (3, 0, 1)), (1, (1, 0, 0)), (0, (1, 1, 1))])
+@pytest.mark.parametrize("metric,params,rlog,side,integrator", [
+    (abi.METRIC_KERR, (0.9,), 1, 17, abi.INTEGRATOR_RK4),
+    (abi.METRIC_KERR, (0.9,), 1, 17, abi.INTEGRATOR_VERLET),
+    (abi.METRIC_FLAT, (), 0, 5, abi.INTEGRATOR_RK4),
+    (abi.METRIC_JOHANNSEN, (0.7, 1.5, 0.0, 0.0, 0.0), 1, 17, abi.INTEGRATOR_VERLET),
+    (abi.METRIC_JOHANNSEN, (0.7, 1.5, 0.0, 0.0, 0.0), 1, 17, abi.INTEGRATOR_RK4),
+    (abi.METRIC_RASHEED_LARSEN, LORENZO, 1, 9, abi.INTEGRATOR_RK4),
+])
+def test_lean_kernels_record_the_general_kernels_positions(eng, metric, params, rlog, side, integrator, keep_steps,
+                                                          freq):
+    px = abi.square_pixels(side)
+    d, keep = describe(metric, params, rlog, 63.0, integrator=integrator, timeout=900)
+    d.diag_flags |= abi.DIAG_GEODESIC_POSITION
+    d.geopos_output_steps, d.geopos_freq = keep_steps, abi.UpdateFreq(*freq)
+    got = {}
+    for name, options, lanes in (("general", abi.MIXED_FP64_DECISIONS, 1), ("one lane", 0, 1), ("two lanes", 0, 2)):
+        d.mixed_options = options
+        with eng.Engine(d) as e:
+            e.set_lanes(lanes)
+            got[name] = e.positions(px, e.integrate(px))
+    for name in ("one lane", "two lanes"):
+        np.testing.assert_array_equal(got[name][0], got["general"][0])
+        np.testing.assert_array_equal(got[name][1], got["general"][1])
+    assert np.isfinite(got["general"][1]).all()
+    del keep
