@@ -6,6 +6,10 @@ namespace foort {
 
 const void* mixed_lean_kernel_flat(bool positions) { return lean_kernel<LeanEngine<kFlat, false>, 1, 3>(positions); }
 
+const void* mixed_lean_verlet_kernel_flat(bool positions) {
+    return lean_kernel<LeanVerletEngine<kFlat, false>, 1, 3>(positions);
+}
+
 const void* mixed_lean_pair_kernel_flat(bool positions) { return lean_kernel<LeanEngine<kFlat, false>, 2>(positions); }
 
 }  // namespace foort

@@ -51,6 +51,7 @@ const void* mixed_lean_kernel_joh13(bool rlog, bool positions);
 const void* mixed_lean_pair_kernel_joh13(bool rlog, bool positions);
 const void* mixed_lean_verlet_kernel_kerr(bool rlog, bool positions);
 const void* mixed_lean_verlet_kernel_joh13(bool rlog, bool positions);
+const void* mixed_lean_verlet_kernel_flat(bool positions);
 const void* mixed_lean_pair_kernel_rl(bool positions);
 const void* analytic_pair_kernel_kerr(bool positions);
 const void* analytic_pair_kernel_joh(bool positions);
@@ -78,6 +79,7 @@ const void* mixed_lean_kernel(const RunConst& R, bool pair, bool positions) {
     if (!lean_options(R)) return nullptr;
     if (R.integrator == FOORT_INTEGRATOR_VERLET) {
         if (pair || R.precision != FOORT_PREC_MIXED || fp64_regions(R)) return nullptr;
+        if (R.metric_id == kFlat && !R.rlog) return mixed_lean_verlet_kernel_flat(positions);
         if (R.metric_id == kKerr) return mixed_lean_verlet_kernel_kerr(R.rlog != 0, positions);
         if (R.metric_id == kJohannsen && R.only_alpha13) return mixed_lean_verlet_kernel_joh13(R.rlog != 0, positions);
         return nullptr;

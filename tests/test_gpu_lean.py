@@ -89,6 +89,8 @@ def test_lean_kernels_give_the_general_kernels_records(eng, metric, params, rlog
     (abi.METRIC_KERR, (0.998,), 1, 17.0, 33, None, 0.001),
     (abi.METRIC_KERR, (0.0,), 1, 90.0, 17, None, 1e-5),
     (abi.METRIC_KERR, (0.7,), 0, 63.0, 5, 20000, 0.001),
+    (abi.METRIC_FLAT, (), 0, 63.0, 7, 20000, 0.001),
+    (abi.METRIC_FLAT, (), 0, 63.0, 5, 3000, 1e-7),
     (abi.METRIC_JOHANNSEN, (0.9, 0.4, 0.0, 0.0, 0.0), 1, 63.0, 33, None, -1.0),
     (abi.METRIC_JOHANNSEN, (0.3, -0.9, 0.0, 0.0, 0.0), 1, 2.0, 33, None, 1e-5),
     (abi.METRIC_JOHANNSEN, (0.9, 0.4, 0.0, 0.0, 0.0), 0, 30.0, 5, 20000, 0.001),
