@@ -40,6 +40,8 @@ struct foort_ctx {
     foort_pixel* d_px = nullptr;
     foort_result* d_out = nullptr;
     uint64_t cap = 0;
+    void* d_pos = nullptr;  // foort_gpu_positions: the plan and the points
+    uint64_t pos_cap = 0;
     uint64_t budget = 0;
     uint64_t last_n = 0;
     uint32_t block_size = 0, blocks_per_sm = 0;
@@ -393,6 +395,16 @@ int ensure_capacity(foort_ctx* ctx, uint64_t n) {
     return FOORT_OK;
 }
 
+// Bytes of the positions workspace that a context keeps between calls: allocating and
+// freeing it took 0.2 ms a call on 3,600 rays.
+constexpr uint64_t kKeepPositions = 64ull << 20;
+
+void release_positions(foort_ctx* ctx) {
+    if (ctx->d_pos) cudaFree(ctx->d_pos);
+    ctx->d_pos = nullptr;
+    ctx->pos_cap = 0;
+}
+
 int autotune_launch(foort_ctx* ctx, const foort_pixel* d_px, uint64_t n, foort_result* d_out, cudaStream_t st,
                     foort_launch_shape* best);
 
@@ -703,8 +715,15 @@ int foort_gpu_positions(foort_ctx* ctx, const foort_pixel* px, uint64_t n, const
     std::vector<foort_result> again(n);
     auto body = [&]() -> int {
         cudaStream_t st = ctx->stream;
-        CK(cudaMalloc(&d_plan, plan.size() * sizeof(GeoposRec)));
-        CK(cudaMalloc(&d_pts, std::max<uint64_t>(1, total) * 4 * sizeof(double)));
+        const uint64_t pts_bytes = std::max<uint64_t>(1, total) * 4 * sizeof(double);
+        const uint64_t bytes = pts_bytes + plan.size() * sizeof(GeoposRec);
+        if (bytes > ctx->pos_cap) {
+            release_positions(ctx);
+            CK(cudaMalloc(&ctx->d_pos, bytes));
+            ctx->pos_cap = bytes;
+        }
+        d_pts = static_cast<double*>(ctx->d_pos);
+        d_plan = reinterpret_cast<GeoposRec*>(static_cast<char*>(ctx->d_pos) + pts_bytes);
         CK(cudaMemsetAsync(d_pts, 0xFF, std::max<uint64_t>(1, total) * 4 * sizeof(double), st));  // NaN
         for (uint64_t i = 0; i < n; ++i) plan[i].dst = d_pts + 4 * first_slot[i];  // device addresses
         CK(cudaMemcpyAsync(ctx->d_px, px, n * sizeof(foort_pixel), cudaMemcpyHostToDevice, st));
@@ -721,8 +740,7 @@ int foort_gpu_positions(foort_ctx* ctx, const foort_pixel* px, uint64_t n, const
         return finish(ctx);
     };
     rc = body();
-    if (d_plan) cudaFree(d_plan);
-    if (d_pts) cudaFree(d_pts);
+    if (rc != FOORT_OK || ctx->pos_cap > kKeepPositions) release_positions(ctx);
     if (rc != FOORT_OK) return rc;
     // the second pass must retrace the first: same steps for every recorded geodesic
     for (uint64_t i = 0; i < n; ++i)
@@ -916,6 +934,7 @@ void foort_gpu_destroy(foort_ctx* ctx) {
     if (ctx->pending && ctx->last_stream) cudaStreamSynchronize(ctx->last_stream);
     if (ctx->d_px) cudaFree(ctx->d_px);
     if (ctx->d_out) cudaFree(ctx->d_out);
+    release_positions(ctx);
     if (ctx->d_images) cudaFree(ctx->d_images);
     if (ctx->d_ctr) cudaFree(ctx->d_ctr);
     if (ctx->h_cancel) cudaFreeHost(ctx->h_cancel);
