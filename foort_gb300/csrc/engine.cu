@@ -267,7 +267,9 @@ struct LaunchShape {
 //   parts that both lanes do: FP64-analytic Kerr in log r, 25,600 geodesics 82 ms on one lane
 //   and 69 on two, 62,500 123 and 111, 90,000 133 and 154. Johannsen's FP64-analytic body is
 //   called, and two lanes call it half as often each: every size (25,600 273 and 186, 250,000
-//   1,411 and 1,198).
+//   1,411 and 1,198). In plain r rays differ less in length, and a wave of two lanes each
+//   (64 x SMs) is the most that pays (flat space in FP64, 9,604 rays cut at 900 steps 20 ms on
+//   two lanes and 29 on one, 19,044 42 and 29).
 // - Lean kernels: one lane already evaluates two stages at a time, so two lanes pay only
 //   while they leave each scheduler one warp (n <= 64 x SMs), and only in log r, where
 //   each half of a packed stage needs its own exponentials and division: Kerr, 3,721
@@ -284,7 +286,7 @@ struct LaunchShape {
 uint64_t pair_limit(const RunConst& R, bool positions, int per_sm, int num_sms, uint32_t bs) {
     const uint64_t sms = static_cast<uint64_t>(num_sms);
     if (R.precision == FOORT_PREC_FP64_ANALYTIC && R.metric_id == kJohannsen) return UINT64_MAX;
-    if (R.precision != FOORT_PREC_MIXED) return 512 * sms;
+    if (R.precision != FOORT_PREC_MIXED) return (R.rlog ? 512 : 64) * sms;
     if (mixed_lean_kernel(R, true, positions)) {
         if (!mixed_lean_kernel(R, false, positions)) return UINT64_MAX;
         if (R.metric_id == kJohannsen) return (R.rlog ? 1024 : 192) * sms;
@@ -304,12 +306,14 @@ uint64_t pair_limit(const RunConst& R, bool positions, int per_sm, int num_sms, 
 //    25,600      103 /  87 / 103;  99 / 124    139 / 113 / 134; 122 / 163     38 / 38; 46     46 / 45; 53
 //    62,500      238 / 174 / 173; 179 / 214    323 / 210 / 218; 212 / 263     88 / 57; 64    108 / 67; 74
 //   250,000      931 / 658 / 600; 658 / 597   1264 / 804 / 815; 803 / 803    344 / 202; 203  424 / 243; 244
-// Past some ten refills of every lane a launch's end is a small part of it.
+// Past some ten refills of every lane a launch's end is a small part of it. In plain r rays
+// differ less in length, and the fewest lanes whose waves of 32, 64 and 128 x SMs geodesics
+// hold the launch win (Kerr RK4, a wave of rays cut at 900 steps 26 / 38 / 64).
 int split_start(const RunConst& R, uint64_t n, int num_sms, bool forced) {
     const uint64_t sms = static_cast<uint64_t>(num_sms);
     const bool rk4 = R.integrator == FOORT_INTEGRATOR_RK4;
-    if (n <= (rk4 ? 64 : 160) * sms) return 4;
-    if (rk4 && n <= 384 * sms) return 2;
+    if (n <= (R.rlog ? (rk4 ? 64 : 160) : rk4 ? 32 : 64) * sms) return 4;
+    if (rk4 && n <= (R.rlog ? 384 : 64) * sms) return 2;
     return (forced || n <= 1024 * sms) ? 1 : 0;
 }
 
@@ -320,13 +324,20 @@ int split_start(const RunConst& R, uint64_t n, int num_sms, bool forced) {
 // its FP64 pipe, more only leave rays unevenly spread over lanes at the end (62,500
 // Johannsen rays in FP64 130 ms with two CTAs of 128 per SM, 110 with four of 32), and small
 // CTAs spread a launch that does not fill the GPU evenly (4,096 Kerr rays 65.8 and 62.5 ms).
+// Eight per SM hide 5 % more latency where rays of like lengths (plain r) need more than the
+// lanes of four (62,500 Kerr rays cut at 900 steps 253 and 238 ms), or where a launch is so
+// large that its end counts little (250,000 in log r 623 and 601, 62,500 170 and 186).
 int choose_launch(foort_ctx* ctx, const RunConst& R, uint64_t n, int num_sms, const foort_launch_shape& want,
                   LaunchShape& out, bool positions = false) {
     const bool fp64 = R.precision != FOORT_PREC_MIXED;
     const uint32_t bs = want.block_size ? want.block_size : fp64 ? 32 : 128;
-    auto resident = [&](const void* fn, int& per_sm) -> int {
+    const uint64_t sms = static_cast<uint64_t>(num_sms);
+    auto resident = [&](const void* fn, uint64_t width, int& per_sm) -> int {
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, static_cast<int>(bs), 0));
-        if (fp64 && !want.blocks_per_sm) per_sm = std::min<int>(per_sm, std::max<int>(1, 128 / static_cast<int>(bs)));
+        if (fp64 && !want.blocks_per_sm) {
+            const bool two = n > 1024 * sms || (!R.rlog && width * n > 128 * sms);
+            per_sm = std::min<int>(per_sm, std::max<int>(1, (two ? 256 : 128) / static_cast<int>(bs)));
+        }
         if (want.blocks_per_sm) per_sm = std::min<int>(per_sm, static_cast<int>(want.blocks_per_sm));
         return FOORT_OK;
     };
@@ -334,30 +345,31 @@ int choose_launch(foort_ctx* ctx, const RunConst& R, uint64_t n, int num_sms, co
     if (!fn) return fail(ctx, FOORT_E_UNSUPPORTED, "no kernel for this metric / integrator / precision");
     int per_sm = 0, rc = 0;
     uint32_t lanes = 1;    // 2 stands for several, as in foort_launch_shape
-    uint32_t threads = 1;  // per geodesic of a launch that does not fill the GPU
-    const int start = (R.precision == FOORT_PREC_FP64 && !positions && want.lanes != 1)
-                          ? split_start(R, n, num_sms, want.lanes == 2)
-                          : 0;
-    const void* split = start ? fp64_split_kernel(R, start) : nullptr;
+    uint64_t threads = n;  // to hold every geodesic at once
+    const bool may_split = R.precision == FOORT_PREC_FP64 && !positions && want.lanes != 1;
+    const int start = may_split ? split_start(R, n, num_sms, want.lanes == 2) : 0;
+    const void* split = may_split ? fp64_split_kernel(R, start) : nullptr;
     const void* pair = (split || want.lanes == 1) ? nullptr : select_pair_kernel(R, positions);
     if (split) {
         fn = split;
-        lanes = 2;
-        threads = 4;  // no more than eight geodesics per warp while that spreads them wider
-        if ((rc = resident(fn, per_sm))) return rc;
+        lanes = start ? 2 : 1;
+        // one warp per scheduler before any is full, as long as each has eight geodesics
+        threads = std::max(std::max(start, 1) * n, std::min(4 * n, 128 * sms));
+        if ((rc = resident(fn, std::max(start, 1), per_sm))) return rc;
     } else if (pair) {
         int per_sm2 = 0;
-        if ((rc = resident(pair, per_sm2))) return rc;
+        if ((rc = resident(pair, 2, per_sm2))) return rc;
         if (per_sm2 > 0 && (want.lanes == 2 || n <= pair_limit(R, positions, per_sm2, num_sms, bs))) {
             fn = pair;
             per_sm = per_sm2;
-            lanes = threads = 2;
+            lanes = 2;
+            threads = 2 * n;
         }
     }
-    if (lanes == 1 && (rc = resident(fn, per_sm))) return rc;
+    if (per_sm == 0 && lanes == 1 && (rc = resident(fn, 1, per_sm))) return rc;
     if (per_sm <= 0) return fail(ctx, FOORT_E_CUDA, "kernel does not fit on an SM with this block size");
     const uint64_t full = static_cast<uint64_t>(per_sm) * static_cast<uint64_t>(num_sms);
-    const uint64_t need = (threads * n + bs - 1) / bs;
+    const uint64_t need = (threads + bs - 1) / bs;
     out.fn = fn;
     out.grid = static_cast<uint32_t>(std::max<uint64_t>(1, std::min(full, need)));
     out.block = bs;
@@ -1010,7 +1022,8 @@ const void* fp64_pair_kernel_joh();
 const void* fp64_split_kernel_kerr(int, int);
 const void* fp64_split_kernel_joh(int, bool, int);
 
-// Four lanes per geodesic in the end: from a start with 4, 2 (RK4 only) or 1.
+// Four lanes per geodesic in the end: from a start with 4, 2 (RK4 only) or 1; 0: one lane to
+// the end (Johannsen with alpha13 alone).
 const void* fp64_split_kernel(const RunConst& R, int start) {
     switch (R.metric_id) {
     case kKerr: return fp64_split_kernel_kerr(R.integrator, start);

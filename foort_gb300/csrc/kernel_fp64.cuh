@@ -18,9 +18,27 @@ struct FdParts {
     G5 dr, dh, gu;
 };
 
-template <int MID>
+// g_dd at one of the four points. own_r: no other point has this r; metrics whose roundings
+// are written out (Mt::kOwnR, SplitMetric) need to know.
+template <class Mt>
+constexpr bool takes_own_r(...) {
+    return false;
+}
+template <class Mt>
+constexpr bool takes_own_r(decltype(Mt::kOwnR)*) {
+    return true;
+}
+template <class Mt>
+__device__ __forceinline__ G5 dd_at(const MetricConst& M, double r, double s, double c, bool rlog, bool own_r) {
+    if constexpr (takes_own_r<Mt>(nullptr)) {
+        return Mt::dd(M.q, r, s, c, rlog, own_r);
+    } else {
+        return Mt::dd(M, r, s, c, rlog);
+    }
+}
+
+template <int MID, class Mt = MetricFP64<MID>>
 __device__ __forceinline__ FdParts fd_parts_fp64(const MetricConst& M, bool rlog, double hfd, const double x[4]) {
-    using Mt = MetricFP64<MID>;
     double r0, rp, rm;
     if (rlog) {
         r0 = exp(x[1]);
@@ -35,10 +53,10 @@ __device__ __forceinline__ FdParts fd_parts_fp64(const MetricConst& M, bool rlog
     sincos(x[2], &s0, &c0);
     sincos(x[2] + hfd, &sp, &cp);
     sincos(x[2] - hfd, &sm, &cm);
-    const G5 a = Mt::dd(M, rp, s0, c0, rlog);
-    const G5 b = Mt::dd(M, rm, s0, c0, rlog);
-    const G5 c = Mt::dd(M, r0, sp, cp, rlog);
-    const G5 d = Mt::dd(M, r0, sm, cm, rlog);
+    const G5 a = dd_at<Mt>(M, rp, s0, c0, rlog, true);
+    const G5 b = dd_at<Mt>(M, rm, s0, c0, rlog, true);
+    const G5 c = dd_at<Mt>(M, r0, sp, cp, rlog, false);
+    const G5 d = dd_at<Mt>(M, r0, sm, cm, rlog, false);
     const G5 gu = Mt::uu(M, r0, s0, c0, rlog);
     const double inv = 1 / (2 * hfd);
     FdParts P;
@@ -61,13 +79,14 @@ __device__ __forceinline__ void contract_fp64(const FdParts& P, const double v[4
 #include "gen_fd_christoffel.inc"
 }
 
-template <int MID>
+template <int MID, class Mt>
 __device__ __forceinline__ void rhs_fd_fp64(const MetricConst& M, bool rlog, double hfd, const double x[4],
                                             const double v[4], double acc[4]) {
-    contract_fp64(fd_parts_fp64<MID>(M, rlog, hfd, x), v, acc);
+    contract_fp64(fd_parts_fp64<MID, Mt>(M, rlog, hfd, x), v, acc);
 }
 
-template <int MID, int INTEG>
+// Mt: the metric's functions (MetricFP64, or SplitMetric's for Johannsen with alpha13 alone).
+template <int MID, int INTEG, class Mt = MetricFP64<MID>>
 struct Fp64Engine {
     static constexpr bool kCopyImage = false;
     static constexpr bool kRecords = true;
@@ -89,7 +108,7 @@ struct Fp64Engine {
 
     static __device__ __forceinline__ void init(Lane& L, const ImageConst& I, const RunConst& R, const foort_pixel& p) {
         initial_conditions(I, p, L.x, L.v);
-        if (INTEG == FOORT_INTEGRATOR_VERLET) L.P = fd_parts_fp64<MID>(I.m, R.rlog != 0, R.hfd, L.x);
+        if (INTEG == FOORT_INTEGRATOR_VERLET) L.P = fd_parts_fp64<MID, Mt>(I.m, R.rlog != 0, R.hfd, L.x);
         L.lam = 0.0;
         L.steps = 0;
         L.err = 0;
@@ -107,17 +126,17 @@ struct Fp64Engine {
         double nx[4], nv[4];
         if (INTEG == FOORT_INTEGRATOR_RK4) {  // Integrators.cpp:51-94
             double k1[4], k2[4], k3[4], k4[4], l2[4], l3[4], l4[4], t[4];
-            rhs_fd_fp64<MID>(M, rlog, R.hfd, L.x, L.v, k1);
+            rhs_fd_fp64<MID, Mt>(M, rlog, R.hfd, L.x, L.v, k1);
             const double hh = 0.5 * h;
 #pragma unroll
             for (int i = 0; i < 4; ++i) { t[i] = L.x[i] + L.v[i] * hh; l2[i] = L.v[i] + k1[i] * hh; }
-            rhs_fd_fp64<MID>(M, rlog, R.hfd, t, l2, k2);
+            rhs_fd_fp64<MID, Mt>(M, rlog, R.hfd, t, l2, k2);
 #pragma unroll
             for (int i = 0; i < 4; ++i) { t[i] = L.x[i] + l2[i] * hh; l3[i] = L.v[i] + k2[i] * hh; }
-            rhs_fd_fp64<MID>(M, rlog, R.hfd, t, l3, k3);
+            rhs_fd_fp64<MID, Mt>(M, rlog, R.hfd, t, l3, k3);
 #pragma unroll
             for (int i = 0; i < 4; ++i) { t[i] = L.x[i] + l3[i] * h; l4[i] = L.v[i] + k3[i] * h; }
-            rhs_fd_fp64<MID>(M, rlog, R.hfd, t, l4, k4);
+            rhs_fd_fp64<MID, Mt>(M, rlog, R.hfd, t, l4, k4);
             rk4_combine(L, h, k1, k2, k3, k4, l2, l3, l4, nx, nv);
             L.rhs += 4;
         } else {  // Integrators.cpp:99-152
@@ -133,7 +152,7 @@ struct Fp64Engine {
                 nx[i] = (L.x[i] + L.v[i] * h) + a0[i] * hh2;
                 vi[i] = L.v[i] + a0[i] * h;
             }
-            const FdParts Pn = fd_parts_fp64<MID>(M, rlog, R.hfd, nx);
+            const FdParts Pn = fd_parts_fp64<MID, Mt>(M, rlog, R.hfd, nx);
             contract_fp64(Pn, vi, a1);
             const double h2 = h / 2.0;
 #pragma unroll
@@ -188,7 +207,7 @@ struct Fp64Engine {
         };
 #pragma unroll
         for (int i = 0; i < 4; ++i) t[i] = odd ? L.x[i] + L.v[i] * hh : L.x[i];
-        FdParts P = fd_parts_fp64<MID>(M, rlog, R.hfd, t);
+        FdParts P = fd_parts_fp64<MID, Mt>(M, rlog, R.hfd, t);
         contract_fp64(P, L.v, ka);
         share(k1, 0);
 #pragma unroll
@@ -199,7 +218,7 @@ struct Fp64Engine {
         for (int i = 0; i < 4; ++i) l3[i] = L.v[i] + k2[i] * hh;
 #pragma unroll
         for (int i = 0; i < 4; ++i) t[i] = L.x[i] + (odd ? l3[i] : l2[i]) * (odd ? h : hh);
-        P = fd_parts_fp64<MID>(M, rlog, R.hfd, t);
+        P = fd_parts_fp64<MID, Mt>(M, rlog, R.hfd, t);
         contract_fp64(P, l3, ka);
         share(k3, 0);
 #pragma unroll

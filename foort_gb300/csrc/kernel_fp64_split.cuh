@@ -17,6 +17,8 @@
 // compiler contracts Fp64Engine (kernel_fp64.cuh; found by comparing evaluations).
 #pragma once
 
+#include <type_traits>
+
 #include "kernel_fp64.cuh"
 
 namespace foort {
@@ -72,6 +74,8 @@ struct SplitMetric<kKerr, false> {
 // Johannsen. A13: alpha22, alpha52 and epsilon3 are 0, whose terms vanish exactly.
 template <bool A13>
 struct SplitMetric<kJohannsen, A13> {
+    static constexpr bool kOwnR = true;
+
     struct Parts {
         double A1, A2, A5, rho2, del, ra, aa, rr;
     };
@@ -127,6 +131,15 @@ struct SplitMetric<kJohannsen, A13> {
         const double w = d_fma(A13 ? p.A1 : d_mul(p.A2, p.A1), x, -p.del);
         g2 = -(d_mul(a, w) / dr);
         if (rlog && i == 1) g1 = d_mul(g1, 1.0 / p.rr);
+    }
+    // All of them (fd_parts_fp64).
+    static __device__ __forceinline__ G5 uu(const MetricConst& M, double r, double s, double c, bool rlog) {
+        G5 g;
+        uu(M.q, r, s, c, rlog, 0, g.tt, g.tp);
+        uu(M.q, r, s, c, rlog, 1, g.rr, g.tp);
+        uu(M.q, r, s, c, rlog, 2, g.hh, g.tp);
+        uu(M.q, r, s, c, rlog, 3, g.pp, g.tp);
+        return g;
     }
 };
 
@@ -368,7 +381,7 @@ struct SplitEngine {
 // launch alone: 62,500 Johannsen rays in FP64 Verlet 122 ms on one lane throughout, 111 on
 // four, 98 on one and then four; 10,000 Kerr rays in RK4 72 on two lanes, 67 on four, 63 on
 // two and then four.
-template <int MID, bool A13, int INTEG>
+template <int MID, bool A13, int INTEG, class Engine>
 struct SplitTail {
     using S = SplitEngine<MID, A13, INTEG>;
     static constexpr bool kIs = true;
@@ -391,7 +404,7 @@ struct SplitTail {
 
     // left: the lanes that hold the geodesics; every lane of the warp calls it.
     static __device__ __forceinline__ void run(const LaunchArgs& A, const RunConst& R,
-                                               const typename Fp64Engine<MID, INTEG>::Lane& L, unsigned left,
+                                               const typename Engine::Lane& L, unsigned left,
                                                uint64_t idx) {
         const int lane = threadIdx.x & 31, i = lane & 3, group = lane >> 2;
         unsigned rest = left;
@@ -417,26 +430,48 @@ struct SplitTail {
     }
 };
 
-// START: lanes per geodesic until a warp has eight geodesics left.
+// START: lanes per geodesic until a warp has eight geodesics left; 0: one to the end (A13).
+// Without the zero terms Johannsen's right-hand side saves nine divisions of 34: one-lane
+// Verlet, 176,400 rays in log r 200 to 157 ms, RK4 653 to 475; 62,500 rays of the reference's
+// debug view with the tail 98 to 79.
 template <int MID, bool A13, int INTEG, int START>
 __global__ void __launch_bounds__(128) integrate_fp64_split_kernel(const __grid_constant__ LaunchArgs A,
                                                                    const __grid_constant__ RunConst R) {
     if constexpr (START == 4) {
         persistent_loop<SplitEngine<MID, A13, INTEG>, 4>(A, R);
     } else {
-        persistent_loop<Fp64Engine<MID, INTEG>, START, SplitTail<MID, A13, INTEG>>(A, R);
+        using E = Fp64Engine<MID, INTEG, std::conditional_t<A13, SplitMetric<MID, A13>, MetricFP64<MID>>>;
+        if constexpr (START == 0) {
+            persistent_loop<E, 1>(A, R);
+        } else {
+            persistent_loop<E, START, SplitTail<MID, A13, INTEG, E>>(A, R);
+        }
+    }
+}
+
+template <int MID, bool A13, int INTEG, int START>
+const void* split_instance() {
+    return reinterpret_cast<const void*>(&integrate_fp64_split_kernel<MID, A13, INTEG, START>);
+}
+
+template <int MID, bool A13, int INTEG>
+const void* split_kernel(int start) {
+    switch (start) {
+    case 0:
+        if constexpr (A13) return split_instance<MID, A13, INTEG, 0>();
+        return nullptr;
+    case 1: return split_instance<MID, A13, INTEG, 1>();
+    case 2:
+        if constexpr (INTEG == FOORT_INTEGRATOR_RK4) return split_instance<MID, A13, INTEG, 2>();
+        return nullptr;
+    default: return split_instance<MID, A13, INTEG, 4>();
     }
 }
 
 template <int MID, bool A13>
 const void* split_kernel(int integrator, int start) {
-    constexpr int kRk4 = FOORT_INTEGRATOR_RK4, kVerlet = FOORT_INTEGRATOR_VERLET;
-    const void* rk4[] = {reinterpret_cast<const void*>(&integrate_fp64_split_kernel<MID, A13, kRk4, 1>),
-                         reinterpret_cast<const void*>(&integrate_fp64_split_kernel<MID, A13, kRk4, 2>),
-                         reinterpret_cast<const void*>(&integrate_fp64_split_kernel<MID, A13, kRk4, 4>)};
-    const void* verlet[] = {reinterpret_cast<const void*>(&integrate_fp64_split_kernel<MID, A13, kVerlet, 1>), nullptr,
-                            reinterpret_cast<const void*>(&integrate_fp64_split_kernel<MID, A13, kVerlet, 4>)};
-    return (integrator == FOORT_INTEGRATOR_RK4 ? rk4 : verlet)[start / 2];
+    return integrator == FOORT_INTEGRATOR_RK4 ? split_kernel<MID, A13, FOORT_INTEGRATOR_RK4>(start)
+                                              : split_kernel<MID, A13, FOORT_INTEGRATOR_VERLET>(start);
 }
 
 }  // namespace foort
