@@ -295,25 +295,29 @@ uint64_t pair_limit(const RunConst& R, bool positions, int per_sm, int num_sms, 
     return static_cast<uint64_t>(per_sm) * sms * bs / 2;
 }
 
-// Lanes per geodesic that an FP64 launch of Kerr or Johannsen starts with in the kernels that
-// end on four lanes per geodesic (kernel_fp64_split.cuh): 4, 2 (RK4) or 1; 0: the plain
-// one-lane kernel, unless several lanes are forced. Four lanes finish a step soonest, but cost
-// 1.5 times the instructions of one lane and 1.4 times those of two per geodesic. Log r, ms
-// (starting with 4 / 2 / 1 lanes; the plain kernel on 2 / 1 lanes):
-//                Kerr RK4                      Johannsen RK4                  Verlet (4 / 1; 1): Kerr, Johannsen
-//     3,600       36 /  42 /  56;  50 /  83     57 /  62 /  81;  71 / 122     14 / 21; 30     16 / 24; 35
-//    10,000       67 /  63 /  92;  72 / 114     91 /  78 / 124;  90 / 149     24 / 33; 39     29 / 41; 47
-//    25,600      103 /  87 / 103;  99 / 124    139 / 113 / 134; 122 / 163     38 / 38; 46     46 / 45; 53
-//    62,500      238 / 174 / 173; 179 / 214    323 / 210 / 218; 212 / 263     88 / 57; 64    108 / 67; 74
-//   250,000      931 / 658 / 600; 658 / 597   1264 / 804 / 815; 803 / 803    344 / 202; 203  424 / 243; 244
+// Lanes per geodesic that an FP64 launch of Kerr or Johannsen starts with in the kernels of
+// kernel_fp64_split.cuh: 8 or 2 (RK4), 4 (Verlet) or 1; 0: one lane to the end, unless several
+// lanes are forced. The most lanes finish a step soonest but cost more instructions per
+// geodesic. ms in log r (the plain kernel on one lane last):
+//               RK4 from 8 / 2 / 1: Kerr       Johannsen            Verlet from 4 / 1: Kerr, Johannsen
+//     3,600      24 /  42 /  57;  83           34 /  54 /  74; 122     14 / 21; 30     16 / 24; 35
+//    10,000      53 /  63 /  83; 114           64 /  76 / 100; 149     24 / 33; 39     29 / 41; 47
+//    15,625      74 /  67 /  89; 107           95 /  73 / 114; 169     40 / 62; 73     51 / 78; 93
+//    25,600       - /  87 / 103; 124            - / 113 / 134; 163     38 / 38; 46     46 / 45; 53
+//    62,500       - / 174 / 173; 214            - / 210 / 218; 263     88 / 57; 64    108 / 67; 74
+//   250,000       - / 658 / 600; 597            - / 804 / 815; 803    344 / 202; 203  424 / 243; 244
 // Past some ten refills of every lane a launch's end is a small part of it. In plain r rays
-// differ less in length, and the fewest lanes whose waves of 32, 64 and 128 x SMs geodesics
-// hold the launch win (Kerr RK4, a wave of rays cut at 900 steps 26 / 38 / 64).
+// differ less in length, and the fewest lanes whose waves hold the launch win (a wave of Kerr
+// rays cut at 900 steps: RK4 15 / 22 / 32 / 64 on 8, 4, 2 lanes and 1, Verlet 10 / 23 on 4 and
+// 1, of 16, 32, 64 and 128 x SMs geodesics).
 int split_start(const RunConst& R, uint64_t n, int num_sms, bool forced) {
     const uint64_t sms = static_cast<uint64_t>(num_sms);
-    const bool rk4 = R.integrator == FOORT_INTEGRATOR_RK4;
-    if (n <= (R.rlog ? (rk4 ? 64 : 160) : rk4 ? 32 : 64) * sms) return 4;
-    if (rk4 && n <= (R.rlog ? 384 : 64) * sms) return 2;
+    if (R.integrator == FOORT_INTEGRATOR_RK4) {
+        if (n <= (R.rlog ? 72 : 32) * sms) return 8;
+        if (n <= (R.rlog ? 384 : 64) * sms) return 2;
+    } else if (n <= (R.rlog ? 160 : 64) * sms) {
+        return 4;
+    }
     return (forced || n <= 1024 * sms) ? 1 : 0;
 }
 
@@ -1022,8 +1026,8 @@ const void* fp64_pair_kernel_joh();
 const void* fp64_split_kernel_kerr(int, int);
 const void* fp64_split_kernel_joh(int, bool, int);
 
-// Four lanes per geodesic in the end: from a start with 4, 2 (RK4 only) or 1; 0: one lane to
-// the end (Johannsen with alpha13 alone).
+// Several lanes per geodesic in the end: from a start with 8 or 2 (RK4), 4 (Verlet) or 1; 0:
+// one lane to the end (Johannsen with alpha13 alone).
 const void* fp64_split_kernel(const RunConst& R, int start) {
     switch (R.metric_id) {
     case kKerr: return fp64_split_kernel_kerr(R.integrator, start);

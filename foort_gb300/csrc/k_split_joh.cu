@@ -1,4 +1,4 @@
-// FP64 kernels that end on four lanes per geodesic, metric kJohannsen.
+// FP64 kernels whose lanes share a geodesic's step, metric kJohannsen.
 #include "kernel_fp64_split.cuh"
 #include "kernels.h"
 

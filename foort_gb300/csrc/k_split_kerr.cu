@@ -1,4 +1,4 @@
-// FP64 kernels that end on four lanes per geodesic, metric kKerr.
+// FP64 kernels whose lanes share a geodesic's step, metric kKerr.
 #include "kernel_fp64_split.cuh"
 #include "kernels.h"
 

@@ -266,8 +266,8 @@ __device__ __forceinline__ bool finite4(const double a[4]) {
 //
 // LANES = 2: lanes 2k and 2k+1 integrate one geodesic together (E::step_pair). Both take the
 // same pixel, hold the same state and so leave the loop together; the even lane writes
-// the record and counts the step. LANES = 4: four lanes do, each with its component of
-// the state (E::step_split); each writes its part of the record.
+// the record and counts the step. LANES = 4 and 8: each lane has its component of the state
+// (E::step_split); each writes its part of the record.
 template <class E>
 constexpr bool is_lean(...) {
     return false;
@@ -297,10 +297,10 @@ constexpr bool is_fp64_steps(decltype(E::kFp64Steps)*) {
     return true;
 }
 
-// TAIL: once the queue is empty and a warp has at most 8 geodesics left, it hands them to
-// Tail, four lanes each (Tail::take_over).
+// TAIL: once the queue is empty and a warp has at most Tail::kLeft geodesics left, it hands
+// them to Tail::run, more lanes each.
 struct NoTail {
-    static constexpr bool kIs = false;
+    static constexpr unsigned kLeft = 0;
 };
 
 // Engines that record positions (E::kRecords): the general ones, and Recording's.
@@ -316,24 +316,24 @@ constexpr bool is_recording(decltype(E::kRecords)*) {
 template <class E, int LANES, class Tail>
 __device__ __forceinline__ void work_loop(const LaunchArgs& A, const RunConst& R, typename E::Lane& L, bool active,
                                           uint64_t idx, bool drained) {
-    static_assert(LANES == 1 || LANES == 2 || LANES == 4, "lanes per geodesic");
-    constexpr bool PAIR = LANES == 2, SPLIT = LANES == 4;
+    static_assert(LANES == 1 || LANES == 2 || LANES == 4 || LANES == 8, "lanes per geodesic");
+    constexpr bool PAIR = LANES == 2, SPLIT = LANES >= 4;
     const unsigned lane = threadIdx.x & 31u;
     const unsigned sub = lane & (LANES - 1u);
     const bool odd = sub != 0;  // not the lane that counts the geodesic
     const unsigned slot_lane = lane - sub;  // the lane that numbers the slot
     const unsigned lt_mask = (1u << slot_lane) - 1u;
-    const unsigned slots = SPLIT ? 0x11111111u : PAIR ? 0x55555555u : kFullMask;  // one bit per geodesic slot
+    const unsigned slots = kFullMask / ((1u << LANES) - 1u);  // one bit per geodesic slot
     const unsigned pmask = ((1u << LANES) - 1u) << slot_lane;
     constexpr bool kLean = is_lean<E>(nullptr);
-    constexpr bool kTail = Tail::kIs;
+    constexpr bool kTail = Tail::kLeft != 0;
     // With a tail: geodesics per warp at a time, an even share of a launch that does not fill
-    // the lanes (but the tail's 8 at least).
+    // the lanes (but the tail's at least).
     unsigned share = 32 / LANES;
     if constexpr (kTail) {
         const uint64_t warps = static_cast<uint64_t>(gridDim.x) * (blockDim.x >> 5);
         const uint64_t even = (A.n + warps - 1) / warps;
-        share = (even < 8) ? 8 : (even < share) ? static_cast<unsigned>(even) : share;
+        share = (even < Tail::kLeft) ? Tail::kLeft : (even < share) ? static_cast<unsigned>(even) : share;
     }
     ImageConst Ic;  // PAIR, E::kCopyImage: the lane's image constants in registers, copied at each refill
     bool stopping = false;
@@ -403,7 +403,7 @@ __device__ __forceinline__ void work_loop(const LaunchArgs& A, const RunConst& R
             continue;
         }
         if constexpr (kTail) {
-            if (drained && __popc(__ballot_sync(kFullMask, active) & slots) <= 8) break;
+            if (drained && __popc(__ballot_sync(kFullMask, active) & slots) <= Tail::kLeft) break;
         }
         // Integrate until a lane needs new work (while work remains) or a poll is due.
         for (;;) {
@@ -440,7 +440,7 @@ __device__ __forceinline__ void work_loop(const LaunchArgs& A, const RunConst& R
             if (idle == kFullMask) break;
             if constexpr (kTail) {
                 const unsigned left = __popc(~idle & slots);
-                if (drained ? left <= 8 : left < share && since_refill >= R.refill_steps) break;
+                if (drained ? left <= Tail::kLeft : left < share && since_refill >= R.refill_steps) break;
                 continue;
             }
             if (idle && !drained && since_refill >= R.refill_steps) break;

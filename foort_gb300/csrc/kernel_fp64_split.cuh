@@ -1,18 +1,19 @@
-// The plain FP64 kernel on four lanes per geodesic (Kerr, Johannsen), throughout or for the
-// last eight geodesics of each warp.
+// The plain FP64 kernel on four (RK4 also: eight) lanes per geodesic for Kerr and Johannsen,
+// throughout or for the last geodesics of each warp.
 //
 // An FP64 instruction occupies its scheduler's pipe for 64 cycles per warp on GB300, however
 // many lanes are active: a launch that leaves lanes idle costs the instructions of one
-// lane's step. Four lanes share a step here:
+// lane's step. Four lanes share a step here, or eight two stages of one (RK4):
 // - finite differences: lane 0 evaluates the metric at r + h, lane 1 at r - h, lane 2 at
 //   theta + h, lane 3 at theta - h (one exp, one sincos and one g_dd each instead of 3, 3
 //   and 4);
 // - lane i holds component i of position and velocity, divides out the inverse metric
 //   components that a^i needs and sums the eight terms of a^i;
 // - the step rule's three quotients are lanes 1 to 3's.
-// A step takes 0.41 (RK4) to 0.44 (Verlet) of the one-lane kernel's time while the geodesics
-// fit on the GPU (log r, 3,721 geodesics, one lane to four: Kerr RK4 82 to 34 ms, Verlet 55 to
-// 25; Johannsen 110 to 49 and 95 to 43); still bound by the FP64 instructions in series.
+// A step takes 0.41 (RK4) to 0.44 (Verlet) of the one-lane kernel's time on four lanes and
+// 0.30 on eight while the geodesics fit on the GPU (log r, 3,600 geodesics, on one, four and
+// eight lanes: Kerr RK4 83, 35 and 24 ms, Johannsen 122, 48 and 34; Verlet 30 and 14, 35 and
+// 16); still bound by the FP64 instructions in series.
 // The values are the one-lane kernel's bit for bit: each rounding is written out as the
 // compiler contracts Fp64Engine (kernel_fp64.cuh; found by comparing evaluations).
 #pragma once
@@ -143,7 +144,7 @@ struct SplitMetric<kJohannsen, A13> {
     }
 };
 
-template <int MID, bool A13, int INTEG>
+template <int MID, bool A13, int INTEG, int LANES = 4>
 struct SplitEngine {
     using Metric = SplitMetric<MID, A13>;
     static constexpr bool kSplit = true;
@@ -151,7 +152,7 @@ struct SplitEngine {
 
     struct Lane {
         double x, v;  // this lane's component
-        double C[6];  // Verlet: the lane's Christoffel symbols at the position
+        double C[INTEG == FOORT_INTEGRATOR_VERLET ? 6 : 1];  // the lane's Christoffel symbols at the position
         double lam;
         uint64_t steps;
         TermState T;
@@ -256,12 +257,13 @@ struct SplitEngine {
     }
 
     static __device__ __forceinline__ void init(Lane& L, const ImageConst& I, const RunConst& R, const foort_pixel& p,
-                                                int i, unsigned m) {
+                                                int sub, unsigned m) {
+        const int i = sub & 3;
         double x[4], v[4];
         initial_conditions(I, p, x, v);
         L.x = (i == 0) ? x[0] : (i == 1) ? x[1] : (i == 2) ? x[2] : x[3];
         L.v = (i == 0) ? v[0] : (i == 1) ? v[1] : (i == 2) ? v[2] : v[3];
-        if (INTEG == FOORT_INTEGRATOR_VERLET) {
+        if constexpr (INTEG == FOORT_INTEGRATOR_VERLET) {
             double r;
             symbols(I.m, R, x[1], x[2], i, m, L.C, r, L.C);
         }
@@ -273,13 +275,40 @@ struct SplitEngine {
         reset_lane_state(R, x, L.D, L.T);
     }
 
-    // One Geodesic::Update (Geodesic.cpp:61-88); i: this lane's component, m: the four lanes.
-    static __device__ __forceinline__ bool step_split(Lane& L, const ImageConst& I, const RunConst& R, int i, unsigned m) {
+    // One Geodesic::Update (Geodesic.cpp:61-88). sub: this lane among the geodesic's, m: those
+    // lanes; i: its component.
+    static __device__ __forceinline__ bool step_split(Lane& L, const ImageConst& I, const RunConst& R, int sub,
+                                                      unsigned m) {
+        const int i = sub & 3;
         const MetricConst& M = I.m;
         const double h = adaptive_step(R, L, i, m);
         double va[4], nx, nv, r;
         gather(L.v, m, va);
-        if (INTEG == FOORT_INTEGRATOR_RK4) {  // Integrators.cpp:51-94
+        if constexpr (LANES == 8) {
+            // The stage positions need only the velocities of earlier stages: lanes 0 to 3
+            // evaluate the symbols of stages 1 and 3, lanes 4 to 7 those of 2 and 4, and both
+            // contract them with both stages' velocities.
+            const bool odd = sub & 4;
+            const double hh = 0.5 * h, h6 = h / 6.0;
+            double C[6], l[4], k, l2, l3, l4, t;
+            t = odd ? d_fma(L.v, hh, L.x) : L.x;
+            symbols(M, R, from(t, 1, m), from(t, 2, m), i, m, C, r);
+            const double k1 = __shfl_sync(m, accel(C, va, i), i, 8);
+            l2 = d_fma(k1, hh, L.v);
+            gather(l2, m, l);
+            const double k2 = __shfl_sync(m, accel(C, l, i), i + 4, 8);
+            l3 = d_fma(k2, hh, L.v);
+            t = d_fma(odd ? l3 : l2, odd ? h : hh, L.x);
+            symbols(M, R, from(t, 1, m), from(t, 2, m), i, m, C, r);
+            gather(l3, m, l);
+            const double k3 = __shfl_sync(m, accel(C, l, i), i, 8);
+            l4 = d_fma(k3, h, L.v);
+            gather(l4, m, l);
+            const double k4 = __shfl_sync(m, accel(C, l, i), i + 4, 8);
+            nv = d_fma(d_add(d_fma(k3, 2.0, d_fma(k2, 2.0, k1)), k4), h6, L.v);
+            nx = d_fma(d_add(d_fma(l3, 2.0, d_fma(l2, 2.0, L.v)), l4), h6, L.x);
+            L.rhs += (sub == 0) ? 4 : 0;
+        } else if constexpr (INTEG == FOORT_INTEGRATOR_RK4) {  // Integrators.cpp:51-94
             const double hh = 0.5 * h, h6 = h / 6.0;
             double C[6], l[4], k1, k2, k3, k4, l2, l3, l4, t;
             symbols(M, R, from(L.x, 1, m), from(L.x, 2, m), i, m, C, r);
@@ -356,6 +385,7 @@ struct SplitEngine {
 
     // Every lane writes its component, lane 0 the rest of the record.
     static __device__ __forceinline__ void write(const Lane& L, foort_result* o, int term, uint32_t err, int i) {
+        if (i >= 4) return;
         o->pos[i] = L.x;
         o->vel[i] = L.v;
         if (i) return;
@@ -375,30 +405,59 @@ struct SplitEngine {
     }
 };
 
+// a of another lane of the warp.
+template <class T>
+__device__ __forceinline__ T from_lane(const T& a, int lane) {
+    static_assert(sizeof(T) % 4 == 0, "whole words");
+    T b;
+    uint32_t w[sizeof(T) / 4];
+    memcpy(w, &a, sizeof(T));
+#pragma unroll
+    for (unsigned k = 0; k < sizeof(T) / 4; ++k) w[k] = __shfl_sync(kFullMask, w[k], lane);
+    memcpy(&b, w, sizeof(T));
+    return b;
+}
+
+// RK4: at most 4 geodesics of a warp on four lanes each continue on eight.
+template <int MID, bool A13>
+struct OctTail {
+    using S = SplitEngine<MID, A13, FOORT_INTEGRATOR_RK4, 8>;
+    static constexpr unsigned kLeft = 4;
+
+    static __device__ __forceinline__ void run(const LaunchArgs& A, const RunConst& R,
+                                               const typename SplitEngine<MID, A13, FOORT_INTEGRATOR_RK4>::Lane& L,
+                                               unsigned left, uint64_t idx) {
+        const int lane = threadIdx.x & 31;
+        unsigned rest = left;
+        for (int k = 0; k < (lane >> 3); ++k) rest &= rest - 1;
+        const bool active = rest != 0;
+        const int src = __ffs(active ? rest : left) - 1 + (lane & 3);  // the same component's lane
+        typename S::Lane T;
+        T.x = from_lane(L.x, src);
+        T.v = from_lane(L.v, src);
+        T.lam = from_lane(L.lam, src);
+        T.steps = from_lane(L.steps, src);
+        T.T = from_lane(L.T, src);
+        T.D = from_lane(L.D, src);
+        T.err = from_lane(L.err, src);
+        T.img = from_lane(L.img, src);
+        T.term = from_lane(L.term, src);
+        work_loop<S, 8, NoTail>(A, R, T, active, from_lane(idx, src), true);
+    }
+};
+
 // The tail of a launch of Fp64Engine (one or two lanes per geodesic): at most 8 geodesics of
 // a warp continue on four lanes each, from the state between two steps. A warp's step takes
 // the same time with one geodesic left as with all its lanes busy, and the longest rays end a
 // launch alone: 62,500 Johannsen rays in FP64 Verlet 122 ms on one lane throughout, 111 on
-// four, 98 on one and then four; 10,000 Kerr rays in RK4 72 on two lanes, 67 on four, 63 on
-// two and then four.
+// four, 98 on one and then four; 15,625 Kerr rays in RK4 107 on one lane, 67 from two.
 template <int MID, bool A13, int INTEG, class Engine>
 struct SplitTail {
     using S = SplitEngine<MID, A13, INTEG>;
-    static constexpr bool kIs = true;
+    static constexpr unsigned kLeft = 8;
 
-    template <class T>
-    static __device__ __forceinline__ T from(const T& a, int lane) {
-        static_assert(sizeof(T) % 4 == 0, "whole words");
-        T b;
-        uint32_t w[sizeof(T) / 4];
-        memcpy(w, &a, sizeof(T));
-#pragma unroll
-        for (unsigned k = 0; k < sizeof(T) / 4; ++k) w[k] = __shfl_sync(kFullMask, w[k], lane);
-        memcpy(&b, w, sizeof(T));
-        return b;
-    }
     static __device__ __forceinline__ double component(const double a[4], int i, int lane) {
-        const double a0 = from(a[0], lane), a1 = from(a[1], lane), a2 = from(a[2], lane), a3 = from(a[3], lane);
+        const double a0 = from_lane(a[0], lane), a1 = from_lane(a[1], lane), a2 = from_lane(a[2], lane), a3 = from_lane(a[3], lane);
         return (i == 0) ? a0 : (i == 1) ? a1 : (i == 2) ? a2 : a3;
     }
 
@@ -410,27 +469,29 @@ struct SplitTail {
         unsigned rest = left;
         for (int k = 0; k < group; ++k) rest &= rest - 1;  // drops the groups before this one
         const bool active = rest != 0;
-        const int src = active ? __ffs(rest) - 1 : __ffs(left) - 1;
+        const int src = __ffs(active ? rest : left) - 1;
         typename S::Lane T;
         T.x = component(L.x, i, src);
         T.v = component(L.v, i, src);
-        T.lam = from(L.lam, src);
-        T.steps = from(L.steps, src);
-        T.T = from(L.T, src);
-        T.D = from(L.D, src);
-        T.err = from(L.err, src);
-        T.img = from(L.img, src);
-        T.term = from(L.term, src);
-        if (INTEG == FOORT_INTEGRATOR_VERLET) {
-            const G5 dr = from(L.P.dr, src), dh = from(L.P.dh, src), gu = from(L.P.gu, src);
+        T.lam = from_lane(L.lam, src);
+        T.steps = from_lane(L.steps, src);
+        T.T = from_lane(L.T, src);
+        T.D = from_lane(L.D, src);
+        T.err = from_lane(L.err, src);
+        T.img = from_lane(L.img, src);
+        T.term = from_lane(L.term, src);
+        if constexpr (INTEG == FOORT_INTEGRATOR_VERLET) {
+            const G5 dr = from_lane(L.P.dr, src), dh = from_lane(L.P.dh, src), gu = from_lane(L.P.gu, src);
             const double g1 = (i == 0) ? gu.tt : (i == 1) ? gu.rr : (i == 2) ? gu.hh : gu.pp;
             S::christoffel(dr, dh, g1, gu.tp, i, T.C, T.C);
         }
-        work_loop<S, 4, NoTail>(A, R, T, active, from(idx, src), true);
+        using Next = std::conditional_t<INTEG == FOORT_INTEGRATOR_RK4, OctTail<MID, A13>, NoTail>;
+        work_loop<S, 4, Next>(A, R, T, active, from_lane(idx, src), true);
     }
 };
 
-// START: lanes per geodesic until a warp has eight geodesics left; 0: one to the end (A13).
+// START: lanes per geodesic, from 1 and 2 until a warp has eight geodesics left; 0: one lane
+// to the end (A13).
 // Without the zero terms Johannsen's right-hand side saves nine divisions of 34: one-lane
 // Verlet, 176,400 rays in log r 200 to 157 ms, RK4 653 to 475; 62,500 rays of the reference's
 // debug view with the tail 98 to 79.
@@ -439,6 +500,8 @@ __global__ void __launch_bounds__(128) integrate_fp64_split_kernel(const __grid_
                                                                    const __grid_constant__ RunConst R) {
     if constexpr (START == 4) {
         persistent_loop<SplitEngine<MID, A13, INTEG>, 4>(A, R);
+    } else if constexpr (START == 8) {
+        persistent_loop<SplitEngine<MID, A13, INTEG, 8>, 8>(A, R);
     } else {
         using E = Fp64Engine<MID, INTEG, std::conditional_t<A13, SplitMetric<MID, A13>, MetricFP64<MID>>>;
         if constexpr (START == 0) {
@@ -456,16 +519,18 @@ const void* split_instance() {
 
 template <int MID, bool A13, int INTEG>
 const void* split_kernel(int start) {
-    switch (start) {
-    case 0:
-        if constexpr (A13) return split_instance<MID, A13, INTEG, 0>();
-        return nullptr;
-    case 1: return split_instance<MID, A13, INTEG, 1>();
-    case 2:
-        if constexpr (INTEG == FOORT_INTEGRATOR_RK4) return split_instance<MID, A13, INTEG, 2>();
-        return nullptr;
-    default: return split_instance<MID, A13, INTEG, 4>();
+    constexpr bool kRk4 = INTEG == FOORT_INTEGRATOR_RK4;
+    if constexpr (A13) {
+        if (start == 0) return split_instance<MID, A13, INTEG, 0>();
     }
+    if (start == 1) return split_instance<MID, A13, INTEG, 1>();
+    if constexpr (kRk4) {
+        if (start == 2) return split_instance<MID, A13, INTEG, 2>();
+        if (start == 8) return split_instance<MID, A13, INTEG, 8>();
+    } else {
+        if (start == 4) return split_instance<MID, A13, INTEG, 4>();
+    }
+    return nullptr;
 }
 
 template <int MID, bool A13>

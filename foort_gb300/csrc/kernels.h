@@ -8,8 +8,8 @@ namespace foort {
 
 // Returns the __global__ function for (metric, integrator), or nullptr.
 const void* fp64_kernel(int metric_id, int integrator);
-// four lanes per geodesic after a start with 4, 2 or 1, and two throughout; nullptr where
-// that kernel does not exist
+// four or eight lanes per geodesic after that start, and two throughout; nullptr where that
+// kernel does not exist
 const void* fp64_split_kernel(const RunConst& R, int start);
 const void* fp64_pair_kernel(int metric_id, int integrator);
 const void* mixed_kernel(int metric_id, int integrator);

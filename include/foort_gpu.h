@@ -286,7 +286,7 @@ int foort_gpu_cancel(foort_ctx* ctx);
  * built-in rule (128 threads, as many CTAs as fit) where the cache has none. */
 int foort_gpu_set_launch(foort_ctx* ctx, uint32_t block_size, uint32_t blocks_per_sm);
 
-/* Lanes per geodesic: 0 chooses per launch, 1 one lane, 2 several (two or four) where such
+/* Lanes per geodesic: 0 chooses per launch, 1 one lane, 2 several (two to eight) where such
  * a kernel exists: RK4 except Manko-Novikov's, Kerr's and Johannsen's FP64 Verlet; other
  * configurations always use one. Small launches take several: a step's latency then sets
  * the pace, and lanes that share a step's metric work shorten it. Results are the same

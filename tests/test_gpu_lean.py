@@ -209,9 +209,9 @@ def several_lanes_and_one(eng, d, px, **run):
     (abi.METRIC_JOHANNSEN, (0.9, 0.4, 0.0, 0.0, 0.0), 0, 30.0, 2, 3000, abi.INTEGRATOR_RK4, 0.001),
     (abi.METRIC_JOHANNSEN, (0.9, 0.4, 0.0, 0.0, 0.0), 1, 30.0, 2, 0, abi.INTEGRATOR_VERLET, 0.001),
 ])
-def test_four_lanes_in_fp64_give_the_one_lane_results(eng, metric, params, rlog, inclination, side, timeout, integrator,
-                                                      tolerance):
-    """The FP64 kernels that share a step between four lanes write each rounding out as the
+def test_shared_steps_in_fp64_give_the_one_lane_results(eng, metric, params, rlog, inclination, side, timeout,
+                                                        integrator, tolerance):
+    """The FP64 kernels that share a step between four or eight lanes write each rounding out as the
     one-lane kernel has it: the same records bit for bit, and the same counts."""
     d, keep = describe(metric, params, rlog, inclination, integrator=integrator, timeout=timeout)
     d.precision, d.verlet_tol = abi.PREC_FP64, tolerance
@@ -223,7 +223,7 @@ def test_four_lanes_in_fp64_give_the_one_lane_results(eng, metric, params, rlog,
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("metric,integrator,side", [
-    (abi.METRIC_KERR, abi.INTEGRATOR_RK4, 60),         # four lanes from the start
+    (abi.METRIC_KERR, abi.INTEGRATOR_RK4, 60),         # eight lanes from the start
     (abi.METRIC_KERR, abi.INTEGRATOR_RK4, 100),        # from two
     (abi.METRIC_KERR, abi.INTEGRATOR_RK4, 180),        # from one
     (abi.METRIC_KERR, abi.INTEGRATOR_VERLET, 120),     # from one
@@ -232,7 +232,7 @@ def test_four_lanes_in_fp64_give_the_one_lane_results(eng, metric, params, rlog,
     (abi.METRIC_JOHANNSEN, abi.INTEGRATOR_VERLET, 120),
 ])
 def test_fp64_lanes_are_refilled_and_run_two_images(eng, metric, integrator, side):
-    """More pixels than the kernels that end on four lanes hold at a time, two images side by
+    """More pixels than the kernels with shared steps hold at a time, two images side by
     side: one lane, several lanes and the built-in choice give the same records, also where
     a step budget ends some of them."""
     d, _ = describe(metric, (0.9,), 1, 70.0, integrator=integrator, timeout=600)
