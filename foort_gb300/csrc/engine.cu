@@ -295,8 +295,8 @@ uint64_t pair_limit(const RunConst& R, bool positions, int per_sm, int num_sms, 
     return static_cast<uint64_t>(per_sm) * sms * bs / 2;
 }
 
-// Lanes per geodesic that an FP64 launch of Kerr or Johannsen starts with in the kernels of
-// kernel_fp64_split.cuh: 8 or 2 (RK4), 4 (Verlet) or 1; 0: one lane to the end, unless several
+// Lanes per geodesic that an FP64 launch of Kerr or Johannsen starts with in the kernels whose
+// lanes share a step (kernel_fp64_split.cuh): 8 or 2 (RK4), 4 (Verlet) or 1; 0: one lane to the end, unless several
 // lanes are forced. The most lanes finish a step soonest but cost more instructions per
 // geodesic. ms in log r (the plain kernel on one lane last):
 //               RK4 from 8 / 2 / 1: Kerr       Johannsen            Verlet from 4 / 1: Kerr, Johannsen
@@ -310,8 +310,16 @@ uint64_t pair_limit(const RunConst& R, bool positions, int per_sm, int num_sms, 
 // differ less in length, and the fewest lanes whose waves hold the launch win (a wave of Kerr
 // rays cut at 900 steps: RK4 15 / 22 / 32 / 64 on 8, 4, 2 lanes and 1, Verlet 10 / 23 on 4 and
 // 1, of 16, 32, 64 and 128 x SMs geodesics).
+// FP64-analytic Kerr in RK4 starts with 8 or 2 lanes (0: select_pair_kernel's or one): eight
+// share less of a step there, and pay for a wave or two (ms on 8 lanes, on 2 and then 8, on 2:
+// log r, 4,096 geodesics 33 / 39 / 40, 6,400 48 / 43 / 46, 15,625 88 / 61 / 67, 62,500 - / 113 /
+// 114; plain r cut at 900 steps, 1,600 15 / 20 / 20, 4,096 25 / 22 / 20).
 int split_start(const RunConst& R, uint64_t n, int num_sms, bool forced) {
     const uint64_t sms = static_cast<uint64_t>(num_sms);
+    if (R.precision == FOORT_PREC_FP64_ANALYTIC) {
+        if (n <= (R.rlog ? 32 : 16) * sms) return 8;
+        return (R.rlog && n <= 512 * sms) ? 2 : 0;
+    }
     if (R.integrator == FOORT_INTEGRATOR_RK4) {
         if (n <= (R.rlog ? 72 : 32) * sms) return 8;
         if (n <= (R.rlog ? 384 : 64) * sms) return 2;
@@ -350,9 +358,11 @@ int choose_launch(foort_ctx* ctx, const RunConst& R, uint64_t n, int num_sms, co
     int per_sm = 0, rc = 0;
     uint32_t lanes = 1;    // 2 stands for several, as in foort_launch_shape
     uint64_t threads = n;  // to hold every geodesic at once
-    const bool may_split = R.precision == FOORT_PREC_FP64 && !positions && want.lanes != 1;
+    const bool may_split = R.precision != FOORT_PREC_MIXED && !positions && want.lanes != 1;
     const int start = may_split ? split_start(R, n, num_sms, want.lanes == 2) : 0;
-    const void* split = may_split ? fp64_split_kernel(R, start) : nullptr;
+    const void* split = !may_split                        ? nullptr
+                        : R.precision == FOORT_PREC_FP64 ? fp64_split_kernel(R, start)
+                                                         : analytic_split_kernel(R, start);
     const void* pair = (split || want.lanes == 1) ? nullptr : select_pair_kernel(R, positions);
     if (split) {
         fn = split;

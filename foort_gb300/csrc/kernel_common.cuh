@@ -297,6 +297,19 @@ constexpr bool is_fp64_steps(decltype(E::kFp64Steps)*) {
     return true;
 }
 
+// a of another lane of the warp.
+template <class T>
+__device__ __forceinline__ T from_lane(const T& a, int lane) {
+    static_assert(sizeof(T) % 4 == 0, "whole words");
+    T b;
+    uint32_t w[sizeof(T) / 4];
+    memcpy(w, &a, sizeof(T));
+#pragma unroll
+    for (unsigned k = 0; k < sizeof(T) / 4; ++k) w[k] = __shfl_sync(kFullMask, w[k], lane);
+    memcpy(&b, w, sizeof(T));
+    return b;
+}
+
 // TAIL: once the queue is empty and a warp has at most Tail::kLeft geodesics left, it hands
 // them to Tail::run, more lanes each.
 struct NoTail {
@@ -410,7 +423,11 @@ __device__ __forceinline__ void work_loop(const LaunchArgs& A, const RunConst& R
             if (active) {
                 bool more;
                 if constexpr (SPLIT) {
-                    more = E::step_split(L, A.images[L.img], R, sub, pmask);
+                    if constexpr (kLean) {
+                        more = E::step_split(L, R, sub, pmask);
+                    } else {
+                        more = E::step_split(L, A.images[L.img], R, sub, pmask);
+                    }
                 } else if constexpr (PAIR && kLean) {
                     more = E::step_pair(L, R, odd, pmask);
                 } else if constexpr (PAIR) {

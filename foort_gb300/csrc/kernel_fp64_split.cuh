@@ -405,19 +405,6 @@ struct SplitEngine {
     }
 };
 
-// a of another lane of the warp.
-template <class T>
-__device__ __forceinline__ T from_lane(const T& a, int lane) {
-    static_assert(sizeof(T) % 4 == 0, "whole words");
-    T b;
-    uint32_t w[sizeof(T) / 4];
-    memcpy(w, &a, sizeof(T));
-#pragma unroll
-    for (unsigned k = 0; k < sizeof(T) / 4; ++k) w[k] = __shfl_sync(kFullMask, w[k], lane);
-    memcpy(&b, w, sizeof(T));
-    return b;
-}
-
 // RK4: at most 4 geodesics of a warp on four lanes each continue on eight.
 template <int MID, bool A13>
 struct OctTail {

@@ -683,6 +683,150 @@ struct AnalyticPairEngine : LeanState<ImageRef> {
     }
 };
 
+// The same on eight lanes: lanes 0 to 3 hold stages 1 and 3, lanes 4 to 7 stages 2 and 4. Each
+// evaluates its stage's metric part; lane i of four contracts, sums and rounds component i.
+// accel_lean<0>'s roundings, with a product alone as fma(x, y, -0): the pair's values. The
+// metric part, over half of a step, is the same on all four lanes; the rest is a quarter:
+// 4,096 Kerr rays in log r 40 ms on two lanes, 33 on eight.
+struct SplitK {
+    double k, F;  // a^i, and the sum it is the inverse metric's product with
+};
+struct SplitTwoK {
+    double a, b, bg, bf;
+};
+static __device__ __forceinline__ double lane4(double a, int lane, unsigned m) { return __shfl_sync(m, a, lane, 4); }
+
+static __device__ __forceinline__ SplitK contract_split(const MetricAt<double>& m, bool rlog, double u, int i,
+                                                        unsigned pmask) {
+    const bool ends = i == 0 || i == 3;
+    double v[4], w1s[4], w2s[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[k] = lane4(u, k, pmask);
+    const double ua = ends ? v[0] : u;
+    auto lower = [&](const G5T<double>& d) {
+        const double A = (i == 0) ? d.tt : (i == 1) ? d.rr : (i == 2) ? d.hh : d.tp, B = (i == 0) ? d.tp : d.pp;
+        const double p = __dmul_rn(B, v[3]);
+        return __fma_rn(A, ua, ends ? p : -0.0);
+    };
+    const double w1 = lower(m.d1), w2 = lower(m.d2);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        w1s[k] = lane4(w1, k, pmask);
+        w2s[k] = lane4(w2, k, pmask);
+    }
+    auto of = [&](int k) { return (i == 2) ? w2s[k] : w1s[k]; };
+    const double qa = __fma_rn(v[0], of(0), __dmul_rn(v[1], of(1))), qh = __dmul_rn(v[2], of(2));
+    const double qb = __fma_rn((i == 2) ? 1.0 : v[2], (i == 2) ? qh : of(2), qa);  // q2's product is rounded
+    const double q = __fma_rn(v[3], of(3), qb);
+    const double s = __fma_rn(v[1], w1, __dmul_rn(v[2], w2));
+    SplitK k;
+    const double sq = __fma_rn(2.0, s, -q);
+    k.F = ends ? s : sq;
+    const double Ft = lane4(k.F, 0, pmask), Fp = lane4(k.F, 3, pmask);
+    const double c1 = (i == 0) ? m.gu.tt : (i == 1) ? m.gu.rr : (i == 2) ? m.gu.hh : m.gu.tp;
+    const double p = __dmul_rn((i == 0) ? m.gu.tp : m.gu.pp, Fp);
+    k.k = __fma_rn(c1, ends ? Ft : k.F, ends ? p : -0.0);
+    k.k = ends ? -k.k : k.k;
+    if (rlog) {
+        const double al = __fma_rn(-u, u, k.k);
+        k.k = (i == 1) ? al : k.k;
+    }
+    return k;
+}
+
+// As round_fp64: a of lanes 0 to 3, b of lanes 4 to 7.
+template <int MID>
+__device__ __noinline__ SplitTwoK round_split(const double* q, const MixedConst& mc, bool rlog, double x, double uf,
+                                              double u, double t, int i, unsigned pmask) {
+    MetricAt<double> m = metric_part_d<MID>(q, mc, rlog, lane4(x, 1, pmask), lane4(x, 2, pmask));
+    m.gu.rr = __dmul_rn(-0.5, m.gu.rr);
+    m.gu.hh = __dmul_rn(-0.5, m.gu.hh);
+    SplitTwoK k;
+    k.a = __shfl_sync(pmask, contract_split(m, rlog, u, i, pmask).k, i, 8);
+    const SplitK b = contract_split(m, rlog, __fma_rn(t, k.a, uf), i, pmask);
+    k.b = __shfl_sync(pmask, b.k, i + 4, 8);
+    k.bg = __shfl_sync(pmask, m.gu.hh, i + 4, 8);
+    k.bf = __shfl_sync(pmask, b.F, i + 4, 8);
+    return k;
+}
+
+template <int MID>
+struct AnalyticSplitEngine : LeanState<ImageRef> {
+    static constexpr unsigned kRhsPerStep = 4;
+    static constexpr bool kFp64Steps = true;
+
+    static __device__ __forceinline__ double own(const f2 h[2], const f2 l[2], int i) {
+        const f2 a = (i == 0 || i == 3) ? h[0] : h[1], b = (i == 0 || i == 3) ? l[0] : l[1];
+        return (i < 2) ? ff_d({lo2(a), lo2(b)}) : ff_d({hi2(a), hi2(b)});
+    }
+    // Every lane gets the four components, in parts.
+    static __device__ __forceinline__ void share(double a, unsigned pmask, f2 h[2], f2 l[2]) {
+        const ff f = ff_from_d(a);
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            h[k] = pack2(__shfl_sync(pmask, f.hi, k, 4), __shfl_sync(pmask, f.hi, 3 - k, 4));
+            l[k] = pack2(__shfl_sync(pmask, f.lo, k, 4), __shfl_sync(pmask, f.lo, 3 - k, 4));
+        }
+    }
+    // adaptive_step_fp64: lanes 1 to 3 each divide for their component.
+    static __device__ __forceinline__ double step_size(const RunConst& R, double x, double u, int i, unsigned pmask) {
+        const double pt = __dsub_rn(kRefPi, x), mth = (pt < x) ? pt : x;
+        const double num = (i == 2) ? __dmul_rn(R.eps, mth) : R.eps;
+        const double w = 1 / fabs(num / fabs(__dadd_rn((i == 3) ? u : fabs(u), 1e-20)));
+        const double h = 1 / __dadd_rn(__dadd_rn(lane4(w, 1, pmask), lane4(w, 2, pmask)), lane4(w, 3, pmask));
+        return (h < R.hmin) ? R.hmin : h;
+    }
+
+    static __device__ __forceinline__ void init(Lane& L, const ImageConst& I, const RunConst& R, const foort_pixel& p,
+                                                int, unsigned) {
+        LeanState<ImageRef>::init(L, I, R, p);
+    }
+    static __device__ __forceinline__ bool step_split(Lane& L, const RunConst& R, int sub, unsigned pmask) {
+        const bool rlog = R.rlog != 0, odd = sub & 4;
+        const int i = sub & 3;
+        const double x = own(L.xh, L.xl, i), u = own(L.vh, L.vl, i);
+        const double h = step_size(R, x, u, i, pmask), hh = 0.5 * h;
+        auto ahead = [](double a, double t, double b) { return __fma_rn(t, b, a); };  // a + t b
+        const SplitTwoK k12 =
+            round_split<MID>(L.c.qa, *L.c.mx, rlog, odd ? ahead(x, hh, u) : x, u, u, hh, i, pmask);
+        const SplitTwoK k34 =
+            round_split<MID>(L.c.qa, *L.c.mx, rlog, ahead(x, odd ? h : hh, ahead(u, hh, odd ? k12.b : k12.a)), u,
+                             ahead(u, hh, k12.b), h, i, pmask);
+        const double h6 = h / 6.0, hh6 = __dmul_rn(h, h6);
+        const double s3 = __fma_rn(k34.a, 2.0, __fma_rn(k12.b, 2.0, k12.a));
+        // as the pair's: k4 of theta joins unrounded
+        const double dv = __dmul_rn(__fma_rn((i == 2) ? k34.bg : 1.0, (i == 2) ? k34.bf : k34.b, s3), h6);
+        const double dx = __fma_rn(u, h, __dmul_rn(__dadd_rn(__dadd_rn(k12.a, k12.b), k34.a), hh6));
+        share(__dadd_rn(x, dx), pmask, L.xh, L.xl);
+        share(__dadd_rn(u, dv), pmask, L.vh, L.vl);
+        return after_step(L, R, ff_add(L.lam, ff_from_d(h)));
+    }
+    static __device__ __forceinline__ void finish(const Lane& L, const RunConst& R, foort_result* o, int sub) {
+        if (sub == 0) LeanState<ImageRef>::finish(L, R, o);
+    }
+    static __device__ __forceinline__ void stop(const Lane& L, const RunConst& R, foort_result* o, uint32_t err,
+                                                int sub) {
+        if (sub == 0) LeanState<ImageRef>::stop(L, R, o, err);
+    }
+};
+
+// The tail of a launch of AnalyticPairEngine: a warp's last four geodesics, eight lanes each.
+template <int MID>
+struct AnalyticTail {
+    using S = AnalyticSplitEngine<MID>;
+    static constexpr unsigned kLeft = 4;
+
+    static __device__ __forceinline__ void run(const LaunchArgs& A, const RunConst& R, const typename S::Lane& L,
+                                               unsigned left, uint64_t idx) {
+        unsigned rest = left;
+        for (unsigned k = 0; k < (threadIdx.x & 31) >> 3; ++k) rest &= rest - 1;
+        const bool active = rest != 0;
+        const int src = __ffs(active ? rest : left) - 1;
+        typename S::Lane T = from_lane(L, src);
+        work_loop<S, 8, NoTail>(A, R, T, active, from_lane(idx, src), true);
+    }
+};
+
 // A lean engine that records positions (Fp64Engine's and MixedEngine's samples): the second
 // pass of foort_gpu_positions takes the first one's steps. 3,600 Kerr rays in Verlet, ln r, 25
 // positions kept of each: 2.06 ms with the general kernel, 1.25 with this (1.09 without
@@ -719,10 +863,10 @@ struct Recording : E {
     }
 };
 
-template <class E, int LANES, int CTAS>
+template <class E, int LANES, int CTAS, class Tail = NoTail>
 __global__ void __launch_bounds__(128, CTAS) integrate_lean_kernel(const __grid_constant__ LaunchArgs A,
                                                                    const __grid_constant__ RunConst R) {
-    persistent_loop<E, LANES>(A, R);
+    persistent_loop<E, LANES, Tail>(A, R);
 }
 
 template <class E, int LANES, int CTAS = 1>

@@ -22,6 +22,10 @@ const void* mixed_pair_kernel_variant(int metric_id, int integrator, bool decide
 // or nullptr where they need the general one.
 const void* mixed_lean_kernel(const RunConst& R, bool pair, bool positions);
 
+// FP64-analytic: eight lanes per geodesic, throughout (start 8) or for the last ones of a warp
+// (start 2); nullptr where that kernel does not exist.
+const void* analytic_split_kernel(const RunConst& R, int start);
+
 // Host-side helpers of the mixed-precision kernels (per-image FP32 constants).
 void fill_mixed_constants(int metric_id, ImageConst& ic, const RunConst& rc);
 void fill_mixed_run(RunConst& rc);

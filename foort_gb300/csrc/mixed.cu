@@ -54,6 +54,7 @@ const void* mixed_lean_verlet_kernel_joh13(bool rlog, bool positions);
 const void* mixed_lean_verlet_kernel_flat(bool positions);
 const void* mixed_lean_pair_kernel_rl(bool positions);
 const void* analytic_pair_kernel_kerr(bool positions);
+const void* analytic_split_kernel_kerr(int start);
 const void* analytic_pair_kernel_joh(bool positions);
 const void* analytic_pair_kernel_flat(bool positions);
 
@@ -104,6 +105,13 @@ const void* mixed_lean_kernel(const RunConst& R, bool pair, bool positions) {
     case kRasheedLarsen: return pair ? mixed_lean_pair_kernel_rl(positions) : nullptr;
     default: return nullptr;
     }
+}
+
+const void* analytic_split_kernel(const RunConst& R, int start) {
+    if (R.precision != FOORT_PREC_FP64_ANALYTIC || R.integrator != FOORT_INTEGRATOR_RK4 || R.metric_id != kKerr ||
+        !lean_options(R))
+        return nullptr;
+    return (start == 8 || start == 2) ? analytic_split_kernel_kerr(start) : nullptr;
 }
 
 void fill_mixed_run(RunConst& rc) {

@@ -222,21 +222,23 @@ def test_shared_steps_in_fp64_give_the_one_lane_results(eng, metric, params, rlo
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("metric,integrator,side", [
-    (abi.METRIC_KERR, abi.INTEGRATOR_RK4, 60),         # eight lanes from the start
-    (abi.METRIC_KERR, abi.INTEGRATOR_RK4, 100),        # from two
-    (abi.METRIC_KERR, abi.INTEGRATOR_RK4, 180),        # from one
-    (abi.METRIC_KERR, abi.INTEGRATOR_VERLET, 120),     # from one
-    (abi.METRIC_JOHANNSEN, abi.INTEGRATOR_RK4, 100),
-    (abi.METRIC_JOHANNSEN, abi.INTEGRATOR_VERLET, 100),
-    (abi.METRIC_JOHANNSEN, abi.INTEGRATOR_VERLET, 120),
+@pytest.mark.parametrize("metric,integrator,side,precision", [
+    (abi.METRIC_KERR, abi.INTEGRATOR_RK4, 60, abi.PREC_FP64),        # eight lanes from the start
+    (abi.METRIC_KERR, abi.INTEGRATOR_RK4, 100, abi.PREC_FP64),       # from two
+    (abi.METRIC_KERR, abi.INTEGRATOR_RK4, 180, abi.PREC_FP64),       # from one
+    (abi.METRIC_KERR, abi.INTEGRATOR_VERLET, 120, abi.PREC_FP64),    # from one
+    (abi.METRIC_JOHANNSEN, abi.INTEGRATOR_RK4, 100, abi.PREC_FP64),
+    (abi.METRIC_JOHANNSEN, abi.INTEGRATOR_VERLET, 100, abi.PREC_FP64),
+    (abi.METRIC_JOHANNSEN, abi.INTEGRATOR_VERLET, 120, abi.PREC_FP64),
+    (abi.METRIC_KERR, abi.INTEGRATOR_RK4, 40, abi.PREC_FP64_ANALYTIC),   # eight from the start
+    (abi.METRIC_KERR, abi.INTEGRATOR_RK4, 120, abi.PREC_FP64_ANALYTIC),  # from two
 ])
-def test_fp64_lanes_are_refilled_and_run_two_images(eng, metric, integrator, side):
+def test_fp64_lanes_are_refilled_and_run_two_images(eng, metric, integrator, side, precision):
     """More pixels than the kernels with shared steps hold at a time, two images side by
     side: one lane, several lanes and the built-in choice give the same records, also where
     a step budget ends some of them."""
     d, _ = describe(metric, (0.9,), 1, 70.0, integrator=integrator, timeout=600)
-    d.precision = abi.PREC_FP64
+    d.precision = precision
     pars = [(a,) if metric == abi.METRIC_KERR else (a, 0.5, 0.0, 0.0, 0.0) for a in (0.9, 0.2)]
     keep = abi.attach_images(d, [abi.make_image(p, r=1000.0, theta=1.2, half_width=8.0) for p in pars])
     px = np.concatenate([abi.square_pixels(side, image=i) for i in (0, 1)])
