@@ -884,8 +884,15 @@ int foort_gpu_run_launch(const foort_ctx* ctx, uint32_t k, foort_pixel* out, uin
 }
 
 uint32_t foort_ctx_schedule(const foort_ctx* ctx) { return ctx->schedule; }
+// Automatic: one warp per scheduler at a geodesic per lane, or two with the one-lane lean
+// kernel in plain r (19,456 Kerr geodesics 0.99 us a step, 58,000 2.1), where a launch saved
+// is a ray's 67 ms: adaptive runs of 19,000 to 37,000 geodesics with caps of 128 and 256 x SMs
+// 202 and 198, 270 and 210, 197 and 197, 185 and 185 ms (with 320: 197, 209, 243, 186).
 uint64_t foort_ctx_lookahead(const foort_ctx* ctx) {
-    return ctx->lookahead == FOORT_LOOKAHEAD_AUTO ? 128ull * static_cast<uint64_t>(ctx->num_sms) : ctx->lookahead;
+    if (ctx->lookahead != FOORT_LOOKAHEAD_AUTO) return ctx->lookahead;
+    const RunConst& R = ctx->rc;
+    const bool lean = !R.rlog && (R.metric_id == kKerr || R.metric_id == kFlat) && mixed_lean_kernel(R, false, false);
+    return (lean ? 256ull : 128ull) * static_cast<uint64_t>(ctx->num_sms);
 }
 void foort_ctx_launched(foort_ctx* ctx, const foort_pixel* px, uint64_t n, bool first) {
     if (first) ctx->launch_px.clear();
