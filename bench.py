@@ -65,15 +65,15 @@ OPS_PER_STEP = {("kerr", "rk4"): 1130, ("johannsen", "rk4"): 1650, ("johannsen",
 SINCOS_PER_STEP = {("kerr", "rk4"): 20, ("johannsen", "rk4"): 20, ("johannsen", "verlet"): 10}
 OPS_PER_EXTRA_VERLET_RHS = 380
 # DRAM traffic per geodesic of the mixed kernel: dram__bytes_read.sum + dram__bytes_write.sum
-# of one ncu capture of the two-lane kernel on a 6,000-pixel sample of the C2 grid, divided
-# by its geodesics
-DRAM_BYTES_PER_GEODESIC = {("kerr", "rk4"): 120.4}
-# Executed thread instructions per geodesic step of the mixed kernel (ncu
-# smsp__inst_executed x 32 / steps): two lanes of ~929 each and one lane of 1,270 on a
-# 6,000-pixel sample of the C2 grid; Johannsen Verlet (one lane) 1,754 on 20,000 pixels
-# of C4's. With the GPU's issue rate (one warp instruction per cycle on each of its
+# of one ncu capture of the lean kernel on a 6,000-pixel sample of the C2 grid, divided by its
+# geodesics (the records stay in L2)
+DRAM_BYTES_PER_GEODESIC = {("kerr", "rk4"): 44.0}
+# Executed thread instructions per geodesic step of the lean mixed kernels (ncu
+# smsp__inst_executed x 32 / steps; many are packed, two operations each): one lane of 855 on
+# a 6,000-pixel sample of the C2 grid and two of ~686 each on 3,000; Johannsen Verlet (one
+# lane, alpha13 alone) 871 on 20,000 pixels of C4's. With the GPU's issue rate (one warp instruction per cycle on each of its
 # 4 x 152 sub-partitions) they give the fraction of issue slots the path fills.
-EXEC_INSTR_PER_STEP = {("kerr", "rk4", 2): 1857, ("kerr", "rk4", 1): 1270, ("johannsen", "verlet", 1): 1754}
+EXEC_INSTR_PER_STEP = {("kerr", "rk4", 2): 1372, ("kerr", "rk4", 1): 855, ("johannsen", "verlet", 1): 871}
 SUBPARTITIONS = 4
 # runs of more geodesics take the FP64 legs on a seeded sample (1 %, at least 20,000)
 FP64_SAMPLE_ABOVE = 60000
@@ -776,7 +776,7 @@ def main():
                 "ops_per_step": ops, "sincos_per_step": SINCOS_PER_STEP.get(mkind, 20),
                 "peak_source": "FP32 FMA microbenchmark on this GPU (foort_measure_peaks); MEASURED_PEAKS.json "
                                "has no FP32/FP64 entry",
-                "kernel": "integrate_mixed_pair_kernel" if mixed_lanes[big] == 2 else "integrate_mixed_kernel",
+                "kernel": "integrate_lean_kernel",
                 "lanes_per_geodesic": mixed_lanes,
                 "largest_launch": {"geodesics": len(launches_px[big]), "launch_ms": big_ms, "steps": big_steps,
                                    "achieved": big_ops / (big_ms * 1e-3) / 1e12,
@@ -785,7 +785,7 @@ def main():
                                                               if k[:2] == mkind},
                              "warp_instructions_per_s": issue, "issue_peak_per_s": issue_peak,
                              "issue_frac": issue / issue_peak if instr else None,
-                             "source": "instructions per step from ncu captures (C2: 6,000-pixel sample; "
+                             "source": "instructions per step from ncu captures (C2: 6,000- and 3,000-pixel samples; "
                                        "Johannsen Verlet: 20,000 C4 pixels); issue peak = 4 x SMs x median SM clock"},
                 "fp64_peak_tflops": peaks[1]}
 
