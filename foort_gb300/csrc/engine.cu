@@ -265,9 +265,7 @@ struct LaunchShape {
 //   many lanes are active, so two lanes halve the metric work of a launch that leaves lanes
 //   idle, and shorten the last rays of a larger one. Past several refills they only add the
 //   parts that both lanes do: FP64-analytic Kerr in log r, 25,600 geodesics 82 ms on one lane
-//   and 69 on two, 62,500 123 and 111, 90,000 133 and 154. Johannsen's FP64-analytic body is
-//   called, and two lanes call it half as often each: every size (25,600 273 and 186, 250,000
-//   1,411 and 1,198). In plain r rays differ less in length, and a wave of two lanes each
+//   and 69 on two, 62,500 123 and 111, 90,000 133 and 154. In plain r rays differ less in length, and a wave of two lanes each
 //   (64 x SMs) is the most that pays (flat space in FP64, 9,604 rays cut at 900 steps 20 ms on
 //   two lanes and 29 on one, 19,044 42 and 29).
 // - Lean kernels: one lane already evaluates two stages at a time, so two lanes pay only
@@ -285,7 +283,6 @@ struct LaunchShape {
 //   than the general one-lane kernel: every size.
 uint64_t pair_limit(const RunConst& R, bool positions, int per_sm, int num_sms, uint32_t bs) {
     const uint64_t sms = static_cast<uint64_t>(num_sms);
-    if (R.precision == FOORT_PREC_FP64_ANALYTIC && R.metric_id == kJohannsen) return UINT64_MAX;
     if (R.precision != FOORT_PREC_MIXED) return (R.rlog ? 512 : 64) * sms;
     if (mixed_lean_kernel(R, true, positions)) {
         if (!mixed_lean_kernel(R, false, positions)) return UINT64_MAX;

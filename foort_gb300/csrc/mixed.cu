@@ -55,7 +55,6 @@ const void* mixed_lean_verlet_kernel_flat(bool positions);
 const void* mixed_lean_pair_kernel_rl(bool positions);
 const void* analytic_pair_kernel_kerr(bool positions);
 const void* analytic_split_kernel_kerr(int start);
-const void* analytic_pair_kernel_joh(bool positions);
 const void* analytic_pair_kernel_flat(bool positions);
 
 // Lean options: every termination and diagnostic in use updates at each step (the
@@ -89,7 +88,6 @@ const void* mixed_lean_kernel(const RunConst& R, bool pair, bool positions) {
         if (!pair) return nullptr;
         switch (R.metric_id) {
         case kKerr: return analytic_pair_kernel_kerr(positions);
-        case kJohannsen: return analytic_pair_kernel_joh(positions);
         case kFlat: return analytic_pair_kernel_flat(positions);
         default: return nullptr;
         }
