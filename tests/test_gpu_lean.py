@@ -278,3 +278,32 @@ def test_lean_kernels_record_the_general_kernels_positions(eng, metric, params, 
         np.testing.assert_array_equal(got[name][1], got["general"][1])
     assert np.isfinite(got["general"][1]).all()
     del keep
+
+
+# rays whose last step overflows FP32: a velocity iteration that diverges before the horizon,
+# a step from the rotation axis that ends at an infinite theta
+@pytest.mark.gpu
+@pytest.mark.parametrize("view,seed,pixel", [
+    (dict(integrator="verlet", side=82, a=0.0877, inclination=15.93, half_width=12.989, diags="all"), 89670267,
+     (4468 // 82, 4468 % 82, 82)),
+    (dict(integrator="rk4", side=42, a=0.0693, inclination=12.78, half_width=9.337, diags="quadrant+passes"), 855370547,
+     (164, 326, 329)),
+])
+def test_lean_kernels_overflow_where_the_general_ones_do(eng, view, seed, pixel):
+    import importlib.util
+    spec = importlib.util.spec_from_file_location("performance_cases", os.path.join(ROOT, "perf", "cases.py"))
+    cases = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(cases)
+    case = dict(call="integrate", metric="kerr", precision="mixed", logr=False, alpha13=0.0, alpha3=0.0, tolerance=0.001,
+                timeout=100000)
+    case.update(view)
+    state = cases.prepare(case, seed)
+    d, px = state["desc"], np.zeros(1, dtype=abi.PIXEL_DTYPE)
+    px["row"], px["col"], px["grid"] = pixel
+    got = {}
+    for options in (0, abi.MIXED_FP64_DECISIONS):
+        d.mixed_options = options
+        with eng.Engine(d) as e:
+            got[options] = e.integrate(px)
+    assert got[0]["err"][0] & abi.ERR_NONFINITE
+    same_records(got[0], got[abi.MIXED_FP64_DECISIONS])
