@@ -70,12 +70,14 @@ FOORT_DEFINE_PACKED_METRIC(kJohannsen, JOHANNSEN13)
 // accel_part (kernel_mixed.cuh) with the compiler's contraction written out. Where a sum has
 // two products, it depends on the code around which of them joins as a fused multiply-add:
 // FORM 0 is the step with an inlined plugin, 1 and 2 the called right-hand side of
-// Johannsen and of Rasheed-Larsen. m.gu.rr and m.gu.hh come multiplied by -1/2; the other
-// factors of 2 and 1/2, which are exact, are left out where they cancel.
-// a[2] is the product of m.gu.hh and *f2 (where asked for). SCALED keeps those factors, so that
-// sums overflow where the general kernel's do: Verlet's velocity iteration diverges inside the
-// last step before some horizons.
-template <int FORM, typename T, bool SCALED = false>
+// Johannsen and of Rasheed-Larsen. m.gu.rr and m.gu.hh come multiplied by -1/2. The other
+// factors of 2 and -1/2 change no rounding, but they are multiplied out as the general kernel
+// does: where a sum is within a factor of 2 of the type's largest value its double overflows, and the
+// ray ends otherwise than with the factors left out (steps that diverge next to the axis or
+// inside a horizon). They cost 1 % of a Kerr launch (RK4, eight images 583 -> 589 ms) and 2 % of
+// Johannsen's in Verlet (147,456 rays 281 -> 286 ms).
+// a[2] is the product of m.gu.hh and *f2 (where asked for).
+template <int FORM, typename T>
 __device__ __forceinline__ void accel_lean(const MetricAt<T>& m, const T u[4], T a[4], T* f2 = nullptr) {
     // x y + z w with the first or the second product fused
     auto first = [](T x, T y, T z, T w) { return p_fma(x, y, p_mul(z, w)); };
@@ -90,18 +92,13 @@ __device__ __forceinline__ void accel_lean(const MetricAt<T>& m, const T u[4], T
     const T q2a = first(u[0], w2t, u[1], w2r);
     const T q2b = FORM ? p_fma(u[2], w2h, q2a) : p_add(q2a, p_mul(u[2], w2h));
     const T q2 = p_fma(u[3], w2p, q2b);
-    const T Ft = kSecond ? second(u[1], w1t, u[2], w2t) : first(u[1], w1t, u[2], w2t);
-    const T Fp = kSecond ? second(u[1], w1p, u[2], w2p) : first(u[1], w1p, u[2], w2p);
-    const T Fr = p_fma(T(2), first(u[1], w1r, u[2], w2r), -q1);
-    const T Fh = p_fma(T(2), kSecond ? second(u[1], w1h, u[2], w2h) : first(u[1], w1h, u[2], w2h), -q2);
-    if constexpr (SCALED) {
-        const T F2t = p_mul(T(2), Ft), F2p = p_mul(T(2), Fp);
-        a[0] = p_mul(T(-0.5), first(m.gu.tt, F2t, m.gu.tp, F2p));
-        a[3] = p_mul(T(-0.5), first(m.gu.tp, F2t, m.gu.pp, F2p));
-    } else {
-        a[0] = -first(m.gu.tt, Ft, m.gu.tp, Fp);
-        a[3] = -first(m.gu.tp, Ft, m.gu.pp, Fp);
-    }
+    const T two = T(2), half = T(-0.5);
+    const T Ft = p_mul(two, kSecond ? second(u[1], w1t, u[2], w2t) : first(u[1], w1t, u[2], w2t));
+    const T Fp = p_mul(two, kSecond ? second(u[1], w1p, u[2], w2p) : first(u[1], w1p, u[2], w2p));
+    const T Fr = p_sub(p_mul(two, first(u[1], w1r, u[2], w2r)), q1);
+    const T Fh = p_sub(p_mul(two, kSecond ? second(u[1], w1h, u[2], w2h) : first(u[1], w1h, u[2], w2h)), q2);
+    a[0] = p_mul(half, first(m.gu.tt, Ft, m.gu.tp, Fp));
+    a[3] = p_mul(half, first(m.gu.tp, Ft, m.gu.pp, Fp));
     a[1] = p_mul(m.gu.rr, Fr);
     a[2] = p_mul(m.gu.hh, Fh);
     if (f2) *f2 = Fh;
@@ -109,9 +106,9 @@ __device__ __forceinline__ void accel_lean(const MetricAt<T>& m, const T u[4], T
 // The form of each metric's FP32 right-hand side.
 constexpr int accel_form(int mid) { return mid == kJohannsen ? 1 : mid == kRasheedLarsen ? 2 : 0; }
 // In log-r mode the coordinate term -(u^1)^2 joins a^1 (accel_log_r).
-template <int FORM, typename T, bool SCALED = false>
+template <int FORM, typename T>
 __device__ __forceinline__ void accel_lean(const MetricAt<T>& m, bool rlog, const T u[4], T a[4], T* f2 = nullptr) {
-    accel_lean<FORM, T, SCALED>(m, u, a, f2);
+    accel_lean<FORM, T>(m, u, a, f2);
     if (rlog) a[1] = p_fma(-u[1], u[1], a[1]);
 }
 
@@ -479,7 +476,7 @@ struct LeanVerletEngine : LeanState<LeanConst<MID>> {
         const float uf[4] = {lo2(uf03), lo2(uf12), hi2(uf12), hi2(uf03)};
         const float h = adaptive_step_lean(G, hi2(L.xh[1]), hi2(L.xl[1]), uf[1], uf[2], uf[3]);
         float a0[4], a1[4], vi[4];
-        accel_lean<0, float, true>(L.m, RLOG, uf, a0);
+        accel_lean<0>(L.m, RLOG, uf, a0);
         const float h2 = 0.5f * h, hh2 = __fmul_rn(h2, h);
         const f2 ph = p_all<f2>(h), ph2 = p_all<f2>(h2), phh2 = p_all<f2>(hh2);
         const f2 a03 = pack2(a0[0], a0[3]), a12 = pack2(a0[1], a0[2]);
@@ -496,7 +493,7 @@ struct LeanVerletEngine : LeanState<LeanConst<MID>> {
         p_two_sum(L.xh[0], th, s, e);
         p_fast_two_sum(s, p_add(e, p_add(L.xl[0], tl)), L.xh[0], L.xl[0]);
         L.m = metric_lean<MID, RLOG, float>(L.c, lo2(L.xh[1]), lo2(L.xl[1]), hi2(L.xh[1]), hi2(L.xl[1]));
-        accel_lean<0, float, true>(L.m, RLOG, vi, a1);
+        accel_lean<0>(L.m, RLOG, vi, a1);
         L.rhs += 2;
         f2 b03 = pack2(a1[0], a1[3]), b12 = pack2(a1[1], a1[2]);
         f2 du03 = p_mul(ph2, p_add(a03, b03)), du12 = p_mul(ph2, p_add(a12, b12));
@@ -518,7 +515,7 @@ struct LeanVerletEngine : LeanState<LeanConst<MID>> {
                     break;
                 }
                 // (in log-r mode the compiled loop rounds (u^1)^2 before it subtracts it)
-                accel_lean<0, float, true>(L.m, false, nv, a1);
+                accel_lean<0>(L.m, false, nv, a1);
                 if (RLOG) a1[1] = __fsub_rn(a1[1], __fmul_rn(nv[1], nv[1]));
                 const f2 c03 = pack2(a1[0], a1[3]), c12 = pack2(a1[1], a1[2]);
                 dv03 = p_mul(ph2, p_sub(c03, b03));
@@ -730,13 +727,12 @@ static __device__ __forceinline__ SplitK contract_split(const MetricAt<double>& 
     const double q = __fma_rn(v[3], of(3), qb);
     const double s = __fma_rn(v[1], w1, __dmul_rn(v[2], w2));
     SplitK k;
-    const double sq = __fma_rn(2.0, s, -q);
-    k.F = ends ? s : sq;
+    k.F = __dsub_rn(__dmul_rn(2.0, s), ends ? 0.0 : q);
     const double Ft = lane4(k.F, 0, pmask), Fp = lane4(k.F, 3, pmask);
     const double c1 = (i == 0) ? m.gu.tt : (i == 1) ? m.gu.rr : (i == 2) ? m.gu.hh : m.gu.tp;
     const double p = __dmul_rn((i == 0) ? m.gu.tp : m.gu.pp, Fp);
     k.k = __fma_rn(c1, ends ? Ft : k.F, ends ? p : -0.0);
-    k.k = ends ? -k.k : k.k;
+    k.k = __dmul_rn(ends ? -0.5 : 1.0, k.k);
     if (rlog) {
         const double al = __fma_rn(-u, u, k.k);
         k.k = (i == 1) ? al : k.k;

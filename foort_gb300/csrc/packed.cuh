@@ -64,6 +64,7 @@ __device__ __forceinline__ float p_sub(float a, float b) { return __fsub_rn(a, b
 __device__ __forceinline__ double p_fma(double a, double b, double c) { return __fma_rn(a, b, c); }
 __device__ __forceinline__ double p_mul(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ double p_add(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ double p_sub(double a, double b) { return __dsub_rn(a, b); }
 
 // A float in every half, and a function of a float on every half.
 template <typename T>

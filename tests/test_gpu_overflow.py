@@ -1,0 +1,75 @@
+"""Rays whose state overflows: the specialised kernels (kernel_lean.cuh, kernel_fp64_split.cuh)
+end them as the general kernels do, with the same codes, counts and bits. The screens look
+along the rotation axis, or take coarse steps, so that some of their rays step past it or
+inside the horizon and diverge there."""
+import numpy as np
+import pytest
+
+from foort_gb300 import abi, workloads
+
+
+@pytest.fixture(scope="module")
+def eng():
+    import foort_gb300
+    from foort_gb300 import build as engine_build
+    engine_build.build()
+    foort_gb300.check_layout()
+    return foort_gb300
+
+
+def describe(precision, metric, params, integrator, rlog, inclination, r, half_width, epsilon, smallest_step, timeout,
+             boundary, tolerance, term_flags):
+    d = workloads.base_desc(precision)
+    d.metric_id, d.integrator_id, d.rlog = metric, integrator, rlog
+    d.epsilon, d.smallest_step, d.timeout_max_steps = epsilon, smallest_step, timeout
+    d.boundary_radius, d.verlet_tol, d.term_flags = boundary, tolerance, term_flags
+    d.diag_flags = abi.DIAG_FOUR_COLOR_SCREEN | abi.DIAG_CLOSEST_RADIUS
+    keep = abi.attach_images(d, [abi.make_image(params, r=r, theta=np.radians(inclination), half_width=half_width)])
+    return d, keep
+
+
+def same_records(a, b):
+    for name in abi.RESULT_DTYPE.names:
+        if name != "equat_passes":
+            np.testing.assert_array_equal(a[name], b[name], err_msg=name)
+
+
+RK4, VERLET = abi.INTEGRATOR_RK4, abi.INTEGRATOR_VERLET
+STOPS = abi.TERM_HORIZON | abi.TERM_BOUNDARY_SPHERE | abi.TERM_TIMEOUT
+ALL_STOPS = STOPS | abi.TERM_THETA_SINGULARITY
+
+
+# sums of the contraction between half the largest float and the largest one: the general
+# kernels double them
+@pytest.mark.gpu
+@pytest.mark.parametrize("metric,params,integrator,rlog,view,side", [
+    (abi.METRIC_FLAT, (), RK4, 0, (0.01, 5.0, 40.0, 0.03, 0.01, 50, 1000.0, 0.001, STOPS), 64),
+    (abi.METRIC_KERR, (0.0,), RK4, 0, (0.01, 30.0, 0.5, 3.0, 1e-7, 900, 1e5, 0.001, STOPS), 64),
+    (abi.METRIC_JOHANNSEN, (0.9563767844865592, 0.5064812267713692, 0.0, 0.0, 0.0), RK4, 0,
+     (0.01, 5.0, 12.0, 10.0, 1e-12, 300, 1000.0, -1.0, ALL_STOPS), 64),
+    (abi.METRIC_JOHANNSEN, (0.0, 0.408884871033909, 0.0, 0.0, 0.0), VERLET, 1,
+     (0.01, 1000.0, 0.5, 1.0, 1e-7, 50, 1e12, 0.001, ALL_STOPS & ~abi.TERM_BOUNDARY_SPHERE), 64),
+    (abi.METRIC_JOHANNSEN, (0.0, 1.0380233096005593, 0.0, 0.0, 0.001), RK4, 0,
+     (2.0, 5.0, 40.0, 10.0, 1e-7, 1, 1000.0, 0.001, ALL_STOPS & ~abi.TERM_BOUNDARY_SPHERE), 7),
+])
+def test_lean_contractions_overflow_where_the_general_ones_do(eng, metric, params, integrator, rlog, view, side):
+    """A diagnostic that does not update at each step takes the general kernel, with the same
+    float-float decisions."""
+    inclination, r, half_width, *rest = view
+    d, keep = describe(abi.PREC_MIXED, metric, params, integrator, rlog, inclination, r, half_width, *rest)
+    px = abi.square_pixels(side)
+    got = []
+    for lanes in (1, 2):
+        with eng.Engine(d) as e:
+            e.set_lanes(lanes)
+            got.append((e.integrate(px), e.stats()["steps"]))
+    d.diag_flags |= abi.DIAG_EQUATORIAL_PASSES
+    d.equat_freq = abi.UpdateFreq(2, 0, 0)
+    with eng.Engine(d) as e:
+        e.set_lanes(1)
+        want = e.integrate(px), e.stats()["steps"]
+    assert (want[0]["err"] & abi.ERR_NONFINITE).any()
+    for records, steps in got:
+        same_records(records, want[0])
+        assert steps == want[1]
+    del keep
