@@ -200,11 +200,12 @@ struct SplitEngine {
         const double h1 = d_mul(0.5, g1), h2 = d_mul(0.5, g2);
         const bool ends = i == 0 || i == 3;
         // t: 0.5 g^tt d_. g_t. + 0.5 g^tphi d_. g_phi.; phi: 0.5 g^tphi d_. g_t. + 0.5 g^phiphi d_. g_phi.
-        const double ha = (i == 3) ? h2 : h1, hb = (i == 3) ? h1 : h2;
-        const double a0 = ends ? dr.tt : (i == 1) ? -dr.tt : -dh.tt, b0 = ends ? dr.tp : 0.0;
-        const double a1 = ends ? dh.tt : (i == 1) ? -dr.tp : -dh.tp, b1 = ends ? dh.tp : 0.0;
-        const double a2 = ends ? dr.tp : (i == 1) ? dr.rr : -dh.rr, b2 = ends ? dr.pp : 0.0;
-        const double a3 = ends ? dh.tp : (i == 1) ? dh.rr : dr.hh, b3 = ends ? dh.pp : 0.0;
+        // (r and theta have no second product: 1 times -0, which adds nothing; g^tphi may be infinite)
+        const double ha = (i == 3) ? h2 : h1, hb = (i == 3) ? h1 : (i == 0) ? h2 : 1.0;
+        const double a0 = ends ? dr.tt : (i == 1) ? -dr.tt : -dh.tt, b0 = ends ? dr.tp : -0.0;
+        const double a1 = ends ? dh.tt : (i == 1) ? -dr.tp : -dh.tp, b1 = ends ? dh.tp : -0.0;
+        const double a2 = ends ? dr.tp : (i == 1) ? dr.rr : -dh.rr, b2 = ends ? dr.pp : -0.0;
+        const double a3 = ends ? dh.tp : (i == 1) ? dh.rr : dr.hh, b3 = ends ? dh.pp : -0.0;
         const double a4 = (i == 1) ? -dr.hh : dh.hh, a5 = (i == 1) ? -dr.pp : -dh.pp;
         // The compiler fuses the first product of a sum, but the second in Kerr's Gamma^t_01 and
         // Gamma^t_02; not so in Verlet's symbols of the position it starts from, kept for it.

@@ -73,3 +73,21 @@ def test_lean_contractions_overflow_where_the_general_ones_do(eng, metric, param
         same_records(records, want[0])
         assert steps == want[1]
     del keep
+
+
+# g^tphi infinite beside finite derivatives: r and theta take no product with it
+@pytest.mark.gpu
+@pytest.mark.parametrize("integrator", [RK4, VERLET])
+def test_shared_fp64_steps_end_where_one_lane_does(eng, integrator):
+    d, keep = describe(abi.PREC_FP64, abi.METRIC_KERR, (0.0,), integrator, 1, 0.3, 30.0, 0.5, 100.0, 0.01, 1, 1e5, -1.0,
+                       ALL_STOPS & ~abi.TERM_BOUNDARY_SPHERE)
+    d.theta_eps = 0.01
+    px = abi.square_pixels(33)
+    got = {}
+    for lanes in (1, 2):
+        with eng.Engine(d) as e:
+            e.set_lanes(lanes)
+            got[lanes] = e.integrate(px)
+    assert (got[1]["err"] & abi.ERR_NONFINITE).any()
+    same_records(got[2], got[1])
+    del keep
