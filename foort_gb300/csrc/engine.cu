@@ -329,23 +329,23 @@ int split_start(const RunConst& R, uint64_t n, int num_sms, bool forced) {
 // Kernel and grid of a launch of n geodesics in the requested shape (zero fields: the
 // built-in rule): a persistent grid of at most the resident CTAs. The rule takes 128
 // threads, as many CTAs per SM as fit, and two lanes per geodesic up to pair_limit().
-// FP64 kernels take CTAs of 32 threads, four per SM: one warp per scheduler already fills
-// its FP64 pipe, more only leave rays unevenly spread over lanes at the end (62,500
-// Johannsen rays in FP64 130 ms with two CTAs of 128 per SM, 110 with four of 32), and small
+// Where neither CTA size nor cap is asked for, FP64 kernels take CTAs of 32 threads, four per
+// SM: one warp per scheduler already fills its FP64 pipe, more only leave rays unevenly spread
+// over lanes at the end (62,500 Johannsen rays in FP64 130 ms with two CTAs of 128 per SM, 110 with four of 32), and small
 // CTAs spread a launch that does not fill the GPU evenly (4,096 Kerr rays 65.8 and 62.5 ms).
 // Eight per SM hide 5 % more latency where rays of like lengths (plain r) need more than the
 // lanes of four (62,500 Kerr rays cut at 900 steps 253 and 238 ms), or where a launch is so
 // large that its end counts little (250,000 in log r 623 and 601, 62,500 170 and 186).
 int choose_launch(foort_ctx* ctx, const RunConst& R, uint64_t n, int num_sms, const foort_launch_shape& want,
                   LaunchShape& out, bool positions = false) {
-    const bool fp64 = R.precision != FOORT_PREC_MIXED;
+    const bool fp64 = R.precision != FOORT_PREC_MIXED && !want.block_size && !want.blocks_per_sm;
     const uint32_t bs = want.block_size ? want.block_size : fp64 ? 32 : 128;
     const uint64_t sms = static_cast<uint64_t>(num_sms);
     auto resident = [&](const void* fn, uint64_t width, int& per_sm) -> int {
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, static_cast<int>(bs), 0));
-        if (fp64 && !want.blocks_per_sm) {
+        if (fp64) {
             const bool two = n > 1024 * sms || (!R.rlog && width * n > 128 * sms);
-            per_sm = std::min<int>(per_sm, std::max<int>(1, (two ? 256 : 128) / static_cast<int>(bs)));
+            per_sm = std::min<int>(per_sm, two ? 8 : 4);
         }
         if (want.blocks_per_sm) per_sm = std::min<int>(per_sm, static_cast<int>(want.blocks_per_sm));
         return FOORT_OK;

@@ -283,7 +283,8 @@ int foort_gpu_cancel(foort_ctx* ctx);
 
 /* Launch shape override: CTA size (a multiple of 32, at most 128) and a cap on resident
  * CTAs per SM; 0 leaves each to the autotuner's cached shape for the launch, or to the
- * built-in rule (128 threads, as many CTAs as fit) where the cache has none. */
+ * built-in rule where the cache has none: 128 threads, as many CTAs as fit; with both 0 in
+ * FP64 and FP64-analytic, 32 threads and four or eight CTAs per SM. */
 int foort_gpu_set_launch(foort_ctx* ctx, uint32_t block_size, uint32_t blocks_per_sm);
 
 /* Lanes per geodesic: 0 chooses per launch, 1 one lane, 2 several (two to eight) where such

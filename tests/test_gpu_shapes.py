@@ -1,0 +1,56 @@
+"""Launch shapes: what a caller asks for is what a launch takes."""
+import numpy as np
+import pytest
+
+from foort_gb300 import abi, workloads
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def eng():
+    import foort_gb300
+    from foort_gb300 import build as engine_build
+    engine_build.build()
+    foort_gb300.check_layout()
+    return foort_gb300
+
+
+@pytest.fixture(scope="module")
+def sms():
+    import torch
+    return torch.cuda.get_device_properties(0).multi_processor_count
+
+
+def describe(precision, metric=abi.METRIC_KERR, params=(0.9,), integrator=abi.INTEGRATOR_RK4, rlog=1, timeout=0):
+    d = workloads.base_desc(precision)
+    d.metric_id, d.integrator_id, d.rlog, d.timeout_max_steps = metric, integrator, rlog, timeout
+    d.diag_flags = abi.DIAG_FOUR_COLOR_SCREEN | abi.DIAG_EQUATORIAL_PASSES | abi.DIAG_CLOSEST_RADIUS
+    keep = abi.attach_images(d, [abi.make_image(params, r=1000.0, theta=1.1, half_width=9.0)])
+    return d, keep
+
+
+# a CTA size alone takes as many CTAs as fit, a cap alone CTAs of 128 threads, in every
+# precision; 0 and 0 is the built-in shape
+@pytest.mark.parametrize("precision", [abi.PREC_MIXED, abi.PREC_FP64, abi.PREC_FP64_ANALYTIC])
+@pytest.mark.parametrize("integrator", [abi.INTEGRATOR_RK4, abi.INTEGRATOR_VERLET])
+@pytest.mark.parametrize("lanes", [0, 1])
+def test_a_forced_size_or_cap_leaves_the_other_as_documented(eng, sms, precision, integrator, lanes):
+    d, keep = describe(precision, integrator=integrator)
+    px = abi.square_pixels(316)
+    with eng.Engine(d) as e:
+        e.set_lanes(lanes)
+        want = e.integrate(px)
+        for block in (64, 96, 128):
+            e.set_launch(block, 0)
+            got, st = e.integrate(px), e.stats()
+            assert st["block_size"] == block and st["n_blocks"] % sms == 0
+            assert st["n_blocks"] * block >= 192 * sms  # every kernel here fits at least this many threads on an SM
+            for name in abi.RESULT_DTYPE.names:
+                np.testing.assert_array_equal(got[name], want[name], err_msg=name)
+        for cap in (1, 2):
+            e.set_launch(0, cap)
+            e.integrate(px)
+            st = e.stats()
+            assert (st["block_size"], st["n_blocks"]) == (128, cap * sms)
+    del keep
