@@ -279,13 +279,18 @@ struct LaunchShape {
 //   plain r, 19,600 geodesics 174 ms on two and 211 on one, 39,204 291 and 255), and in log r,
 //   where the longest rays end a launch alone, several refills further (62,500 4.9 and 5.9 ms,
 //   160,000 9.0 and 9.2).
-// - Lean kernels with a called plugin exist on two lanes only and cost a geodesic no more
-//   than the general one-lane kernel: every size.
+// - Lean kernels with a called plugin exist on two lanes only. Rasheed-Larsen costs a geodesic
+//   less there than in the general one-lane kernel at every size (log r, 1,000,000 geodesics
+//   265 and 226, plain r 345 and 336). Johannsen's does while a launch's latency counts: log
+//   r, 250,000 29.8 and 27.7, 290,000 30.1 and 32.0, 1,000,000 98 and 109; plain r cut at 900
+//   steps, 36,000 6.23 and 6.09, 40,000 8.47 and 9.02, 1,000,000 142 and 156.
 uint64_t pair_limit(const RunConst& R, bool positions, int per_sm, int num_sms, uint32_t bs) {
     const uint64_t sms = static_cast<uint64_t>(num_sms);
     if (R.precision != FOORT_PREC_MIXED) return (R.rlog ? 512 : 64) * sms;
     if (mixed_lean_kernel(R, true, positions)) {
-        if (!mixed_lean_kernel(R, false, positions)) return UINT64_MAX;
+        const bool called = !mixed_lean_kernel(R, false, positions);
+        if (called && R.metric_id == kRasheedLarsen) return UINT64_MAX;
+        if (called) return (R.rlog ? 1792 : 256) * sms;
         if (R.metric_id == kJohannsen) return (R.rlog ? 1024 : 192) * sms;
         return (R.rlog ? 64 : 24) * sms;
     }

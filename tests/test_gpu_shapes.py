@@ -54,3 +54,22 @@ def test_a_forced_size_or_cap_leaves_the_other_as_documented(eng, sms, precision
             st = e.stats()
             assert (st["block_size"], st["n_blocks"]) == (128, cap * sms)
     del keep
+
+
+# two lanes per geodesic only where they are the faster kernel: on both sides of each limit
+# (in geodesics per SM)
+@pytest.mark.parametrize("metric,params,rlog,limit", [
+    (abi.METRIC_JOHANNSEN, (0.8, 1.0, 0.5, 0.2, 0.1), 0, 256),
+    (abi.METRIC_JOHANNSEN, (0.8, 1.0, 0.5, 0.2, 0.1), 1, 1792),
+    (abi.METRIC_JOHANNSEN, (0.8, 1.0, 0.0, 0.0, 0.0), 0, 192),
+])
+def test_two_lanes_up_to_the_limit_of_each_metric(eng, sms, metric, params, rlog, limit):
+    d, keep = describe(abi.PREC_MIXED, metric, params, rlog=rlog)
+    n = limit * sms
+    px = abi.square_pixels(int(np.ceil(np.sqrt(n + 2))))
+    with eng.Engine(d) as e:
+        for count, lanes in ((n, 2), (n + 1, 1)):
+            if count:
+                e.integrate(px[:count])
+                assert e.stats()["lanes_per_geodesic"] == lanes
+    del keep
