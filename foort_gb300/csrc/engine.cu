@@ -268,12 +268,15 @@ struct LaunchShape {
 //   and 69 on two, 62,500 123 and 111, 90,000 133 and 154. In plain r rays differ less in length, and a wave of two lanes each
 //   (64 x SMs) is the most that pays (flat space in FP64, 9,604 rays cut at 900 steps 20 ms on
 //   two lanes and 29 on one, 19,044 42 and 29).
-// - Lean kernels: one lane already evaluates two stages at a time, so two lanes pay only
-//   while they leave each scheduler one warp (n <= 64 x SMs), and only in log r, where
-//   each half of a packed stage needs its own exponentials and division: Kerr, 3,721
-//   geodesics in log r 1.31 ms on two lanes and 1.58 on one. In plain r both take the same
-//   within 3 % (3,000 geodesics 66 and 64 ms, 1.00 and 0.97 us a step): the smallest launches
-//   stay on two, the rest take one.
+// - Lean Kerr: one lane already evaluates two stages at a time, but scalar stages of a lane each
+//   have a shorter chain than packed ones. In plain r two lanes pay while they leave each
+//   scheduler one warp (ms on one lane and on two: 1,000 geodesics 68.7 and 65.3, 9,728 69.3 and
+//   66.3; 10,000 cut at 20,000 steps 20.0 and 24.1). In log r, where each half of a packed stage needs
+//   its own exponentials and division and the longest rays end a launch alone, up to 448 x SMs
+//   (3,000 1.84 and 1.42, 19,000 2.40 and 2.01, 58,000 3.37 and 2.98, 70,000 3.19 and 3.16, 80,000
+//   3.37 and 3.49).
+// - Lean flat space: its metric is too small for its half to be worth an exchange (100
+//   geodesics 46.0 and 54.0, 3,000 68.0 and 78.2): one lane.
 // - Johannsen with alpha13 alone: its packed body spills on one lane at three CTAs per SM and
 //   is held to two, so two lanes pay as long as they fit on the GPU (192 x SMs geodesics;
 //   plain r, 19,600 geodesics 174 ms on two and 211 on one, 39,204 291 and 255), and in log r,
@@ -292,7 +295,8 @@ uint64_t pair_limit(const RunConst& R, bool positions, int per_sm, int num_sms, 
         if (called && R.metric_id == kRasheedLarsen) return UINT64_MAX;
         if (called) return (R.rlog ? 1792 : 256) * sms;
         if (R.metric_id == kJohannsen) return (R.rlog ? 1024 : 192) * sms;
-        return (R.rlog ? 64 : 24) * sms;
+        if (R.metric_id == kFlat) return 0;
+        return (R.rlog ? 448 : 64) * sms;
     }
     return static_cast<uint64_t>(per_sm) * sms * bs / 2;
 }

@@ -59,6 +59,9 @@ def test_a_forced_size_or_cap_leaves_the_other_as_documented(eng, sms, precision
 # two lanes per geodesic only where they are the faster kernel: on both sides of each limit
 # (in geodesics per SM)
 @pytest.mark.parametrize("metric,params,rlog,limit", [
+    (abi.METRIC_KERR, (0.9,), 0, 64),
+    (abi.METRIC_KERR, (0.9,), 1, 448),
+    (abi.METRIC_FLAT, (), 0, 0),
     (abi.METRIC_JOHANNSEN, (0.8, 1.0, 0.5, 0.2, 0.1), 0, 256),
     (abi.METRIC_JOHANNSEN, (0.8, 1.0, 0.5, 0.2, 0.1), 1, 1792),
     (abi.METRIC_JOHANNSEN, (0.8, 1.0, 0.0, 0.0, 0.0), 0, 192),
