@@ -345,6 +345,11 @@ int split_start(const RunConst& R, uint64_t n, int num_sms, bool forced) {
 // Eight per SM hide 5 % more latency where rays of like lengths (plain r) need more than the
 // lanes of four (62,500 Kerr rays cut at 900 steps 253 and 238 ms), or where a launch is so
 // large that its end counts little (250,000 in log r 623 and 601, 62,500 170 and 186).
+// In plain r a wave's lanes end together: as many CTAs as fit (12 in FP64-analytic and flat space)
+// where their waves come to at most a tenth more threads than those of eight (FP64-analytic
+// Verlet cut at 300 steps, eight and twelve: Kerr 40,000 rays 18.1 and 14.7 ms, 62,000 24.3 and
+// 24.6, 90,000 36.4 and 30.4, 250,000 85.0 and 79.4; Johannsen 69.1 and 54.5, 90.6 and 93.7, 130
+// and 115, 318 and 320).
 int choose_launch(foort_ctx* ctx, const RunConst& R, uint64_t n, int num_sms, const foort_launch_shape& want,
                   LaunchShape& out, bool positions = false) {
     const bool fp64 = R.precision != FOORT_PREC_MIXED && !want.block_size && !want.blocks_per_sm;
@@ -354,7 +359,13 @@ int choose_launch(foort_ctx* ctx, const RunConst& R, uint64_t n, int num_sms, co
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, static_cast<int>(bs), 0));
         if (fp64) {
             const bool two = n > 1024 * sms || (!R.rlog && width * n > 128 * sms);
-            per_sm = std::min<int>(per_sm, two ? 8 : 4);
+            const int fit = per_sm;
+            per_sm = std::min<int>(fit, two ? 8 : 4);
+            auto in_waves = [&](int ctas) {  // the threads of all waves
+                const uint64_t wave = 32ull * static_cast<uint64_t>(ctas) * sms;
+                return (width * n + wave - 1) / wave * wave;
+            };
+            if (!R.rlog && fit > 8 && 10 * in_waves(fit) <= 11 * in_waves(8)) per_sm = fit;
         }
         if (want.blocks_per_sm) per_sm = std::min<int>(per_sm, static_cast<int>(want.blocks_per_sm));
         return FOORT_OK;

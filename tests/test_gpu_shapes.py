@@ -76,3 +76,18 @@ def test_two_lanes_up_to_the_limit_of_each_metric(eng, sms, metric, params, rlog
                 e.integrate(px[:count])
                 assert e.stats()["lanes_per_geodesic"] == lanes
     del keep
+
+
+@pytest.mark.parametrize("metric,params", [(abi.METRIC_KERR, (0.9,)), (abi.METRIC_JOHANNSEN, (0.8, 1.0, 0.5, 0.2, 0.1))])
+def test_fp64_waves_in_plain_r_leave_few_lanes_idle(eng, sms, metric, params):
+    """FP64-analytic Verlet fits twelve CTAs of 32 threads on an SM and takes eight, unless
+    twelve make fewer waves of threads."""
+    d, keep = describe(abi.PREC_FP64_ANALYTIC, metric, params, abi.INTEGRATOR_VERLET, rlog=0)
+    px = abi.square_pixels(int(np.ceil(np.sqrt(600 * sms))))
+    with eng.Engine(d) as e:
+        for per_sm, threads in ((100, 100), (250, 250), (256, 256), (300, 300), (384, 384), (400, 256), (600, 384)):
+            n = per_sm * sms
+            e.integrate(px[:n])
+            st = e.stats()
+            assert (st["block_size"], st["n_blocks"]) == (32, -(-threads * sms // 32))
+    del keep
