@@ -234,10 +234,12 @@ __global__ void expand_positions(double* x, uint64_t n) {
     }
 }
 
+// The one-lane kernel for these options.
 const void* select_kernel(const RunConst& R, bool positions) {
     if (const void* lean = mixed_lean_kernel(R, false, positions)) return lean;
     if (analytic_family(R.precision))
         return mixed_kernel_variant(R.metric_id, R.integrator, (R.mixed_options & FOORT_MIXED_FP64_DECISIONS) != 0);
+    if (const void* reduced = fp64_split_kernel(R, 0)) return reduced;
     return fp64_kernel(R.metric_id, R.integrator);
 }
 
