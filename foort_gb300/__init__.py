@@ -95,6 +95,8 @@ def load():
     lib.foort_gpu_launch_shape.argtypes = [vp, u64, C.POINTER(abi.LaunchShape)]
     lib.foort_tune_bucket.argtypes = [u64]
     lib.foort_tune_bucket.restype = u32
+    lib.foort_tune_candidates.argtypes = [C.c_int32, C.c_int32, C.c_void_p, u32]
+    lib.foort_tune_candidates.restype = u32
     lib.foort_tune_key.argtypes = [C.POINTER(abi.RunDesc), i32, u64, C.c_char_p, u64]
     lib.foort_tune_put.argtypes = [C.c_char_p, C.POINTER(abi.LaunchShape)]
     lib.foort_tune_get.argtypes = [C.c_char_p, C.POINTER(abi.LaunchShape)]
@@ -318,6 +320,14 @@ def tune_key(desc, num_sms, n):
     if rc != 0:
         raise FoortError(rc, "tune key")
     return buf.value.decode()
+
+
+def tune_candidates(precision, several):
+    """The first shapes of foort_gpu_autotune's search (foort_tune_candidates)."""
+    n = load().foort_tune_candidates(precision, int(several), None, 0)
+    out = (abi.LaunchShape * n)()
+    load().foort_tune_candidates(precision, int(several), out, n)
+    return [s.as_dict() for s in out]
 
 
 def tune_get(key):

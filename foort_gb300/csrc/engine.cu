@@ -352,20 +352,23 @@ int split_start(const RunConst& R, uint64_t n, int num_sms, bool forced) {
 // Verlet cut at 300 steps, eight and twelve: Kerr 40,000 rays 18.1 and 14.7 ms, 62,000 24.3 and
 // 24.6, 90,000 36.4 and 30.4, 250,000 85.0 and 79.4; Johannsen 69.1 and 54.5, 90.6 and 93.7, 130
 // and 115, 318 and 320).
+// whole: the geodesics of the launch that n of them stand for (0: n), by which lanes and
+// occupancy are chosen.
 int choose_launch(foort_ctx* ctx, const RunConst& R, uint64_t n, int num_sms, const foort_launch_shape& want,
-                  LaunchShape& out, bool positions = false) {
+                  LaunchShape& out, bool positions = false, uint64_t whole = 0) {
+    const uint64_t all = whole ? whole : n;
     const bool fp64 = R.precision != FOORT_PREC_MIXED && !want.block_size && !want.blocks_per_sm;
     const uint32_t bs = want.block_size ? want.block_size : fp64 ? 32 : 128;
     const uint64_t sms = static_cast<uint64_t>(num_sms);
     auto resident = [&](const void* fn, uint64_t width, int& per_sm) -> int {
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, static_cast<int>(bs), 0));
         if (fp64) {
-            const bool two = n > 1024 * sms || (!R.rlog && width * n > 128 * sms);
+            const bool two = all > 1024 * sms || (!R.rlog && width * all > 128 * sms);
             const int fit = per_sm;
             per_sm = std::min<int>(fit, two ? 8 : 4);
             auto in_waves = [&](int ctas) {  // the threads of all waves
                 const uint64_t wave = 32ull * static_cast<uint64_t>(ctas) * sms;
-                return (width * n + wave - 1) / wave * wave;
+                return (width * all + wave - 1) / wave * wave;
             };
             if (!R.rlog && fit > 8 && 10 * in_waves(fit) <= 11 * in_waves(8)) per_sm = fit;
         }
@@ -378,7 +381,7 @@ int choose_launch(foort_ctx* ctx, const RunConst& R, uint64_t n, int num_sms, co
     uint32_t lanes = 1;    // 2 stands for several, as in foort_launch_shape
     uint64_t threads = n;  // to hold every geodesic at once
     const bool may_split = R.precision != FOORT_PREC_MIXED && !positions && want.lanes != 1;
-    const int start = may_split ? split_start(R, n, num_sms, want.lanes == 2) : 0;
+    const int start = may_split ? split_start(R, all, num_sms, want.lanes == 2) : 0;
     const void* split = !may_split                        ? nullptr
                         : R.precision == FOORT_PREC_FP64 ? fp64_split_kernel(R, start)
                                                          : analytic_split_kernel(R, start);
@@ -392,7 +395,7 @@ int choose_launch(foort_ctx* ctx, const RunConst& R, uint64_t n, int num_sms, co
     } else if (pair) {
         int per_sm2 = 0;
         if ((rc = resident(pair, 2, per_sm2))) return rc;
-        if (per_sm2 > 0 && (want.lanes == 2 || n <= pair_limit(R, positions, per_sm2, num_sms, bs))) {
+        if (per_sm2 > 0 && (want.lanes == 2 || all <= pair_limit(R, positions, per_sm2, num_sms, bs))) {
             fn = pair;
             per_sm = per_sm2;
             lanes = 2;
@@ -421,7 +424,10 @@ foort_launch_shape requested_shape(const foort_ctx* ctx, uint64_t n, bool* cache
                      foort_tune_get(key, &s) == FOORT_OK;
     if (!hit) s = foort_launch_shape{};
     if (cached) *cached = hit;
-    if (ctx->block_size) s.block_size = ctx->block_size;
+    if (ctx->block_size) {
+        if (s.block_size != ctx->block_size) s.blocks_per_sm = 0;  // a cap for the cached size
+        s.block_size = ctx->block_size;
+    }
     if (ctx->blocks_per_sm) s.blocks_per_sm = ctx->blocks_per_sm;
     if (ctx->lanes) s.lanes = ctx->lanes;
     return s;
@@ -454,14 +460,14 @@ int autotune_launch(foort_ctx* ctx, const foort_pixel* d_px, uint64_t n, foort_r
                     foort_launch_shape* best);
 
 // One launch over n pixels: the explicit shape if given, else the requested one (with
-// the search first where autotuning is on and the cache has no entry).
+// the search first where autotuning is on and the cache has no entry). whole: choose_launch.
 int launch(foort_ctx* ctx, const foort_pixel* d_px, uint64_t n, foort_result* d_out, cudaStream_t st,
-           GeoposRec* gp_plan = nullptr, const foort_launch_shape* shape = nullptr) {
+           GeoposRec* gp_plan = nullptr, const foort_launch_shape* shape = nullptr, uint64_t whole = 0) {
     bool cached = false;
     const foort_launch_shape want = shape ? *shape : requested_shape(ctx, n, &cached);
     if (!shape && !cached && ctx->autotune && !gp_plan && n > 0) return autotune_launch(ctx, d_px, n, d_out, st, nullptr);
     LaunchShape ls;
-    int rc = choose_launch(ctx, ctx->rc, n, ctx->num_sms, want, ls, gp_plan != nullptr);
+    int rc = choose_launch(ctx, ctx->rc, n, ctx->num_sms, want, ls, gp_plan != nullptr, whole);
     if (rc) return rc;
     const void* fn = ls.fn;
     const uint32_t bs = ls.block, grid = ls.grid;
@@ -542,12 +548,11 @@ int finish(foort_ctx* ctx) {
     return rc;
 }
 
-// The search (foort_gpu_autotune). Candidates: lanes per geodesic (1, and 2 where the
-// two-lane kernel exists) times CTA sizes 32, 64, 128, at refill cadence 1 and the default
-// poll interval; then, around the fastest, refill cadences 4 and 16 and poll intervals
-// 128 and 2048; the two fastest are timed once more and the smaller time counts. Each
-// candidate is one launch over the pixels (or a prefix, for launches much larger than the
-// GPU's resident lanes), timed with CUDA events. The last launch integrates all n pixels
+// The search (foort_gpu_autotune). Candidates: foort_tune_candidates, at refill cadence 1
+// and the default poll interval; then, around the fastest, refill cadences 4 and 16 and poll
+// intervals 128 and 2048; the two fastest are timed once more and the smaller time counts.
+// Each candidate is one launch over the pixels (or a prefix, for launches much larger than the
+// GPU's resident lanes, in the whole launch's kernel), timed with CUDA events. The last launch integrates all n pixels
 // in the winning shape.
 int autotune_launch(foort_ctx* ctx, const foort_pixel* d_px, uint64_t n, foort_result* d_out, cudaStream_t st,
                     foort_launch_shape* best_out) {
@@ -563,7 +568,7 @@ int autotune_launch(foort_ctx* ctx, const foort_pixel* d_px, uint64_t n, foort_r
                           (ctx->rc.precision == FOORT_PREC_FP64 && fp64_split_kernel(ctx->rc, 1));
     std::vector<foort_launch_shape> tried;
     auto time_shape = [&](foort_launch_shape s, double& ms) -> int {
-        int r = launch(ctx, d_px, m, d_out, st, nullptr, &s);
+        int r = launch(ctx, d_px, m, d_out, st, nullptr, &s, n);
         if (r) return r;
         r = finish(ctx);
         if (r != FOORT_OK) return r;
@@ -591,9 +596,10 @@ int autotune_launch(foort_ctx* ctx, const foort_pixel* d_px, uint64_t n, foort_r
     // one untimed launch: module load and first-touch costs stay out of the comparison
     double warm = 0.0;
     if ((rc = time_shape(foort_launch_shape{128, 0, 1, 1, kDefaultPollSteps, 0, 0.0}, warm))) return rc;
-    for (uint32_t lanes = 1; lanes <= (has_pair ? 2u : 1u); ++lanes)
-        for (uint32_t bs : {32u, 64u, 128u})
-            if ((rc = consider(foort_launch_shape{bs, 0, lanes, 1, kDefaultPollSteps, 0, 0.0}))) return rc;
+    foort_launch_shape first[16];
+    const uint32_t shapes = foort_tune_candidates(ctx->rc.precision, has_pair, first, 16);
+    for (uint32_t i = 0; i < shapes; ++i)
+        if ((rc = consider(first[i]))) return rc;
     foort_launch_shape b = fastest();
     for (uint32_t refill : {4u, 16u}) {
         foort_launch_shape c = b;

@@ -102,7 +102,7 @@ enum Ctr {
 };
 
 // Steps between budget / cancel polls unless a launch shape says otherwise.
-constexpr uint32_t kDefaultPollSteps = 512;
+constexpr uint32_t kDefaultPollSteps = FOORT_DEFAULT_POLL_STEPS;
 
 // Status bits written by the kernel.
 constexpr unsigned long long kStatusBudget = 1ull;

@@ -55,6 +55,21 @@ int foort_tune_key(const foort_run_desc* d, int32_t num_sms, uint64_t n, char* b
     return (w > 0 && static_cast<uint64_t>(w) < cap) ? FOORT_OK : FOORT_E_BADARG;
 }
 
+uint32_t foort_tune_candidates(int32_t precision, int32_t several, foort_launch_shape* out, uint32_t cap) {
+    const bool fp64 = precision != FOORT_PREC_MIXED;
+    uint32_t n = 0;
+    auto add = [&](uint32_t block, uint32_t blocks_per_sm, uint32_t lanes) {
+        if (out && n < cap) out[n] = foort_launch_shape{block, blocks_per_sm, lanes, 1, FOORT_DEFAULT_POLL_STEPS, 0, 0.0};
+        ++n;
+    };
+    for (uint32_t lanes = 1; lanes <= (several ? 2u : 1u); ++lanes) {
+        if (fp64)
+            for (uint32_t per_sm : {4u, 8u}) add(32, per_sm, lanes);
+        for (uint32_t block : {32u, 64u, 128u}) add(block, 0, lanes);
+    }
+    return n;
+}
+
 int foort_tune_put(const char* key, const foort_launch_shape* shape) {
     if (!valid_key(key) || !shape || !valid_shape(*shape)) return FOORT_E_BADARG;
     std::lock_guard<std::mutex> lk(g_mu);

@@ -312,10 +312,11 @@ typedef struct foort_launch_shape {
     uint32_t reserved;
     double ms;              /* the search's measured time for this shape (0: none)     */
 } foort_launch_shape;
+#define FOORT_DEFAULT_POLL_STEPS 512u
 
 /* Autotune the launch of n pixels held in DEVICE memory: time candidate shapes with CUDA
- * events on `cuda_stream` (lanes x CTA size, then the regrouping cadence and the poll
- * interval around the best), on all n pixels or, for launches of more than
+ * events on `cuda_stream` (foort_tune_candidates, then the regrouping cadence and the
+ * poll interval around the best), on all n pixels or, for launches of more than
  * FOORT_TUNE_SAMPLE_LANES_X times the resident lanes, on a prefix of that many. The
  * fastest goes into the launch-shape cache under this context's key for n (see
  * foort_tune_key) and into *best (may be NULL). The call ends with a launch of all n
@@ -324,6 +325,12 @@ typedef struct foort_launch_shape {
 #define FOORT_TUNE_SAMPLE_LANES_X 4u
 int foort_gpu_autotune(foort_ctx* ctx, const foort_pixel* d_px, uint64_t n, foort_result* d_out,
                        void* cuda_stream, foort_launch_shape* best);
+
+/* The search's first shapes: one lane per geodesic, and several where `several` is set, times
+ * CTAs of 32, 64 and 128 threads with as many on an SM as fit, and in FP64 and
+ * FP64-analytic four and eight of 32 threads (one and two warps per scheduler). Returns
+ * their number and writes up to cap of them to out (may be NULL). */
+uint32_t foort_tune_candidates(int32_t precision, int32_t several, foort_launch_shape* out, uint32_t cap);
 
 /* on = 1: a launch whose key has no cache entry first runs the search (that launch waits
  * for its stream and takes several times longer); on = 0 (default): launches use the

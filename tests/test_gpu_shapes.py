@@ -91,3 +91,34 @@ def test_fp64_waves_in_plain_r_leave_few_lanes_idle(eng, sms, metric, params):
             st = e.stats()
             assert (st["block_size"], st["n_blocks"]) == (32, -(-threads * sms // 32))
     del keep
+
+
+# more pixels than a search times: the sample runs in the whole launch's kernel and shape
+@pytest.mark.parametrize("precision,metric,params,integrator", [
+    (abi.PREC_FP64, abi.METRIC_JOHANNSEN, (0.7, 1.0, 0.0, 0.0, 0.0), abi.INTEGRATOR_VERLET),
+    (abi.PREC_FP64_ANALYTIC, abi.METRIC_KERR, (0.9,), abi.INTEGRATOR_RK4),
+])
+def test_tuned_fp64_shapes_are_launched_as_they_were_timed(eng, sms, precision, metric, params, integrator):
+    import torch
+    d, keep = describe(precision, metric, params, integrator, timeout=12)
+    px = abi.square_pixels(int(np.ceil(np.sqrt(1100 * sms))))
+    eng.tune_clear()
+    with eng.Engine(d) as e:
+        want = e.integrate(px)
+        d_px = torch.from_numpy(px.view(np.uint8).copy()).cuda()
+        d_out = torch.zeros(len(px) * abi.RESULT_DTYPE.itemsize, dtype=torch.uint8, device="cuda")
+        best = e.autotune(d_px.data_ptr(), len(px), d_out.data_ptr())
+        shapes = {(s["block_size"], s["blocks_per_sm"], s["lanes"]) for s in eng.tune_candidates(precision, True)}
+        assert (best["block_size"], best["blocks_per_sm"], best["lanes"]) in shapes
+        got, st = e.integrate(px), e.stats()
+        assert st["block_size"] == best["block_size"] and st["lanes_per_geodesic"] == best["lanes"]
+        if best["blocks_per_sm"]:
+            assert st["n_blocks"] <= best["blocks_per_sm"] * sms
+        e.set_launch(96, 0)  # a forced size takes no cap that was found for another
+        e.integrate(px)
+        assert e.stats()["n_blocks"] * 96 >= 192 * sms
+    eng.tune_clear()
+    for name in abi.RESULT_DTYPE.names:
+        np.testing.assert_array_equal(got[name], want[name], err_msg=name)
+        np.testing.assert_array_equal(d_out.cpu().numpy().view(abi.RESULT_DTYPE)[name], want[name], err_msg=name)
+    del keep
