@@ -15,6 +15,7 @@
 
 #include "engine.h"
 #include "kernels.h"
+#include "variant.h"
 
 using namespace foort;
 
@@ -173,10 +174,8 @@ int validate(const foort_run_desc* d, std::string& why) {
 
 RunConst make_run_const(const foort_run_desc& d) {
     RunConst R{};
-    R.only_alpha13 = 1;
-    for (uint32_t i = 0; i < d.n_images; ++i)
-        for (int k = 2; k < 5; ++k)  // alpha22, alpha52, epsilon3
-            if (d.images[i].metric_params[k] != 0.0) R.only_alpha13 = 0;
+    R.only_alpha13 = only_alpha13(d);
+    R.each_step = updates_each_step(d);
     R.metric_id = d.metric_id;
     // Flat space is not a SphericalHorizonMetric: no log-r scale (ViewScreen.h:49-50)
     // and no Horizon termination (Config.cpp:649-657).

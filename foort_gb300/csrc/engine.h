@@ -86,8 +86,7 @@ struct RunConst {
     uint64_t gp_every;  // GeodesicPosition update frequency (recorded on a second pass)
     int32_t gp_start, gp_finish;
     MixedRun mr;
-    int32_t only_alpha13;  // Johannsen: the other deviation parameters are 0 in every image
-    int32_t pad;
+    int32_t only_alpha13, each_step;  // variant.h
 };
 
 // Scratch counters of one launch (device memory, zeroed before each launch).

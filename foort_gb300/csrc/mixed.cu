@@ -59,16 +59,7 @@ const void* analytic_pair_kernel_flat(bool positions);
 
 // Lean options: every termination and diagnostic in use updates at each step (the
 // default), with decisions on the float-float state.
-static bool lean_options(const RunConst& R) {
-    if (R.mixed_options & FOORT_MIXED_FP64_DECISIONS) return false;
-    auto each_step = [](uint32_t flags, uint32_t flag, uint64_t every) { return !(flags & flag) || every == 1; };
-    return each_step(R.term_flags, FOORT_TERM_HORIZON, R.h_every) &&
-           each_step(R.term_flags, FOORT_TERM_BOUNDARY_SPHERE, R.b_every) &&
-           each_step(R.term_flags, FOORT_TERM_TIMEOUT, R.t_every) &&
-           each_step(R.term_flags, FOORT_TERM_THETA_SINGULARITY, R.th_every) &&
-           each_step(R.diag_flags, FOORT_DIAG_EQUATORIAL_PASSES, R.eq_every) &&
-           each_step(R.diag_flags, FOORT_DIAG_CLOSEST_RADIUS, R.cr_every);
-}
+static bool lean_options(const RunConst& R) { return R.each_step && !(R.mixed_options & FOORT_MIXED_FP64_DECISIONS); }
 
 // Whether some steps of a mixed launch are taken in FP64 (near the horizon, at turning points).
 static bool fp64_regions(const RunConst& R) {

@@ -1,7 +1,8 @@
 // Launch-shape cache of the engine's autotuner (include/foort_gpu.h, foort_tune_*).
 //
 // One process-wide table maps a tuning key -- the GPU's SM count, the kernel variant
-// (metric, integrator, precision, decision and strong-field options) and the launch-size
+// (metric, integrator, precision, decision and strong-field options, Johannsen's deviation
+// parameters besides alpha13, updates not made at each step) and the launch-size
 // bucket floor(log2 n) -- to the launch shape measured fastest for it. The search itself
 // (foort_gpu_autotune, engine.cu) times candidate shapes on the GPU; this file only keeps
 // and persists its results, so it needs no GPU. The reference has no counterpart: its
@@ -13,6 +14,7 @@
 #include <string>
 
 #include "../../include/foort_gpu.h"
+#include "variant.h"
 
 namespace {
 
@@ -49,9 +51,15 @@ int foort_tune_key(const foort_run_desc* d, int32_t num_sms, uint64_t n, char* b
     const int region = ((d->mixed_options & FOORT_MIXED_FP64_NEAR_HORIZON) && d->mixed_fp64_margin > 0.0 ? 1 : 0) |
                        ((d->mixed_options & FOORT_MIXED_FP64_TURNING_POINTS) ? 2 : 0);
     const int decide64 = (d->mixed_options & FOORT_MIXED_FP64_DECISIONS) != 0;
-    const int w = std::snprintf(buf, cap, "sm%d:m%d:i%d:p%d:r%d:d%d:f%d:b%u", num_sms, d->metric_id,
+    // the lean kernels, and of Johannsen's those with alpha13 alone, have their own shapes
+    const bool mixed = d->precision == FOORT_PREC_MIXED;
+    const bool lean_kinds = !decide64 && (mixed ? region == 0 : d->precision == FOORT_PREC_FP64_ANALYTIC);
+    const bool general = lean_kinds && !foort::updates_each_step(*d);
+    const bool full = d->metric_id == FOORT_METRIC_JOHANNSEN && !general &&
+                      ((mixed && lean_kinds) || d->precision == FOORT_PREC_FP64) && !foort::only_alpha13(*d);
+    const int w = std::snprintf(buf, cap, "sm%d:m%d:i%d:p%d:r%d:d%d:f%d%s%s:b%u", num_sms, d->metric_id,
                                 d->integrator_id, d->precision, d->rlog ? 1 : 0, decide64, region,
-                                foort_tune_bucket(n));
+                                general ? ":u1" : "", full ? ":j1" : "", foort_tune_bucket(n));
     return (w > 0 && static_cast<uint64_t>(w) < cap) ? FOORT_OK : FOORT_E_BADARG;
 }
 

@@ -342,8 +342,9 @@ int foort_gpu_launch_shape(foort_ctx* ctx, uint64_t n, foort_launch_shape* shape
 
 /* The launch-shape cache: one table per process, shared by every context. A key names
  * the GPU's SM count, the kernel variant (metric, integrator, precision, log-r, FP64
- * decisions, FP64 steps by radius or at turning points) and the size bucket
- * floor(log2 n) of the launch.
+ * decisions, FP64 steps by radius or at turning points; where the lean kernels could
+ * serve, that a termination or diagnostic does not update at each step; Johannsen's
+ * parameters besides alpha13) and the size bucket floor(log2 n) of the launch.
  * save / load write and read one text line per entry (load adds to the table). */
 uint32_t foort_tune_bucket(uint64_t n);
 int foort_tune_key(const foort_run_desc* desc, int32_t num_sms, uint64_t n, char* buf, uint64_t cap);
