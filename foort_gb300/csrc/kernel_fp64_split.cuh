@@ -201,12 +201,13 @@ struct SplitEngine {
         const bool ends = i == 0 || i == 3;
         // t: 0.5 g^tt d_. g_t. + 0.5 g^tphi d_. g_phi.; phi: 0.5 g^tphi d_. g_t. + 0.5 g^phiphi d_. g_phi.
         // (r and theta have no second product: 1 times -0, which adds nothing; g^tphi may be infinite)
+        const double own = (i == 1) ? dr.rr : dh.hh, self = twice_less_once(own);
         const double ha = (i == 3) ? h2 : h1, hb = (i == 3) ? h1 : (i == 0) ? h2 : 1.0;
         const double a0 = ends ? dr.tt : (i == 1) ? -dr.tt : -dh.tt, b0 = ends ? dr.tp : -0.0;
         const double a1 = ends ? dh.tt : (i == 1) ? -dr.tp : -dh.tp, b1 = ends ? dh.tp : -0.0;
-        const double a2 = ends ? dr.tp : (i == 1) ? dr.rr : -dh.rr, b2 = ends ? dr.pp : -0.0;
+        const double a2 = ends ? dr.tp : (i == 1) ? self : -dh.rr, b2 = ends ? dr.pp : -0.0;
         const double a3 = ends ? dh.tp : (i == 1) ? dh.rr : dr.hh, b3 = ends ? dh.pp : -0.0;
-        const double a4 = (i == 1) ? -dr.hh : dh.hh, a5 = (i == 1) ? -dr.pp : -dh.pp;
+        const double a4 = (i == 1) ? -dr.hh : self, a5 = (i == 1) ? -dr.pp : -dh.pp;
         // The compiler fuses the first product of a sum, but the second in Kerr's Gamma^t_01 and
         // Gamma^t_02; not so in Verlet's symbols of the position it starts from, kept for it.
         const bool swap = MID == kKerr && i == 0;
@@ -220,6 +221,11 @@ struct SplitEngine {
         C[3] = two(ha, a3, hb, b3);
         C[4] = d_mul(ha, a4);
         C[5] = d_mul(ha, a5);
+    }
+    // (x + x) - x of the symbols with three like indices (gen_fd_christoffel.inc): x, but NaN or
+    // infinite where the sum is.
+    static __device__ __forceinline__ double twice_less_once(double x) {
+        return ((__double2hiint(x) & 0x7fffffff) < 0x7fe00000) ? x : d_sub(d_add(x, x), x);
     }
     static __device__ __forceinline__ double two(double a, double x, double b, double y) {
         return d_fma(a, x, d_mul(b, y));

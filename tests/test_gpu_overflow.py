@@ -91,3 +91,23 @@ def test_shared_fp64_steps_end_where_one_lane_does(eng, integrator):
     assert (got[1]["err"] & abi.ERR_NONFINITE).any()
     same_records(got[2], got[1])
     del keep
+
+
+# a finite difference across Delta = 0, where d_r g_rr is infinite
+@pytest.mark.gpu
+@pytest.mark.parametrize("integrator", [RK4, VERLET])
+@pytest.mark.parametrize("side", [4, 90])
+def test_shared_fp64_steps_cross_the_horizon_as_one_lane_does(eng, integrator, side):
+    h = 2.0 ** -23
+    d, keep = describe(abi.PREC_FP64, abi.METRIC_KERR, (0.0,), integrator, 0, 60.0, 2.0 - h, 0.5, 0.03, 1e-12, 3, 1e5, -1.0,
+                       abi.TERM_BOUNDARY_SPHERE | abi.TERM_TIMEOUT)
+    d.derivative_h = h
+    px = abi.square_pixels(side)
+    got = {}
+    for lanes in (1, 2):
+        with eng.Engine(d) as e:
+            e.set_lanes(lanes)
+            got[lanes] = e.integrate(px)
+    assert (got[1]["err"] & abi.ERR_NONFINITE).all()
+    same_records(got[2], got[1])
+    del keep
