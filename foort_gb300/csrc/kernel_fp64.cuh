@@ -8,6 +8,9 @@
 // argument: the two radial shifts share theta, the two angular shifts share r.
 #pragma once
 
+#include <type_traits>
+
+#include "fp64_rounded.cuh"
 #include "kernel_common.cuh"
 
 namespace foort {
@@ -18,26 +21,30 @@ struct FdParts {
     G5 dr, dh, gu;
 };
 
-// g_dd at one of the four points. own_r: no other point has this r; metrics whose roundings
-// are written out (Mt::kOwnR, SplitMetric) need to know.
+// Metrics whose right-hand side has its roundings written out (RoundedMetric, with the functions
+// of fp64_rounded.cuh); the others' (Mt = MetricFP64) are the compiler's.
 template <class Mt>
-constexpr bool takes_own_r(...) {
+constexpr bool is_rounded(...) {
     return false;
 }
 template <class Mt>
-constexpr bool takes_own_r(decltype(Mt::kOwnR)*) {
+constexpr bool is_rounded(decltype(Mt::kOwnR)*) {
     return true;
 }
+template <int MID>
+using FdMetric = std::conditional_t<MID == kKerr || MID == kJohannsen, RoundedMetric<MID, false>, MetricFP64<MID>>;
+
+// g_dd at one of the four points. own_r: no other point has this r; written-out roundings need to know.
 template <class Mt>
 __device__ __forceinline__ G5 dd_at(const MetricConst& M, double r, double s, double c, bool rlog, bool own_r) {
-    if constexpr (takes_own_r<Mt>(nullptr)) {
+    if constexpr (is_rounded<Mt>(nullptr)) {
         return Mt::dd(M.q, r, s, c, rlog, own_r);
     } else {
         return Mt::dd(M, r, s, c, rlog);
     }
 }
 
-template <int MID, class Mt = MetricFP64<MID>>
+template <class Mt>
 __device__ __forceinline__ FdParts fd_parts_fp64(const MetricConst& M, bool rlog, double hfd, const double x[4]) {
     double r0, rp, rm;
     if (rlog) {
@@ -57,7 +64,12 @@ __device__ __forceinline__ FdParts fd_parts_fp64(const MetricConst& M, bool rlog
     const G5 b = dd_at<Mt>(M, rm, s0, c0, rlog, true);
     const G5 c = dd_at<Mt>(M, r0, sp, cp, rlog, false);
     const G5 d = dd_at<Mt>(M, r0, sm, cm, rlog, false);
-    const G5 gu = Mt::uu(M, r0, s0, c0, rlog);
+    G5 gu;
+    if constexpr (is_rounded<Mt>(nullptr)) {
+        gu = rounded_inverse<Mt>(M, r0, s0, c0, rlog);
+    } else {
+        gu = Mt::uu(M, r0, s0, c0, rlog);
+    }
     const double inv = 1 / (2 * hfd);
     FdParts P;
     G5& dr = P.dr;
@@ -71,25 +83,46 @@ __device__ __forceinline__ FdParts fd_parts_fp64(const MetricConst& M, bool rlog
 }
 
 // The Christoffel symbols from the parts and their contraction with v (Metric.cpp:39-53,
-// Integrators.cpp:60-68).
+// Integrators.cpp:60-68). KEPT: with parts kept from the last step (Verlet).
+template <int MID, class Mt, bool KEPT = false>
 __device__ __forceinline__ void contract_fp64(const FdParts& P, const double v[4], double acc[4]) {
     const G5& dr = P.dr;
     const G5& dh = P.dh;
     const G5& gu = P.gu;
+    if constexpr (is_rounded<Mt>(nullptr)) {
+        const double g1[4] = {gu.tt, gu.rr, gu.hh, gu.pp};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            double C[6];
+            rounded_symbols<MID>(dr, dh, g1[i], gu.tp, i, C, (KEPT && i == 0) ? C : nullptr);
+            acc[i] = rounded_accel(C, v, i);
+        }
+    } else {
 #include "gen_fd_christoffel.inc"
+    }
 }
 
 template <int MID, class Mt>
 __device__ __forceinline__ void rhs_fd_fp64(const MetricConst& M, bool rlog, double hfd, const double x[4],
                                             const double v[4], double acc[4]) {
-    contract_fp64(fd_parts_fp64<MID, Mt>(M, rlog, hfd, x), v, acc);
+    contract_fp64<MID, Mt>(fd_parts_fp64<Mt>(M, rlog, hfd, x), v, acc);
 }
 
-// Mt: the metric's functions (MetricFP64, or SplitMetric's for Johannsen with alpha13 alone).
-template <int MID, int INTEG, class Mt = MetricFP64<MID>>
+// Mt: the metric's functions (FdMetric, or RoundedMetric's for Johannsen with alpha13 alone).
+template <int MID, int INTEG, class Mt = FdMetric<MID>>
 struct Fp64Engine {
     static constexpr bool kCopyImage = false;
     static constexpr bool kRecords = true;
+    static constexpr bool kRounded = is_rounded<Mt>(nullptr);
+
+    // a + b t
+    static __device__ __forceinline__ double ahead(double a, double b, double t) {
+        if constexpr (kRounded) {
+            return d_fma(b, t, a);
+        } else {
+            return a + b * t;
+        }
+    }
 
     struct Lane {
         double x[4], v[4];
@@ -108,7 +141,7 @@ struct Fp64Engine {
 
     static __device__ __forceinline__ void init(Lane& L, const ImageConst& I, const RunConst& R, const foort_pixel& p) {
         initial_conditions(I, p, L.x, L.v);
-        if (INTEG == FOORT_INTEGRATOR_VERLET) L.P = fd_parts_fp64<MID, Mt>(I.m, R.rlog != 0, R.hfd, L.x);
+        if (INTEG == FOORT_INTEGRATOR_VERLET) L.P = fd_parts_fp64<Mt>(I.m, R.rlog != 0, R.hfd, L.x);
         L.lam = 0.0;
         L.steps = 0;
         L.err = 0;
@@ -129,13 +162,13 @@ struct Fp64Engine {
             rhs_fd_fp64<MID, Mt>(M, rlog, R.hfd, L.x, L.v, k1);
             const double hh = 0.5 * h;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) { t[i] = L.x[i] + L.v[i] * hh; l2[i] = L.v[i] + k1[i] * hh; }
+            for (int i = 0; i < 4; ++i) { t[i] = ahead(L.x[i], L.v[i], hh); l2[i] = ahead(L.v[i], k1[i], hh); }
             rhs_fd_fp64<MID, Mt>(M, rlog, R.hfd, t, l2, k2);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) { t[i] = L.x[i] + l2[i] * hh; l3[i] = L.v[i] + k2[i] * hh; }
+            for (int i = 0; i < 4; ++i) { t[i] = ahead(L.x[i], l2[i], hh); l3[i] = ahead(L.v[i], k2[i], hh); }
             rhs_fd_fp64<MID, Mt>(M, rlog, R.hfd, t, l3, k3);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) { t[i] = L.x[i] + l3[i] * h; l4[i] = L.v[i] + k3[i] * h; }
+            for (int i = 0; i < 4; ++i) { t[i] = ahead(L.x[i], l3[i], h); l4[i] = ahead(L.v[i], k3[i], h); }
             rhs_fd_fp64<MID, Mt>(M, rlog, R.hfd, t, l4, k4);
             rk4_combine(L, h, k1, k2, k3, k4, l2, l3, l4, nx, nv);
             L.rhs += 4;
@@ -145,18 +178,18 @@ struct Fp64Engine {
             // there are computed once and kept for the next step. The reference computes
             // them again from the same nx, so the values are the same.
             double a0[4], a1[4], vi[4];
-            contract_fp64(L.P, L.v, a0);
+            contract_fp64<MID, Mt, true>(L.P, L.v, a0);
             const double hh2 = h * h / 2.0;
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                nx[i] = (L.x[i] + L.v[i] * h) + a0[i] * hh2;
-                vi[i] = L.v[i] + a0[i] * h;
+                nx[i] = ahead(ahead(L.x[i], L.v[i], h), a0[i], hh2);
+                vi[i] = ahead(L.v[i], a0[i], h);
             }
-            const FdParts Pn = fd_parts_fp64<MID, Mt>(M, rlog, R.hfd, nx);
-            contract_fp64(Pn, vi, a1);
+            const FdParts Pn = fd_parts_fp64<Mt>(M, rlog, R.hfd, nx);
+            contract_fp64<MID, Mt>(Pn, vi, a1);
             const double h2 = h / 2.0;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) nv[i] = L.v[i] + (a0[i] + a1[i]) * h2;
+            for (int i = 0; i < 4; ++i) nv[i] = ahead(L.v[i], a0[i] + a1[i], h2);
             L.rhs += 2;
             if (R.vtol > 0.0) {
                 const double tol2 = R.vtol * R.vtol;
@@ -165,8 +198,8 @@ struct Fp64Engine {
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
                         const double d = nv[i] - vi[i];
-                        num += d * d;
-                        den += nv[i] * nv[i];
+                        num = ahead(num, d, d);
+                        den = ahead(den, nv[i], nv[i]);
                     }
                     if (!(num / den > tol2)) break;
                     if (it >= R.verlet_cap) {
@@ -175,9 +208,9 @@ struct Fp64Engine {
                     }
 #pragma unroll
                     for (int i = 0; i < 4; ++i) vi[i] = nv[i];
-                    contract_fp64(Pn, vi, a1);
+                    contract_fp64<MID, Mt>(Pn, vi, a1);
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) nv[i] = L.v[i] + (a0[i] + a1[i]) * h2;
+                    for (int i = 0; i < 4; ++i) nv[i] = ahead(L.v[i], a0[i] + a1[i], h2);
                     L.rhs += 1;
                 }
             }
@@ -206,24 +239,24 @@ struct Fp64Engine {
             for (int i = 0; i < 4; ++i) k[i] = __shfl_sync(pmask, ka[i], from, 2);
         };
 #pragma unroll
-        for (int i = 0; i < 4; ++i) t[i] = odd ? L.x[i] + L.v[i] * hh : L.x[i];
-        FdParts P = fd_parts_fp64<MID, Mt>(M, rlog, R.hfd, t);
-        contract_fp64(P, L.v, ka);
+        for (int i = 0; i < 4; ++i) t[i] = odd ? ahead(L.x[i], L.v[i], hh) : L.x[i];
+        FdParts P = fd_parts_fp64<Mt>(M, rlog, R.hfd, t);
+        contract_fp64<MID, Mt>(P, L.v, ka);
         share(k1, 0);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) l2[i] = L.v[i] + k1[i] * hh;
-        contract_fp64(P, l2, ka);
+        for (int i = 0; i < 4; ++i) l2[i] = ahead(L.v[i], k1[i], hh);
+        contract_fp64<MID, Mt>(P, l2, ka);
         share(k2, 1);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) l3[i] = L.v[i] + k2[i] * hh;
+        for (int i = 0; i < 4; ++i) l3[i] = ahead(L.v[i], k2[i], hh);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) t[i] = L.x[i] + (odd ? l3[i] : l2[i]) * (odd ? h : hh);
-        P = fd_parts_fp64<MID, Mt>(M, rlog, R.hfd, t);
-        contract_fp64(P, l3, ka);
+        for (int i = 0; i < 4; ++i) t[i] = ahead(L.x[i], odd ? l3[i] : l2[i], odd ? h : hh);
+        P = fd_parts_fp64<Mt>(M, rlog, R.hfd, t);
+        contract_fp64<MID, Mt>(P, l3, ka);
         share(k3, 0);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) l4[i] = L.v[i] + k3[i] * h;
-        contract_fp64(P, l4, ka);
+        for (int i = 0; i < 4; ++i) l4[i] = ahead(L.v[i], k3[i], h);
+        contract_fp64<MID, Mt>(P, l4, ka);
         share(k4, 1);
         rk4_combine(L, h, k1, k2, k3, k4, l2, l3, l4, nx, nv);
         L.rhs += 2;  // the pair evaluates four
@@ -237,8 +270,8 @@ struct Fp64Engine {
         const double h6 = h / 6.0;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            nv[i] = L.v[i] + (((k1[i] + k2[i] * 2) + k3[i] * 2) + k4[i]) * h6;
-            nx[i] = L.x[i] + (((L.v[i] + l2[i] * 2) + l3[i] * 2) + l4[i]) * h6;
+            nv[i] = ahead(L.v[i], ahead(ahead(k1[i], k2[i], 2), k3[i], 2) + k4[i], h6);
+            nx[i] = ahead(L.x[i], ahead(ahead(L.v[i], l2[i], 2), l3[i], 2) + l4[i], h6);
         }
     }
 
