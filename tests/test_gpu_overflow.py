@@ -2,6 +2,8 @@
 end them as the general kernels do, with the same codes, counts and bits. The screens look
 along the rotation axis, or take coarse steps, so that some of their rays step past it or
 inside the horizon and diverge there."""
+import random
+
 import numpy as np
 import pytest
 
@@ -111,3 +113,45 @@ def test_shared_fp64_steps_cross_the_horizon_as_one_lane_does(eng, integrator, s
     assert (got[1]["err"] & abi.ERR_NONFINITE).all()
     same_records(got[2], got[1])
     del keep
+
+
+def random_setting(rng, precision):
+    """Views, steps and limits from ordinary to absurd."""
+    metric = rng.choice([abi.METRIC_KERR, abi.METRIC_KERR, abi.METRIC_FLAT, abi.METRIC_RASHEED_LARSEN,
+                         abi.METRIC_JOHANNSEN, abi.METRIC_JOHANNSEN])
+    a = rng.choice([0.0, 1e-3, rng.uniform(0.0, 1.0), 0.998])
+    others = rng.choice([(0.0, 0.0, 0.0), (0.0, 0.0, 0.0), (0.3, 0.2, 0.1), (0.0, 0.0, 1e-3)])
+    params = {abi.METRIC_KERR: (a,), abi.METRIC_FLAT: (),
+              abi.METRIC_RASHEED_LARSEN: (0.3556562853309941, 0.2969060968239216, 3.057664971085168, 0.942335028914832),
+              abi.METRIC_JOHANNSEN: (a, rng.uniform(-1.0, 2.0)) + others}[metric]
+    rlog = 0 if metric == abi.METRIC_FLAT else rng.randint(0, 1)
+    d, keep = describe(precision, metric, params, rng.choice([RK4, VERLET]), rlog,
+                       rng.choice([0.01, 0.3, 2.0, rng.uniform(5.0, 90.0), 90.0]), rng.choice([1000.0, 30.0, 5.0]),
+                       rng.choice([0.5, 6.0, 12.0, 40.0]), rng.choice([0.03, 0.1, 0.3, 1.0, 3.0, 10.0, 100.0]),
+                       rng.choice([1e-12, 1e-7, 1e-2]), rng.choice([0, 1, 50, 300]), rng.choice([1e3, 1e3, 1e5, 1e12, 1e30]),
+                       rng.choice([-1.0, 1e-3, 1e-6]), rng.choice([STOPS, ALL_STOPS, ALL_STOPS & ~abi.TERM_BOUNDARY_SPHERE]))
+    d.theta_eps = rng.choice([1e-5, 1e-2, 0.0])
+    return d, keep, abi.square_pixels(rng.choice([1, 2, 7, 33]) + 1)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [abi.PREC_MIXED, abi.PREC_FP64, abi.PREC_FP64_ANALYTIC])
+@pytest.mark.parametrize("seed", range(8))
+def test_random_views_end_alike_in_every_kernel(eng, precision, seed):
+    rng = random.Random(1000 * precision + seed)
+    for _ in range(12):
+        d, keep, px = random_setting(rng, precision)
+        got = []
+        for lanes in (0, 1, 2):
+            with eng.Engine(d) as e:
+                e.set_lanes(lanes)
+                got.append((e.integrate(px), {k: e.stats()[k] for k in ("steps", "rhs_evals")}))
+        d.diag_flags |= abi.DIAG_EQUATORIAL_PASSES
+        d.equat_freq = abi.UpdateFreq(2, 0, 0)  # the general kernels
+        with eng.Engine(d) as e:
+            e.set_lanes(1)
+            want = e.integrate(px), {k: e.stats()[k] for k in ("steps", "rhs_evals")}
+        for records, counts in got:
+            same_records(records, want[0])
+            assert counts == want[1]
+        del keep
