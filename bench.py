@@ -43,6 +43,7 @@ import argparse
 import json
 import math
 import os
+import re
 import statistics
 import subprocess
 import sys
@@ -511,7 +512,8 @@ def main():
                 if lists:
                     continue
                 shapes[i] = {"geodesics": len(r), "block_size": st["block_size"], "lanes": st["lanes_per_geodesic"],
-                             "refill_steps": st["refill_steps"], "poll_steps": st["poll_steps"]}
+                             "refill_steps": st["refill_steps"], "poll_steps": st["poll_steps"],
+                             "kernel": re.search(r"integrate_\w*?kernel|$", e.kernel_name()).group()}
                 rhs_per_round[i] = st["rhs_evals"]
                 lanes_per_round[i] = st["lanes_per_geodesic"]
         return kms
@@ -776,7 +778,7 @@ def main():
                 "ops_per_step": ops, "sincos_per_step": SINCOS_PER_STEP.get(mkind, 20),
                 "peak_source": "FP32 FMA microbenchmark on this GPU (foort_measure_peaks); MEASURED_PEAKS.json "
                                "has no FP32/FP64 entry",
-                "kernel": "integrate_lean_kernel",
+                "kernel": ", ".join(sorted({sh["kernel"] for sh in tuned_shapes})),
                 "lanes_per_geodesic": mixed_lanes,
                 "largest_launch": {"geodesics": len(launches_px[big]), "launch_ms": big_ms, "steps": big_steps,
                                    "achieved": big_ops / (big_ms * 1e-3) / 1e12,

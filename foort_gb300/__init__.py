@@ -95,6 +95,8 @@ def load():
     lib.foort_gpu_launch_shape.argtypes = [vp, u64, C.POINTER(abi.LaunchShape)]
     lib.foort_tune_bucket.argtypes = [u64]
     lib.foort_tune_bucket.restype = u32
+    lib.foort_gpu_kernel_name.argtypes = [vp]
+    lib.foort_gpu_kernel_name.restype = C.c_char_p
     lib.foort_tune_candidates.argtypes = [C.c_int32, C.c_int32, C.c_void_p, u32]
     lib.foort_tune_candidates.restype = u32
     lib.foort_tune_key.argtypes = [C.POINTER(abi.RunDesc), i32, u64, C.c_char_p, u64]
@@ -291,6 +293,10 @@ class Engine:
         s = abi.Stats()
         self._lib.foort_gpu_get_stats(self._ctx, C.byref(s))
         return {k: getattr(s, k) for k, _ in abi.Stats._fields_}
+
+    def kernel_name(self):
+        """The (mangled) name of the last launch's kernel; empty before the first."""
+        return self._lib.foort_gpu_kernel_name(self._ctx).decode()
 
     def last_error(self):
         return self._lib.foort_gpu_last_error(self._ctx).decode()

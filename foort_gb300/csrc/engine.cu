@@ -45,6 +45,7 @@ struct foort_ctx {
     uint64_t pos_cap = 0;
     uint64_t budget = 0;
     uint64_t last_n = 0;
+    const void* last_fn = nullptr;  // the last launch's kernel
     uint32_t block_size = 0, blocks_per_sm = 0;
     uint32_t lanes = 0;  // lanes per geodesic: 0 chosen per launch, 1, 2
     int device = 0, num_sms = 0;
@@ -501,6 +502,7 @@ int launch(foort_ctx* ctx, const foort_pixel* d_px, uint64_t n, foort_result* d_
     ctx->stats.refill_steps = ls.refill;
     ctx->stats.poll_steps = ls.poll;
     ctx->last_n = n;
+    ctx->last_fn = fn;
     ctx->last_stream = st;
     ctx->pending = true;
     return FOORT_OK;
@@ -984,6 +986,12 @@ int foort_gpu_get_stats(const foort_ctx* ctx, foort_stats* stats) {
     if (!ctx || !stats) return FOORT_E_BADARG;
     *stats = ctx->stats;
     return FOORT_OK;
+}
+
+const char* foort_gpu_kernel_name(const foort_ctx* ctx) {
+    const char* name = nullptr;
+    if (!ctx || !ctx->last_fn || cudaFuncGetName(&name, ctx->last_fn) != cudaSuccess) return "";
+    return name ? name : "";
 }
 
 void foort_gpu_destroy(foort_ctx* ctx) {

@@ -357,6 +357,10 @@ int foort_tune_load(const char* path);
 
 int foort_gpu_get_stats(const foort_ctx* ctx, foort_stats* stats);
 
+/* The (mangled) name of the kernel of the context's last launch; "" before the first.
+ * Never NULL. */
+const char* foort_gpu_kernel_name(const foort_ctx* ctx);
+
 /* The context's run descriptor (its images point to the context's own copy). */
 int foort_gpu_get_desc(const foort_ctx* ctx, foort_run_desc* desc);
 
