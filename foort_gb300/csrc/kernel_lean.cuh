@@ -71,12 +71,15 @@ FOORT_DEFINE_PACKED_METRIC(kJohannsen, JOHANNSEN13)
 // two products, it depends on the code around which of them joins as a fused multiply-add:
 // FORM 0 is the step with an inlined plugin, 1 and 2 the called right-hand side of
 // Johannsen and of Rasheed-Larsen. m.gu.rr and m.gu.hh come multiplied by -1/2. The other
-// factors of 2 and -1/2 change no rounding, but they are multiplied out as the general kernel
-// does: where a sum is within a factor of 2 of the type's largest value its double overflows, and the
-// ray ends otherwise than with the factors left out (steps that diverge next to the axis or
-// inside a horizon). They cost 1 % of a Kerr launch (RK4, eight images 583 -> 589 ms) and 2 % of
-// Johannsen's in Verlet (147,456 rays 281 -> 286 ms).
+// factors of 2 and -1/2 change no rounding, but are multiplied out as the general kernel does:
+// where a sum is within a factor of 2 of the type's largest value its double overflows, and
+// the ray would end otherwise without them (steps that diverge next to the axis or inside a
+// horizon). Taken two at a time they cost next to nothing: 200,000 Kerr rays cut at 1,000 steps 7.20 ms
+// without them, 7.28 one by one, 7.19 so (two lanes, 9,000 cut at 20,000: 18.9, 19.1 and
+// 17.8; Johannsen in Verlet, 147,456 cut at 900: 3.82, 3.89 and 3.81). Flat space takes them
+// one by one (58,368 cut at 3,000: 3.71 without, 3.78 and 3.87).
 // a[2] is the product of m.gu.hh and *f2 (where asked for).
+constexpr int kFlatForm = 3;  // FORM 0 of flat space
 template <int FORM, typename T>
 __device__ __forceinline__ void accel_lean(const MetricAt<T>& m, const T u[4], T a[4], T* f2 = nullptr) {
     // x y + z w with the first or the second product fused
@@ -84,27 +87,42 @@ __device__ __forceinline__ void accel_lean(const MetricAt<T>& m, const T u[4], T
     auto second = [](T x, T y, T z, T w) { return p_fma(z, w, p_mul(x, y)); };
     const T w1t = first(m.d1.tt, u[0], m.d1.tp, u[3]), w1p = first(m.d1.tp, u[0], m.d1.pp, u[3]);
     const T w2t = first(m.d2.tt, u[0], m.d2.tp, u[3]);
-    constexpr bool kSecond = FORM == 1 || FORM == 2;
+    constexpr bool kSecond = FORM == 1 || FORM == 2, kPairs = sizeof(T) == sizeof(float) && FORM != kFlatForm;
     const T w2p = (FORM == 1) ? second(m.d2.tp, u[0], m.d2.pp, u[3]) : first(m.d2.tp, u[0], m.d2.pp, u[3]);
     const T w1r = p_mul(m.d1.rr, u[1]), w1h = p_mul(m.d1.hh, u[2]);
     const T w2r = p_mul(m.d2.rr, u[1]), w2h = p_mul(m.d2.hh, u[2]);
     const T q1 = p_fma(u[3], w1p, p_fma(u[2], w1h, first(u[0], w1t, u[1], w1r)));
     const T q2a = first(u[0], w2t, u[1], w2r);
-    const T q2b = FORM ? p_fma(u[2], w2h, q2a) : p_add(q2a, p_mul(u[2], w2h));
+    const T q2b = kSecond ? p_fma(u[2], w2h, q2a) : p_add(q2a, p_mul(u[2], w2h));
     const T q2 = p_fma(u[3], w2p, q2b);
-    const T two = T(2), half = T(-0.5);
-    const T Ft = p_mul(two, kSecond ? second(u[1], w1t, u[2], w2t) : first(u[1], w1t, u[2], w2t));
-    const T Fp = p_mul(two, kSecond ? second(u[1], w1p, u[2], w2p) : first(u[1], w1p, u[2], w2p));
-    const T Fr = p_sub(p_mul(two, first(u[1], w1r, u[2], w2r)), q1);
-    const T Fh = p_sub(p_mul(two, kSecond ? second(u[1], w1h, u[2], w2h) : first(u[1], w1h, u[2], w2h)), q2);
-    a[0] = p_mul(half, first(m.gu.tt, Ft, m.gu.tp, Fp));
-    a[3] = p_mul(half, first(m.gu.tp, Ft, m.gu.pp, Fp));
+    const T St = kSecond ? second(u[1], w1t, u[2], w2t) : first(u[1], w1t, u[2], w2t);
+    const T Sp = kSecond ? second(u[1], w1p, u[2], w2p) : first(u[1], w1p, u[2], w2p);
+    const T Sr = first(u[1], w1r, u[2], w2r);
+    const T Sh = kSecond ? second(u[1], w1h, u[2], w2h) : first(u[1], w1h, u[2], w2h);
+    T Ft, Fp, Fr, Fh;
+    if constexpr (kPairs) {
+        const foort::f2 tp = pack2(St, Sp), rh = pack2(Sr, Sh);
+        const foort::f2 F = p_add(tp, tp), G = p_sub(p_add(rh, rh), pack2(q1, q2));
+        Ft = lo2(F), Fp = hi2(F), Fr = lo2(G), Fh = hi2(G);
+    } else {
+        Ft = p_mul(T(2), St), Fp = p_mul(T(2), Sp);
+        Fr = p_sub(p_mul(T(2), Sr), q1), Fh = p_sub(p_mul(T(2), Sh), q2);
+    }
+    const T xt = first(m.gu.tt, Ft, m.gu.tp, Fp), xp = first(m.gu.tp, Ft, m.gu.pp, Fp);
+    if constexpr (kPairs) {
+        const foort::f2 x = p_mul(p_all<foort::f2>(-0.5f), pack2(xt, xp));
+        a[0] = lo2(x), a[3] = hi2(x);
+    } else {
+        a[0] = p_mul(T(-0.5), xt), a[3] = p_mul(T(-0.5), xp);
+    }
     a[1] = p_mul(m.gu.rr, Fr);
     a[2] = p_mul(m.gu.hh, Fh);
     if (f2) *f2 = Fh;
 }
 // The form of each metric's FP32 right-hand side.
-constexpr int accel_form(int mid) { return mid == kJohannsen ? 1 : mid == kRasheedLarsen ? 2 : 0; }
+constexpr int accel_form(int mid) {
+    return mid == kJohannsen ? 1 : mid == kRasheedLarsen ? 2 : mid == kFlat ? kFlatForm : 0;
+}
 // In log-r mode the coordinate term -(u^1)^2 joins a^1 (accel_log_r).
 template <int FORM, typename T>
 __device__ __forceinline__ void accel_lean(const MetricAt<T>& m, bool rlog, const T u[4], T a[4], T* f2 = nullptr) {
@@ -459,6 +477,7 @@ template <int MID, bool RLOG>
 struct LeanVerletEngine : LeanState<LeanConst<MID>> {
     using Base = LeanState<LeanConst<MID>>;
     static constexpr bool kCountsRhs = true;
+    static constexpr int kForm = (MID == kFlat) ? kFlatForm : 0;  // Johannsen's is inlined here
 
     struct Lane : Base::Lane {
         MetricAt<float> m;  // at (x1, theta)
@@ -476,7 +495,7 @@ struct LeanVerletEngine : LeanState<LeanConst<MID>> {
         const float uf[4] = {lo2(uf03), lo2(uf12), hi2(uf12), hi2(uf03)};
         const float h = adaptive_step_lean(G, hi2(L.xh[1]), hi2(L.xl[1]), uf[1], uf[2], uf[3]);
         float a0[4], a1[4], vi[4];
-        accel_lean<0>(L.m, RLOG, uf, a0);
+        accel_lean<kForm>(L.m, RLOG, uf, a0);
         const float h2 = 0.5f * h, hh2 = __fmul_rn(h2, h);
         const f2 ph = p_all<f2>(h), ph2 = p_all<f2>(h2), phh2 = p_all<f2>(hh2);
         const f2 a03 = pack2(a0[0], a0[3]), a12 = pack2(a0[1], a0[2]);
@@ -493,7 +512,7 @@ struct LeanVerletEngine : LeanState<LeanConst<MID>> {
         p_two_sum(L.xh[0], th, s, e);
         p_fast_two_sum(s, p_add(e, p_add(L.xl[0], tl)), L.xh[0], L.xl[0]);
         L.m = metric_lean<MID, RLOG, float>(L.c, lo2(L.xh[1]), lo2(L.xl[1]), hi2(L.xh[1]), hi2(L.xl[1]));
-        accel_lean<0>(L.m, RLOG, vi, a1);
+        accel_lean<kForm>(L.m, RLOG, vi, a1);
         L.rhs += 2;
         f2 b03 = pack2(a1[0], a1[3]), b12 = pack2(a1[1], a1[2]);
         f2 du03 = p_mul(ph2, p_add(a03, b03)), du12 = p_mul(ph2, p_add(a12, b12));
@@ -515,7 +534,7 @@ struct LeanVerletEngine : LeanState<LeanConst<MID>> {
                     break;
                 }
                 // (in log-r mode the compiled loop rounds (u^1)^2 before it subtracts it)
-                accel_lean<0>(L.m, false, nv, a1);
+                accel_lean<kForm>(L.m, false, nv, a1);
                 if (RLOG) a1[1] = __fsub_rn(a1[1], __fmul_rn(nv[1], nv[1]));
                 const f2 c03 = pack2(a1[0], a1[3]), c12 = pack2(a1[1], a1[2]);
                 dv03 = p_mul(ph2, p_sub(c03, b03));
