@@ -68,13 +68,14 @@ OPS_PER_EXTRA_VERLET_RHS = 380
 # DRAM traffic per geodesic of the mixed kernel: dram__bytes_read.sum + dram__bytes_write.sum
 # of one ncu capture of the lean kernel on a 6,000-pixel sample of the C2 grid, divided by its
 # geodesics (the records stay in L2)
-DRAM_BYTES_PER_GEODESIC = {("kerr", "rk4"): 44.0}
+DRAM_BYTES_PER_GEODESIC = {("kerr", "rk4"): 107.0}
 # Executed thread instructions per geodesic step of the lean mixed kernels (ncu
-# smsp__inst_executed x 32 / steps; many are packed, two operations each): one lane of 855 on
-# a 6,000-pixel sample of the C2 grid and two of ~686 each on 3,000; Johannsen Verlet (one
-# lane, alpha13 alone) 871 on 20,000 pixels of C4's. With the GPU's issue rate (one warp instruction per cycle on each of its
-# 4 x 152 sub-partitions) they give the fraction of issue slots the path fills.
-EXEC_INSTR_PER_STEP = {("kerr", "rk4", 2): 1372, ("kerr", "rk4", 1): 855, ("johannsen", "verlet", 1): 871}
+# smsp__inst_executed x 32 / steps; many are packed, two operations each): one lane of 865 on
+# a 6,000-pixel sample of the C2 grid and two of 692 each on 3,000; Johannsen Verlet (one
+# lane, alpha13 alone) 871 on 20,000 pixels of C4's. With the GPU's issue rate (one warp
+# instruction per cycle on each of its 4 x 152 sub-partitions) they give the fraction of
+# issue slots the path fills.
+EXEC_INSTR_PER_STEP = {("kerr", "rk4", 2): 1384, ("kerr", "rk4", 1): 865, ("johannsen", "verlet", 1): 871}
 SUBPARTITIONS = 4
 # runs of more geodesics take the FP64 legs on a seeded sample (1 %, at least 20,000)
 FP64_SAMPLE_ABOVE = 60000

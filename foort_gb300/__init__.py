@@ -264,7 +264,8 @@ class Engine:
 
     def set_lookahead(self, max_geodesics=None):
         """Cap of a wave launch that also takes the next wave's candidates (None: the
-        default, 128 x the SM count; 0: off)."""
+        default, 128 x the SM count, or 256 x for Kerr and flat space in mixed precision and
+        plain r; 0: off)."""
         self._check(self._lib.foort_gpu_set_lookahead(self._ctx, (1 << 64) - 1 if max_geodesics is None
                                                       else max_geodesics))
 

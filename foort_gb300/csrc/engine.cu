@@ -266,29 +266,29 @@ struct LaunchShape {
 // - FP64 kernels: an FP64 instruction occupies its scheduler's pipe for 64 cycles however
 //   many lanes are active, so two lanes halve the metric work of a launch that leaves lanes
 //   idle, and shorten the last rays of a larger one. Past several refills they only add the
-//   parts that both lanes do: FP64-analytic Kerr in log r, 25,600 geodesics 82 ms on one lane
-//   and 69 on two, 62,500 123 and 111, 90,000 133 and 154. In plain r rays differ less in length, and a wave of two lanes each
-//   (64 x SMs) is the most that pays (flat space in FP64, 9,604 rays cut at 900 steps 20 ms on
-//   two lanes and 29 on one, 19,044 42 and 29).
+//   parts that both lanes do: FP64-analytic Kerr in log r, 25,600 geodesics 77 ms on one lane
+//   and 63 on two, 62,500 117 and 115, 90,000 149 and 163. In plain r rays differ less in
+//   length, and a wave of two lanes each (64 x SMs) is the most that pays (flat space in FP64,
+//   9,604 rays cut at 900 steps 20 ms on two lanes and 29 on one, 19,044 42 and 29).
 // - Lean Kerr: one lane already evaluates two stages at a time, but scalar stages of a lane each
 //   have a shorter chain than packed ones. In plain r two lanes pay while they leave each
-//   scheduler one warp (ms on one lane and on two: 1,000 geodesics 68.7 and 65.3, 9,728 69.3 and
-//   66.3; 10,000 cut at 20,000 steps 20.0 and 24.1). In log r, where each half of a packed stage needs
-//   its own exponentials and division and the longest rays end a launch alone, up to 448 x SMs
-//   (3,000 1.84 and 1.42, 19,000 2.40 and 2.01, 58,000 3.37 and 2.98, 70,000 3.19 and 3.16, 80,000
-//   3.37 and 3.49).
+//   scheduler one warp (ms on one lane and on two: 1,000 geodesics 68.4 and 61.3, 9,728 69.0 and
+//   61.5, 10,000 68.9 and 74.7). In log r, where each half of a packed stage needs its own
+//   exponentials and division and the longest rays end a launch alone, up to 448 x SMs (3,000
+//   1.84 and 1.40, 19,000 2.41 and 1.97, 58,000 3.5 and 3.1, 70,000 3.19 and 3.19, 80,000 3.40 and
+//   3.44).
 // - Lean flat space: its metric is too small for its half to be worth an exchange (100
-//   geodesics 46.0 and 54.0, 3,000 68.0 and 78.2): one lane.
+//   geodesics 45.7 and 54.0, 3,000 67.5 and 76.2): one lane.
 // - Johannsen with alpha13 alone: its packed body spills on one lane at three CTAs per SM and
-//   is held to two, so two lanes pay as long as they fit on the GPU (192 x SMs geodesics;
-//   plain r, 19,600 geodesics 174 ms on two and 211 on one, 39,204 291 and 255), and in log r,
-//   where the longest rays end a launch alone, several refills further (62,500 4.9 and 5.9 ms,
-//   160,000 9.0 and 9.2).
+//   is held to two, so two lanes pay while they fit on the GPU and somewhat further (192 x SMs
+//   geodesics; plain r, 19,400 geodesics 128 ms on one lane and 123 on two, 25,000 218 and 185,
+//   29,000 215 and 242), and in log r, where the longest rays end a launch alone, several
+//   refills further (62,500 5.7 and 4.5, 150,000 9.4 and 9.3, 170,000 9.7 and 10.5).
 // - Lean kernels with a called plugin exist on two lanes only. Rasheed-Larsen costs a geodesic
 //   less there than in the general one-lane kernel at every size (log r, 1,000,000 geodesics
 //   265 and 226, plain r 345 and 336). Johannsen's does while a launch's latency counts: log
-//   r, 250,000 29.8 and 27.7, 290,000 30.1 and 32.0, 1,000,000 98 and 109; plain r cut at 900
-//   steps, 36,000 6.23 and 6.09, 40,000 8.47 and 9.02, 1,000,000 142 and 156.
+//   r, 250,000 29.9 and 27.4, 290,000 29.9 and 31.6, 1,000,000 98 and 109; plain r cut at 900
+//   steps, 36,000 6.24 and 6.04, 40,000 8.48 and 8.87, 1,000,000 142 and 156.
 uint64_t pair_limit(const RunConst& R, bool positions, int per_sm, int num_sms, uint32_t bs) {
     const uint64_t sms = static_cast<uint64_t>(num_sms);
     if (R.precision != FOORT_PREC_MIXED) return (R.rlog ? 512 : 64) * sms;
@@ -304,9 +304,9 @@ uint64_t pair_limit(const RunConst& R, bool positions, int per_sm, int num_sms, 
 }
 
 // Lanes per geodesic that an FP64 launch of Kerr or Johannsen starts with in the kernels whose
-// lanes share a step (kernel_fp64_split.cuh): 8 or 2 (RK4), 4 (Verlet) or 1; 0: one lane to the end, unless several
-// lanes are forced. The most lanes finish a step soonest but cost more instructions per
-// geodesic. ms in log r (the plain kernel on one lane last):
+// lanes share a step (kernel_fp64_split.cuh): 8 or 2 (RK4), 4 (Verlet) or 1; 0: one lane to
+// the end, unless several lanes are forced. The most lanes finish a step soonest but cost more
+// instructions per geodesic. ms in log r (the plain kernel on one lane last):
 //               RK4 from 8 / 2 / 1: Kerr       Johannsen            Verlet from 4 / 1: Kerr, Johannsen
 //     3,600      24 /  42 /  57;  83           34 /  54 /  74; 122     14 / 21; 30     16 / 24; 35
 //    10,000      53 /  63 /  83; 114           64 /  76 / 100; 149     24 / 33; 39     29 / 41; 47
@@ -342,8 +342,9 @@ int split_start(const RunConst& R, uint64_t n, int num_sms, bool forced) {
 // threads, as many CTAs per SM as fit, and two lanes per geodesic up to pair_limit().
 // Where neither CTA size nor cap is asked for, FP64 kernels take CTAs of 32 threads, four per
 // SM: one warp per scheduler already fills its FP64 pipe, more only leave rays unevenly spread
-// over lanes at the end (62,500 Johannsen rays in FP64 130 ms with two CTAs of 128 per SM, 110 with four of 32), and small
-// CTAs spread a launch that does not fill the GPU evenly (4,096 Kerr rays 65.8 and 62.5 ms).
+// over lanes at the end (22,500 Kerr rays in FP64 Verlet, log r, 46 ms with CTAs of 128 as many
+// as fit, 40 with four of 32), and small CTAs spread a launch that does not fill the GPU evenly
+// (9,000 in FP64-analytic Verlet, plain r, 6.5 and 6.0 ms).
 // Eight per SM hide 5 % more latency where rays of like lengths (plain r) need more than the
 // lanes of four (62,500 Kerr rays cut at 900 steps 253 and 238 ms), or where a launch is so
 // large that its end counts little (250,000 in log r 623 and 601, 62,500 170 and 186).

@@ -250,8 +250,8 @@ __device__ __forceinline__ bool finite4(const double a[4]) {
 //   stop(L, R, out, err)               write a partial record (budget / cancel)
 //   counters: L.rhs, L.fp64            accumulated per lane, flushed at each poll
 // A lean engine (E::kLean, kernel_lean.cuh) has step(L, R) instead: its lanes keep the
-// image constants they need, record no positions and take kRhsPerStep right-hand sides a
-// step.
+// image constants they need and take kRhsPerStep right-hand sides a step, or count them
+// (E::kCountsRhs, Verlet); it records positions only as Recording<E> (E::kRecords).
 //
 // Every warp takes pixels from one global counter (one atomic per warp, shared by the
 // lanes that need work) and keeps integrating until the queue is empty. Lanes whose

@@ -1,25 +1,26 @@
 // Lean mixed-precision kernels: the mixed kernel's arithmetic (kernel_mixed.cuh) for the
 // options nearly every run has, with packed FP32 instructions (packed.cuh).
 //
-// Lean options (lean_options, engine.cu): every termination and diagnostic in use updates
-// at each step, decisions on the float-float state, no FP64 steps, no recorded positions.
-// A lane then carries no update counters, no position record and no copy of the options'
-// constants (they sit in the kernel's parameters, RunConst::mr). Results are the general
-// kernel's bit for bit: each rounding is written out as the compiler contracts the scalar
-// code (gen_packed.py), and the shortcuts below only skip work whose outcome is known.
+// Lean options (lean_options, mixed.cu): every termination and diagnostic in use updates
+// at each step, decisions on the float-float state, no FP64 steps. A lane then carries no
+// update counters and no copy of the options' constants (they sit in the kernel's parameters,
+// RunConst::mr); positions are recorded by a variant of each kernel (Recording). Results are
+// the general kernel's bit for bit, also where a state overflows: each rounding is written out
+// as the compiler contracts the scalar code (gen_packed.py), and the shortcuts below only
+// skip work whose outcome is known.
 //
 // RK4, one lane per geodesic: the metric parts of stages 1 and 2 need only the step's
 // start, those of stages 3 and 4 only k1 and k2, so each of the two pairs is evaluated
 // packed, one stage per half. On two lanes per geodesic each lane evaluates one stage of a
-// pair, and only the state's update is packed.
+// pair, and only the contraction's last sums and the state's update are packed.
 //
-// What bounds it: a warp alone on its scheduler waits for fixed latencies (0.89 of 2.36
-// cycles per issue; 809 instructions and 1,914 cycles a step, 0.95 us, where the general
-// kernels took 1.66 us on one lane and 1.17 us on two); three warps per scheduler take
-// 1,441 cycles per warp and step, near the FP32 pipe (476 packed and 154 scalar
-// instructions) with what mixing scalar and packed ones costs it. Kerr a = 0.99 view of
-// half-width 12 M from r = 1000, random pixels, GB300 at 2,070 MHz: 16,384 geodesics 65 ms
-// (general kernels: 82 to 94), 58,368 geodesics 140 ms.
+// What bounds it: a warp alone on its scheduler waits for fixed latencies (0.93 of 2.42
+// cycles per issue; 799 instructions a step, 0.97 us; on two lanes 692 each, 0.86 us; the
+// general kernels take 1.66 us on one lane and 1.17 us on two). Three warps per scheduler take 1,338
+// cycles per warp and step, near the FP32 pipe (377 packed and 244 scalar instructions, 998
+// cycles) with what mixing scalar and packed ones costs it. Kerr views from r = 1000, GB300 at
+// 2,070 MHz: 9,728 geodesics 61 ms on two lanes and 69 on one, 16,384 64 ms on one (general
+// kernels: 82 to 94), 93,000 278 ms.
 #pragma once
 
 #include "kernel_mixed.cuh"
@@ -555,11 +556,11 @@ struct LeanVerletEngine : LeanState<LeanConst<MID>> {
 // RK4 on two lanes with a plugin too large to pack or to inline (Johannsen,
 // Rasheed-Larsen): the compiler's scalar body, in one function that both rounds of a step
 // call. Its ~900 and ~1,800 instructions set the pace; on one lane the general kernel calls
-// it four times in sequence, which costs as many instructions per geodesic, so two lanes
-// are taken at every size. GB300, log r, one lane before and two lanes now: Johannsen
-// 3,721 geodesics 6.0 and 2.9 ms, 90,000 15.1 and 11.0 ms; Rasheed-Larsen 14.7 and 7.2,
-// 39.7 and 24.5 ms. Without a register cap (226 and 255): capped to three CTAs per SM the
-// largest of these take 11.5 and 29.4 ms.
+// it four times in sequence. GB300, log r, the general kernel's one lane and two lanes:
+// Johannsen 3,721 geodesics 7.4 and 3.6 ms, 90,000 14.2 and 10.6 ms; Rasheed-Larsen 14.9 and
+// 6.9, 38 and 23.5 ms (larger launches: pair_limit, engine.cu). Without a register cap (230
+// and 255, Rasheed-Larsen with 124 bytes of spills): capped to three CTAs per SM 90,000 take
+// 11.5 and 29.4 ms.
 struct ImageRef {
     const MixedConst* mx;
     const double* qa;

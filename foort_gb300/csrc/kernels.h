@@ -8,9 +8,10 @@ namespace foort {
 
 // Returns the __global__ function for (metric, integrator), or nullptr.
 const void* fp64_kernel(int metric_id, int integrator);
-// four or eight lanes per geodesic after that start, and two throughout; nullptr where that
-// kernel does not exist
+// The kernel whose geodesics start on that many lanes (8, 4, 2 or 1) and end on four or eight; start
+// 0: one lane to the end, Johannsen with alpha13 alone. nullptr where there is none.
 const void* fp64_split_kernel(const RunConst& R, int start);
+// Two lanes per geodesic throughout, or nullptr where that kernel does not exist.
 const void* fp64_pair_kernel(int metric_id, int integrator);
 const void* mixed_kernel(int metric_id, int integrator);
 // decide64: terminations and diagnostics decided in FP64 (else in float-float)
