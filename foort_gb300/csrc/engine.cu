@@ -358,12 +358,12 @@ int split_start(const RunConst& R, uint64_t n, int num_sms, bool forced) {
 int choose_launch(foort_ctx* ctx, const RunConst& R, uint64_t n, int num_sms, const foort_launch_shape& want,
                   LaunchShape& out, bool positions = false, uint64_t whole = 0) {
     const uint64_t all = whole ? whole : n;
-    const bool fp64 = R.precision != FOORT_PREC_MIXED && !want.block_size && !want.blocks_per_sm;
-    const uint32_t bs = want.block_size ? want.block_size : fp64 ? 32 : 128;
+    const bool fp64_shape = R.precision != FOORT_PREC_MIXED && !want.block_size && !want.blocks_per_sm;
+    const uint32_t bs = want.block_size ? want.block_size : fp64_shape ? 32 : 128;
     const uint64_t sms = static_cast<uint64_t>(num_sms);
     auto resident = [&](const void* fn, uint64_t width, int& per_sm) -> int {
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, static_cast<int>(bs), 0));
-        if (fp64) {
+        if (fp64_shape) {
             const bool two = all > 1024 * sms || (!R.rlog && width * all > 128 * sms);
             const int fit = per_sm;
             per_sm = std::min<int>(fit, two ? 8 : 4);
